@@ -274,13 +274,11 @@ void free_ctx(sphdem_ctx *c) {
     cudaFree(c->mx_q1);
     cudaFree(c->mx_q2);
     cudaFree(c->mx_dp);
-    cudaFree(c->mx_poslo);
     cudaFree(c->mx_rc4);
     cudaFree(c->mx_shep32);
     cudaFree(c->mx_ds);
     cudaFree(c->mx_nb);
     cudaFree(c->mx_win);
-    cudaFree(c->mx_bandq);
     cudaFree(c->mx_bandn);
     cudaFree(c->dcfg);
     fields_async_free(c);
@@ -542,18 +540,12 @@ int sphdem_create(const SphDemConfig *cfg, const SphDemParticles *init, int64_t 
             SPHDEM_CUDA_CHECK(cudaMalloc(&c->mx_q1, capacity * sizeof(float4)));
             SPHDEM_CUDA_CHECK(cudaMalloc(&c->mx_q2, capacity * sizeof(float4)));
             SPHDEM_CUDA_CHECK(cudaMalloc(&c->mx_dp, capacity * sizeof(float4)));
-            SPHDEM_CUDA_CHECK(cudaMalloc(&c->mx_poslo, capacity * sizeof(float4)));
             SPHDEM_CUDA_CHECK(cudaMalloc(&c->mx_rc4, capacity * sizeof(int4)));
             SPHDEM_CUDA_CHECK(cudaMalloc(&c->mx_shep32, capacity * sizeof(float)));
             SPHDEM_CUDA_CHECK(cudaMalloc(&c->mx_ds, capacity * sizeof(float4)));
             SPHDEM_CUDA_CHECK(cudaMalloc(&c->mx_nb, 3 * capacity * sizeof(float4)));
             c->mx_win_cap = win_cap;
             SPHDEM_CUDA_CHECK(cudaMalloc(&c->mx_win, 3 * (size_t)win_cap * sizeof(int4)));
-            /* list entries that FP32 cannot decide (mostly FP64 ties: a staggered
-             * lattice at rest density has 20 neighbours per particle at exactly
-             * 2h) are recorded per particle for the FP64 fix-up pass */
-            c->mx_band_per_particle = sphdem::mixed::band_records_per_particle();
-            SPHDEM_CUDA_CHECK(cudaMalloc(&c->mx_bandq, capacity * c->mx_band_per_particle * sizeof(int2)));
             SPHDEM_CUDA_CHECK(cudaMalloc(&c->mx_bandn, capacity * sizeof(int)));
             SPHDEM_CUDA_CHECK(cudaMemset(c->mx_bandn, 0, capacity * sizeof(int)));
             SPHDEM_CUDA_CHECK(cudaMemset(c->mx_om, 0, capacity * sizeof(float)));
@@ -760,7 +752,8 @@ int sphdem_get_stats(sphdem_handle h, SphDemStats *out) {
         cudaMemcpy(nb.data(), h->mx_bandn, h->n * sizeof(int), cudaMemcpyDeviceToHost);
         for (int64_t k = 0; k < h->n; k++)
             if (sphdem::is_sph_or_sphb(iam[k])) out->n_band_candidates += nb[k];
-        out->band_queue_capacity = (int64_t)h->cap * h->mx_band_per_particle;
+        /* settled where they are found: bounded by the lists' own capacity */
+        out->band_queue_capacity = (int64_t)h->cap * h->mx_maxn;
     }
     return cudaGetLastError() == cudaSuccess ? SPHDEM_OK : SPHDEM_ERR_CUDA;
 }

@@ -103,7 +103,6 @@ struct sphdem_ctx {
     bool mx_dem_only = false;   /* every particle at creation is DEM: the FP64 phases run */
     float4 *mx_q0 = nullptr, *mx_q1 = nullptr, *mx_q2 = nullptr;  /* FPI fields of fluid particles */
     float4 *mx_dp = nullptr;    /* (m/shep, fdrag) of DEM particles */
-    float4 *mx_poslo = nullptr; /* low FP32 halves of offsets and h (double-float) */
     int4 *mx_rc4 = nullptr;     /* packed reference DEM buckets (own, image -L, image +L) */
     int4 *mx_win = nullptr;     /* coupling windows per SPH bucket index and axis */
     int mx_win_cap = 0;         /* entries per axis */
@@ -121,9 +120,7 @@ struct sphdem_ctx {
     int blk_pair = 128;         /* block size of the list-consumer passes (<= 128) */
     bool force_tile = false;    /* force / continuity: neighbour records staged in shared memory */
     int grid_div = 1;           /* divides the resident-block grid of the slice passes */
-    int2 *mx_bandq = nullptr;   /* per particle: list entries within the FP32 band */
-    int *mx_bandn = nullptr;    /* per particle: how many are recorded */
-    int mx_band_per_particle = 0;
+    int *mx_bandn = nullptr;    /* per particle: list candidates FP32 could not decide */
     sphdem::DevCfg *dcfg = nullptr;  /* device copy of cfg for out-of-line helpers */
     /* staging buffer for field transfers in tag order */
     double *stage = nullptr;
@@ -196,7 +193,6 @@ void nlist(sphdem_ctx *c);
 void prepare(sphdem_ctx *c);
 void zero_shep(sphdem_ctx *c);
 int nlist_max_count(sphdem_ctx *c);
-int band_records_per_particle();
 void omega_eos(sphdem_ctx *c, bool omega, bool eos);
 void force(sphdem_ctx *c);
 void dddt(sphdem_ctx *c);

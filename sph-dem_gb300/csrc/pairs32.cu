@@ -9,11 +9,11 @@
  * the dimension so per-axis arrays live in registers.
  *
  *   k_nlist      after each rebuild, the exact neighbour list of every
- *                sph/sphBoundary particle: one warp per SPH bucket stages the
- *                3^d stencil's candidates in shared memory and tests them in
+ *                sph/sphBoundary particle: a warp stages the 3^d stencil's
+ *                candidates of 32 particles in shared memory and tests them in
  *                FP32 with a proven error bound; candidates inside the bound
- *                go to k_band_fix (double-float, then the reference's FP64
- *                predicate, particle.h:236-238, for true ties).  Periodic
+ *                are settled there by the reference's FP64 predicate
+ *                (particle.h:236-238).  Periodic
  *                images only where the reference holds a ghost.  Entries
  *                b | stencil code << 26 in tiles of 32 particles x 8 slots
  *                (nl_at).
@@ -37,6 +37,7 @@
 #include <algorithm>
 #include <cfloat>
 #include <climits>
+#include <type_traits>
 #include <vector>
 
 #include "internal.cuh"
@@ -82,17 +83,6 @@ __device__ __forceinline__ float wdK32(float q, float wcon) {
     if (q > 2.f) return 0.f;
     const float t = 2.f - q, t2 = t * t;
     return wcon * (-4.f * (t2 * t) * (1.f + 2.f * q) + 2.f * (t2 * t2));
-}
-
-/* error-free transforms for the double-float (hi + lo FP32) refinement */
-__device__ __forceinline__ void two_sum(float a, float b, float &s, float &e) {
-    s = a + b;
-    const float bb = s - a;
-    e = (a - (s - bb)) + (b - bb);
-}
-__device__ __forceinline__ void two_prod(float a, float b, float &p, float &e) {
-    p = a * b;
-    e = fmaf(a, b, -p);
 }
 
 template <int ND>
@@ -208,7 +198,7 @@ __device__ __forceinline__ int pack_cells(const int *k, int nd) {
 template <int ND>
 __global__ void k_pack(DevCfg c, DevState s, const int *__restrict__ skey, const DevGlobals *__restrict__ g,
                        float4 *__restrict__ P0, float4 *__restrict__ P1, float4 *__restrict__ P2,
-                       float4 *__restrict__ P0lo, int *__restrict__ tg, int4 *__restrict__ RC4, int with_rc,
+                       int *__restrict__ tg, int4 *__restrict__ RC4, int with_rc,
                        float4 *__restrict__ DS, float4 *__restrict__ NB, int64_t n) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -216,7 +206,7 @@ __global__ void k_pack(DevCfg c, DevState s, const int *__restrict__ skey, const
     tg[i] = (t & 0xff) | (s.irow(FI_GCODE)[i] << 8);
     if (t == T_DEAD) return;
     const int key = skey[i];
-    float off[3] = {0.f, 0.f, 0.f}, lo[3] = {0.f, 0.f, 0.f};
+    float off[3] = {0.f, 0.f, 0.f};
     int cc[3] = {0, 0, 0};
     const bool dem = c.liq_dem() && t == T_DEM;
     if (dem) {
@@ -229,11 +219,6 @@ __global__ void k_pack(DevCfg c, DevState s, const int *__restrict__ skey, const
     for (int d = 0; d < ND; d++) {
         const double o = s.row(FD_R + d)[i] - (dem ? dem_origin(c, d, cc[d]) : sph_origin(c, g, d, cc[d]));
         off[d] = (float)o;
-        lo[d] = (float)(o - (double)off[d]);
-    }
-    {
-        const double h = s.row(FD_H)[i];
-        P0lo[i] = make_float4(lo[0], lo[1], lo[2], (float)(h - (double)(float)h));
     }
     float vh[3] = {0.f, 0.f, 0.f};
 #pragma unroll
@@ -332,20 +317,6 @@ __global__ void k_pack_fpi(DevState s, float4 *__restrict__ Q0, float4 *__restri
     Q2[i] = make_float4(v[8], v[9], v[10], v[11]);
 }
 
-/* the reference's FP64 neighbour predicate, len2(ra - image(rb)) <= (2 max(ha, hb))^2
- * (dataLL.h neighbour traversal), evaluated without contraction */
-template <int ND>
-__device__ __forceinline__ bool exact_neighbour(const DevCfg &c, const DevState &s, int a, int b, const int *sh) {
-    double dx[3] = {0, 0, 0};
-#pragma unroll
-    for (int d = 0; d < ND; d++)
-        dx[d] = dsub(s.row(FD_R + d)[a], image_pos(s.row(FD_R + d)[b], sh[d], c.rmin[d], c.rmax[d]));
-    const double r2 = exact_len2(dx, ND);
-    const double ha = s.row(FD_H)[a], hb = s.row(FD_H)[b];
-    const double t = 2.0 * (ha > hb ? ha : hb);
-    return r2 <= dmul(t, t);
-}
-
 /* ---------------------------------------------------------------------- */
 /* Half-width of the band around a cut-off T = R^2 inside which an FP32 r^2
  * built from bucket offsets cannot decide: each displacement component is
@@ -353,48 +324,10 @@ __device__ __forceinline__ bool exact_neighbour(const DevCfg &c, const DevState 
  * r^2 by < 1.25e-6 L max(L, R) + 1.8e-7 r^2, and T by < 1.8e-7 T. */
 __device__ __forceinline__ float fp32_band(float T, float L2) { return fmaf(5e-7f, T, 1.5e-6f * fmaxf(L2, T)); }
 
-constexpr int CENTER_CODE = 13 << B_BITS;
-
 __device__ __forceinline__ void nl_decode_code(int code, int *o) {
     o[0] = code / 9 - 1;
     o[1] = (code / 3) % 3 - 1;
     o[2] = code % 3 - 1;
-}
-
-/* Double-float (hi + lo FP32) decision for one candidate near the cut-off:
- * +1 inside, -1 outside, 0 an FP64 tie.  Offsets, bucket size and h as hi+lo
- * pairs carry ~48 bits, so r^2 - (2h)^2 is known to ~1e-13 of (2h)^2 plus
- * ~1e-14 c^2 (c the bucket size); within 1e-12 of (2h)^2 + tol_abs only the
- * FP64 predicate decides. */
-template <int ND>
-__device__ __forceinline__ int nl_refine(const float4 pa, const float4 al, const float4 pb, const float4 bl,
-                                         const int *o, const float *cell, const float *cell_lo, float tol_abs) {
-    const float ah[3] = {pa.x, pa.y, pa.z}, bh[3] = {pb.x, pb.y, pb.z};
-    const float alo[3] = {al.x, al.y, al.z}, blo[3] = {bl.x, bl.y, bl.z};
-    float r2h = 0.f, r2l = 0.f;
-#pragma unroll
-    for (int d = 0; d < ND; d++) {
-        float s1v, e1, s2v, e2;
-        two_sum(ah[d], -bh[d], s1v, e1);
-        two_sum(s1v, -o[d] * cell[d], s2v, e2);
-        const float lo = e1 + e2 + (alo[d] - blo[d]) - o[d] * cell_lo[d];
-        float dh, dl;
-        two_sum(s2v, lo, dh, dl);
-        float p, pe;
-        two_prod(dh, dh, p, pe);
-        float t1, te;
-        two_sum(r2h, p, t1, te);
-        r2h = t1;
-        r2l += te + pe + 2.f * dh * dl;
-    }
-    const bool amax = pa.w > pb.w || (pa.w == pb.w && al.w >= bl.w);
-    const float hh = 2.f * (amax ? pa.w : pb.w), hl = 2.f * (amax ? al.w : bl.w);
-    float Th, Te;
-    two_prod(hh, hh, Th, Te);
-    const float Tl = Te + 2.f * hh * hl;
-    const float diff = (r2h - Th) + (r2l - Tl);
-    if (fabsf(diff) <= 1e-12f * Th + tol_abs) return 0;
-    return diff < 0.f ? 1 : -1;
 }
 
 /* ---------------------------------------------------------------------- */
@@ -406,46 +339,40 @@ __device__ __forceinline__ int nl_refine(const float4 pa, const float4 al, const
  * the warp stages the candidates of the union of the runs' 3^d stencils --
  * 3^(d-1) neighbour columns x the run's z-range +-1 -- in shared memory,
  * with positions moved into the run's frame (coalesced loads; the periodic
- * image filter is applied once per candidate), then every lane tests all
- * staged candidates with broadcast shared-memory reads.  Sharing the stencil
- * across a run keeps all 32 lanes busy whatever the bucket occupancy.
+ * image filter and the distance to the run's bounding box are applied once
+ * per candidate), then every lane tests all staged candidates with broadcast
+ * shared-memory reads.  Sharing the stencil across a run keeps all 32 lanes
+ * busy whatever the bucket occupancy.
+ *
+ * A passing candidate is appended by its lane to the lane's column of a
+ * shared-memory queue (slot-major, so the stores never conflict) with one
+ * predicated store and add, without a branch; when a lane's column is half
+ * full, every lane moves its complete groups of 8 entries to its list tile, a
+ * whole sector per group.  The pass is bound by instruction issue, so two
+ * candidates share each FP32 operation (packed f32x2: 10 instructions a
+ * candidate and warp instead of 13), the append is part of the test loop, and
+ * candidates are cut to those within reach of the run's bounding box (23 %
+ * fewer on a 3D lattice).
  *
  * FP32 error bound of the test (L = largest offset magnitude in the frame,
  * R = 2 max(ha, hb)): each displacement component carries < 6 * 2^-24 L, so
  * r^2 is off by < 1.25e-6 L max(L, R) + 1.8e-7 r^2 and the cut-off
- * 4 max(ha^2, hb^2) by < 1.8e-7 of itself.  Candidates closer than
- * fp32_band(T, L^2) to the cut-off are recorded per particle (up to NL_QB)
- * and decided by k_band_fix; beyond that they are decided inline in FP64. */
-constexpr int NL_WARPS = 8;
-constexpr int NL_CAP = 256;   /* staged candidates per warp before a flush */
-constexpr int NL_QB = 32;     /* band candidates recorded per particle */
+ * 4 max(ha^2, hb^2) by < 1.8e-7 of itself.  A candidate passes up to
+ * 4 h^2 (1 + 5e-7) + 1.5e-6 L^2; one that passes by less than the width of
+ * the band of doubt is settled on the spot (settle_band), which also takes
+ * the particle itself out, so the lists hold exactly the neighbours.  The
+ * lane only keeps the smallest margin of 32 candidates; the rare 32 with a
+ * doubtful one (or the particle itself) are gone over again. */
+constexpr int NL_WARPS = 4;
+constexpr int NL_CAP = 128;   /* staged candidates per warp before they are tested */
+constexpr int NL_QN = 64;     /* queue slots per lane: moved on when over 32 are taken, 32 come at most per round */
+/* buckets of a run, less one: the staged set of a run grows with its length
+ * along the last axis, that of a run cut short with its two ends; in 2D a
+ * bucket holds ~7 particles, so 32 of them span five */
+template <int ND>
+constexpr int NL_RUN = ND == 3 ? 2 : (ND == 2 ? 6 : 14);
 
 __device__ __forceinline__ int code_stride(int d) { return d == 0 ? 9 : (d == 1 ? 3 : 1); }
-
-/* FP64 decision of list entry e of particle a (bucket cc), out of line */
-template <int ND>
-__device__ __noinline__ bool exact_from_code(const DevCfg &c, const DevState &s, const DevGlobals *g, int a, int e,
-                                             const int *cc) {
-    int o[3], sh[3] = {0, 0, 0};
-    nl_decode_code(e >> B_BITS, o);
-    const int dims[3] = {g->sdims[0], g->sdims[1], g->sdims[2]};
-#pragma unroll
-    for (int d = 0; d < ND; d++) {
-        const int t = cc[d] + o[d];
-        sh[d] = t < 0 ? -1 : (t >= dims[d] ? 1 : 0);
-    }
-    return exact_neighbour<ND>(c, s, a, e & B_MASK, sh);
-}
-
-/* FP64 decision of list entry e of particle a, its bucket from the key row */
-template <int ND>
-__device__ __noinline__ bool exact_from_key(const DevCfg &c, const DevState &s, const DevGlobals *g,
-                                            const int *skey, int a, int e) {
-    const int dims[3] = {g->sdims[0], g->sdims[1], g->sdims[2]};
-    int cc[3] = {0, 0, 0};
-    decode<ND>(skey[a], dims, cc);
-    return exact_from_code<ND>(c, s, g, a, e, cc);
-}
 
 /* Neighbour lists: slot j of particle a, in tiles of 32 particles x 8
  * entries -- each particle's 8 entries contiguous, the 32 particles' groups
@@ -456,31 +383,129 @@ __device__ __forceinline__ int64_t nl_at(int64_t a, int j, int64_t maxn) {
     return ((a >> 5) * maxn + (j & ~7)) * 32 + ((a & 31) << 3) + (j & 7);
 }
 
-/* lane bits [lo, hi), 0 <= lo <= hi <= 32 */
-__device__ __forceinline__ unsigned lane_range(int lo, int hi) {
-    const unsigned up = hi >= 32 ? 0xffffffffu : ((1u << hi) - 1u);
-    const unsigned dn = lo >= 32 ? 0xffffffffu : ((1u << lo) - 1u);
-    return up & ~dn;
+/* One lane's entry of a bucket range table around a run of buckets (ccol
+ * on the leading axes, zmin..zmax on the last axis Z): lane = 3 * column +
+ * period piece, for the 3^(d-1) neighbour columns; each entry is a run of
+ * consecutive keys key0 + lin .. (buckets zmin-1 .. zmax+1 of the column,
+ * cut at a periodic seam).  Entries of other lanes are empty. */
+struct RangeEntry {
+    int b0, cnt, lin, zoff, shp, code;
+    float ox, oy;
+};
+
+template <int ND>
+__device__ __forceinline__ RangeEntry range_entry(int lane, const int *ccol, int zmin, int zmax, const int *dims,
+                                                  const int *periodic, const float *cell, int key0,
+                                                  const int *__restrict__ start) {
+    constexpr int Z = ND - 1;
+    constexpr int NCOL = Z == 2 ? 9 : (Z == 1 ? 3 : 1);
+    RangeEntry r = {0, 0, 0, 0, 0x15, 0, 0.f, 0.f};
+    if (lane >= 3 * NCOL) return r;
+    const int colidx = lane / 3, wz = lane % 3 - 1;
+    int o[2] = {0, 0};
+    if (Z == 2) {
+        o[0] = colidx / 3 - 1;
+        o[1] = colidx % 3 - 1;
+    } else if (Z == 1) {
+        o[0] = colidx - 1;
+    }
+    bool ok = wz == 0 || periodic[Z];
+    int col_lin = 0, code = 0, shp = 0;
+    float off[2] = {0.f, 0.f};
+#pragma unroll
+    for (int d = ND; d < 3; d++) {
+        shp |= 1 << (2 * d);
+        code += code_stride(d);
+    }
+#pragma unroll
+    for (int d = 0; d < Z; d++) {
+        int t = ccol[d] + o[d], shd = 0;
+        if (t < 0) {
+            ok = ok && periodic[d];
+            t += dims[d];
+            shd = -1;
+        } else if (t >= dims[d]) {
+            ok = ok && periodic[d];
+            t -= dims[d];
+            shd = 1;
+        }
+        col_lin = col_lin * dims[d] + t;
+        code += (o[d] + 1) * code_stride(d);
+        off[d] = (float)o[d] * cell[d];
+        shp |= (shd + 1) << (2 * d);
+    }
+    shp |= (wz + 1) << (2 * Z);
+    const int zdim = dims[Z];
+    const int zlo = max(zmin - 1, wz * zdim), zhi = min(zmax + 1, (wz + 1) * zdim - 1);
+    if (ok && zlo <= zhi) {
+        r.lin = key0 + col_lin * zdim + (zlo - wz * zdim);
+        r.b0 = start[r.lin];
+        r.cnt = start[r.lin + (zhi - zlo) + 1] - r.b0;
+        r.zoff = zlo - zmin;
+        r.shp = shp;
+        r.code = code << B_BITS;
+        r.ox = off[0];
+        r.oy = off[1];
+    }
+    return r;
 }
 
-template <int ND, bool COUNT>
-__global__ void __launch_bounds__(NL_WARPS * 32, 3) k_nlist(DevCfg c, DevState s, const int *__restrict__ start,
-                                                         const int *__restrict__ skey, DevGlobals *__restrict__ g,
-                                                         const float4 *__restrict__ P0, const int *__restrict__ tg,
-                                                         int *__restrict__ nbr, int *__restrict__ ncnt, int maxn,
-                                                         int64_t ld, int2 *__restrict__ bandq,
-                                                         int *__restrict__ bandn) {
+/* A candidate whose FP32 test leaves doubt: list entry e (candidate and stencil
+ * code) of particle a in bucket cc, zd its bucket on the last axis relative to
+ * a's.  Buckets are at least 2h wide, so one outside a's own 3^d stencil is no
+ * neighbour; for all others the reference's FP64 predicate decides.  (A
+ * double-float refinement before it settled nothing for the exact ties of
+ * particles at rest on a lattice, which are nearly all of these candidates,
+ * and doubled the latency of their chain.) */
+template <int ND>
+__device__ __forceinline__ bool settle_band(const DevCfg *__restrict__ cp, const DevState &s, const int *dims, const int *cc,
+                                            int a, int e, int zd) {
+    if (zd < -1 || zd > 1) return false;
+    int o[3], sh[3] = {0, 0, 0};
+    nl_decode_code(e >> B_BITS, o);
+#pragma unroll
+    for (int d = 0; d < ND; d++) {
+        const int t = cc[d] + o[d];
+        sh[d] = t < 0 ? -1 : (t >= dims[d] ? 1 : 0);
+    }
+    return exact_pair<ND>(cp, s, a, e & B_MASK, sh[0], sh[1], sh[2], 0.0, 0);
+}
+
+__device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
+
+/* append e to the lane's queue column (next free slot at shared address qa) when margin >= 0, without a branch */
+__device__ __forceinline__ void queue_append(unsigned &qa, int e, float margin) {
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ge.f32 p, %2, 0f00000000;\n @p st.shared.u32 [%0], %1;\n @p add.u32 %0, %0, 128;\n}\n"
+        : "+r"(qa)
+        : "r"(e), "f"(margin));
+}
+
+/* G lanes per particle: a warp takes 32 / G consecutive particles and each of
+ * a particle's lanes tests every G-th group of four candidates.  G = 1 reads
+ * the fewest candidates per particle; G = 4 runs four times the warps, each a
+ * third as long, for populations that leave the chip short of warps. */
+template <int ND, bool COUNT, int G>
+__global__ void __launch_bounds__(NL_WARPS * 32, 5) k_nlist(DevCfg c, const DevCfg *__restrict__ cp, DevState s,
+                                                         const int *__restrict__ start, const int *__restrict__ skey,
+                                                         DevGlobals *__restrict__ g, const float4 *__restrict__ P0,
+                                                         const int *__restrict__ tg, int *__restrict__ nbr,
+                                                         int *__restrict__ ncnt, int maxn, int *__restrict__ bandn) {
     constexpr int Z = ND - 1;
     constexpr unsigned FULL = 0xffffffffu;
-    __shared__ float4 s_pos[NL_WARPS][NL_CAP + 32];
-    __shared__ int s_ent[NL_WARPS][NL_CAP + 32];
+    /* staged candidates: negated position in the run's frame, cut-off, list
+     * entry (its code counts buckets on the last axis from the run's first) */
+    __shared__ __align__(16) float s_x[NL_WARPS][3][NL_CAP], s_cut[NL_WARPS][NL_CAP];
+    __shared__ __align__(16) int s_ent[NL_WARPS][NL_CAP];
+    __shared__ int s_queue[NL_WARPS][NL_QN * 32];
     __shared__ unsigned char s_zr[NL_WARPS][NL_CAP];
-    __shared__ float4 s_own[NL_WARPS][32];
     const int lane = threadIdx.x & 31;
     const int w = threadIdx.x >> 5;
-    float4 *cpos = s_pos[w];
+    float(*cx)[NL_CAP] = s_x[w];
+    float *ccut = s_cut[w];
     int *cent = s_ent[w];
     unsigned char *czr = s_zr[w];
+    int *const queue = s_queue[w] + lane;
     const unsigned lt_mask = (1u << lane) - 1u;
     const int nsc = g->n_sph_cells;
     const int n_t = start[nsc];
@@ -494,19 +519,22 @@ __global__ void __launch_bounds__(NL_WARPS * 32, 3) k_nlist(DevCfg c, DevState s
         if (d < Z) l_other = fmaxf(l_other, 2.f * cell[d]);
     }
     const float cz = cell[Z];
-    int code_fixed = 0;
+    /* code of the run's own column, one bucket below its first */
+    int code_own = 0;
 #pragma unroll
-    for (int d = ND; d < 3; d++) code_fixed += code_stride(d);
+    for (int d = 0; d < 3; d++)
+        if (d != Z) code_own += code_stride(d);
     const int zstride = code_stride(Z) << B_BITS;
-    const int self_e = CENTER_CODE;
     const float supp = (float)(2.0 * g->sr) * (1.f + 1e-5f) + 1e-5f * cz;
-    const float K_HI = 4.f * (1.f + 5e-7f), K_LO = 4.f * (1.f - 5e-7f);
+    const float K_HI = 4.f * (1.f + 5e-7f);
 
-    for (int t0 = (blockIdx.x * NL_WARPS + w) * 32; t0 < n_t; t0 += NL_WARPS * gridDim.x * 32) {
-        const int a = t0 + lane;
-        /* the warp's 32 particles share one column of list tiles: entry j of
-         * particle t0 + i sits at tiles + (j & ~7) * 32 + i * 8 + (j & 7) */
-        int *const tiles = nbr + (int64_t)(t0 >> 5) * maxn * 32;
+    constexpr int PP = 32 / G; /* particles per warp */
+    const int sub = lane % G;
+    for (int t0 = (blockIdx.x * NL_WARPS + w) * PP; t0 < n_t; t0 += NL_WARPS * gridDim.x * PP) {
+        const int a = t0 + lane / G;
+        /* the warp's particles share one column of list tiles: entry j of
+         * particle a sits at tiles + (j & ~7) * 32 + (j & 7) */
+        int4 *const tiles = reinterpret_cast<int4 *>(nbr + (int64_t)(a >> 5) * maxn * 32 + (a & 31) * 8);
         bool act = false;
         int key = 0;
         if (a < n_t) {
@@ -518,14 +546,50 @@ __global__ void __launch_bounds__(NL_WARPS * 32, 3) k_nlist(DevCfg c, DevState s
         const int col = key / zdim;
         float4 pa0 = make_float4(0.f, 0.f, 0.f, 0.f);
         if (act) pa0 = P0[a];
-        int cnt = 0, nb = 0;
+        /* entries in the list tiles (a multiple of 8) and waiting in the queue;
+         * band candidates; what turns a staged entry's code into this lane's */
+        int cnt = 0, qn = 0, nb = 0, adj = 0;
+        /* complete groups of 8 go to the tile, the rest to the queue's front; with
+         * several lanes per particle, all entries, one lane's after the other's */
+        auto flush = [&]() {
+            if (G > 1) {
+                int off = qn;
+#pragma unroll
+                for (int o = 1; o < G; o <<= 1) {
+                    const int v = __shfl_up_sync(FULL, off, o, G);
+                    if (sub >= o) off += v;
+                }
+                const int all = __shfl_sync(FULL, off, G - 1, G);
+                off += cnt - qn;
+                int *const e = reinterpret_cast<int *>(tiles);
+                for (int k = 0; k < qn; k++)
+                    if (off + k < maxn) e[((off + k) & ~7) * 32 + ((off + k) & 7)] = queue[k << 5] + adj;
+                cnt += all;
+                qn = 0;
+                return;
+            }
+            int h = 0;
+            for (; __any_sync(FULL, qn - h >= 8); h += 8) {
+                if (qn - h < 8) continue;
+                if (cnt + 8 <= maxn) {
+                    const int *q = queue + (h << 5);
+                    tiles[cnt * 8] = make_int4(q[0] + adj, q[32] + adj, q[64] + adj, q[96] + adj);
+                    tiles[cnt * 8 + 1] = make_int4(q[128] + adj, q[160] + adj, q[192] + adj, q[224] + adj);
+                }
+                cnt += 8;
+            }
+            const int done = qn & ~7;
+            qn &= 7;
+            if (done)
+                for (int k = 0; k < qn; k++) queue[k << 5] = queue[(done + k) << 5];
+        };
         unsigned pending = __ballot_sync(FULL, act);
         while (pending) {
-            /* a run: lanes in the leader's column within 3 buckets of it */
+            /* a run: lanes in the leader's column within a few buckets of it */
             const int leader = __ffs(pending) - 1;
             const int lcol = __shfl_sync(FULL, col, leader);
             const int zmin = __shfl_sync(FULL, cc[Z], leader);
-            const unsigned gmask = __ballot_sync(FULL, act && col == lcol && cc[Z] <= zmin + 2) & pending;
+            const unsigned gmask = __ballot_sync(FULL, act && col == lcol && cc[Z] <= zmin + NL_RUN<ND>) & pending;
             pending &= ~gmask;
             const int zmax = __shfl_sync(FULL, cc[Z], 31 - __clz(gmask));
             int ccol[3] = {0, 0, 0};
@@ -534,325 +598,284 @@ __global__ void __launch_bounds__(NL_WARPS * 32, 3) k_nlist(DevCfg c, DevState s
             const bool mine = (gmask >> lane) & 1u;
             /* this lane's particle in the run's frame; others sit far away */
             float pv[3] = {1e30f, 1e30f, 1e30f};
-            float ha2 = 0.f;
+            const int my_zr = cc[Z] - zmin + 1;
+            float thr_a = -1.f;
+            const float L = fmaxf(l_other, (float)(zmax - zmin + 2) * cz);
+            const float EPS = 1.5e-6f * L * L;
             if (mine) {
                 pv[0] = pa0.x;
                 pv[1] = pa0.y;
                 pv[2] = pa0.z;
-                pv[Z] += (float)(cc[Z] - zmin) * cz;
-                ha2 = pa0.w * pa0.w;
+                pv[Z] += (float)(my_zr - 1) * cz;
+                adj = (int)((unsigned)(1 - my_zr) * (unsigned)zstride);
+                thr_a = fmaf(pa0.w * pa0.w, K_HI, EPS);
             }
-            const int lane_zr = cc[Z] - zmin + 1;
-            const float L = fmaxf(l_other, (float)(zmax - zmin + 2) * cz);
-            const float EPS = 1.5e-6f * L * L;
-            /* the run's extent on the last axis, widened by the largest support
-             * 2 sr >= 2 max(h) and a rounding margin: nothing outside is a neighbour */
-            float zt_lo = mine ? pv[Z] : 1e30f, zt_hi = mine ? pv[Z] : -1e30f;
+            /* width of the band of doubt below the FP32 cut-off: 1e-6 (2h)^2 + 3 EPS */
+            const float W = 1.01f * (1e-6f * supp * supp + 3.f * EPS);
+            /* the run's bounding box: a candidate further from it than the largest
+             * support 2 sr >= 2 max(h), plus a rounding margin, is no neighbour */
+            float blo[3], bhi[3];
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                zt_lo = fminf(zt_lo, __shfl_xor_sync(FULL, zt_lo, o));
-                zt_hi = fmaxf(zt_hi, __shfl_xor_sync(FULL, zt_hi, o));
+            for (int d = 0; d < ND; d++) {
+                blo[d] = pv[d];
+                bhi[d] = mine ? pv[d] : -1e30f;
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) {
+                    blo[d] = fminf(blo[d], __shfl_xor_sync(FULL, blo[d], o));
+                    bhi[d] = fmaxf(bhi[d], __shfl_xor_sync(FULL, bhi[d], o));
+                }
             }
-            zt_lo -= supp;
-            zt_hi += supp;
-            int nst = 0;
-
-            /* Test the staged candidates 32 at a time, branch-free: one bit per
-             * candidate that passes the widened FP32 test (the staged set is
-             * padded to a multiple of 32 with far-away entries; each staged w
-             * holds the candidate's own threshold K_HI h_b^2 + EPS).  The warp
-             * then writes the passing entries of all its lanes together: the
-             * t-th entry of the chunk goes to the lane whose prefix of pass
-             * counts covers t, and each particle's entries land in consecutive
-             * slots of its 8-entry list tiles, so the stores coalesce.  The
-             * particle itself and band candidates outside the particle's own
-             * stencil leave a hole (-1), which every reader skips. */
-            const float thr_a = fmaf(ha2, K_HI, EPS);
-            s_own[w][lane] = make_float4(pv[0], pv[1], pv[2], ha2);
-            __syncwarp();
-            const int my_zr = lane_zr;
-            auto evaluate = [&]() {
-                if (lane < ((32 - (nst & 31)) & 31)) {
-                    cpos[nst + lane] = make_float4(-1e30f, -1e30f, -1e30f, 0.f);
-                    cent[nst + lane] = 0;
+            /* the run's own particles are the first candidates; each lane skips its own */
+            const int self_j = __popc(gmask & lt_mask) / G;
+            int nst = __popc(gmask) / G;
+            if (mine && sub == 0) {
+#pragma unroll
+                for (int d = 0; d < ND; d++) cx[d][self_j] = -pv[d];
+                ccut[self_j] = thr_a;
+                cent[self_j] = (int)((unsigned)(a | (code_own << B_BITS)) + (unsigned)my_zr * (unsigned)zstride);
+                czr[self_j] = (unsigned char)my_zr;
+            }
+            /* the four staged candidates from j on */
+            struct Four {
+                float4 x, y, z, cut;
+                int4 e;
+            };
+            auto load4 = [&](int j) {
+                Four f;
+                f.x = *reinterpret_cast<const float4 *>(cx[0] + j);
+                if (ND > 1) f.y = *reinterpret_cast<const float4 *>(cx[1] + j);
+                if (ND > 2) f.z = *reinterpret_cast<const float4 *>(cx[2] + j);
+                f.cut = *reinterpret_cast<const float4 *>(ccut + j);
+                f.e = *reinterpret_cast<const int4 *>(cent + j);
+                return f;
+            };
+            /* test 32 staged candidates; SELF: the lane's own particle may be among
+             * them.  The next four are loaded before the current four are appended,
+             * as a load cannot pass the appends' stores.  Returns the smallest margin. */
+            auto round32 = [&](auto self_tag, int j0) {
+                constexpr bool SELF = decltype(self_tag)::value;
+                const unsigned qbase = smem_u32(queue);
+                unsigned qa = qbase + (qn << 7);
+                unsigned near = 0xffffffffu;
+                const float2 ax = make_float2(pv[0], pv[0]), ay = make_float2(pv[1], pv[1]), az = make_float2(pv[2], pv[2]);
+                Four f = load4(j0 + 4 * sub);
+#pragma unroll
+                for (int jb = 0; jb < 32; jb += 4 * G) {
+                    const int jj = jb + 4 * sub;
+                    Four nx = f;
+                    if (jb + 4 * G < 32) nx = load4(j0 + jj + 4 * G);
+                    float2 d = __fadd2_rn(ax, make_float2(f.x.x, f.x.y)), e = __fadd2_rn(ax, make_float2(f.x.z, f.x.w));
+                    float2 r = __fmul2_rn(d, d), q = __fmul2_rn(e, e);
+                    if (ND > 1) {
+                        d = __fadd2_rn(ay, make_float2(f.y.x, f.y.y));
+                        e = __fadd2_rn(ay, make_float2(f.y.z, f.y.w));
+                        r = __ffma2_rn(d, d, r);
+                        q = __ffma2_rn(e, e, q);
+                    }
+                    if (ND > 2) {
+                        d = __fadd2_rn(az, make_float2(f.z.x, f.z.y));
+                        e = __fadd2_rn(az, make_float2(f.z.z, f.z.w));
+                        r = __ffma2_rn(d, d, r);
+                        q = __ffma2_rn(e, e, q);
+                    }
+                    const float df[4] = {fmaxf(thr_a, f.cut.x) - r.x, fmaxf(thr_a, f.cut.y) - r.y,
+                                         fmaxf(thr_a, f.cut.z) - q.x, fmaxf(thr_a, f.cut.w) - q.y};
+                    const int ev[4] = {f.e.x, f.e.y, f.e.z, f.e.w};
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        if (COUNT) {
+                            qn += df[u] >= 0.f;
+                            continue;
+                        }
+                        near = min(near, __float_as_uint(df[u])); /* negative: above every width */
+                        queue_append(qa, ev[u], SELF && j0 + jj + u == self_j ? -1.f : df[u]);
+                    }
+                    f = nx;
                 }
-                __syncwarp();
-                for (int j0 = 0; j0 < nst; j0 += 32) {
-                    unsigned pm = 0u;
-#pragma unroll 8
-                    for (int jj = 0; jj < 32; jj++) {
-                        const float4 q = cpos[j0 + jj];
-                        const float dx = pv[0] - q.x;
-                        const float dy = ND > 1 ? pv[1] - q.y : 0.f;
-                        const float dz = ND > 2 ? pv[2] - q.z : 0.f;
-                        const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-                        pm |= (r2 <= fmaxf(thr_a, q.w) ? 1u : 0u) << jj;
-                    }
-                    const int c_i = __popc(pm);
-                    if (COUNT) {
-                        cnt += c_i;
-                        continue;
-                    }
-                    int incl = c_i;
-#pragma unroll
-                    for (int o = 1; o < 32; o <<= 1) {
-                        const int v = __shfl_up_sync(FULL, incl, o);
-                        if (lane >= o) incl += v;
-                    }
-                    const int T = __shfl_sync(FULL, incl, 31);
-                    const int my_ex = incl - c_i;
-                    for (int base = 0; base < T; base += 32) {
-                        const int t = base + lane;
-                        /* owner: the first lane whose inclusive count exceeds t */
-                        int i = 0;
-#pragma unroll
-                        for (int step = 16; step > 0; step >>= 1) {
-                            const int v = __shfl_sync(FULL, incl, i + step - 1);
-                            if (v <= t) i += step;
-                        }
-                        const unsigned pmi = __shfl_sync(FULL, pm, i);
-                        const int exi = __shfl_sync(FULL, my_ex, i);
-                        const int cni = __shfl_sync(FULL, cnt | (nb << 16), i);
-                        const int zri = __shfl_sync(FULL, my_zr, i);
-                        const float4 own = s_own[w][i];
-                        const float pxi = own.x, pyi = own.y, pzi = own.z, h2i = own.w;
-                        const bool on = t < T;
-                        int e = -1, slot = 0, j = 0;
-                        const int ai = t0 + i;
-                        bool band = false;
-                        if (on) {
-                            /* the r-th set bit of the owner's mask */
-                            const int r = t - exi;
-                            unsigned m = pmi;
-                            int bit = 0, rr = r;
-#pragma unroll
-                            for (int w2 = 16; w2 > 0; w2 >>= 1) {
-                                const int cl = __popc(m & ((1u << w2) - 1u));
-                                if (rr >= cl) {
-                                    rr -= cl;
-                                    m >>= w2;
-                                    bit += w2;
-                                }
-                            }
-                            j = j0 + bit;
-                            slot = (cni & 0xffff) + r;
-                            e = (int)((unsigned)cent[j] + (unsigned)(1 - zri) * (unsigned)zstride);
-                            if (e == (ai | self_e)) {
-                                e = -1; /* the particle itself */
-                            } else {
-                                const float4 q = cpos[j];
-                                const float dx = pxi - q.x;
-                                const float dy = ND > 1 ? pyi - q.y : 0.f;
-                                const float dz = ND > 2 ? pzi - q.z : 0.f;
-                                const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-                                band = r2 >= fmaf(fmaxf(h2i, q.w * (1.f / K_HI)), K_LO, -2.f * EPS);
-                            }
-                        }
-                        const unsigned bb = __ballot_sync(FULL, band);
-                        if (band) {
-                            /* buckets are at least 2h wide, so a candidate outside this
-                             * particle's own 3^d stencil is at least 2h away: it can only
-                             * pass the FP32 test inside the band, and is no neighbour */
-                            const bool in_stencil = (unsigned)((int)czr[j] - zri + 1) <= 2u;
-                            const int qb = (cni >> 16) + __popc(bb & lane_range(max(exi - base, 0), lane));
-                            if (qb < NL_QB) {
-                                bandq[(int64_t)ai * NL_QB + qb] =
-                                    in_stencil && slot < maxn ? make_int2(e, slot) : make_int2(-1, -1);
-                                e = in_stencil ? (e | (int)0x80000000u) : -1;
-                            } else if (!in_stencil || !exact_from_key<ND>(c, s, g, skey, ai, e)) {
-                                e = -1; /* record full: decided here (slow but exact) */
-                            }
-                        }
-                        if (on && slot < maxn) tiles[((slot & ~7) << 5) + (i << 3) + (slot & 7)] = e;
-                        /* band records of this lane's own entries in this round
-                         * (bb is warp-uniform and almost always empty) */
-                        if (bb)
-                            nb += __popc(bb & lane_range(min(max(my_ex - base, 0), 32),
-                                                         min(max(my_ex + c_i - base, 0), 32)));
-                    }
-                    cnt += c_i;
-                }
-                __syncwarp();
-                nst = 0;
+                if (!COUNT) qn = (int)(qa - qbase) >> 7;
+                return near;
             };
 
             /* Range table, one lane per (neighbour column, period piece): the
              * column's buckets zmin-1 .. zmax+1 cut at the periodic seam into at
              * most 3 runs of consecutive keys.  All lanes load their bucket range
-             * at once; the candidates of all ranges are then gathered flat. */
-            constexpr int NCOL = Z == 2 ? 9 : (Z == 1 ? 3 : 1);
-            int r_b0 = 0, r_cnt = 0, r_lin = 0, r_zoff = 0, r_code = 0, r_sh = 0;
-            float r_ox = 0.f, r_oy = 0.f;
-            if (lane < 3 * NCOL) {
-                const int colidx = lane / 3, wz = lane % 3 - 1;
-                int o[2] = {0, 0};
-                if (Z == 2) {
-                    o[0] = colidx / 3 - 1;
-                    o[1] = colidx % 3 - 1;
-                } else if (Z == 1) {
-                    o[0] = colidx - 1;
-                }
-                bool ok = wz == 0 || c.periodic[Z];
-                int col_lin = 0, code_o = code_fixed, shp = 0;
+             * at once; the ranges are then gathered one after the other, 64
+             * candidates at a time, and tested when 64 and more are staged. */
+            const RangeEntry re = range_entry<ND>(lane, ccol, zmin, zmax, dims, c.periodic, cell, 0, start);
+            unsigned live = __ballot_sync(FULL, re.cnt > 0);
+            int b0 = 0, num = 0, lin = 0, zoff = 0, code = 0, shp = 0x15, t = 0;
+            float ox = 0.f, oy = 0.f;
+            bool first = true;
+            for (bool last = false; !last;) {
+                while (nst <= NL_CAP - 64) {
+                    if (t >= num) {
+                        last = live == 0;
+                        if (last) break;
+                        const int src = __ffs(live) - 1;
+                        live &= live - 1;
+                        b0 = __shfl_sync(FULL, re.b0, src);
+                        num = __shfl_sync(FULL, re.cnt, src);
+                        lin = __shfl_sync(FULL, re.lin, src);
+                        zoff = __shfl_sync(FULL, re.zoff, src);
+                        code = __shfl_sync(FULL, re.code, src);
+                        shp = __shfl_sync(FULL, re.shp, src);
+                        ox = __shfl_sync(FULL, re.ox, src);
+                        oy = __shfl_sync(FULL, re.oy, src);
+                        t = 0;
+                    }
+                    const int shv[3] = {(shp & 3) - 1, ((shp >> 2) & 3) - 1, ((shp >> 4) & 3) - 1};
+                    float4 pb[2];
+                    int kb[2];
 #pragma unroll
-                for (int d = ND; d < 3; d++) shp |= 1 << (2 * d); /* unused axes: no shift */
-                float off[2] = {0.f, 0.f};
+                    for (int u = 0; u < 2; u++) {
+                        const int k = b0 + min(t + lane + 32 * u, num - 1);
+                        pb[u] = P0[k];
+                        kb[u] = skey[k];
+                    }
 #pragma unroll
-                for (int d = 0; d < Z; d++) {
-                    int t = ccol[d] + o[d], shd = 0;
-                    if (t < 0) {
-                        ok = ok && c.periodic[d];
-                        t += dims[d];
-                        shd = -1;
-                    } else if (t >= dims[d]) {
-                        ok = ok && c.periodic[d];
-                        t -= dims[d];
-                        shd = 1;
+                    for (int u = 0; u < 2; u++) {
+                        const int k = b0 + t + lane + 32 * u;
+                        bool valid = t + lane + 32 * u < num;
+                        const int zrel = zoff + (kb[u] - lin);
+                        float qv[3] = {pb[u].x, pb[u].y, pb[u].z};
+                        if (Z > 0) qv[0] += ox;
+                        if (Z > 1) qv[1] += oy;
+                        qv[Z] += (float)zrel * cz;
+                        float far2 = 0.f;
+#pragma unroll
+                        for (int d = 0; d < ND; d++) {
+                            const float f = fmaxf(0.f, fmaxf(blo[d] - qv[d], qv[d] - bhi[d]));
+                            far2 = fmaf(f, f, far2);
+                        }
+                        valid = valid && far2 <= supp * supp;
+                        if (shp == 0x15)
+                            valid = valid && !((unsigned)(k - t0) < (unsigned)PP && ((gmask >> ((k - t0) * G)) & 1u));
+                        else if (valid)
+                            valid = img_ok<ND>(tg[k] >> 8, shv);
+                        const unsigned m = __ballot_sync(FULL, valid);
+                        if (valid) {
+                            const int pos = nst + __popc(m & lt_mask);
+#pragma unroll
+                            for (int d = 0; d < ND; d++) cx[d][pos] = -qv[d];
+                            ccut[pos] = fmaf(pb[u].w * pb[u].w, K_HI, EPS);
+                            /* k | code of the candidate's bucket relative to the run's
+                             * first bucket - 1; adj adds the lane's own offset */
+                            cent[pos] = (int)((unsigned)(k | code) + (unsigned)(zrel + 1) * (unsigned)zstride);
+                            czr[pos] = (unsigned char)(zrel + 1);
+                        }
+                        nst += __popc(m);
                     }
-                    col_lin = col_lin * dims[d] + t;
-                    code_o += (o[d] + 1) * code_stride(d);
-                    off[d] = (float)o[d] * cell[d];
-                    shp |= (shd + 1) << (2 * d);
+                    t += 64;
                 }
-                shp |= (wz + 1) << (2 * Z);
-                /* unwrapped z range of this piece */
-                const int zlo = max(zmin - 1, wz * zdim), zhi = min(zmax + 1, (wz + 1) * zdim - 1);
-                if (ok && zlo <= zhi) {
-                    r_lin = col_lin * zdim + (zlo - wz * zdim);
-                    r_b0 = start[r_lin];
-                    r_cnt = start[r_lin + (zhi - zlo) + 1] - r_b0;
-                    r_zoff = zlo - zmin;
-                    r_code = code_o << B_BITS;
-                    r_sh = shp;
-                    r_ox = off[0];
-                    r_oy = off[1];
-                    /* buckets hold their particles sorted on the last axis, so the
-                     * run is sorted there: keep only [zt_lo, zt_hi] (binary search) */
-                    int lo = 0, hi = r_cnt;
-                    while (lo < hi) {
-                        const int mid = (lo + hi) >> 1, k = r_b0 + mid;
-                        const float4 q = P0[k];
-                        const float z = (Z == 0 ? q.x : (Z == 1 ? q.y : q.z)) + (float)(r_zoff + skey[k] - r_lin) * cz;
-                        if (z < zt_lo) lo = mid + 1;
-                        else hi = mid;
+                /* test the complete rounds of 32 and keep the rest, or (last) all of
+                 * them, padded with far-away candidates */
+                if (last && lane < ((32 - (nst & 31)) & 31)) {
+#pragma unroll
+                    for (int d = 0; d < ND; d++) cx[d][nst + lane] = 1e30f;
+                    ccut[nst + lane] = -1.f;
+                }
+                __syncwarp();
+                const int end = last ? (nst + 31) & ~31 : nst & ~31;
+#pragma unroll 1
+                for (int j0 = 0; j0 < end; j0 += 32) {
+                    const int q0 = qn;
+                    const unsigned near = first ? round32(std::true_type{}, j0) : round32(std::false_type{}, j0);
+                    const bool own_round = first;
+                    first = false;
+                    if (COUNT) continue;
+                    __syncwarp();
+                    const bool doubt = near <= __float_as_uint(W);
+                    if (__any_sync(FULL, doubt)) {
+                        /* some candidate within the band of doubt: the round's pass mask
+                         * again, its doubtful bits settled, all lanes one of theirs at a
+                         * time (walls at rest have a score of exact ties each), and the
+                         * entries written anew */
+                        unsigned pass = 0u, open = 0u;
+                        if (doubt) {
+#pragma unroll 4
+                            for (int jj = 0; jj < 32; jj++) {
+                                if (G > 1 && ((jj >> 2) % G) != sub) continue;
+                                const int j = j0 + jj;
+                                const float dx = pv[0] + cx[0][j], dy = ND > 1 ? pv[1] + cx[1][j] : 0.f;
+                                const float dz = ND > 2 ? pv[2] + cx[2][j] : 0.f;
+                                const float df = fmaxf(thr_a, ccut[j]) - fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+                                if (df >= 0.f) pass |= 1u << jj;
+                                if (df >= 0.f && df <= W) open |= 1u << jj;
+                            }
+                            if (own_round) {
+                                pass &= ~(1u << self_j);
+                                open &= pass;
+                            }
+                            nb += __popc(open);
+                        }
+                        while (__any_sync(FULL, open)) {
+                            if (open) {
+                                const int jj = __ffs(open) - 1, j = j0 + jj;
+                                open &= open - 1;
+                                if (!settle_band<ND>(cp, s, dims, cc, a, cent[j] + adj, (int)czr[j] - my_zr))
+                                    pass &= ~(1u << jj);
+                            }
+                            __syncwarp();
+                        }
+                        if (doubt) {
+                            qn = q0;
+                            for (; pass; pass &= pass - 1) {
+                                queue[qn << 5] = cent[j0 + __ffs(pass) - 1];
+                                qn++;
+                            }
+                        }
+                        __syncwarp();
                     }
-                    const int first = lo;
-                    hi = r_cnt;
-                    while (lo < hi) {
-                        const int mid = (lo + hi) >> 1, k = r_b0 + mid;
-                        const float4 q = P0[k];
-                        const float z = (Z == 0 ? q.x : (Z == 1 ? q.y : q.z)) + (float)(r_zoff + skey[k] - r_lin) * cz;
-                        if (z <= zt_hi) lo = mid + 1;
-                        else hi = mid;
-                    }
-                    r_b0 += first;
-                    r_cnt = lo - first;
+                    if (__any_sync(FULL, qn > NL_QN - 32)) flush();
+                }
+                if (last) break;
+                nst -= end;
+                float x[3] = {0.f, 0.f, 0.f}, cut = 0.f;
+                int e = 0;
+                unsigned char zr = 0;
+                if (lane < nst) {
+#pragma unroll
+                    for (int d = 0; d < ND; d++) x[d] = cx[d][end + lane];
+                    cut = ccut[end + lane];
+                    e = cent[end + lane];
+                    zr = czr[end + lane];
+                }
+                __syncwarp();
+                if (lane < nst) {
+#pragma unroll
+                    for (int d = 0; d < ND; d++) cx[d][lane] = x[d];
+                    ccut[lane] = cut;
+                    cent[lane] = e;
+                    czr[lane] = zr;
                 }
             }
-            /* exclusive prefix of the range sizes over the lanes */
-            int r_excl = r_cnt;
+            __syncwarp();
+        }
+        if (COUNT) {
+            if (act) ncnt[a] = qn;
+            continue;
+        }
+        flush();
+        if (G > 1) {
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int v = __shfl_up_sync(FULL, r_excl, o);
-                if (lane >= o) r_excl += v;
-            }
-            const int total = __shfl_sync(FULL, r_excl, 31);
-            r_excl -= r_cnt;
-
-            for (int t = 0;;) {
-              for (; t < total && nst + 32 <= NL_CAP; t += 32) {
-                const int j = t + lane;
-                /* the range holding flat index j: the last lane with excl <= j */
-                int src = 0;
-#pragma unroll
-                for (int step = 16; step > 0; step >>= 1) {
-                    const int e = __shfl_sync(FULL, r_excl, src + step);
-                    if (e <= j) src += step;
-                }
-                const int b0 = __shfl_sync(FULL, r_b0, src), ex = __shfl_sync(FULL, r_excl, src);
-                const int lin = __shfl_sync(FULL, r_lin, src), zoff = __shfl_sync(FULL, r_zoff, src);
-                const int code = __shfl_sync(FULL, r_code, src), shp = __shfl_sync(FULL, r_sh, src);
-                const float ox = __shfl_sync(FULL, r_ox, src), oy = __shfl_sync(FULL, r_oy, src);
-                bool valid = j < total;
-                float4 pb = make_float4(0.f, 0.f, 0.f, 0.f);
-                int k = 0, zrel = 0;
-                if (valid) {
-                    k = b0 + (j - ex);
-                    pb = P0[k];
-                    zrel = zoff + (skey[k] - lin);
-                    if (shp != 0x15) {
-                        const int shv[3] = {(shp & 3) - 1, ((shp >> 2) & 3) - 1, ((shp >> 4) & 3) - 1};
-                        valid = img_ok<ND>(tg[k] >> 8, shv);
-                    }
-                }
-                const unsigned m = __ballot_sync(FULL, valid);
-                if (valid) {
-                    const int pos = nst + __popc(m & lt_mask);
-                    float qv[3] = {pb.x, pb.y, pb.z};
-                    if (Z > 0) qv[0] += ox;
-                    if (Z > 1) qv[1] += oy;
-                    qv[Z] += (float)zrel * cz;
-                    cpos[pos] = make_float4(qv[0], qv[1], qv[2], fmaf(pb.w * pb.w, K_HI, EPS));
-                    /* k | code of the candidate's bucket relative to the run's
-                     * first bucket - 1; evaluate adds the lane's own offset */
-                    cent[pos] = (int)((unsigned)(k | code) + (unsigned)(zrel + 1) * (unsigned)zstride);
-                    czr[pos] = (unsigned char)(zrel + 1);
-                }
-                nst += __popc(m);
-              }
-              evaluate();
-              if (t >= total) break;
-            }
+            for (int o = 1; o < G; o <<= 1) nb += __shfl_xor_sync(FULL, nb, o);
+            if (sub) continue;
         }
         if (act) {
-            ncnt[a] = COUNT ? cnt : min(cnt, maxn);
-            if (!COUNT) {
-                bandn[a] = min(nb, NL_QB);
-                /* stored counts never exceed the list depth; an overflow is an error */
-                if (cnt > maxn) set_err(g, SPHDEM_ERR_CAPACITY, cnt);
-            }
-        } else if (!COUNT && a < n_t) {
-            bandn[a] = 0;
-        }
-    }
-}
-
-/* Decide the recorded band candidates of every particle: the double-float
- * refinement settles all but FP64 ties, which take the reference's FP64
- * predicate.  Keep (clear the pending bit) or mark the list slot invalid (-1). */
-template <int ND>
-__global__ void k_band_fix(DevCfg c, DevState s, const DevGlobals *__restrict__ g, const int *__restrict__ start,
-                           const int *__restrict__ skey, const float4 *__restrict__ P0,
-                           const float4 *__restrict__ P0lo, const int2 *__restrict__ bandq,
-                           const int *__restrict__ bandn, int *__restrict__ nbr, int64_t ld) {
-    const int n_t = start[g->n_sph_cells];
-    float cell[3], cell_lo[3];
-    float cmax = 0.f;
+            /* the last, incomplete group */
+            if (G == 1 && qn > 0 && cnt + 8 <= maxn) {
+                int v[8];
 #pragma unroll
-    for (int d = 0; d < 3; d++) {
-        const double cw = c.periodic[d] ? g->scell[d] : g->sr2;
-        cell[d] = (float)cw;
-        cell_lo[d] = (float)(cw - (double)cell[d]);
-        if (d < ND) cmax = fmaxf(cmax, cell[d]);
-    }
-    const int dims[3] = {g->sdims[0], g->sdims[1], g->sdims[2]};
-    for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < n_t; a += gridDim.x * blockDim.x) {
-        const int nb = bandn[a];
-        if (nb == 0) continue;
-        int cc[3] = {0, 0, 0};
-        decode<ND>(skey[a], dims, cc);
-        const float4 pa = P0[a], al = P0lo[a];
-        for (int k = 0; k < nb; k++) {
-            const int2 it = bandq[(int64_t)a * NL_QB + k];
-            if (it.y < 0) continue; /* a blank record */
-            const int e = it.x, b = e & B_MASK;
-            int o[3];
-            nl_decode_code(e >> B_BITS, o);
-            int dec = nl_refine<ND>(pa, al, P0[b], P0lo[b], o, cell, cell_lo, 1e-13f * cmax * cmax);
-            /* an FP64 tie: the reference's predicate on the periodic image */
-            if (dec == 0) dec = exact_from_code<ND>(c, s, g, a, e, cc) ? 1 : -1;
-            nbr[nl_at(a, it.y, ld)] = dec > 0 ? e : -1;
+                for (int k = 0; k < 8; k++) v[k] = k < qn ? queue[k << 5] + adj : -1;
+                tiles[cnt * 8] = make_int4(v[0], v[1], v[2], v[3]);
+                tiles[cnt * 8 + 1] = make_int4(v[4], v[5], v[6], v[7]);
+            }
+            cnt += qn;
+            /* stored counts never exceed the list depth; an overflow is an error */
+            ncnt[a] = min(cnt, maxn);
+            if (cnt > maxn) set_err(g, SPHDEM_ERR_CAPACITY, cnt);
         }
+        if (a < n_t) bandn[a] = nb;
     }
 }
 
@@ -1046,8 +1069,6 @@ __device__ __noinline__ void boundary32(const DevCfg *__restrict__ cp, const flo
  * range cut at the capacity) read from global memory. */
 constexpr int ST_CAP = 1536;    /* staged records per block (2 or 3 x 16 B each) */
 constexpr int ST_MAXSLOT = 9;   /* neighbour columns: 3^(d-1) */
-
-__device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
 
 __device__ __forceinline__ void mbar_init(unsigned long long *bar, unsigned count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
@@ -2001,73 +2022,6 @@ __global__ void k_pack_dem_drag(DevState s, const float *__restrict__ shep32, co
                         (float)s.row(FD_FDRAG + 2)[i]);
 }
 
-/* One lane's entry of a bucket range table around a run of buckets (ccol
- * on the leading axes, zmin..zmax on the last axis Z): lane = 3 * column +
- * period piece, for the 3^(d-1) neighbour columns; each entry is a run of
- * consecutive keys key0 + lin .. (buckets zmin-1 .. zmax+1 of the column,
- * cut at a periodic seam).  Entries of other lanes are empty. */
-struct RangeEntry {
-    int b0, cnt, lin, zoff, shp, code;
-    float ox, oy;
-};
-
-template <int ND>
-__device__ __forceinline__ RangeEntry range_entry(int lane, const int *ccol, int zmin, int zmax, const int *dims,
-                                                  const int *periodic, const float *cell, int key0,
-                                                  const int *__restrict__ start) {
-    constexpr int Z = ND - 1;
-    constexpr int NCOL = Z == 2 ? 9 : (Z == 1 ? 3 : 1);
-    RangeEntry r = {0, 0, 0, 0, 0x15, 0, 0.f, 0.f};
-    if (lane >= 3 * NCOL) return r;
-    const int colidx = lane / 3, wz = lane % 3 - 1;
-    int o[2] = {0, 0};
-    if (Z == 2) {
-        o[0] = colidx / 3 - 1;
-        o[1] = colidx % 3 - 1;
-    } else if (Z == 1) {
-        o[0] = colidx - 1;
-    }
-    bool ok = wz == 0 || periodic[Z];
-    int col_lin = 0, code = 0, shp = 0;
-    float off[2] = {0.f, 0.f};
-#pragma unroll
-    for (int d = ND; d < 3; d++) {
-        shp |= 1 << (2 * d);
-        code += code_stride(d);
-    }
-#pragma unroll
-    for (int d = 0; d < Z; d++) {
-        int t = ccol[d] + o[d], shd = 0;
-        if (t < 0) {
-            ok = ok && periodic[d];
-            t += dims[d];
-            shd = -1;
-        } else if (t >= dims[d]) {
-            ok = ok && periodic[d];
-            t -= dims[d];
-            shd = 1;
-        }
-        col_lin = col_lin * dims[d] + t;
-        code += (o[d] + 1) * code_stride(d);
-        off[d] = (float)o[d] * cell[d];
-        shp |= (shd + 1) << (2 * d);
-    }
-    shp |= (wz + 1) << (2 * Z);
-    const int zdim = dims[Z];
-    const int zlo = max(zmin - 1, wz * zdim), zhi = min(zmax + 1, (wz + 1) * zdim - 1);
-    if (ok && zlo <= zhi) {
-        r.lin = key0 + col_lin * zdim + (zlo - wz * zdim);
-        r.b0 = start[r.lin];
-        r.cnt = start[r.lin + (zhi - zlo) + 1] - r.b0;
-        r.zoff = zlo - zmin;
-        r.shp = shp;
-        r.code = code << B_BITS;
-        r.ox = off[0];
-        r.oy = off[1];
-    }
-    return r;
-}
-
 /* exclusive prefix of v over the warp; *total = the sum */
 __device__ __forceinline__ int warp_excl_scan(int v, int lane, int *total) {
     int x = v;
@@ -2490,17 +2444,18 @@ int dem_end_blocks(int64_t particles) {
 }
 
 /* list build: grid-stride over 32-particle slices, one wave of resident blocks */
-template <int ND, bool COUNT>
+template <int ND, bool COUNT, int G>
 int nlist_blocks(int64_t particles) {
     static int resident = 0;
     if (!resident) {
         int dev = 0, sms = 0, per_sm = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_nlist<ND, COUNT>, NL_WARPS * 32, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_nlist<ND, COUNT, G>, NL_WARPS * 32, 0);
         resident = std::max(1, sms * per_sm);
     }
-    const int64_t need = (particles + 32 * NL_WARPS - 1) / (32 * NL_WARPS);
+    const int per_block = 32 / G * NL_WARPS;
+    const int64_t need = (particles + per_block - 1) / per_block;
     return (int)std::max<int64_t>(1, std::min<int64_t>(resident, need));
 }
 
@@ -2542,7 +2497,7 @@ void pack(sphdem_ctx *c, bool coupling) {
     coupling = coupling && c->cfg.liq_dem();
 #define L_(ND)                                                                                                  \
     SPHDEM_LAUNCH(c, "pack32", k_pack<ND>, grid_for(c->n, 256), 256, 0, c->cfg, c->A, c->buf.skey, c->g,         \
-                  c->mx_pos, c->mx_vel, c->mx_aux, c->mx_poslo, c->mx_tg, c->mx_rc4, (int)coupling, c->mx_ds,      \
+                  c->mx_pos, c->mx_vel, c->mx_aux, c->mx_tg, c->mx_rc4, (int)coupling, c->mx_ds,      \
                   c->mx_nb, c->n)
     SPHDEM_ND_DISPATCH(c->cfg.nd, L_);
 #undef L_
@@ -2563,30 +2518,38 @@ void pack_fpi(sphdem_ctx *c) {
     SPHDEM_LAUNCH(c, "pack_fpi32", k_pack_fpi, grid_for(c->n, 256), 256, 0, c->A, c->mx_q0, c->mx_q1, c->mx_q2, c->n);
 }
 
-int band_records_per_particle() { return NL_QB; }
-
 void nlist(sphdem_ctx *c) {
-#define L_(ND)                                                                                                  \
-    SPHDEM_LAUNCH(c, "nlist32", (k_nlist<ND, false>), (std::max(1, nlist_blocks<ND, false>(c->n) / c->grid_div)), NL_WARPS * 32, 0, c->cfg,  \
-                  c->A, c->buf.start, c->buf.skey, c->g, c->mx_pos, c->mx_tg, c->mx_nbr, c->mx_ncnt, c->mx_maxn,  \
-                  c->cap, c->mx_bandq, c->mx_bandn)
+    /* below these counts the warps of 32 particles do not fill the chip and the
+     * pass is the length of one warp's chain.  Two builds, one / four lanes per
+     * particle: 2D 6.5k 38 / 26 us, 23k 45 / 30, 44k 46 / 38, 86k 50 / 56; 3D
+     * 3.8k 112 / 69, 23k 113 / 82, 47k 123 / 131, 91k 153 / 228 */
+    const bool split = c->n < (c->cfg.nd == 3 ? 40000 : 65000);
+#define LG_(ND, G)                                                                                              \
+    SPHDEM_LAUNCH(c, "nlist32", (k_nlist<ND, false, G>),                                                       \
+                  (std::max(1, nlist_blocks<ND, false, G>(c->n) / c->grid_div)), NL_WARPS * 32, 0, c->cfg, c->dcfg, \
+                  c->A, c->buf.start, c->buf.skey, c->g, c->mx_pos, c->mx_tg, c->mx_nbr, c->mx_ncnt, c->mx_maxn, \
+                  c->mx_bandn)
+#define L_(ND)            \
+    do {                  \
+        if (split)        \
+            LG_(ND, 4);   \
+        else              \
+            LG_(ND, 1);   \
+    } while (0)
     SPHDEM_ND_DISPATCH(c->cfg.nd, L_);
 #undef L_
-#define L_(ND)                                                                                                  \
-    SPHDEM_LAUNCH(c, "band_fix", k_band_fix<ND>, grid_for(c->n, 256), 256, 0, c->cfg, c->A, c->g, c->buf.start,  \
-                  c->buf.skey, c->mx_pos, c->mx_poslo, c->mx_bandq, c->mx_bandn, c->mx_nbr, (int64_t)c->mx_maxn)
-    SPHDEM_ND_DISPATCH(c->cfg.nd, L_);
-#undef L_
+#undef LG_
 }
 
 /* largest neighbour count at the current positions (sizes the lists); band
- * candidates count as neighbours, so this is an upper bound */
+ * candidates and the particle itself count as neighbours, so this is an upper
+ * bound */
 int nlist_max_count(sphdem_ctx *c) {
     SPHDEM_CUDA_CHECK(cudaMemsetAsync(c->mx_ncnt, 0, c->n * sizeof(int), c->stream));
 #define L_(ND)                                                                                                    \
-    k_nlist<ND, true><<<nlist_blocks<ND, true>(c->n), NL_WARPS * 32, 0, c->stream>>>(                           \
-        c->cfg, c->A, c->buf.start, c->buf.skey, c->g, c->mx_pos, c->mx_tg, c->mx_nbr, c->mx_ncnt, 0, c->cap,     \
-        nullptr, nullptr)
+    k_nlist<ND, true, 1><<<nlist_blocks<ND, true, 1>(c->n), NL_WARPS * 32, 0, c->stream>>>(                           \
+        c->cfg, c->dcfg, c->A, c->buf.start, c->buf.skey, c->g, c->mx_pos, c->mx_tg, c->mx_nbr,      \
+        c->mx_ncnt, 0, nullptr)
     SPHDEM_ND_DISPATCH(c->cfg.nd, L_);
 #undef L_
     SPHDEM_CUDA_CHECK(cudaGetLastError());
