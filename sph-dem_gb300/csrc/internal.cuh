@@ -184,9 +184,9 @@ void mixed_list_export(sphdem_ctx *c, int *cnt, const long long *offs, int *idx)
 
 /* pairs32.cu: mixed-precision passes */
 namespace mixed {
-/* pack the FP32 records; `coupling` also packs the reference DEM buckets and
- * the coupling windows the SPH-DEM passes need */
-void pack(sphdem_ctx *c, bool coupling = true);
+/* pack the FP32 records of the middle phase, with the reference DEM buckets and
+ * the coupling windows its SPH-DEM passes need, or those of the end phase */
+void pack(sphdem_ctx *c, bool middle = true);
 void pack_fpi(sphdem_ctx *c);
 void nlist(sphdem_ctx *c);
 /* once per process, outside stream capture: kernel attributes of the step */
@@ -194,6 +194,11 @@ void prepare(sphdem_ctx *c);
 void zero_shep(sphdem_ctx *c);
 int nlist_max_count(sphdem_ctx *c);
 void omega_eos(sphdem_ctx *c, bool omega, bool eos);
+/* lists32.cu: the force / continuity passes specialised on the physics class;
+ * false when the handle's class has none */
+bool force_lists(sphdem_ctx *c);
+bool dddt_lists(sphdem_ctx *c);
+void prepare_lists();
 void force(sphdem_ctx *c);
 void dddt(sphdem_ctx *c);
 void porosity(sphdem_ctx *c);

@@ -35,69 +35,13 @@
  * (~80 FP32 FLOP per listed pair against 4 B of list + 48 B of packed input).
  */
 #include <algorithm>
-#include <cfloat>
-#include <climits>
 #include <type_traits>
 #include <vector>
 
-#include "internal.cuh"
+#include "mixed.cuh"
 
 namespace sphdem {
 namespace {
-
-constexpr int BLK = 128;
-constexpr int B_BITS = 26;
-constexpr int B_MASK = (1 << B_BITS) - 1;
-
-struct Kahan {
-    float s, c;
-    __device__ __forceinline__ void init(float v) {
-        s = v;
-        c = 0.f;
-    }
-    __device__ __forceinline__ void add(float x) {
-        const float y = x - c;
-        const float t = s + y;
-        c = (t - s) - y;
-        s = t;
-    }
-    __device__ __forceinline__ double value() const { return (double)s - (double)c; }
-};
-
-/* A plain FP32 sum with the same interface, for sums whose rounding does
- * not reach the results' tolerance: the calcOmega sum under
- * VAR_H_CORRECTION, where Omega = 1 + h sum / (rho NDIM) is an O(1) factor
- * known to ~1e-6 from ~100 terms. */
-struct Plain {
-    float s;
-    __device__ __forceinline__ void init(float v) { s = v; }
-    __device__ __forceinline__ void add(float x) { s += x; }
-};
-
-__device__ __forceinline__ float wK32(float q, float wcon) {
-    if (q > 2.f) return 0.f;
-    const float t = 2.f - q, t2 = t * t;
-    return wcon * (t2 * t2) * (1.f + 2.f * q);
-}
-__device__ __forceinline__ float wdK32(float q, float wcon) {
-    if (q > 2.f) return 0.f;
-    const float t = 2.f - q, t2 = t * t;
-    return wcon * (-4.f * (t2 * t) * (1.f + 2.f * q) + 2.f * (t2 * t2));
-}
-
-template <int ND>
-__device__ __forceinline__ float powi(float x) {
-    float r = x;
-#pragma unroll
-    for (int k = 1; k < ND; k++) r *= x;
-    return r;
-}
-
-__device__ __forceinline__ float warp_sum(float v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
 
 /* FP64 origin of SPH bucket `cell` on axis d, and its size */
 __device__ __forceinline__ double sph_origin(const DevCfg &c, const DevGlobals *g, int d, int cell) {
@@ -108,21 +52,6 @@ __device__ __forceinline__ double sph_width(const DevCfg &c, const DevGlobals *g
 }
 __device__ __forceinline__ double dem_origin(const DevCfg &c, int d, int cell) {
     return c.dorig[d] + cell * c.dcell[d];
-}
-
-template <int ND>
-__device__ __forceinline__ void decode(int key, const int *dims, int *cc) {
-    if (ND == 3) {
-        cc[2] = key % dims[2];
-        key /= dims[2];
-        cc[1] = key % dims[1];
-        cc[0] = key / dims[1];
-    } else if (ND == 2) {
-        cc[1] = key % dims[1];
-        cc[0] = key / dims[1];
-    } else {
-        cc[0] = key;
-    }
 }
 
 /* stencil neighbour (offsets o) with periodic wrap; -1 when off the grid */
@@ -184,8 +113,11 @@ __device__ __noinline__ bool exact_pair(const DevCfg *__restrict__ cp, const Dev
 
 /* ---------------------------------------------------------------------- */
 /* P0 = (offset from own bucket origin, h), P1 = (vhat, mass; negated for
- * particles that are neither sph / sphBoundary nor DEM),
- * P2 = (dens, pdr2, porosity, 1/h), tg = type | gcode << 8 */
+ * particles that are neither sph / sphBoundary nor DEM), P2 = (dens, pdr2, cF,
+ * 1/h) for the middle phase and (dens, cF, porosity, 1/h) for the end phase,
+ * where cF = -10 C / h^(d+2) is the factor of the Wendland gradient F(r, h) =
+ * cF (2 - r/h)^3 and a DEM particle's second place holds its radius,
+ * tg = type | gcode << 8 */
 /* reference DEM bucket indices packed 10 bits per axis (biased by 512) */
 constexpr int CP_BIAS = 512;
 
@@ -198,7 +130,7 @@ __device__ __forceinline__ int pack_cells(const int *k, int nd) {
 template <int ND>
 __global__ void k_pack(DevCfg c, DevState s, const int *__restrict__ skey, const DevGlobals *__restrict__ g,
                        float4 *__restrict__ P0, float4 *__restrict__ P1, float4 *__restrict__ P2,
-                       int *__restrict__ tg, int4 *__restrict__ RC4, int with_rc,
+                       int *__restrict__ tg, int4 *__restrict__ RC4, int with_rc, int middle,
                        float4 *__restrict__ DS, float4 *__restrict__ NB, int64_t n) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -231,8 +163,9 @@ __global__ void k_pack(DevCfg c, DevState s, const int *__restrict__ skey, const
     P1[i] = make_float4(vh[0], vh[1], vh[2], (is_sph_or_sphb(t) || dem) ? mpk : -mpk);
     /* a DEM particle's pdr2 slot holds its radius (the contact pre-test) */
     const double rad = s.row(FD_RADIUS)[i] > 0 ? s.row(FD_RADIUS)[i] : c.dem_radius;
-    P2[i] = make_float4((float)s.row(FD_DENS)[i], (float)(t == T_DEM ? rad : s.row(FD_PDR2)[i]),
-                        (float)s.row(FD_POR)[i], (float)s.row(FD_IH)[i]);
+    const float cF = (float)(-10.0 * c.wcon * s.row(FD_IHN2)[i]);
+    P2[i] = make_float4((float)s.row(FD_DENS)[i], t == T_DEM ? (float)rad : (middle ? (float)s.row(FD_PDR2)[i] : cF),
+                        middle ? cF : (float)s.row(FD_POR)[i], (float)s.row(FD_IH)[i]);
     if (is_boundary(t)) {
         float nv[3][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
 #pragma unroll
@@ -372,17 +305,6 @@ constexpr int NL_QN = 64;     /* queue slots per lane: moved on when over 32 are
 template <int ND>
 constexpr int NL_RUN = ND == 3 ? 2 : (ND == 2 ? 6 : 14);
 
-__device__ __forceinline__ int code_stride(int d) { return d == 0 ? 9 : (d == 1 ? 3 : 1); }
-
-/* Neighbour lists: slot j of particle a, in tiles of 32 particles x 8
- * entries -- each particle's 8 entries contiguous, the 32 particles' groups
- * back to back -- so a warp of consecutive particles reads 8 entries each
- * with two coalesced int4 loads and the build writes a particle's entries in
- * runs.  maxn (the list depth) is a multiple of 8. */
-__device__ __forceinline__ int64_t nl_at(int64_t a, int j, int64_t maxn) {
-    return ((a >> 5) * maxn + (j & ~7)) * 32 + ((a & 31) << 3) + (j & 7);
-}
-
 /* One lane's entry of a bucket range table around a run of buckets (ccol
  * on the leading axes, zmin..zmax on the last axis Z): lane = 3 * column +
  * period piece, for the 3^(d-1) neighbour columns; each entry is a run of
@@ -470,8 +392,6 @@ __device__ __forceinline__ bool settle_band(const DevCfg *__restrict__ cp, const
     }
     return exact_pair<ND>(cp, s, a, e & B_MASK, sh[0], sh[1], sh[2], 0.0, 0);
 }
-
-__device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
 
 /* append e to the lane's queue column (next free slot at shared address qa) when margin >= 0, without a branch */
 __device__ __forceinline__ void queue_append(unsigned &qa, int e, float margin) {
@@ -879,35 +799,6 @@ __global__ void __launch_bounds__(NL_WARPS * 32, 5) k_nlist(DevCfg c, const DevC
     }
 }
 
-__device__ __forceinline__ void load_cell32(const DevCfg &c, const DevGlobals *g, float *cell) {
-#pragma unroll
-    for (int d = 0; d < 3; d++) cell[d] = (float)(c.periodic[d] ? g->scell[d] : g->sr2);
-}
-
-/* The 27 stencil shifts o * bucket size, indexed by the list entry's code,
- * in shared memory: one load per pair instead of a decode and three
- * int-to-float conversions.  Every thread of the block must call this. */
-__device__ __forceinline__ const float4 *stencil_shifts(const DevCfg &c, const DevGlobals *g) {
-    __shared__ float4 tab[27];
-    if (threadIdx.x < 27) {
-        const int code = threadIdx.x;
-        const float o0 = (float)(code / 9 - 1), o1 = (float)((code / 3) % 3 - 1), o2 = (float)(code % 3 - 1);
-        float cell[3];
-        load_cell32(c, g, cell);
-        tab[code] = make_float4(o0 * cell[0], o1 * cell[1], o2 * cell[2], 0.f);
-    }
-    __syncthreads();
-    return tab;
-}
-
-template <int ND>
-__device__ __forceinline__ void nb_delta_t(int e, const float4 *tab, float4 pa, float4 pb, float *d) {
-    const float4 sft = tab[e >> B_BITS];
-    d[0] = pa.x - pb.x - sft.x;
-    d[1] = ND > 1 ? pa.y - pb.y - sft.y : 0.f;
-    d[2] = ND > 2 ? pa.z - pb.z - sft.z : 0.f;
-}
-
 /* ---------------------------------------------------------------------- */
 template <int ND>
 __global__ void __launch_bounds__(BLK) k_omega_eos(DevCfg c, DevState s, const DevGlobals *__restrict__ g,
@@ -978,252 +869,15 @@ __global__ void __launch_bounds__(BLK) k_omega_eos(DevCfg c, DevState s, const D
         const double pdr2 = press * (rd * rd);
         s.row(FD_PRESS)[a] = press;
         s.row(FD_PDR2)[a] = pdr2;
-        float4 p2 = P2[a];
-        p2.y = (float)pdr2;
-        p2.z = (float)s.row(FD_POR)[a];
-        P2[a] = p2;
+        P2[a].y = (float)pdr2;
     }
 }
 
 /* ---------------------------------------------------------------------- */
-__device__ __forceinline__ void block_min_atomic(float v, unsigned long long *target) {
-    __shared__ float smin[32];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fminf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if (lane == 0) smin[w] = v;
-    __syncthreads();
-    if (w == 0) {
-        v = lane < (int)(blockDim.x >> 5) ? smin[lane] : FLT_MAX;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v = fminf(v, __shfl_xor_sync(0xffffffffu, v, o));
-        if (lane == 0 && v < FLT_MAX) atomic_min_pos(target, (double)v);
-    }
-}
-
-/* boundary force of sph.h:736-918 in FP32 (b is a repulsive boundary particle) */
-template <int ND>
-__device__ __noinline__ void boundary32(const DevCfg *__restrict__ cp, const float4 *__restrict__ NB, int b, float d0,
-                                        float d1, float d2, float r, float dv0, float dv1, float dv2, float ma, float mb,
-                                        float *fbx) {
-    const DevCfg &c = *cp;
-    const float d[3] = {d0, d1, d2}, dv[3] = {dv0, dv1, dv2};
-    const float4 N1 = NB[3 * b], N2 = NB[3 * b + 1], N3 = NB[3 * b + 2];
-    const float n1[3] = {N1.x, N1.y, N1.z}, n2[3] = {N2.x, N2.y, N2.z}, nt[3] = {N3.x, N3.y, N3.z};
-    float np[3];
-    if (n2[0] == 0.f && n2[1] == 0.f && n2[2] == 0.f) {
-        for (int k = 0; k < 3; k++) np[k] = n1[k];
-    } else {
-        const float rd1 = d[0] * n1[0] + d[1] * n1[1] + d[2] * n1[2];
-        const float rd2 = d[0] * n2[0] + d[1] * n2[1] + d[2] * n2[2];
-        const float rnt = r * r * (n1[0] * n2[0] + n1[1] * n2[1] + n1[2] * n2[2]) - rd1 * rd2;
-        if (rnt <= 0.f) {
-            for (int k = 0; k < 3; k++) np[k] = d[k] / r;
-        } else {
-            const float con = N1.w;
-            for (int k = 0; k < 3; k++) np[k] = con * (rd1 - rd2) > 0.f ? n1[k] : n2[k];
-        }
-    }
-    const float rperp = np[0] * d[0] + np[1] * d[1] + np[2] * d[2];
-    const float rt0 = d[0] - rperp * np[0], rt1 = d[1] - rperp * np[1], rt2 = d[2] - rperp * np[2];
-    const float rdelp = c.f_rdelp;
-    float pt0, pt1;
-    if (ND == 3) {
-        pt0 = fabsf(rt0 * nt[0] + rt1 * nt[1] + rt2 * nt[2]);
-        const float cx = rt1 * nt[2] - rt2 * nt[1], cy = rt2 * nt[0] - rt0 * nt[2], cz = rt0 * nt[1] - rt1 * nt[0];
-        pt1 = sqrtf(cx * cx + cy * cy + cz * cz);
-    } else {
-        pt0 = sqrtf(rt0 * rt0 + rt1 * rt1);
-        pt1 = 0.f;
-    }
-    const float pd0 = pt0 * rdelp, pd1 = pt1 * rdelp;
-    if (!(pd0 <= 1.f && pd1 <= 1.f)) return;
-    const float pif = c.f_pi, c0 = c.f_c0;
-    const float pesky = 0.25f * (1.f + cosf(pif * pd0)) * (1.f + cosf(pif * pd1));
-    const float q = fabsf(rperp) * c.f_rpsep;
-    if (!(q < 2.f)) return;
-    const int beta = (d[0] * dv[0] + d[1] * dv[1] + d[2] * dv[2]) < 0.f ? 1 : 0;
-    const float bigA = 0.01f * c0 * c0 - beta * c0 * (dv[0] * np[0] + dv[1] * np[1] + dv[2] * np[2]);
-    const float bfact = 1.f / fabsf(rperp);
-    const float QIN = 2.f / 3.f;
-    float bforce;
-    if (q <= QIN) bforce = bfact * QIN;
-    else if (q <= 1.f) bforce = bfact * (2.f * q - 1.5f * q * q);
-    else bforce = bfact * 0.5f * (2.f - q) * (2.f - q);
-    const float sc = (rperp < 0.f ? -1.f : 1.f) * (2.f * ma / (ma + mb)) * bigA * bforce * pesky;
-    for (int k = 0; k < 3; k++) fbx[k] = sc * np[k];
-}
-
-/* ---------------------------------------------------------------------- */
-/* Neighbour-record staging for the list consumers (TMA bulk copies).
- *
- * A block takes consecutive particles of the bucket order, so most of them
- * lie in one column of buckets along the last axis, and their neighbours in
- * the 3^(d-1) columns around it, over the block's bucket range on the last
- * axis +- one bucket.  Each of those column ranges is a contiguous run of
- * particle slots, so its packed records (P0, P1, P2) are copied global ->
- * shared with one cp.async.bulk per array, completing on one mbarrier.  A
- * list entry's stencil code names its neighbour column, so its record is
- * found in shared memory when its slot lies in that column's staged range,
- * else (another column of the block, a periodic image on the last axis, a
- * range cut at the capacity) read from global memory. */
-constexpr int ST_CAP = 1536;    /* staged records per block (2 or 3 x 16 B each) */
-constexpr int ST_MAXSLOT = 9;   /* neighbour columns: 3^(d-1) */
-
-__device__ __forceinline__ void mbar_init(unsigned long long *bar, unsigned count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-
-__device__ __forceinline__ void mbar_expect_tx(unsigned long long *bar, unsigned bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-                 : "memory");
-}
-
-__device__ __forceinline__ void bulk_g2s(void *dst, const void *src, unsigned bytes, unsigned long long *bar) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-            smem_u32(dst)),
-        "l"(src), "r"(bytes), "r"(smem_u32(bar))
-        : "memory");
-}
-
-__device__ __forceinline__ bool mbar_try_wait(unsigned long long *bar, unsigned parity) {
-    unsigned ok = 0;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-
-/* bounded wait for phase 0 of the staging barrier: false after the limit */
-__device__ __forceinline__ bool mbar_wait_bounded(unsigned long long *bar) {
-    for (int it = 0; it < (1 << 22); it++)
-        if (mbar_try_wait(bar, 0)) return true;
-    return false;
-}
-
-struct Staged {
-    const float4 *S0, *S1, *S2;
-    const int *lo, *num, *base;
-    bool ok;
-};
-
-/* the neighbour column of a stencil code (3D: code / 3, 2D: code / 9) */
-template <int ND>
-__device__ __forceinline__ int st_slot(int code) {
-    return ND == 3 ? code / 3 : (ND == 2 ? code / 9 : 0);
-}
-
-/* Called by every thread of the block.  a0: the block's first slot, n_t:
- * the particles in SPH buckets (sorted by bucket key). */
-template <int ND, int NARR>
-__device__ Staged stage_neighbours(const DevCfg &c, DevGlobals *g, const int *__restrict__ start,
-                                   const int *__restrict__ skey, const float4 *__restrict__ P0,
-                                   const float4 *__restrict__ P1, const float4 *__restrict__ P2, int64_t a0,
-                                   int n_t, float4 *smem) {
-    constexpr int Z = ND - 1;
-    constexpr int NS = ND == 3 ? 9 : (ND == 2 ? 3 : 1);
-    __shared__ int s_lo[ST_MAXSLOT], s_num[ST_MAXSLOT], s_base[ST_MAXSLOT];
-    __shared__ int s_col, s_zmin, s_zmax;
-    __shared__ __align__(8) unsigned long long s_bar;
-    const int dims[3] = {g->sdims[0], g->sdims[1], g->sdims[2]};
-    const int zdim = dims[Z];
-    if (threadIdx.x == 0) {
-        s_col = skey[a0] / zdim;
-        s_zmin = INT_MAX;
-        s_zmax = -1;
-        mbar_init(&s_bar, 1);
-    }
-    __syncthreads();
-    const int64_t a = a0 + threadIdx.x;
-    if (a < n_t) {
-        const int key = skey[a];
-        if (key / zdim == s_col) {
-            atomicMin(&s_zmin, key % zdim);
-            atomicMax(&s_zmax, key % zdim);
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x < NS) {
-        const int t = threadIdx.x;
-        int o[2] = {0, 0}, cc[2] = {0, 0};
-        if (ND == 3) {
-            o[0] = t / 3 - 1;
-            o[1] = t % 3 - 1;
-            cc[0] = s_col / dims[1];
-            cc[1] = s_col % dims[1];
-        } else if (ND == 2) {
-            o[0] = t - 1;
-            cc[0] = s_col;
-        }
-        bool ok = true;
-        int col = 0;
-#pragma unroll
-        for (int d = 0; d < Z; d++) {
-            int x = cc[d] + o[d];
-            if (x < 0 || x >= dims[d]) {
-                ok = ok && c.periodic[d];
-                x = x < 0 ? x + dims[d] : x - dims[d];
-            }
-            col = col * dims[d] + x;
-        }
-        const int zlo = max(s_zmin - 1, 0), zhi = min(s_zmax + 1, zdim - 1);
-        int lo = 0, num = 0;
-        if (ok && zlo <= zhi) {
-            lo = start[col * zdim + zlo];
-            num = start[col * zdim + zhi + 1] - lo;
-        }
-        s_lo[t] = lo;
-        s_num[t] = num;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int base = 0;
-        for (int t = 0; t < NS; t++) {
-            const int num = min(s_num[t], ST_CAP - base);
-            s_num[t] = num;
-            s_base[t] = base;
-            base += num;
-        }
-        mbar_expect_tx(&s_bar, (unsigned)(NARR * 16 * base));
-        for (int t = 0; t < NS; t++) {
-            const int num = s_num[t];
-            if (num <= 0) continue;
-            const unsigned bytes = (unsigned)(16 * num);
-            bulk_g2s(smem + s_base[t], P0 + s_lo[t], bytes, &s_bar);
-            bulk_g2s(smem + ST_CAP + s_base[t], P1 + s_lo[t], bytes, &s_bar);
-            if (NARR > 2) bulk_g2s(smem + 2 * ST_CAP + s_base[t], P2 + s_lo[t], bytes, &s_bar);
-        }
-    }
-    __syncthreads();
-    Staged st;
-    st.S0 = smem;
-    st.S1 = smem + ST_CAP;
-    st.S2 = smem + 2 * ST_CAP;
-    st.lo = s_lo;
-    st.num = s_num;
-    st.base = s_base;
-    bool ok = mbar_wait_bounded(&s_bar);
-    if (!ok) {
-        /* gave up: record it, and keep the block alive (again bounded) until
-         * the copies into its shared memory have landed */
-        set_err(g, SPHDEM_ERR_TIMEOUT, 1);
-        mbar_wait_bounded(&s_bar);
-    }
-    /* the whole block gives up together */
-    st.ok = !__syncthreads_or(!ok);
-    return st;
-}
-
-/* Physics classes the force pass is specialised on (so that the unused
- * viscosity forms, accumulators and branches compile away): the coupled
- * sedimentation form (Morris viscosity, VAR_H_CORRECTION, no anticlumping),
- * the dam-break form (artificial viscosity, constant h, no anticlumping),
- * and every other combination read from the configuration. */
-enum : int { PHYS_GENERIC = 0, PHYS_MORRIS_VARH = 1, PHYS_ARTIFICIAL = 2, PHYS_CG = 3 };
+/* The general force and continuity passes: every physics class that
+ * lists32.cu has no specialised pass for (1D, Monaghan viscosity,
+ * anticlumping, CORRECTED_GRADIENT), read from the configuration. */
+enum : int { PHYS_GENERIC = 0, PHYS_CG = 3 };
 
 /* CORRECTED_GRADIENT in FP32 (sph.h:325-326): the corrected gradient of a
  * pair is invM_a ((dr F - sumGrad_a/sum_a) / sum_a); invM_a, sumGrad_a and
@@ -1254,13 +908,6 @@ struct Cg32 {
     }
 };
 
-inline int phys_class(const DevCfg &c) {
-    const bool anti = !(c.flags & SPHDEM_F_NO_ANTICLUMPING);
-    if (!anti && c.visc == SPHDEM_VISC_MORRIS && c.var_h()) return PHYS_MORRIS_VARH;
-    if (!anti && c.visc == SPHDEM_VISC_ARTIFICIAL && !c.var_h()) return PHYS_ARTIFICIAL;
-    return PHYS_GENERIC;
-}
-
 template <int ND, int PHYS, bool TILE>
 __global__ void __launch_bounds__(BLK) k_force(DevCfg c, const DevCfg *__restrict__ cp, DevState s, DevGlobals *__restrict__ g,
                                                const float4 *__restrict__ P0, const float4 *__restrict__ P1,
@@ -1277,12 +924,11 @@ __global__ void __launch_bounds__(BLK) k_force(DevCfg c, const DevCfg *__restric
         const int n_t = start[g->n_sph_cells];
         const int64_t a0 = blockIdx.x * (int64_t)blockDim.x;
         if (a0 >= n_t) return;  /* no list owner in this block */
-        st = stage_neighbours<ND, 3>(c, g, start, skey, P0, P1, P2, a0, n_t, st_smem);
+        st = stage_neighbours<ND, 3, 1>(c, g, start, skey, P0, P1, P2, a0, n_t, st_smem);
         if (!st.ok) return;
     }
-    const int visc = PHYS == PHYS_MORRIS_VARH ? SPHDEM_VISC_MORRIS
-                     : (PHYS == PHYS_ARTIFICIAL ? SPHDEM_VISC_ARTIFICIAL : c.visc);
-    const bool var_h = PHYS == PHYS_MORRIS_VARH ? true : (PHYS == PHYS_ARTIFICIAL ? false : c.var_h());
+    const int visc = c.visc;
+    const bool var_h = c.var_h();
     const int64_t a = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     float ndt = FLT_MAX;
     const int ta = a < n ? (tg[a] & 0xff) : -1;
@@ -1300,7 +946,7 @@ __global__ void __launch_bounds__(BLK) k_force(DevCfg c, const DevCfg *__restric
         Plain om;
         om.init(-ma * pd_coef * wK32(0.f, wcon));
         const bool sph = ta == T_SPH;
-        const bool anti = PHYS == PHYS_GENERIC && !(c.flags & SPHDEM_F_NO_ANTICLUMPING);
+        const bool anti = !(c.flags & SPHDEM_F_NO_ANTICLUMPING);
         const float visc_nu = (float)c.viscosity, c0 = (float)c.spsound;
         const float liq_visc = (float)(2.0 * c.viscosity * c.dens);
         const float alpha_mon = (float)c.alpha_mon, alpha_art = (float)c.alpha_art;
@@ -1499,7 +1145,7 @@ __global__ void __launch_bounds__(BLK) k_dddt(DevCfg c, DevState s, const DevGlo
         const int n_t = start[g->n_sph_cells];
         const int64_t a0 = blockIdx.x * (int64_t)blockDim.x;
         if (a0 >= n_t) return;  /* no list owner in this block */
-        st = stage_neighbours<ND, 2>(c, const_cast<DevGlobals *>(g), start, skey, P0, P1, P2, a0, n_t, st_smem);
+        st = stage_neighbours<ND, 2, 1>(c, const_cast<DevGlobals *>(g), start, skey, P0, P1, P2, a0, n_t, st_smem);
         if (!st.ok) return;
     }
     const int64_t a = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -2493,11 +2139,11 @@ void mixed_adj_pairs(sphdem_ctx *c, int *nb, int2 *oc, int *cnt, int64_t cap, co
 
 namespace mixed {
 
-void pack(sphdem_ctx *c, bool coupling) {
-    coupling = coupling && c->cfg.liq_dem();
+void pack(sphdem_ctx *c, bool middle) {
+    const bool coupling = middle && c->cfg.liq_dem();
 #define L_(ND)                                                                                                  \
     SPHDEM_LAUNCH(c, "pack32", k_pack<ND>, grid_for(c->n, 256), 256, 0, c->cfg, c->A, c->buf.skey, c->g,         \
-                  c->mx_pos, c->mx_vel, c->mx_aux, c->mx_tg, c->mx_rc4, (int)coupling, c->mx_ds,      \
+                  c->mx_pos, c->mx_vel, c->mx_aux, c->mx_tg, c->mx_rc4, (int)coupling, (int)middle, c->mx_ds,      \
                   c->mx_nb, c->n)
     SPHDEM_ND_DISPATCH(c->cfg.nd, L_);
 #undef L_
@@ -2572,42 +2218,25 @@ void omega_eos(sphdem_ctx *c, bool omega, bool eos) {
 }
 
 void force(sphdem_ctx *c) {
-    const int phys = phys_class(c->cfg);
+    if (force_lists(c)) return;
     const double *cgrows = corrected_gradient(c) ? c->cg : nullptr;
     /* neighbour records staged through shared memory (2D and 3D) */
     const bool tile = c->cfg.nd > 1 && c->force_tile;
     const size_t st_bytes = tile ? (size_t)3 * ST_CAP * sizeof(float4) : 0;
-#define LP_(ND, P)                                                                                              \
-    do {                                                                                                        \
-        if (tile) {                                                                                             \
-            SPHDEM_LAUNCH(c, "force32", (k_force<ND, P, true>), grid_for(c->n, c->blk_pair), c->blk_pair,      \
-                          st_bytes, c->cfg, c->dcfg, c->A, c->g, c->mx_pos, c->mx_vel, c->mx_aux, c->mx_om,     \
-                          c->mx_tg, c->mx_nbr, c->mx_ncnt, (int64_t)c->mx_maxn, c->n, c->mx_nb, cgrows,        \
-                          c->buf.start, c->buf.skey);                                                          \
-        } else {                                                                                                \
-            SPHDEM_LAUNCH(c, "force32", (k_force<ND, P, false>), grid_for(c->n, c->blk_pair), c->blk_pair, 0,  \
-                          c->cfg, c->dcfg, c->A, c->g, c->mx_pos, c->mx_vel, c->mx_aux, c->mx_om, c->mx_tg,     \
-                          c->mx_nbr, c->mx_ncnt, (int64_t)c->mx_maxn, c->n, c->mx_nb, cgrows, c->buf.start,    \
-                          c->buf.skey);                                                                        \
-        }                                                                                                       \
-    } while (0)
-#define L_(ND)                                                                                                  \
-    do {                                                                                                        \
-        if (cgrows) {                                                                                           \
-            LP_(ND, PHYS_CG);                                                                                   \
-            break;                                                                                              \
-        }                                                                                                       \
-        if constexpr (ND > 1) {                                                                                 \
-            if (phys == PHYS_MORRIS_VARH) {                                                                     \
-                LP_(ND, PHYS_MORRIS_VARH);                                                                      \
-                break;                                                                                          \
-            }                                                                                                   \
-            if (phys == PHYS_ARTIFICIAL) {                                                                      \
-                LP_(ND, PHYS_ARTIFICIAL);                                                                       \
-                break;                                                                                          \
-            }                                                                                                   \
-        }                                                                                                       \
-        LP_(ND, PHYS_GENERIC);                                                                                  \
+#define LP_(ND, P, T)                                                                                           \
+    SPHDEM_LAUNCH(c, "force32", (k_force<ND, P, T>), grid_for(c->n, c->blk_pair), c->blk_pair, st_bytes, c->cfg, \
+                  c->dcfg, c->A, c->g, c->mx_pos, c->mx_vel, c->mx_aux, c->mx_om, c->mx_tg, c->mx_nbr,         \
+                  c->mx_ncnt, (int64_t)c->mx_maxn, c->n, c->mx_nb, cgrows, c->buf.start, c->buf.skey)
+#define L_(ND)                              \
+    do {                                    \
+        if (cgrows && tile)                 \
+            LP_(ND, PHYS_CG, true);         \
+        else if (cgrows)                    \
+            LP_(ND, PHYS_CG, false);        \
+        else if (tile)                      \
+            LP_(ND, PHYS_GENERIC, true);    \
+        else                                \
+            LP_(ND, PHYS_GENERIC, false);   \
     } while (0)
     SPHDEM_ND_DISPATCH(c->cfg.nd, L_);
 #undef L_
@@ -2623,54 +2252,46 @@ void prepare(sphdem_ctx *) {
 #define A_(ND, P) \
     SPHDEM_CUDA_CHECK(cudaFuncSetAttribute(k_force<ND, P, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes))
     A_(2, PHYS_GENERIC);
-    A_(2, PHYS_MORRIS_VARH);
-    A_(2, PHYS_ARTIFICIAL);
     A_(2, PHYS_CG);
     A_(3, PHYS_GENERIC);
-    A_(3, PHYS_MORRIS_VARH);
-    A_(3, PHYS_ARTIFICIAL);
     A_(3, PHYS_CG);
 #undef A_
     const int bytes2 = (int)(2 * ST_CAP * sizeof(float4));
-#define D_(ND, CGF, VH) \
-    SPHDEM_CUDA_CHECK(cudaFuncSetAttribute(k_dddt<ND, CGF, VH, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes2))
-    D_(2, true, -1);
-    D_(2, false, 1);
-    D_(2, false, 0);
-    D_(3, true, -1);
-    D_(3, false, 1);
-    D_(3, false, 0);
+#define D_(ND) \
+    SPHDEM_CUDA_CHECK(cudaFuncSetAttribute(k_dddt<ND, true, -1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes2))
+    D_(2);
+    D_(3);
 #undef D_
+    prepare_lists();
     done = true;
 }
 
 void dddt(sphdem_ctx *c) {
+    if (dddt_lists(c)) return;
+    /* CORRECTED_GRADIENT, or 1D */
     const double *cgrows = corrected_gradient(c) ? c->cg : nullptr;
-    const bool vh = c->cfg.var_h();
     const bool tile = c->cfg.nd > 1 && c->force_tile;
-    const size_t st_bytes = (size_t)2 * ST_CAP * sizeof(float4);
-#define LD_(ND, CGF, VH)                                                                                        \
-    do {                                                                                                        \
-        if (tile)                                                                                               \
-            SPHDEM_LAUNCH(c, "dddt32", (k_dddt<ND, CGF, VH, true>), grid_for(c->n, c->blk_pair), c->blk_pair,  \
-                          st_bytes, c->cfg, c->A, c->g, c->mx_pos, c->mx_vel, c->mx_aux, c->mx_om, c->mx_tg,    \
-                          c->mx_nbr, c->mx_ncnt, (int64_t)c->mx_maxn, c->n, cgrows, c->buf.start, c->buf.skey); \
-        else                                                                                                    \
-            SPHDEM_LAUNCH(c, "dddt32", (k_dddt<ND, CGF, VH, false>), grid_for(c->n, c->blk_pair), c->blk_pair, \
-                          0, c->cfg, c->A, c->g, c->mx_pos, c->mx_vel, c->mx_aux, c->mx_om, c->mx_tg,           \
-                          c->mx_nbr, c->mx_ncnt, (int64_t)c->mx_maxn, c->n, cgrows, c->buf.start, c->buf.skey); \
-    } while (0)
-#define L_(ND)                       \
-    do {                             \
-        if (cgrows)                  \
-            LD_(ND, true, -1);       \
-        else if (vh)                 \
-            LD_(ND, false, 1);       \
-        else                         \
-            LD_(ND, false, 0);       \
-    } while (0)
-    SPHDEM_ND_DISPATCH(c->cfg.nd, L_);
-#undef L_
+    const size_t st_bytes = tile ? (size_t)2 * ST_CAP * sizeof(float4) : 0;
+#define LD_(ND, CGF, T)                                                                                         \
+    SPHDEM_LAUNCH(c, "dddt32", (k_dddt<ND, CGF, -1, T>), grid_for(c->n, c->blk_pair), c->blk_pair, st_bytes,   \
+                  c->cfg, c->A, c->g, c->mx_pos, c->mx_vel, c->mx_aux, c->mx_om, c->mx_tg, c->mx_nbr,          \
+                  c->mx_ncnt, (int64_t)c->mx_maxn, c->n, cgrows, c->buf.start, c->buf.skey)
+    if (c->cfg.nd == 1) {
+        if (cgrows)
+            LD_(1, true, false);
+        else
+            LD_(1, false, false);
+    } else if (c->cfg.nd == 2) {
+        if (tile)
+            LD_(2, true, true);
+        else
+            LD_(2, true, false);
+    } else {
+        if (tile)
+            LD_(3, true, true);
+        else
+            LD_(3, true, false);
+    }
 #undef LD_
 }
 

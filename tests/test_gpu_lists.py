@@ -52,3 +52,44 @@ def test_lists_equal_the_fp64_bucket_scan(lib, nd, n, tie):
         sim.close()
     assert n < 30 or sets[0].size > 0
     assert np.array_equal(sets[0], sets[1])
+
+
+def list_pass_case(kind, n):
+    """Moving, slightly disordered fluid with walls; `n` sets the lanes per particle."""
+    rng = np.random.default_rng(3)
+    if kind == "artificial":
+        case = cases.dambreak2d(dx=float(np.sqrt(2.0 / n)))
+    else:
+        nx = int(round((n / 2.0) ** (1.0 / 3.0)))
+        case = cases.sediment3d(nx=nx, L=0.0025 * nx, height=0.005 * nx, n_dem=20, viscosity=1e-4,
+                                var_h=kind == "morris_varh")
+    p, nd, dx = case.particles, case.cfg["ndim"], case.cfg["psep"]
+    fluid = p["iam"] == cases.SPH
+    p["r"][fluid, :nd] += rng.uniform(-0.05 * dx, 0.05 * dx, (int(fluid.sum()), nd))
+    p["v"][fluid, :nd] += 0.05 * rng.standard_normal((int(fluid.sum()), nd))
+    for d in range(nd):
+        if case.cfg["periodic"][d]:
+            p["r"][fluid, d] %= case.cfg["rmax"][d]
+    p["dens"][fluid] *= 1.0 + 1e-3 * rng.standard_normal(int(fluid.sum()))
+    return case, fluid
+
+
+@pytest.mark.parametrize("kind", ["artificial", "morris", "morris_varh"])
+@pytest.mark.parametrize("n", [1800, 7000, 16000, 132000])
+def test_list_passes_equal_fp64(lib, kind, n):
+    """Force and continuity passes, one to eight lanes per particle: pressure,
+    viscous and wall forces, density rate and Omega against the FP64 path.
+    Tolerance: FP32 terms good to ~20 roundings (1.2e-6) of which a sum
+    cancels at most nine tenths (2-norm over the fluid)."""
+    case, fluid = list_pass_case(kind, n)
+    got = []
+    for prec in (cases.PREC_FP64, cases.PREC_MIXED):
+        sim = capi.Simulation(lib, case.cfg, case.particles, precision=prec)
+        sim.step(1)
+        a = sim.get()
+        got.append({k: a[k][fluid].copy() for k in ("f", "fp", "fv", "fb", "dddt", "omega")})
+        sim.close()
+    for k, x in got[0].items():
+        norm = np.linalg.norm(x)
+        if norm > 0:
+            assert np.linalg.norm(got[1][k] - x) <= 1.2e-5 * norm, k
