@@ -284,11 +284,46 @@ void free_ctx(sphdem_ctx *c) {
     fields_async_free(c);
     cudaFree(c->cg);
     cudaFree(c->hpred);
+    cudaFree(c->reinit_wide);
     cudaFree(c->delmark);
     for (int k = 0; k < 4; k++)
         if (c->graph[k]) cudaGraphExecDestroy(c->graph[k]);
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c;
+}
+
+/* list depth for the largest neighbour count at creation: headroom for
+ * compression, a multiple of 32 */
+int list_depth(int count) { return (std::max(32, (int)(1.6 * count) + 16) + 31) / 32 * 32; }
+
+/* Neighbour lists of an FP64 handle with fluid.  They only spare the FP64
+ * passes the search: without them (no memory to spare, lengths outside FP32's
+ * range, more particles than an entry can name) every particle scans its
+ * buckets. */
+void alloc_lists64(sphdem_ctx *c, double hmax) {
+    bool fluid = false;
+    std::vector<int> iam(c->n);
+    SPHDEM_CUDA_CHECK(cudaMemcpy(iam.data(), c->A.irow(FI_IAM), c->n * sizeof(int), cudaMemcpyDeviceToHost));
+    for (int t : iam) fluid = fluid || is_sph_or_sphb(t);
+    const double hs = std::min(c->host_cfg.h, hmax), hl = std::max(c->host_cfg.h, hmax);
+    if (!fluid || c->cap > (int64_t)1 << 26 || !(hs > 1e-12) || !(hl < 1e12)) return;
+    const int64_t cap = c->cap;
+    auto get = [](auto **p, size_t bytes) {
+        size_t room = 0, total = 0;
+        if (cudaMemGetInfo(&room, &total) != cudaSuccess || bytes > room / 4) return false;
+        if (cudaMalloc(p, bytes) == cudaSuccess) return true;
+        *p = nullptr;
+        cudaGetLastError();
+        return false;
+    };
+    if (!get(&c->mx_pos, cap * sizeof(float4)) || !get(&c->mx_tg, cap * sizeof(int)) ||
+        !get(&c->mx_ncnt, cap * sizeof(int)) || !get(&c->mx_bandn, cap * sizeof(int)))
+        return;
+    pack_positions(c);
+    const int m = mixed::nlist_max_count(c);
+    if (m <= 0) return;
+    const int depth = list_depth(m);
+    if (get(&c->mx_nbr, (size_t)depth * ((cap + 31) / 32 * 32) * sizeof(int))) c->f64_maxn = depth;
 }
 
 void run_phase_mixed(sphdem_ctx *c, int phase) {
@@ -299,7 +334,7 @@ void run_phase_mixed(sphdem_ctx *c, int phase) {
             globals_op(c, OP_MIDDLE_BEGIN);
             rebuild(c);
             mixed::pack(c);
-            if (lists) mixed::nlist(c);
+            if (lists) mixed::nlist(c, c->mx_maxn);
             /* calcInvM in FP64 once per rebuild; the pair passes apply it in FP32 */
             if (corrected_gradient(c)) run_invm(c);
             if (liq) {
@@ -320,9 +355,9 @@ void run_phase_mixed(sphdem_ctx *c, int phase) {
             run_end_drift(c);
             rebuild(c);
             mixed::pack(c, false);
+            if (lists) mixed::nlist(c, c->mx_maxn);
             if (corrected_gradient(c)) run_invm(c);
             if (lists) {
-                mixed::nlist(c);
                 mixed::dddt(c);  /* Omega (VAR_H_CORRECTION) is summed inside the continuity pass */
             }
             if (liq) mixed::dem_end(c);
@@ -356,13 +391,14 @@ void run_phase(sphdem_ctx *c, int phase) {
         case SPHDEM_PHASE_MIDDLE:
             globals_op(c, OP_MIDDLE_BEGIN);
             rebuild(c);
+            run_lists64(c);
             if (liq) {
                 run_porosity(c);
                 run_dem_drag(c);
             }
             if (corrected_gradient(c)) run_invm(c);
-            run_omega_eos(c, c->cfg.var_h(), true);
-            run_force(c);
+            run_eos(c);
+            run_force(c);  /* Omega (VAR_H_CORRECTION) is summed inside */
             if (liq) run_dem_accel(c);
             globals_op(c, OP_SET_DT);
             run_middle_tail(c);
@@ -373,9 +409,9 @@ void run_phase(sphdem_ctx *c, int phase) {
         case SPHDEM_PHASE_END:
             run_end_drift(c);
             rebuild(c);
+            run_lists64(c);
             if (corrected_gradient(c)) run_invm(c);
-            if (c->cfg.var_h()) run_omega_eos(c, true, false);
-            run_dddt(c);
+            run_dddt(c);   /* Omega (VAR_H_CORRECTION) is summed inside */
             if (liq) run_dem_end(c);
             if (c->host_cfg.flags & SPHDEM_F_DEM_BLOCK) run_dem_block(c);
             run_end_tail(c);
@@ -498,7 +534,10 @@ int sphdem_create(const SphDemConfig *cfg, const SphDemParticles *init, int64_t 
         setup_rebuild_buffers(c);
         if (cfg->flags & SPHDEM_F_CORRECTED_GRADIENT)
             SPHDEM_CUDA_CHECK(cudaMalloc(&c->cg, (size_t)CG_ROWS * capacity * sizeof(double)));
-        if (reinit_configured(*cfg)) SPHDEM_CUDA_CHECK(cudaMalloc(&c->hpred, capacity * sizeof(double)));
+        if (reinit_configured(*cfg)) {
+            SPHDEM_CUDA_CHECK(cudaMalloc(&c->hpred, capacity * sizeof(double)));
+            SPHDEM_CUDA_CHECK(cudaMalloc(&c->reinit_wide, sizeof(int)));
+        }
         SPHDEM_CUDA_CHECK(cudaMalloc(&c->delmark, capacity));
         SPHDEM_CUDA_CHECK(cudaMemset(c->delmark, 0, capacity));
 
@@ -563,16 +602,17 @@ int sphdem_create(const SphDemConfig *cfg, const SphDemParticles *init, int64_t 
             mixed::pack(c);
             const int m = mixed::nlist_max_count(c);
             if (m > 0) {
-                /* headroom for compression; a run that outgrows it stops with
-                 * SPHDEM_ERR_CAPACITY rather than dropping neighbours */
-                int maxn = std::max(32, (int)(1.6 * m) + 16);
-                maxn = (maxn + 31) / 32 * 32;
+                /* a run that outgrows the depth stops with SPHDEM_ERR_CAPACITY
+                 * rather than dropping neighbours */
+                const int maxn = list_depth(m);
                 c->mx_maxn = maxn;
                 /* list tiles of 32 particles x 8 entries */
                 SPHDEM_CUDA_CHECK(cudaMalloc(&c->mx_nbr, (size_t)maxn * ((capacity + 31) / 32 * 32) * sizeof(int)));
                 /* the lists of the creation's rebuild, for exports before any step */
-                mixed::nlist(c);
+                mixed::nlist(c, c->mx_maxn);
             }
+        } else {
+            alloc_lists64(c, hmax0);
         }
         int rc = check_device(c);
         if (rc != SPHDEM_OK) {
@@ -683,7 +723,7 @@ int sphdem_rebuild(sphdem_handle h) {
         rebuild(h);
         if (h->mx_maxn > 0) {
             mixed::pack(h);
-            mixed::nlist(h);
+            mixed::nlist(h, h->mx_maxn);
         }
     } catch (const std::string &e) {
         return fail(h, SPHDEM_ERR_CUDA, e);
@@ -747,7 +787,7 @@ int sphdem_get_stats(sphdem_handle h, SphDemStats *out) {
     out->n_dem_cells = h->cfg.n_dem_cells;
     out->h_max = hg.hmax;
     out->search_radius = hg.sr;
-    if (h->mx_bandn) {
+    if (h->mx_maxn > 0) {
         std::vector<int> nb(h->n);
         cudaMemcpy(nb.data(), h->mx_bandn, h->n * sizeof(int), cudaMemcpyDeviceToHost);
         for (int64_t k = 0; k < h->n; k++)

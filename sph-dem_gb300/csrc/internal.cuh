@@ -100,6 +100,8 @@ struct sphdem_ctx {
     int *mx_nbr = nullptr;      /* lists in tiles of 32 particles x 8 slots, mx_maxn x cap (rounded to 32) */
     int *mx_ncnt = nullptr;
     int mx_maxn = 0;
+    int f64_maxn = 0;           /* FP64 handle: depth of its neighbour lists (mx_nbr), 0 without */
+    int *reinit_wide = nullptr; /* density re-initialisation: some first-round h outgrew the buckets */
     bool mx_dem_only = false;   /* every particle at creation is DEM: the FP64 phases run */
     float4 *mx_q0 = nullptr, *mx_q1 = nullptr, *mx_q2 = nullptr;  /* FPI fields of fluid particles */
     float4 *mx_dp = nullptr;    /* (m/shep, fdrag) of DEM particles */
@@ -167,11 +169,13 @@ void run_hook_before_end(sphdem_ctx *c);
 void run_hook_after_end(sphdem_ctx *c);
 void run_h_derived(sphdem_ctx *c);
 
-/* pairs64.cu / pairs32.cu: pair passes */
+/* pairs64.cu, lists64.cu: FP64 pair passes */
 void run_porosity(sphdem_ctx *c);      /* calcPorosity + calcShepSum        */
 void run_dem_drag(sphdem_ctx *c);      /* calcDEMtoSPHDrag + finalisePorosity */
-void run_omega_eos(sphdem_ctx *c, bool omega, bool eos);
-void run_force(sphdem_ctx *c);         /* calcForce + accelCondition        */
+void run_eos(sphdem_ctx *c);
+void pack_positions(sphdem_ctx *c);    /* FP32 records of the list build    */
+void run_lists64(sphdem_ctx *c);       /* neighbour lists of an FP64 handle */
+void run_force(sphdem_ctx *c);         /* calcForce + calcOmega + accelCondition */
 void run_dem_accel(sphdem_ctx *c);
 void run_dddt(sphdem_ctx *c);          /* calcDddtDudt                      */
 void run_invm(sphdem_ctx *c);
@@ -188,7 +192,9 @@ namespace mixed {
  * the coupling windows its SPH-DEM passes need, or those of the end phase */
 void pack(sphdem_ctx *c, bool middle = true);
 void pack_fpi(sphdem_ctx *c);
-void nlist(sphdem_ctx *c);
+/* the neighbour lists of the last rebuild, `depth` entries per particle; more
+ * neighbours are an error, or (soft) leave the particle without a list */
+void nlist(sphdem_ctx *c, int depth, bool soft = false);
 /* once per process, outside stream capture: kernel attributes of the step */
 void prepare(sphdem_ctx *c);
 void zero_shep(sphdem_ctx *c);

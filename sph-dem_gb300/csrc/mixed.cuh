@@ -120,6 +120,20 @@ __device__ __forceinline__ void decode(int key, const int *dims, int *cc) {
 
 __device__ __forceinline__ int code_stride(int d) { return d == 0 ? 9 : (d == 1 ? 3 : 1); }
 
+__device__ __forceinline__ void nl_decode_code(int code, int *o) {
+    o[0] = code / 9 - 1;
+    o[1] = (code / 3) % 3 - 1;
+    o[2] = code % 3 - 1;
+}
+
+/* FP64 origin of SPH bucket `cell` on axis d, and its size */
+__device__ __forceinline__ double sph_origin(const DevCfg &c, const DevGlobals *g, int d, int cell) {
+    return c.periodic[d] ? c.dmin[d] + cell * g->scell[d] : c.dmin[d] + (cell - 3) * g->sr2;
+}
+__device__ __forceinline__ double sph_width(const DevCfg &c, const DevGlobals *g, int d) {
+    return c.periodic[d] ? g->scell[d] : g->sr2;
+}
+
 /* Neighbour lists: slot j of particle a, in tiles of 32 particles x 8
  * entries -- each particle's 8 entries contiguous, the 32 particles' groups
  * back to back -- so a warp of consecutive particles reads 8 entries each

@@ -43,13 +43,6 @@
 namespace sphdem {
 namespace {
 
-/* FP64 origin of SPH bucket `cell` on axis d, and its size */
-__device__ __forceinline__ double sph_origin(const DevCfg &c, const DevGlobals *g, int d, int cell) {
-    return c.periodic[d] ? c.dmin[d] + cell * g->scell[d] : c.dmin[d] + (cell - 3) * g->sr2;
-}
-__device__ __forceinline__ double sph_width(const DevCfg &c, const DevGlobals *g, int d) {
-    return c.periodic[d] ? g->scell[d] : g->sr2;
-}
 __device__ __forceinline__ double dem_origin(const DevCfg &c, int d, int cell) {
     return c.dorig[d] + cell * c.dcell[d];
 }
@@ -257,12 +250,6 @@ __global__ void k_pack_fpi(DevState s, float4 *__restrict__ Q0, float4 *__restri
  * r^2 by < 1.25e-6 L max(L, R) + 1.8e-7 r^2, and T by < 1.8e-7 T. */
 __device__ __forceinline__ float fp32_band(float T, float L2) { return fmaf(5e-7f, T, 1.5e-6f * fmaxf(L2, T)); }
 
-__device__ __forceinline__ void nl_decode_code(int code, int *o) {
-    o[0] = code / 9 - 1;
-    o[1] = (code / 3) % 3 - 1;
-    o[2] = code % 3 - 1;
-}
-
 /* ---------------------------------------------------------------------- */
 /* Neighbour-list build.
  *
@@ -410,7 +397,8 @@ __global__ void __launch_bounds__(NL_WARPS * 32, 5) k_nlist(DevCfg c, const DevC
                                                          const int *__restrict__ start, const int *__restrict__ skey,
                                                          DevGlobals *__restrict__ g, const float4 *__restrict__ P0,
                                                          const int *__restrict__ tg, int *__restrict__ nbr,
-                                                         int *__restrict__ ncnt, int maxn, int *__restrict__ bandn) {
+                                                         int *__restrict__ ncnt, int maxn, int soft,
+                                                         int *__restrict__ bandn) {
     constexpr int Z = ND - 1;
     constexpr unsigned FULL = 0xffffffffu;
     /* staged candidates: negated position in the run's frame, cut-off, list
@@ -791,9 +779,10 @@ __global__ void __launch_bounds__(NL_WARPS * 32, 5) k_nlist(DevCfg c, const DevC
                 tiles[cnt * 8 + 1] = make_int4(v[4], v[5], v[6], v[7]);
             }
             cnt += qn;
-            /* stored counts never exceed the list depth; an overflow is an error */
-            ncnt[a] = min(cnt, maxn);
-            if (cnt > maxn) set_err(g, SPHDEM_ERR_CAPACITY, cnt);
+            /* stored counts never exceed the list depth; an overflow is an error, or
+             * (soft) marked for the reader, which then scans the buckets */
+            ncnt[a] = cnt <= maxn ? cnt : (soft ? -1 : maxn);
+            if (cnt > maxn && !soft) set_err(g, SPHDEM_ERR_CAPACITY, cnt);
         }
         if (a < n_t) bandn[a] = nb;
     }
@@ -2164,7 +2153,7 @@ void pack_fpi(sphdem_ctx *c) {
     SPHDEM_LAUNCH(c, "pack_fpi32", k_pack_fpi, grid_for(c->n, 256), 256, 0, c->A, c->mx_q0, c->mx_q1, c->mx_q2, c->n);
 }
 
-void nlist(sphdem_ctx *c) {
+void nlist(sphdem_ctx *c, int depth, bool soft) {
     /* below these counts the warps of 32 particles do not fill the chip and the
      * pass is the length of one warp's chain.  Two builds, one / four lanes per
      * particle: 2D 6.5k 38 / 26 us, 23k 45 / 30, 44k 46 / 38, 86k 50 / 56; 3D
@@ -2173,8 +2162,8 @@ void nlist(sphdem_ctx *c) {
 #define LG_(ND, G)                                                                                              \
     SPHDEM_LAUNCH(c, "nlist32", (k_nlist<ND, false, G>),                                                       \
                   (std::max(1, nlist_blocks<ND, false, G>(c->n) / c->grid_div)), NL_WARPS * 32, 0, c->cfg, c->dcfg, \
-                  c->A, c->buf.start, c->buf.skey, c->g, c->mx_pos, c->mx_tg, c->mx_nbr, c->mx_ncnt, c->mx_maxn, \
-                  c->mx_bandn)
+                  c->A, c->buf.start, c->buf.skey, c->g, c->mx_pos, c->mx_tg, c->mx_nbr, c->mx_ncnt, depth,      \
+                  (int)soft, c->mx_bandn)
 #define L_(ND)            \
     do {                  \
         if (split)        \
@@ -2195,7 +2184,7 @@ int nlist_max_count(sphdem_ctx *c) {
 #define L_(ND)                                                                                                    \
     k_nlist<ND, true, 1><<<nlist_blocks<ND, true, 1>(c->n), NL_WARPS * 32, 0, c->stream>>>(                           \
         c->cfg, c->dcfg, c->A, c->buf.start, c->buf.skey, c->g, c->mx_pos, c->mx_tg, c->mx_nbr,      \
-        c->mx_ncnt, 0, nullptr)
+        c->mx_ncnt, 0, 0, nullptr)
     SPHDEM_ND_DISPATCH(c->cfg.nd, L_);
 #undef L_
     SPHDEM_CUDA_CHECK(cudaGetLastError());

@@ -93,3 +93,36 @@ def test_list_passes_equal_fp64(lib, kind, n):
         norm = np.linalg.norm(x)
         if norm > 0:
             assert np.linalg.norm(got[1][k] - x) <= 1.2e-5 * norm, k
+
+
+@pytest.mark.parametrize("kind,n", [("artificial", 1800), ("options", 1800)])
+def test_fp64_particles_beyond_the_list_depth(lib, kind, n):
+    """An FP64 handle squeezed beyond the depth its lists were given at
+    creation scans the buckets instead: the step equals that of a handle
+    created at the squeezed positions (whose lists are deep enough), up to
+    the order of the FP64 sums (1e-12 of each field's 2-norm)."""
+    if kind == "options":
+        case = cases.dambreak2d(dx=0.05, visc_model=cases.VISC_MONAGHAN, anticlumping=True, const_h=False, var_h=True,
+                                viscosity=1e-2, reinit_every=1, fixed_dt=False)
+        fluid = case.particles["iam"] == cases.SPH
+    else:
+        case, fluid = list_pass_case(kind, n)
+    nd = case.cfg["ndim"]
+    r = case.particles["r"].copy()
+    mid = r[fluid].mean(axis=0)
+    r[fluid, nd - 1] = mid[nd - 1] + 0.3 * (r[fluid, nd - 1] - mid[nd - 1])
+    r[fluid, 0] = mid[0] + 0.5 * (r[fluid, 0] - mid[0])
+    got = []
+    for squeezed in (False, True):
+        p = dict(case.particles, r=r) if squeezed else case.particles
+        sim = capi.Simulation(lib, case.cfg, p, precision=cases.PREC_FP64)
+        buf = capi.ParticleBuffers(case.n, {"r": r}, fields=("r",))
+        sim.set(buf, capi.FIELD_R)
+        sim.rebuild()
+        sim.rebuild()   # the ghost widths of both handles follow the same h
+        sim.step(1)
+        a = sim.get()
+        got.append({k: a[k][fluid].copy() for k in ("f", "fp", "dddt", "dens")})
+        sim.close()
+    for k in got[0]:
+        assert np.linalg.norm(got[0][k] - got[1][k]) <= 1e-12 * np.linalg.norm(got[1][k]), k
