@@ -249,6 +249,14 @@ std::string validate(const SphDemConfig *cfg, const SphDemParticles *p, int64_t 
     return "";
 }
 
+void drop_kept_pairs(sphdem_ctx *c) {
+    cudaFree(c->cp_id);
+    cudaFree(c->cp_w);
+    cudaFree(c->cp_num);
+    c->cp_id = c->cp_num = nullptr;
+    c->cp_w = nullptr;
+}
+
 void free_ctx(sphdem_ctx *c) {
     if (!c) return;
     adjoint_free(c);
@@ -272,13 +280,10 @@ void free_ctx(sphdem_ctx *c) {
     cudaFree(c->stage);
     cudaFree(c->mx_q0);
     cudaFree(c->mx_q1);
-    cudaFree(c->mx_q2);
     cudaFree(c->mx_dp);
-    cudaFree(c->mx_rc4);
-    cudaFree(c->mx_shep32);
     cudaFree(c->mx_ds);
+    drop_kept_pairs(c);
     cudaFree(c->mx_nb);
-    cudaFree(c->mx_win);
     cudaFree(c->mx_bandn);
     cudaFree(c->dcfg);
     fields_async_free(c);
@@ -296,30 +301,35 @@ void free_ctx(sphdem_ctx *c) {
  * compression, a multiple of 32 */
 int list_depth(int count) { return (std::max(32, (int)(1.6 * count) + 16) + 31) / 32 * 32; }
 
-/* Neighbour lists of an FP64 handle with fluid.  They only spare the FP64
- * passes the search: without them (no memory to spare, lengths outside FP32's
- * range, more particles than an entry can name) every particle scans its
- * buckets. */
-void alloc_lists64(sphdem_ctx *c, double hmax) {
-    bool fluid = false;
-    std::vector<int> iam(c->n);
-    SPHDEM_CUDA_CHECK(cudaMemcpy(iam.data(), c->A.irow(FI_IAM), c->n * sizeof(int), cudaMemcpyDeviceToHost));
-    for (int t : iam) fluid = fluid || is_sph_or_sphb(t);
-    const double hs = std::min(c->host_cfg.h, hmax), hl = std::max(c->host_cfg.h, hmax);
-    if (!fluid || c->cap > (int64_t)1 << 26 || !(hs > 1e-12) || !(hl < 1e12)) return;
+/* Neighbour lists of an FP64 handle with fluid, and the FP32 records its
+ * searches read.  They only spare the FP64 passes work: without them (no memory
+ * to spare, lengths outside FP32's range, more particles than an entry can name)
+ * every particle scans its buckets in FP64. */
+void alloc_lists64(sphdem_ctx *c, double hmax, bool fluid) {
+    const bool liq = c->cfg.liq_dem();
+    double hs = std::min(c->host_cfg.h, hmax), hl = std::max(c->host_cfg.h, hmax);
+    if (liq) {
+        hs = std::min({hs, c->cfg.rc, c->cfg.dem_sr});
+        hl = std::max({hl, c->cfg.rc, c->cfg.dem_sr});
+    }
+    if (c->cap > (int64_t)1 << 26 || !(hs > 1e-12) || !(hl < 1e12)) return;
     const int64_t cap = c->cap;
     auto get = [](auto **p, size_t bytes) {
         size_t room = 0, total = 0;
+        if (*p) return true;
         if (cudaMemGetInfo(&room, &total) != cudaSuccess || bytes > room / 4) return false;
         if (cudaMalloc(p, bytes) == cudaSuccess) return true;
         *p = nullptr;
         cudaGetLastError();
         return false;
     };
-    if (!get(&c->mx_pos, cap * sizeof(float4)) || !get(&c->mx_tg, cap * sizeof(int)) ||
-        !get(&c->mx_ncnt, cap * sizeof(int)) || !get(&c->mx_bandn, cap * sizeof(int)))
-        return;
-    pack_positions(c);
+    if (!get(&c->mx_pos, cap * sizeof(float4)) || !get(&c->mx_tg, cap * sizeof(int))) return;
+    if (liq && get(&c->mx_ds, cap * sizeof(float4))) c->f64_dem = true;
+    if (c->f64_dem && fluid && !(get(&c->cp_id, kept_entries(cap) * sizeof(int)) && get(&c->cp_w, kept_entries(cap) * sizeof(double)) &&
+                                 get(&c->cp_num, 4 * cap * sizeof(int))))
+        drop_kept_pairs(c);
+    if (!fluid || !get(&c->mx_ncnt, cap * sizeof(int)) || !get(&c->mx_bandn, cap * sizeof(int))) return;
+    pack_positions(c, false);
     const int m = mixed::nlist_max_count(c);
     if (m <= 0) return;
     const int depth = list_depth(m);
@@ -338,7 +348,6 @@ void run_phase_mixed(sphdem_ctx *c, int phase) {
             /* calcInvM in FP64 once per rebuild; the pair passes apply it in FP32 */
             if (corrected_gradient(c)) run_invm(c);
             if (liq) {
-                mixed::zero_shep(c);
                 mixed::porosity(c);
                 mixed::dem_drag(c);
             }
@@ -391,14 +400,16 @@ void run_phase(sphdem_ctx *c, int phase) {
         case SPHDEM_PHASE_MIDDLE:
             globals_op(c, OP_MIDDLE_BEGIN);
             rebuild(c);
-            run_lists64(c);
+            run_lists64(c, true);
             if (liq) {
                 run_porosity(c);
                 run_dem_drag(c);
             }
-            if (corrected_gradient(c)) run_invm(c);
-            run_eos(c);
-            run_force(c);  /* Omega (VAR_H_CORRECTION) is summed inside */
+            if (!c->only_dem) {
+                if (corrected_gradient(c)) run_invm(c);
+                run_eos(c);
+                run_force(c);  /* Omega (VAR_H_CORRECTION) is summed inside */
+            }
             if (liq) run_dem_accel(c);
             globals_op(c, OP_SET_DT);
             run_middle_tail(c);
@@ -409,9 +420,11 @@ void run_phase(sphdem_ctx *c, int phase) {
         case SPHDEM_PHASE_END:
             run_end_drift(c);
             rebuild(c);
-            run_lists64(c);
-            if (corrected_gradient(c)) run_invm(c);
-            run_dddt(c);   /* Omega (VAR_H_CORRECTION) is summed inside */
+            run_lists64(c, false);
+            if (!c->only_dem) {
+                if (corrected_gradient(c)) run_invm(c);
+                run_dddt(c);   /* Omega (VAR_H_CORRECTION) is summed inside */
+            }
             if (liq) run_dem_end(c);
             if (c->host_cfg.flags & SPHDEM_F_DEM_BLOCK) run_dem_block(c);
             run_end_tail(c);
@@ -514,11 +527,9 @@ int sphdem_create(const SphDemConfig *cfg, const SphDemParticles *init, int64_t 
         for (int64_t i = 0; i < n; i++) hmax0 = std::max(hmax0, init->h[i]);
         const double sr_min = 0.5 * std::min(cfg->h, hmax0);
         long long sc = 1;
-        int win_cap = 1; /* bucket indices along any one axis */
         for (int d = 0; d < cfg->ndim; d++) {
             const long long nd = (long long)((cfg->domain_max[d] - cfg->domain_min[d]) / (2.0 * sr_min)) + 9;
             sc *= nd;
-            win_cap = (int)std::max<long long>(win_cap, std::min<long long>(nd, 1ll << 30));
         }
         if (sc > (1ll << 30)) throw std::string("bucket grid too large for the domain / smoothing length");
         c->cfg.sph_cells_cap = (int)sc;
@@ -576,15 +587,15 @@ int sphdem_create(const SphDemConfig *cfg, const SphDemParticles *init, int64_t 
             SPHDEM_CUDA_CHECK(cudaMalloc(&c->mx_om, capacity * sizeof(float)));
             SPHDEM_CUDA_CHECK(cudaMalloc(&c->mx_ncnt, capacity * sizeof(int)));
             SPHDEM_CUDA_CHECK(cudaMalloc(&c->mx_q0, capacity * sizeof(float4)));
-            SPHDEM_CUDA_CHECK(cudaMalloc(&c->mx_q1, capacity * sizeof(float4)));
-            SPHDEM_CUDA_CHECK(cudaMalloc(&c->mx_q2, capacity * sizeof(float4)));
+            SPHDEM_CUDA_CHECK(cudaMalloc(&c->mx_q1, capacity * sizeof(float2)));
             SPHDEM_CUDA_CHECK(cudaMalloc(&c->mx_dp, capacity * sizeof(float4)));
-            SPHDEM_CUDA_CHECK(cudaMalloc(&c->mx_rc4, capacity * sizeof(int4)));
-            SPHDEM_CUDA_CHECK(cudaMalloc(&c->mx_shep32, capacity * sizeof(float)));
             SPHDEM_CUDA_CHECK(cudaMalloc(&c->mx_ds, capacity * sizeof(float4)));
             SPHDEM_CUDA_CHECK(cudaMalloc(&c->mx_nb, 3 * capacity * sizeof(float4)));
-            c->mx_win_cap = win_cap;
-            SPHDEM_CUDA_CHECK(cudaMalloc(&c->mx_win, 3 * (size_t)win_cap * sizeof(int4)));
+            if (c->cfg.liq_dem()) {
+                SPHDEM_CUDA_CHECK(cudaMalloc(&c->cp_id, kept_entries(capacity) * sizeof(int)));
+                SPHDEM_CUDA_CHECK(cudaMalloc(&c->cp_w, kept_entries(capacity) * sizeof(float)));
+                SPHDEM_CUDA_CHECK(cudaMalloc(&c->cp_num, 4 * capacity * sizeof(int)));
+            }
             SPHDEM_CUDA_CHECK(cudaMalloc(&c->mx_bandn, capacity * sizeof(int)));
             SPHDEM_CUDA_CHECK(cudaMemset(c->mx_bandn, 0, capacity * sizeof(int)));
             SPHDEM_CUDA_CHECK(cudaMemset(c->mx_om, 0, capacity * sizeof(float)));
@@ -611,9 +622,15 @@ int sphdem_create(const SphDemConfig *cfg, const SphDemParticles *init, int64_t 
                 /* the lists of the creation's rebuild, for exports before any step */
                 mixed::nlist(c, c->mx_maxn);
             }
-        } else {
-            alloc_lists64(c, hmax0);
         }
+        bool fluid = false;
+        c->only_dem = c->cfg.liq_dem();
+        for (int64_t i = 0; i < n; i++) {
+            fluid = fluid || is_sph_or_sphb(init->iam[i]);
+            c->only_dem = c->only_dem && init->iam[i] == T_DEM;
+        }
+        /* a mixed handle whose particles are all DEM runs the FP64 phases */
+        if (cfg->precision != SPHDEM_PREC_MIXED || c->mx_dem_only) alloc_lists64(c, hmax0, fluid);
         int rc = check_device(c);
         if (rc != SPHDEM_OK) {
             g_create_err = c->err;

@@ -56,5 +56,50 @@ __device__ __forceinline__ void block_min_atomic(double v, unsigned long long *t
     }
 }
 
+/* 1/x for x > 0: an FP32 estimate y (relative error d ~ 1e-7) and one step of
+ * the series 1/x = y (1 + e + e^2 + ..), e = 1 - x y, which leaves d^3 */
+__device__ __forceinline__ double rcp_pos(double x) {
+    const float xf = (float)x;
+    if (!(xf > 1e-30f && xf < 1e30f)) return 1.0 / x;
+    float yf;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(yf) : "f"(xf));
+    const double y = (double)yf, e = fma(-x, y, 1.0);
+    return fma(y, fma(e, e, e), y);
+}
+
+/* sqrt(x) and, where asked, 1/sqrt(x) of x >= 0: an FP32 estimate y of 1/sqrt
+ * and one step of the series 1/sqrt(1 - e) = 1 + e/2 + 3 e^2/8 + .., e = 1 - x y^2 */
+__device__ __forceinline__ double sqrt_pos(double x, double *inv = nullptr) {
+    const float xf = (float)x;
+    if (!(xf > 1e-30f && xf < 1e30f)) {
+        const double r = sqrt(x);
+        if (inv) *inv = r > 0.0 ? 1.0 / r : 0.0;
+        return r;
+    }
+    float yf;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(yf) : "f"(xf));
+    const double y = (double)yf, s = x * y;
+    const double e = fma(-s, y, 1.0), k = e * fma(e, 0.375, 0.5);
+    if (inv) *inv = fma(y, k, y);
+    return fma(s, k, s);
+}
+
+/* max(x, 0) by the sign bit (an integer operation) */
+__device__ __forceinline__ double positive_part(double x) {
+    return __double_as_longlong(x) < 0 ? 0.0 : x;
+}
+
+/* the smaller of two non-negative doubles by their bit patterns */
+__device__ __forceinline__ double min_pos(double a, double b) {
+    return __double_as_longlong(a) < __double_as_longlong(b) ? a : b;
+}
+
+template <int G>
+__device__ __forceinline__ double lane_sum(double v) {
+#pragma unroll
+    for (int o = 1; o < G; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
 }  // namespace
 }  // namespace sphdem

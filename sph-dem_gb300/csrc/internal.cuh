@@ -100,15 +100,18 @@ struct sphdem_ctx {
     int *mx_nbr = nullptr;      /* lists in tiles of 32 particles x 8 slots, mx_maxn x cap (rounded to 32) */
     int *mx_ncnt = nullptr;
     int mx_maxn = 0;
+    /* coupling pairs of the porosity pass, kept for the drag pass: entry (DEM slot |
+     * image code), kernel value (the handle's precision), pairs per thread */
+    int *cp_id = nullptr, *cp_num = nullptr;
+    void *cp_w = nullptr;
+    bool f64_dem = false;       /* FP64 phases with DEM: the FP32 records of their searches exist */
+    bool only_dem = false;      /* every particle is DEM */
     int f64_maxn = 0;           /* FP64 handle: depth of its neighbour lists (mx_nbr), 0 without */
     int *reinit_wide = nullptr; /* density re-initialisation: some first-round h outgrew the buckets */
     bool mx_dem_only = false;   /* every particle at creation is DEM: the FP64 phases run */
-    float4 *mx_q0 = nullptr, *mx_q1 = nullptr, *mx_q2 = nullptr;  /* FPI fields of fluid particles */
+    float4 *mx_q0 = nullptr;    /* FPI fields of fluid particles */
+    float2 *mx_q1 = nullptr;
     float4 *mx_dp = nullptr;    /* (m/shep, fdrag) of DEM particles */
-    int4 *mx_rc4 = nullptr;     /* packed reference DEM buckets (own, image -L, image +L) */
-    int4 *mx_win = nullptr;     /* coupling windows per SPH bucket index and axis */
-    int mx_win_cap = 0;         /* entries per axis */
-    float *mx_shep32 = nullptr; /* FP32 Shepard sums of DEM particles */
     float4 *mx_ds = nullptr;    /* DEM particles: offset in their SPH bucket, bucket key */
     float4 *mx_nb = nullptr;    /* boundary particles: FP32 normals n1 (+concave), n2, n3 */
     sphdem::AdjointData *adj = nullptr; /* checkpoints and buffers of the adjoint */
@@ -137,6 +140,16 @@ struct sphdem_ctx {
 };
 
 namespace sphdem {
+
+/* coupling passes: populations below this take four threads per fluid particle;
+ * pairs a thread keeps (a partner's bucket column gives one thread of four most
+ * of a particle's pairs at times); entries and threads to allocate for */
+constexpr int64_t CP_SPLIT_BELOW = 60000;
+__host__ __device__ constexpr int kept_pairs(int threads_per_particle) { return threads_per_particle > 1 ? 16 : 32; }
+inline int64_t kept_entries(int64_t cap) {
+    const int64_t split = (cap < CP_SPLIT_BELOW ? cap : CP_SPLIT_BELOW) * 4 * kept_pairs(4);
+    return cap * kept_pairs(1) > split ? cap * kept_pairs(1) : split;
+}
 
 /* CORRECTED_GRADIENT rows per particle: invM (nd x nd, row-major),
  * sumGrad/sum, sum */
@@ -173,8 +186,9 @@ void run_h_derived(sphdem_ctx *c);
 void run_porosity(sphdem_ctx *c);      /* calcPorosity + calcShepSum        */
 void run_dem_drag(sphdem_ctx *c);      /* calcDEMtoSPHDrag + finalisePorosity */
 void run_eos(sphdem_ctx *c);
-void pack_positions(sphdem_ctx *c);    /* FP32 records of the list build    */
-void run_lists64(sphdem_ctx *c);       /* neighbour lists of an FP64 handle */
+/* FP32 records of the searches of an FP64 handle, and its neighbour lists */
+void pack_positions(sphdem_ctx *c, bool middle);
+void run_lists64(sphdem_ctx *c, bool middle);
 void run_force(sphdem_ctx *c);         /* calcForce + calcOmega + accelCondition */
 void run_dem_accel(sphdem_ctx *c);
 void run_dddt(sphdem_ctx *c);          /* calcDddtDudt                      */
@@ -188,16 +202,14 @@ void mixed_list_export(sphdem_ctx *c, int *cnt, const long long *offs, int *idx)
 
 /* pairs32.cu: mixed-precision passes */
 namespace mixed {
-/* pack the FP32 records of the middle phase, with the reference DEM buckets and
- * the coupling windows its SPH-DEM passes need, or those of the end phase */
+/* pack the FP32 records of the middle phase (which also starts the Shepard sums
+ * at zero) or those of the end phase */
 void pack(sphdem_ctx *c, bool middle = true);
-void pack_fpi(sphdem_ctx *c);
 /* the neighbour lists of the last rebuild, `depth` entries per particle; more
  * neighbours are an error, or (soft) leave the particle without a list */
 void nlist(sphdem_ctx *c, int depth, bool soft = false);
 /* once per process, outside stream capture: kernel attributes of the step */
 void prepare(sphdem_ctx *c);
-void zero_shep(sphdem_ctx *c);
 int nlist_max_count(sphdem_ctx *c);
 void omega_eos(sphdem_ctx *c, bool omega, bool eos);
 /* lists32.cu: the force / continuity passes specialised on the physics class;
@@ -211,6 +223,11 @@ void porosity(sphdem_ctx *c);
 void dem_drag(sphdem_ctx *c);
 void dem_end(sphdem_ctx *c);
 }  // namespace mixed
+
+/* coupling.cu: porosity + Shepard sums (0) / DEM -> SPH drag (1), and calcFPI +
+ * drag + contacts, of an FP64 handle with the records (c->f64_dem) */
+void couple64(sphdem_ctx *c, int mode);
+void dem_end64(sphdem_ctx *c, bool fluid);
 
 /* pairs32.cu: the mixed lists of the last rebuild as the adjoint's pair
  * tables (tag space, slot *slot of nb / oc / cnt) */

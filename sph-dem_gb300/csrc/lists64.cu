@@ -35,51 +35,6 @@ namespace {
 template <int ND>
 constexpr int LANES64 = ND == 3 ? 8 : (ND == 2 ? 4 : 1);
 
-/* 1/x for x > 0: an FP32 estimate y (relative error d ~ 1e-7) and one step of
- * the series 1/x = y (1 + e + e^2 + ..), e = 1 - x y, which leaves d^3 */
-__device__ __forceinline__ double rcp_pos(double x) {
-    const float xf = (float)x;
-    if (!(xf > 1e-30f && xf < 1e30f)) return 1.0 / x;
-    float yf;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(yf) : "f"(xf));
-    const double y = (double)yf, e = fma(-x, y, 1.0);
-    return fma(y, fma(e, e, e), y);
-}
-
-/* sqrt(x) and, where asked, 1/sqrt(x) of x >= 0: an FP32 estimate y of 1/sqrt
- * and one step of the series 1/sqrt(1 - e) = 1 + e/2 + 3 e^2/8 + .., e = 1 - x y^2 */
-__device__ __forceinline__ double sqrt_pos(double x, double *inv = nullptr) {
-    const float xf = (float)x;
-    if (!(xf > 1e-30f && xf < 1e30f)) {
-        const double r = sqrt(x);
-        if (inv) *inv = r > 0.0 ? 1.0 / r : 0.0;
-        return r;
-    }
-    float yf;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(yf) : "f"(xf));
-    const double y = (double)yf, s = x * y;
-    const double e = fma(-s, y, 1.0), k = e * fma(e, 0.375, 0.5);
-    if (inv) *inv = fma(y, k, y);
-    return fma(s, k, s);
-}
-
-/* max(x, 0) by the sign bit (an integer operation) */
-__device__ __forceinline__ double positive_part(double x) {
-    return __double_as_longlong(x) < 0 ? 0.0 : x;
-}
-
-/* the smaller of two non-negative doubles by their bit patterns */
-__device__ __forceinline__ double min_pos(double a, double b) {
-    return __double_as_longlong(a) < __double_as_longlong(b) ? a : b;
-}
-
-template <int G>
-__device__ __forceinline__ double lane_sum(double v) {
-#pragma unroll
-    for (int o = 1; o < G; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
 struct Lists64 {
     const int *nbr, *ncnt;
     int64_t ld;
@@ -685,22 +640,28 @@ __global__ void __launch_bounds__(BLK) k_reinit_dens(DevCfg c, DevState s, Lists
     }
 }
 
-/* the records the list build reads: offset in the particle's bucket and h, type
- * and ghost code */
+/* the records of the FP32 searches: offset in the particle's own bucket and h,
+ * type and ghost code, a DEM particle's place in the SPH grid; in the middle
+ * phase the Shepard sums start at zero */
 template <int ND>
 __global__ void k_pack_pos(DevCfg c, DevState s, const int *__restrict__ skey, const DevGlobals *__restrict__ g,
-                           float4 *__restrict__ P0, int *__restrict__ tg, int64_t n) {
+                           float4 *__restrict__ P0, int *__restrict__ tg, float4 *__restrict__ DS, int middle, int64_t n) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int t = s.irow(FI_IAM)[i];
     tg[i] = (t & 0xff) | (s.irow(FI_GCODE)[i] << 8);
-    if (t == T_DEAD || (c.liq_dem() && t == T_DEM)) return;
+    if (t == T_DEAD) return;
+    const bool dem = c.liq_dem() && t == T_DEM;
     const int dims[3] = {g->sdims[0], g->sdims[1], g->sdims[2]};
     int cc[3] = {0, 0, 0};
-    decode<ND>(skey[i], dims, cc);
+    if (dem) decode<ND>(skey[i] - g->n_sph_cells, c.ddims, cc);
+    else decode<ND>(skey[i], dims, cc);
     float off[3] = {0.f, 0.f, 0.f};
 #pragma unroll
-    for (int d = 0; d < ND; d++) off[d] = (float)(s.row(FD_R + d)[i] - sph_origin(c, g, d, cc[d]));
+    for (int d = 0; d < ND; d++)
+        off[d] = (float)(s.row(FD_R + d)[i] - (dem ? dem_origin(c, d, cc[d]) : sph_origin(c, g, d, cc[d])));
+    if (dem && middle) s.row(FD_SHEP)[i] = 0.0;
+    if (dem && !middle && DS) DS[i] = dem_in_sph_grid<ND>(c, s, g, i);
     P0[i] = make_float4(off[0], off[1], off[2], (float)s.row(FD_H)[i]);
 }
 
@@ -716,29 +677,17 @@ int blocks64(int64_t n) {
 
 }  // namespace
 
-#define SPHDEM_ND_DISPATCH(nd, F) \
-    do {                          \
-        if ((nd) == 3) {          \
-            F(3);                 \
-        } else if ((nd) == 2) {   \
-            F(2);                 \
-        } else {                  \
-            F(1);                 \
-        }                         \
-    } while (0)
-
-void pack_positions(sphdem_ctx *c) {
+void pack_positions(sphdem_ctx *c, bool middle) {
 #define L_(ND)                                                                                                   \
     SPHDEM_LAUNCH(c, "pack_pos", k_pack_pos<ND>, grid_for(c->n, 256), 256, 0, c->cfg, c->A, c->buf.skey, c->g, \
-                  c->mx_pos, c->mx_tg, c->n)
+                  c->mx_pos, c->mx_tg, c->mx_ds, (int)middle, c->n)
     SPHDEM_ND_DISPATCH(c->cfg.nd, L_);
 #undef L_
 }
 
-void run_lists64(sphdem_ctx *c) {
-    if (c->f64_maxn <= 0) return;
-    pack_positions(c);
-    mixed::nlist(c, c->f64_maxn, true);
+void run_lists64(sphdem_ctx *c, bool middle) {
+    if (c->f64_maxn > 0 || c->f64_dem) pack_positions(c, middle);
+    if (c->f64_maxn > 0) mixed::nlist(c, c->f64_maxn, true);
 }
 
 void run_force(sphdem_ctx *c) {
@@ -790,7 +739,7 @@ void run_reinit_density(sphdem_ctx *c) {
     SPHDEM_LAUNCH(c, "reinit_h", k_reinit_h, grid_for(c->n, 256), 256, 0, c->cfg, c->A, c->g, c->hpred, c->reinit_wide,
                   c->n);
     if (L.nbr) {
-        pack_positions(c);
+        pack_positions(c, false);
         mixed::nlist(c, (int)L.ld, true);
     }
 #define L_(ND)                                                                                                    \

@@ -126,12 +126,132 @@ __device__ __forceinline__ void nl_decode_code(int code, int *o) {
     o[2] = code % 3 - 1;
 }
 
-/* FP64 origin of SPH bucket `cell` on axis d, and its size */
+/* FP64 origin of SPH bucket `cell` on axis d */
 __device__ __forceinline__ double sph_origin(const DevCfg &c, const DevGlobals *g, int d, int cell) {
     return c.periodic[d] ? c.dmin[d] + cell * g->scell[d] : c.dmin[d] + (cell - 3) * g->sr2;
 }
-__device__ __forceinline__ double sph_width(const DevCfg &c, const DevGlobals *g, int d) {
-    return c.periodic[d] ? g->scell[d] : g->sr2;
+
+__device__ __forceinline__ double dem_origin(const DevCfg &c, int d, int cell) {
+    return c.dorig[d] + cell * c.dcell[d];
+}
+
+
+template <int ND>
+__device__ __forceinline__ bool img_ok(int gcode, const int *sh) {
+#pragma unroll
+    for (int d = 0; d < ND; d++) {
+        if (sh[d] == 0) continue;
+        const int ic = (gcode >> (2 * d)) & 3;
+        if (sh[d] < 0 ? ic != 2 : ic != 0) return false;
+    }
+    return true;
+}
+
+/* The reference's FP64 predicate for a pair inside the FP32 band. */
+template <int ND>
+__device__ __noinline__ bool exact_pair(const DevCfg *__restrict__ cp, const DevState s, int a, int b, int sh0,
+                                        int sh1, int sh2, double lim2, int strict) {
+    const int sh[3] = {sh0, sh1, sh2};
+    double dx[3] = {0, 0, 0};
+#pragma unroll
+    for (int d = 0; d < ND; d++)
+        dx[d] = dsub(s.row(FD_R + d)[a], image_pos(s.row(FD_R + d)[b], sh[d], cp->rmin[d], cp->rmax[d]));
+    const double r2 = exact_len2(dx, ND);
+    if (lim2 > 0) return strict ? r2 < lim2 : r2 <= lim2;
+    const double ha = s.row(FD_H)[a], hb = s.row(FD_H)[b];
+    const double t = 2.0 * (ha > hb ? ha : hb);
+    return r2 <= dmul(t, t);
+}
+
+/* Half-width of the band around a cut-off T = R^2 inside which an FP32 r^2
+ * built from bucket offsets cannot decide: each displacement component is
+ * off by < 6 * 2^-24 L when L bounds the magnitudes of the offset terms, so
+ * r^2 by < 1.25e-6 L max(L, R) + 1.8e-7 r^2, and T by < 1.8e-7 T. */
+__device__ __forceinline__ float fp32_band(float T, float L2) { return fmaf(5e-7f, T, 1.5e-6f * fmaxf(L2, T)); }
+
+/* One lane's entry of a bucket range table around a run of buckets (ccol
+ * on the leading axes, zmin..zmax on the last axis Z): lane = 3 * column +
+ * period piece, for the 3^(d-1) neighbour columns; each entry is a run of
+ * consecutive keys key0 + lin .. (buckets zmin-1 .. zmax+1 of the column,
+ * cut at a periodic seam).  Entries of other lanes are empty. */
+struct RangeEntry {
+    int b0, cnt, lin, zoff, shp, code;
+    float ox, oy;
+};
+
+template <int ND>
+__device__ __forceinline__ RangeEntry range_entry(int lane, const int *ccol, int zmin, int zmax, const int *dims,
+                                                  const int *periodic, const float *cell, int key0,
+                                                  const int *__restrict__ start) {
+    constexpr int Z = ND - 1;
+    constexpr int NCOL = Z == 2 ? 9 : (Z == 1 ? 3 : 1);
+    RangeEntry r = {0, 0, 0, 0, 0x15, 0, 0.f, 0.f};
+    if (lane >= 3 * NCOL) return r;
+    const int colidx = lane / 3, wz = lane % 3 - 1;
+    int o[2] = {0, 0};
+    if (Z == 2) {
+        o[0] = colidx / 3 - 1;
+        o[1] = colidx % 3 - 1;
+    } else if (Z == 1) {
+        o[0] = colidx - 1;
+    }
+    bool ok = wz == 0 || periodic[Z];
+    int col_lin = 0, code = 0, shp = 0;
+    float off[2] = {0.f, 0.f};
+#pragma unroll
+    for (int d = ND; d < 3; d++) {
+        shp |= 1 << (2 * d);
+        code += code_stride(d);
+    }
+#pragma unroll
+    for (int d = 0; d < Z; d++) {
+        int t = ccol[d] + o[d], shd = 0;
+        if (t < 0) {
+            ok = ok && periodic[d];
+            t += dims[d];
+            shd = -1;
+        } else if (t >= dims[d]) {
+            ok = ok && periodic[d];
+            t -= dims[d];
+            shd = 1;
+        }
+        col_lin = col_lin * dims[d] + t;
+        code += (o[d] + 1) * code_stride(d);
+        off[d] = (float)o[d] * cell[d];
+        shp |= (shd + 1) << (2 * d);
+    }
+    shp |= (wz + 1) << (2 * Z);
+    const int zdim = dims[Z];
+    const int zlo = max(zmin - 1, wz * zdim), zhi = min(zmax + 1, (wz + 1) * zdim - 1);
+    if (ok && zlo <= zhi) {
+        r.lin = key0 + col_lin * zdim + (zlo - wz * zdim);
+        r.b0 = start[r.lin];
+        r.cnt = start[r.lin + (zhi - zlo) + 1] - r.b0;
+        r.zoff = zlo - zmin;
+        r.shp = shp;
+        r.code = code << B_BITS;
+        r.ox = off[0];
+        r.oy = off[1];
+    }
+    return r;
+}
+
+/* the SPH bucket of a DEM particle (as calcFPI searches it) and its FP32 offset there: (offset, bucket key) */
+template <int ND>
+__device__ __forceinline__ float4 dem_in_sph_grid(const DevCfg &c, const DevState &s, const DevGlobals *g, int64_t i) {
+    const int dims[3] = {g->sdims[0], g->sdims[1], g->sdims[2]};
+    int key = 0;
+    float o[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+    for (int d = 0; d < ND; d++) {
+        const double r = s.row(FD_R + d)[i];
+        int kd = c.periodic[d] ? (int)floor((r - c.dmin[d]) * g->rscell[d])
+                               : trunc_index(r, c.dmin[d], g->sr2, g->rsr2_f, 3.0);
+        kd = kd < 0 ? 0 : (kd >= dims[d] ? dims[d] - 1 : kd);
+        key = key * dims[d] + kd;
+        o[d] = (float)(r - sph_origin(c, g, d, kd));
+    }
+    return make_float4(o[0], o[1], o[2], __int_as_float(key));
 }
 
 /* Neighbour lists: slot j of particle a, in tiles of 32 particles x 8
@@ -408,3 +528,14 @@ __device__ Staged stage_neighbours(const DevCfg &c, DevGlobals *g, const int *__
 
 }  // namespace
 }  // namespace sphdem
+
+#define SPHDEM_ND_DISPATCH(nd, F) \
+    do {                          \
+        if ((nd) == 3) {          \
+            F(3);                 \
+        } else if ((nd) == 2) {   \
+            F(2);                 \
+        } else {                  \
+            F(1);                 \
+        }                         \
+    } while (0)

@@ -21,14 +21,7 @@
  *                cancels too much for FP32)
  *   k_force      calcForce + the Courant/viscous/accel dt conditions
  *   k_dddt       calcDddtDudt
- *   k_couple     calcPorosity + calcShepSum (mode 0) and calcDEMtoSPHDrag +
- *                finalisePorosity (mode 1): 32-particle slices stage the DEM
- *                particles of the DEM buckets within Rc in shared memory and
- *                test them with the reference's asymmetric bucket rule
- *                (dataLL.cpp:1154-1190); the Shepard scatter is reduced over
- *                the warp and lands as one FP64 atomic per (warp, DEM particle)
- *   k_dem_end    calcFPI + calcParticleDrag + calcDEMContacts: one warp per
- *                DEM particle, lanes split the candidates, warp reductions
+ * The SPH-DEM coupling and contact passes are in coupling.cu.
  *
  * Sums are Kahan-compensated in FP32 and added to the FP64 state once per
  * particle.  Roofline: the list passes are FP32-pipe-bound on 3D workloads
@@ -43,67 +36,6 @@
 namespace sphdem {
 namespace {
 
-__device__ __forceinline__ double dem_origin(const DevCfg &c, int d, int cell) {
-    return c.dorig[d] + cell * c.dcell[d];
-}
-
-/* stencil neighbour (offsets o) with periodic wrap; -1 when off the grid */
-template <int ND>
-__device__ __forceinline__ int nb_cell(const int *cc, const int *o, const int *dims, const int *periodic, int *sh) {
-    int lin = 0;
-#pragma unroll
-    for (int d = 0; d < ND; d++) {
-        int t = cc[d] + o[d];
-        sh[d] = 0;
-        if (t < 0) {
-            if (!periodic[d]) return -1;
-            t += dims[d];
-            sh[d] = -1;
-        } else if (t >= dims[d]) {
-            if (!periodic[d]) return -1;
-            t -= dims[d];
-            sh[d] = 1;
-        }
-        lin = lin * dims[d] + t;
-    }
-    return lin;
-}
-
-template <int ND>
-__device__ __forceinline__ bool img_ok(int gcode, const int *sh) {
-#pragma unroll
-    for (int d = 0; d < ND; d++) {
-        if (sh[d] == 0) continue;
-        const int ic = (gcode >> (2 * d)) & 3;
-        if (sh[d] < 0 ? ic != 2 : ic != 0) return false;
-    }
-    return true;
-}
-
-template <int ND>
-__device__ __forceinline__ bool any_shift(const int *sh) {
-    bool a = false;
-#pragma unroll
-    for (int d = 0; d < ND; d++) a |= sh[d] != 0;
-    return a;
-}
-
-/* The reference's FP64 predicate for a pair inside the FP32 band. */
-template <int ND>
-__device__ __noinline__ bool exact_pair(const DevCfg *__restrict__ cp, const DevState s, int a, int b, int sh0,
-                                        int sh1, int sh2, double lim2, int strict) {
-    const int sh[3] = {sh0, sh1, sh2};
-    double dx[3] = {0, 0, 0};
-#pragma unroll
-    for (int d = 0; d < ND; d++)
-        dx[d] = dsub(s.row(FD_R + d)[a], image_pos(s.row(FD_R + d)[b], sh[d], cp->rmin[d], cp->rmax[d]));
-    const double r2 = exact_len2(dx, ND);
-    if (lim2 > 0) return strict ? r2 < lim2 : r2 <= lim2;
-    const double ha = s.row(FD_H)[a], hb = s.row(FD_H)[b];
-    const double t = 2.0 * (ha > hb ? ha : hb);
-    return r2 <= dmul(t, t);
-}
-
 /* ---------------------------------------------------------------------- */
 /* P0 = (offset from own bucket origin, h), P1 = (vhat, mass; negated for
  * particles that are neither sph / sphBoundary nor DEM), P2 = (dens, pdr2, cF,
@@ -111,20 +43,10 @@ __device__ __noinline__ bool exact_pair(const DevCfg *__restrict__ cp, const Dev
  * where cF = -10 C / h^(d+2) is the factor of the Wendland gradient F(r, h) =
  * cF (2 - r/h)^3 and a DEM particle's second place holds its radius,
  * tg = type | gcode << 8 */
-/* reference DEM bucket indices packed 10 bits per axis (biased by 512) */
-constexpr int CP_BIAS = 512;
-
-__device__ __forceinline__ int pack_cells(const int *k, int nd) {
-    int p = 0;
-    for (int d = 0; d < nd; d++) p |= ((k[d] + CP_BIAS) & 1023) << (10 * d);
-    return p;
-}
-
 template <int ND>
 __global__ void k_pack(DevCfg c, DevState s, const int *__restrict__ skey, const DevGlobals *__restrict__ g,
                        float4 *__restrict__ P0, float4 *__restrict__ P1, float4 *__restrict__ P2,
-                       int *__restrict__ tg, int4 *__restrict__ RC4, int with_rc, int middle,
-                       float4 *__restrict__ DS, float4 *__restrict__ NB, int64_t n) {
+                       int *__restrict__ tg, int middle, float4 *__restrict__ DS, float4 *__restrict__ NB, int64_t n) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int t = s.irow(FI_IAM)[i];
@@ -171,84 +93,9 @@ __global__ void k_pack(DevCfg c, DevState s, const int *__restrict__ skey, const
         NB[3 * i + 1] = make_float4(nv[1][0], nv[1][1], nv[1][2], 0.f);
         NB[3 * i + 2] = make_float4(nv[2][0], nv[2][1], nv[2][2], 0.f);
     }
-    if (dem) {
-        /* the SPH bucket of a DEM particle and its FP32 offset there (calcFPI) */
-        const int dims[3] = {g->sdims[0], g->sdims[1], g->sdims[2]};
-        int k[3] = {0, 0, 0}, key = 0;
-        float o[3] = {0.f, 0.f, 0.f};
-#pragma unroll
-        for (int d = 0; d < ND; d++) {
-            const double r = s.row(FD_R + d)[i];
-            int kd = c.periodic[d] ? (int)floor((r - c.dmin[d]) * g->rscell[d])
-                                   : trunc_index(r, c.dmin[d], g->sr2, g->rsr2_f, 3.0);
-            kd = kd < 0 ? 0 : (kd >= dims[d] ? dims[d] - 1 : kd);
-            k[d] = kd;
-            key = key * dims[d] + kd;
-            o[d] = (float)(r - sph_origin(c, g, d, kd));
-        }
-        DS[i] = make_float4(o[0], o[1], o[2], __int_as_float(key));
-    }
-    if (with_rc) {
-        /* reference DEM buckets (dem_getCellI) of the particle and, for DEM
-         * particles, of its periodic images one period below / above */
-        int k[3] = {0, 0, 0}, km[3] = {0, 0, 0}, kp[3] = {0, 0, 0};
-#pragma unroll
-        for (int d = 0; d < ND; d++) {
-            const double r = s.row(FD_R + d)[i];
-            k[d] = ref_dem_cell(r, c, d);
-            if (dem && c.periodic[d]) {
-                km[d] = ref_dem_cell(image_pos(r, -1, c.rmin[d], c.rmax[d]), c, d);
-                kp[d] = ref_dem_cell(image_pos(r, 1, c.rmin[d], c.rmax[d]), c, d);
-            }
-        }
-        RC4[i] = make_int4(pack_cells(k, ND), pack_cells(km, ND), pack_cells(kp, ND), 0);
-    }
+    if (dem && middle) s.row(FD_SHEP)[i] = 0.0; /* the porosity pass adds into it */
+    if (dem && !middle) DS[i] = dem_in_sph_grid<ND>(c, s, g, i);
 }
-
-/* Coupling windows: for SPH bucket index i on axis d, the DEM buckets
- * [klo, khi] within Rc of it and the FP32 offset of its origin from the
- * origin of DEM bucket klo (one FP64 evaluation per bucket per rebuild). */
-template <int ND>
-__global__ void k_win(DevCfg c, const DevGlobals *__restrict__ g, int4 *__restrict__ win, int win_cap) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int d = t / win_cap, i = t - d * win_cap;
-    if (d >= ND || i >= g->sdims[d]) return;
-    const double lo = sph_origin(c, g, d, i);
-    const double hi = lo + sph_width(c, g, d);
-    int klo = (int)floor((lo - c.rc - c.dorig[d]) * c.rdcell[d]);
-    int khi = (int)floor((hi + c.rc - c.dorig[d]) * c.rdcell[d]);
-    if (!c.periodic[d]) {
-        klo = max(klo, 0);
-        khi = min(khi, c.ddims[d] - 1);
-    }
-    win[t] = make_int4(klo, khi, __float_as_int((float)(lo - (c.dorig[d] + klo * c.dcell[d]))), 0);
-}
-
-/* fields the DEM side gathers from fluid neighbours in calcFPI (sph.h:1708-1792):
- * Q0 = (fp+fb, fv.x), Q1 = (fv.y, fv.z, f.x, f.y), Q2 = (f.z, fdrag) */
-__global__ void k_pack_fpi(DevState s, float4 *__restrict__ Q0, float4 *__restrict__ Q1, float4 *__restrict__ Q2,
-                           int64_t n) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float v[12];
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-        v[d] = (float)(s.row(FD_FP + d)[i] + s.row(FD_FB + d)[i]);
-        v[3 + d] = (float)s.row(FD_FV + d)[i];
-        v[6 + d] = (float)s.row(FD_F + d)[i];
-        v[9 + d] = (float)s.row(FD_FDRAG + d)[i];
-    }
-    Q0[i] = make_float4(v[0], v[1], v[2], v[3]);
-    Q1[i] = make_float4(v[4], v[5], v[6], v[7]);
-    Q2[i] = make_float4(v[8], v[9], v[10], v[11]);
-}
-
-/* ---------------------------------------------------------------------- */
-/* Half-width of the band around a cut-off T = R^2 inside which an FP32 r^2
- * built from bucket offsets cannot decide: each displacement component is
- * off by < 6 * 2^-24 L when L bounds the magnitudes of the offset terms, so
- * r^2 by < 1.25e-6 L max(L, R) + 1.8e-7 r^2, and T by < 1.8e-7 T. */
-__device__ __forceinline__ float fp32_band(float T, float L2) { return fmaf(5e-7f, T, 1.5e-6f * fmaxf(L2, T)); }
 
 /* ---------------------------------------------------------------------- */
 /* Neighbour-list build.
@@ -291,73 +138,6 @@ constexpr int NL_QN = 64;     /* queue slots per lane: moved on when over 32 are
  * bucket holds ~7 particles, so 32 of them span five */
 template <int ND>
 constexpr int NL_RUN = ND == 3 ? 2 : (ND == 2 ? 6 : 14);
-
-/* One lane's entry of a bucket range table around a run of buckets (ccol
- * on the leading axes, zmin..zmax on the last axis Z): lane = 3 * column +
- * period piece, for the 3^(d-1) neighbour columns; each entry is a run of
- * consecutive keys key0 + lin .. (buckets zmin-1 .. zmax+1 of the column,
- * cut at a periodic seam).  Entries of other lanes are empty. */
-struct RangeEntry {
-    int b0, cnt, lin, zoff, shp, code;
-    float ox, oy;
-};
-
-template <int ND>
-__device__ __forceinline__ RangeEntry range_entry(int lane, const int *ccol, int zmin, int zmax, const int *dims,
-                                                  const int *periodic, const float *cell, int key0,
-                                                  const int *__restrict__ start) {
-    constexpr int Z = ND - 1;
-    constexpr int NCOL = Z == 2 ? 9 : (Z == 1 ? 3 : 1);
-    RangeEntry r = {0, 0, 0, 0, 0x15, 0, 0.f, 0.f};
-    if (lane >= 3 * NCOL) return r;
-    const int colidx = lane / 3, wz = lane % 3 - 1;
-    int o[2] = {0, 0};
-    if (Z == 2) {
-        o[0] = colidx / 3 - 1;
-        o[1] = colidx % 3 - 1;
-    } else if (Z == 1) {
-        o[0] = colidx - 1;
-    }
-    bool ok = wz == 0 || periodic[Z];
-    int col_lin = 0, code = 0, shp = 0;
-    float off[2] = {0.f, 0.f};
-#pragma unroll
-    for (int d = ND; d < 3; d++) {
-        shp |= 1 << (2 * d);
-        code += code_stride(d);
-    }
-#pragma unroll
-    for (int d = 0; d < Z; d++) {
-        int t = ccol[d] + o[d], shd = 0;
-        if (t < 0) {
-            ok = ok && periodic[d];
-            t += dims[d];
-            shd = -1;
-        } else if (t >= dims[d]) {
-            ok = ok && periodic[d];
-            t -= dims[d];
-            shd = 1;
-        }
-        col_lin = col_lin * dims[d] + t;
-        code += (o[d] + 1) * code_stride(d);
-        off[d] = (float)o[d] * cell[d];
-        shp |= (shd + 1) << (2 * d);
-    }
-    shp |= (wz + 1) << (2 * Z);
-    const int zdim = dims[Z];
-    const int zlo = max(zmin - 1, wz * zdim), zhi = min(zmax + 1, (wz + 1) * zdim - 1);
-    if (ok && zlo <= zhi) {
-        r.lin = key0 + col_lin * zdim + (zlo - wz * zdim);
-        r.b0 = start[r.lin];
-        r.cnt = start[r.lin + (zhi - zlo) + 1] - r.b0;
-        r.zoff = zlo - zmin;
-        r.shp = shp;
-        r.code = code << B_BITS;
-        r.ox = off[0];
-        r.oy = off[1];
-    }
-    return r;
-}
 
 /* A candidate whose FP32 test leaves doubt: list entry e (candidate and stencil
  * code) of particle a in bucket cc, zd its bucket on the last axis relative to
@@ -1229,750 +1009,6 @@ __global__ void __launch_bounds__(BLK) k_dddt(DevCfg c, DevState s, const DevGlo
     s.row(FD_DDDT)[a] += (double)(acc.s * roma);
 }
 
-/* ---------------------------------------------------------------------- */
-/* SPH <-> DEM coupling sums over the reference's coupling neighbours
- * (calcNeighboursCoupling, dataLL.cpp:1104-1192: DEM within Rc, with the
- * asymmetric bucket rule).  MODE 0: calcPorosity + the DEM Shepard sums
- * (sph.h calcPorosity / calcShepSum); MODE 1: calcDEMtoSPHDrag +
- * finalisePorosity.
- *
- * Work split as in k_nlist: a warp takes 32 consecutive particles of the
- * bucket order, forms runs of buckets along the last axis, and stages the DEM
- * particles of every DEM bucket within Rc of the run in shared memory
- * (position in the run's frame, reference DEM bucket of the image, the
- * partner's packed fields); every lane then tests all staged partners.  The
- * Shepard contribution of one partner is reduced over the warp and added
- * with one FP64 atomic. */
-constexpr int CP_WARPS = 8;
-constexpr int CP_CAP = 128;
-
-/* coupling_rule on packed bucket indices; lim_ceil = ceil(couple_lim), so
- * that for the integer sums rP < couple_lim <=> rP < lim_ceil */
-template <int ND>
-__device__ __forceinline__ bool coupling_rule_packed(int cs, int cd, int num, int lim_ceil) {
-    int rP = 0, rM = 0;
-#pragma unroll
-    for (int d = 0; d < ND; d++) {
-        const int o = ((cd >> (10 * d)) & 1023) - ((cs >> (10 * d)) & 1023);
-        if (o < -num || o > num) return false;
-        rP += (o + 1) * (o + 1);
-        rM += (o - 1) * (o - 1);
-    }
-    if (ND == 1) return true;
-    return rP < lim_ceil || rM < lim_ceil;
-}
-
-/* one warp-aggregated atomic reserves k entries per lane of cnt; every lane
- * of the warp calls it; returns this lane's first entry */
-__device__ __forceinline__ int64_t tap_reserve(int k, int *cnt) {
-    const int lane = threadIdx.x & 31;
-    int incl = k;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += t;
-    }
-    const int total = __shfl_sync(0xffffffffu, incl, 31);
-    int base = 0;
-    if (lane == 31 && total > 0) base = atomicAdd(cnt, total);
-    base = __shfl_sync(0xffffffffu, base, 31);
-    return (int64_t)base + incl - k;
-}
-
-/* TAP (adjoint replay only): the coupling pairs each fluid particle takes
- * go to the tap table tt of step *tslot -- mode 0 counts them and reserves
- * the particle's entries, mode 1 (same pairs, same order) writes them. */
-template <int ND, int MODE, bool TAP>
-__global__ void __launch_bounds__(CP_WARPS * 32, 3) k_couple(DevCfg c, const DevCfg *__restrict__ cp, DevState s,
-                                                          const int *__restrict__ start, const int *__restrict__ skey,
-                                                          const DevGlobals *__restrict__ g,
-                                                          const float4 *__restrict__ P0, const float4 *__restrict__ P1,
-                                                          const float4 *__restrict__ P2, const float4 *__restrict__ DP,
-                                                          const int *__restrict__ tg, const int4 *__restrict__ RC4,
-                                                          const int4 *__restrict__ win, int win_cap,
-                                                          float *__restrict__ shep32, TapTable tt,
-                                                          const int *__restrict__ tslot, int64_t n_all) {
-    constexpr int Z = ND - 1;
-    constexpr unsigned FULL = 0xffffffffu;
-    __shared__ float4 s_pos[CP_WARPS][CP_CAP];
-    __shared__ float4 s_aux[CP_WARPS][CP_CAP];
-    __shared__ int2 s_id[CP_WARPS][CP_CAP];
-    const int lane = threadIdx.x & 31;
-    const int w = threadIdx.x >> 5;
-    float4 *cpos = s_pos[w];
-    float4 *caux = s_aux[w];
-    int2 *cid = s_id[w];
-    const unsigned lt_mask = (1u << lane) - 1u;
-    const int nsc = g->n_sph_cells;
-    const int n_t = start[nsc];
-    const int sdims[3] = {g->sdims[0], g->sdims[1], g->sdims[2]};
-    const int zdim = sdims[Z];
-    float cell[3];
-    load_cell32(c, g, cell);
-    const float cz = cell[Z];
-    const float wcon = (float)c.wcon, two_over_rc = (float)c.two_over_rc;
-    const float c_ihn = (float)c.c_ihn, c_ihn2 = (float)c.c_ihn2;
-    const float por_incr = (float)c.por_incr, dem_vol = (float)c.dem_vol;
-    const float rc2 = (float)c.rc2;
-    const float rdens2d = (float)(1.0 / (2.0 * c.dem_radius));
-    const int lim_ceil = (int)ceil(c.couple_lim);
-    const float rc2x = (float)(2.0 * c.rc);
-    const float rc_w = (float)c.rc * (1.f + 1e-5f);
-    float dcf[3] = {0.f, 0.f, 0.f};
-#pragma unroll
-    for (int d = 0; d < ND; d++) dcf[d] = (float)c.dcell[d];
-
-    for (int t0 = (blockIdx.x * CP_WARPS + w) * 32; t0 < n_t; t0 += CP_WARPS * gridDim.x * 32) {
-        const int a = t0 + lane;
-        int ta = -1, key = 0;
-        if (a < n_t) {
-            key = skey[a];
-            ta = tg[a] & 0xff;
-        }
-        const bool act = is_sph_or_sphb(ta);
-        if (MODE == 1 && is_boundary(ta)) s.row(FD_POR)[a] = 1.0;
-        int ntap = 0, tag_a = 0, tlim = 0, js = 0;
-        int *tout = nullptr;
-        if (TAP) {
-            js = *tslot;
-            if (act) tag_a = s.irow(FI_TAG)[a];
-            if (MODE == 1 && act) {
-                const int2 o = tt.oc[(int64_t)js * n_all + tag_a];
-                tout = tt.nb + (int64_t)js * tt.cap + o.x;
-                tlim = o.y;
-            }
-        }
-        int cc[3] = {0, 0, 0};
-        decode<ND>(key, sdims, cc);
-        const int col = key / zdim;
-        /* this lane's particle: packed fields and reference DEM bucket */
-        float4 pa0 = make_float4(0.f, 0.f, 0.f, 0.f), va = make_float4(0.f, 0.f, 0.f, 0.f);
-        float dvol = 0.f, rdens = 0.f;
-        int cs = 0;
-        if (act) {
-            pa0 = P0[a];
-            va = P1[a];
-            cs = RC4[a].x;
-            const float densa = P2[a].x;
-            dvol = va.w / densa;
-            rdens = ND == 2 ? rdens2d / densa : 1.f / densa;
-        }
-        Kahan por, dpd, acc[ND];
-        por.init(0.f);
-        dpd.init(0.f);
-#pragma unroll
-        for (int k = 0; k < ND; k++) acc[k].init(0.f);
-
-        unsigned pending = __ballot_sync(FULL, act);
-        while (pending) {
-            const int leader = __ffs(pending) - 1;
-            const int lcol = __shfl_sync(FULL, col, leader);
-            const int zmin = __shfl_sync(FULL, cc[Z], leader);
-            const unsigned gmask = __ballot_sync(FULL, act && col == lcol && cc[Z] <= zmin + 2) & pending;
-            pending &= ~gmask;
-            const int zmax = __shfl_sync(FULL, cc[Z], 31 - __clz(gmask));
-            int ccol[3] = {0, 0, 0};
-#pragma unroll
-            for (int d = 0; d < ND; d++) ccol[d] = __shfl_sync(FULL, cc[d], leader);
-            const bool mine = (gmask >> lane) & 1u;
-            float pv[3] = {1e30f, 1e30f, 1e30f};
-            if (mine) {
-                pv[0] = pa0.x;
-                pv[1] = pa0.y;
-                pv[2] = pa0.z;
-                pv[Z] += (float)(cc[Z] - zmin) * cz;
-            }
-            /* DEM buckets within Rc of the run; the origin of DEM bucket k in
-             * the run's frame (origin of bucket (ccol, zmin)) is
-             * obase - (k - klo) * dcell, one FP64 difference per axis */
-            int klo[3] = {0, 0, 0}, khi[3] = {0, 0, 0};
-            float obase[3] = {0.f, 0.f, 0.f};
-            float lmax = 0.f;
-#pragma unroll
-            for (int d = 0; d < ND; d++) {
-                const int4 wlo = win[d * win_cap + (d == Z ? zmin : ccol[d])];
-                klo[d] = wlo.x;
-                khi[d] = d == Z ? win[d * win_cap + zmax].y : wlo.y;
-                obase[d] = __int_as_float(wlo.z);
-                if (c.periodic[d] && khi[d] - klo[d] + 1 > c.ddims[d]) khi[d] = klo[d] + c.ddims[d] - 1;
-                lmax = fmaxf(lmax, (d == Z ? (float)(zmax - zmin + 1) : 1.f) * cell[d] + rc2x + 2.f * dcf[d]);
-            }
-            const float band_c = fp32_band(rc2, lmax * lmax);
-            /* the run's extent on the last axis, widened by Rc and a rounding
-             * margin: no DEM partner lies outside */
-            float zw_lo = mine ? pv[Z] : 1e30f, zw_hi = mine ? pv[Z] : -1e30f;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                zw_lo = fminf(zw_lo, __shfl_xor_sync(FULL, zw_lo, o));
-                zw_hi = fmaxf(zw_hi, __shfl_xor_sync(FULL, zw_hi, o));
-            }
-            zw_lo -= rc_w + 1e-5f * lmax;
-            zw_hi += rc_w + 1e-5f * lmax;
-            int nst = 0;
-
-            auto evaluate = [&]() {
-                __syncwarp();
-                for (int j = 0; j < nst; j++) {
-                    const float4 q = cpos[j];
-                    const float dd0 = pv[0] - q.x;
-                    const float dd1 = ND > 1 ? pv[1] - q.y : 0.f;
-                    const float dd2 = ND > 2 ? pv[2] - q.z : 0.f;
-                    const float r2 = fmaf(dd2, dd2, fmaf(dd1, dd1, dd0 * dd0));
-                    float wgt = 0.f;
-                    if (r2 < rc2 + band_c) {
-                        const int2 id = cid[j];
-                        bool in = coupling_rule_packed<ND>(cs, id.y, c.couple_num, lim_ceil);
-                        if (in && r2 >= rc2 - band_c) {
-                            const int shp = (unsigned)id.x >> B_BITS;
-                            in = exact_pair<ND>(cp, s, a, id.x & B_MASK, (shp & 3) - 1, ((shp >> 2) & 3) - 1,
-                                                ((shp >> 4) & 3) - 1, c.rc2, 1);
-                        }
-                        if (in) {
-                            if (TAP) {
-                                if (MODE == 1 && ntap < tlim) tout[ntap] = s.irow(FI_TAG)[id.x & B_MASK] | (id.x & ~B_MASK);
-                                ntap++;
-                            }
-                            const float r = sqrtf(r2);
-                            const float qq = r * two_over_rc;
-                            wgt = c_ihn * wK32(qq, wcon);
-                            const float4 x = caux[j];
-                            if (MODE == 0) {
-                                por.add(por_incr * wgt);
-                                if (r != 0.f) {
-                                    const float Fq = c_ihn2 * wdK32(qq, wcon) / qq;
-                                    const float vd = (va.x - x.x) * dd0 + (va.y - x.y) * dd1 + (va.z - x.z) * dd2;
-                                    dpd.add(-dem_vol * vd * Fq);
-                                    const float ddv[3] = {dd0, dd1, dd2};
-#pragma unroll
-                                    for (int k = 0; k < ND; k++) acc[k].add(dem_vol * ddv[k] * Fq);
-                                }
-                            } else {
-                                /* x = (m/shep, fdrag) of the DEM particle */
-                                const float sc = x.x * rdens * wgt;
-                                const float fdb[3] = {x.y, x.z, x.w};
-#pragma unroll
-                                for (int k = 0; k < ND; k++) acc[k].add(-sc * fdb[k]);
-                            }
-                        }
-                    }
-                    if (MODE == 0 && __any_sync(FULL, wgt != 0.f)) {
-                        const float sum = warp_sum(dvol * wgt);
-                        if (lane == 0 && sum != 0.f) atomicAdd(&shep32[cid[j].x & B_MASK], sum);
-                    }
-                }
-                __syncwarp();
-                nst = 0;
-            };
-
-            /* Range table in rounds of 32 lanes: one lane per (DEM column of the
-             * window, period piece along the last axis), each a run of
-             * consecutive DEM keys.  All lanes load their ranges at once; the
-             * candidates of a round are then gathered flat. */
-            int nwcol = 1;
-#pragma unroll
-            for (int d = 0; d < Z; d++) nwcol *= khi[d] - klo[d] + 1;
-            const int nranges = 3 * nwcol;
-            const int ddz = c.ddims[Z];
-            const int dstart = nsc;
-            int r0 = -32, t = 0, total = 0;
-            int r_b0 = 0, r_cnt = 0, r_lin = 0, r_zq = 0, r_sh = 0, r_excl = 0;
-            float r_dx = 0.f, r_dy = 0.f;
-            /* next round of ranges with at least one candidate */
-            auto load_round = [&]() -> bool {
-                for (r0 += 32; r0 < nranges; r0 += 32) {
-                    r_b0 = r_cnt = r_lin = r_zq = r_sh = 0;
-                    r_dx = r_dy = 0.f;
-                    const int ri = r0 + lane;
-                    if (ri < nranges) {
-                        const int colq = ri / 3, wz = ri % 3 - 1;
-                        int kq[2] = {0, 0};
-                        if (Z == 2) {
-                            const int nwy = khi[1] - klo[1] + 1;
-                            kq[0] = klo[0] + colq / nwy;
-                            kq[1] = klo[1] + colq % nwy;
-                        } else if (Z == 1) {
-                            kq[0] = klo[0] + colq;
-                        }
-                        int col_lin = 0, shp = 0;
-                        float dl[2] = {0.f, 0.f};
-#pragma unroll
-                        for (int d = ND; d < 3; d++) shp |= 1 << (2 * d);
-#pragma unroll
-                        for (int d = 0; d < Z; d++) {
-                            int tt = kq[d], shd = 0;
-                            if (tt < 0) {
-                                tt += c.ddims[d];
-                                shd = -1;
-                            } else if (tt >= c.ddims[d]) {
-                                tt -= c.ddims[d];
-                                shd = 1;
-                            }
-                            col_lin = col_lin * c.ddims[d] + tt;
-                            dl[d] = (float)(kq[d] - klo[d]) * dcf[d] - obase[d];
-                            shp |= (shd + 1) << (2 * d);
-                        }
-                        shp |= (wz + 1) << (2 * Z);
-                        const bool ok = wz == 0 || c.periodic[Z];
-                        const int zlo = max(klo[Z], wz * ddz), zhi = min(khi[Z], (wz + 1) * ddz - 1);
-                        if (ok && zlo <= zhi) {
-                            r_lin = dstart + col_lin * ddz + (zlo - wz * ddz);
-                            r_b0 = start[r_lin];
-                            r_cnt = start[r_lin + (zhi - zlo) + 1] - r_b0;
-                            r_zq = zlo - klo[Z];
-                            r_sh = shp;
-                            r_dx = dl[0];
-                            r_dy = dl[1];
-                            /* DEM buckets hold their particles sorted on the last axis:
-                             * keep those within Rc of the run there (binary search) */
-                            int lo = 0, hi = r_cnt;
-                            while (lo < hi) {
-                                const int mid = (lo + hi) >> 1, b = r_b0 + mid;
-                                const float4 q = P0[b];
-                                const float z = (Z == 0 ? q.x : (Z == 1 ? q.y : q.z)) +
-                                                ((float)(r_zq + skey[b] - r_lin) * dcf[Z] - obase[Z]);
-                                if (z < zw_lo) lo = mid + 1;
-                                else hi = mid;
-                            }
-                            const int first = lo;
-                            hi = r_cnt;
-                            while (lo < hi) {
-                                const int mid = (lo + hi) >> 1, b = r_b0 + mid;
-                                const float4 q = P0[b];
-                                const float z = (Z == 0 ? q.x : (Z == 1 ? q.y : q.z)) +
-                                                ((float)(r_zq + skey[b] - r_lin) * dcf[Z] - obase[Z]);
-                                if (z <= zw_hi) lo = mid + 1;
-                                else hi = mid;
-                            }
-                            r_b0 += first;
-                            r_cnt = lo - first;
-                        }
-                    }
-                    r_excl = r_cnt;
-#pragma unroll
-                    for (int o = 1; o < 32; o <<= 1) {
-                        const int v = __shfl_up_sync(FULL, r_excl, o);
-                        if (lane >= o) r_excl += v;
-                    }
-                    total = __shfl_sync(FULL, r_excl, 31);
-                    r_excl -= r_cnt;
-                    t = 0;
-                    if (total > 0) return true;
-                }
-                return false;
-            };
-
-            bool more = load_round();
-            for (;;) {
-                while (more && nst + 32 <= CP_CAP) {
-                    const int j = t + lane;
-                    int src = 0;
-#pragma unroll
-                    for (int step = 16; step > 0; step >>= 1) {
-                        const int e = __shfl_sync(FULL, r_excl, src + step);
-                        if (e <= j) src += step;
-                    }
-                    const int b0 = __shfl_sync(FULL, r_b0, src), ex = __shfl_sync(FULL, r_excl, src);
-                    const int lin = __shfl_sync(FULL, r_lin, src), zq = __shfl_sync(FULL, r_zq, src);
-                    const int shp = __shfl_sync(FULL, r_sh, src);
-                    const float dx = __shfl_sync(FULL, r_dx, src), dy = __shfl_sync(FULL, r_dy, src);
-                    bool valid = false;
-                    float4 pb = make_float4(0.f, 0.f, 0.f, 0.f), xb = make_float4(0.f, 0.f, 0.f, 0.f);
-                    int b = 0, cdp = 0;
-                    float dzl = 0.f;
-                    if (j < total) {
-                        b = b0 + (j - ex);
-                        const int tgb = tg[b];
-                        const int shv[3] = {(shp & 3) - 1, ((shp >> 2) & 3) - 1, ((shp >> 4) & 3) - 1};
-                        valid = (tgb & 0xff) == T_DEM && (shp == 0x15 || img_ok<ND>(tgb >> 8, shv));
-                        if (valid) {
-                            pb = P0[b];
-                            xb = MODE == 0 ? P1[b] : DP[b];
-                            dzl = (float)(zq + (skey[b] - lin)) * dcf[Z] - obase[Z];
-                            const int4 rc = RC4[b];
-                            cdp = rc.x;
-#pragma unroll
-                            for (int d = 0; d < ND; d++) {
-                                const int m = 1023 << (10 * d);
-                                if (shv[d]) cdp = (cdp & ~m) | ((shv[d] < 0 ? rc.y : rc.z) & m);
-                            }
-                        }
-                    }
-                    const unsigned m = __ballot_sync(FULL, valid);
-                    if (valid) {
-                        const int pos = nst + __popc(m & lt_mask);
-                        float qv[3] = {pb.x, pb.y, pb.z};
-                        if (Z > 0) qv[0] += dx;
-                        if (Z > 1) qv[1] += dy;
-                        qv[Z] += dzl;
-                        cpos[pos] = make_float4(qv[0], qv[1], qv[2], 0.f);
-                        caux[pos] = xb;
-                        cid[pos] = make_int2(b | (shp << B_BITS), cdp);
-                    }
-                    nst += __popc(m);
-                    t += 32;
-                    if (t >= total) more = load_round();
-                }
-                evaluate();
-                if (!more) break;
-            }
-        }
-        if (TAP && MODE == 0) {
-            const int64_t off = tap_reserve(ntap, tt.cnt + js);
-            if (act) tt.oc[(int64_t)js * n_all + tag_a] = make_int2((int)off, off + ntap <= tt.cap ? ntap : 0);
-        }
-        if (!act) continue;
-        if (MODE == 0) {
-            s.row(FD_POR)[a] = por.s;
-            s.row(FD_DPORDT)[a] = dpd.s;
-#pragma unroll
-            for (int k = 0; k < ND; k++) s.row(FD_GPOR + k)[a] = acc[k].s;
-        } else {
-#pragma unroll
-            for (int k = 0; k < ND; k++) {
-                const double v = acc[k].s;
-                s.row(FD_FDRAG + k)[a] = v;
-                s.row(FD_F + k)[a] += v;
-            }
-            double p = 1.0 - s.row(FD_POR)[a];
-            if (p < 0.37) {
-                p = 0.37;
-                s.row(FD_DPORDT)[a] = 0.0;
-                for (int k = 0; k < 3; k++) s.row(FD_GPOR + k)[a] = 0.0;
-            }
-            s.row(FD_POR)[a] = p;
-        }
-    }
-}
-
-/* (m/shep, fdrag) of every DEM particle for the DEM->SPH drag (sph.h:1359) */
-__global__ void k_pack_dem_drag(DevState s, const float *__restrict__ shep32, const float4 *__restrict__ P1,
-                                float4 *__restrict__ DP, int64_t n) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (s.irow(FI_IAM)[i] != T_DEM) return;
-    /* the Shepard sum was accumulated in FP32 by k_couple<.., 0> */
-    const float sh = shep32[i];
-    s.row(FD_SHEP)[i] = sh;
-    DP[i] = make_float4(sh != 0.f ? P1[i].w / sh : 0.f, (float)s.row(FD_FDRAG)[i], (float)s.row(FD_FDRAG + 1)[i],
-                        (float)s.row(FD_FDRAG + 2)[i]);
-}
-
-/* exclusive prefix of v over the warp; *total = the sum */
-__device__ __forceinline__ int warp_excl_scan(int v, int lane, int *total) {
-    int x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
-    *total = __shfl_sync(0xffffffffu, x, 31);
-    return x - v;
-}
-
-/* the lane whose range holds flat index j: the last lane with excl <= j */
-__device__ __forceinline__ int warp_range_src(int excl, int j) {
-    int src = 0;
-#pragma unroll
-    for (int step = 16; step > 0; step >>= 1) {
-        const int e = __shfl_sync(0xffffffffu, excl, src + step);
-        if (e <= j) src += step;
-    }
-    return src;
-}
-
-/* One DEM-DEM contact in FP64 (calcDEMContacts, sph.h:1676-1706): the
- * overlap (Ra + Rb) - r cancels, so r and the spring-dashpot force are FP64 */
-template <int ND>
-__device__ __noinline__ bool dem_contact(const DevCfg *__restrict__ cp, const DevState s, int a, int b,
-                                         const int *sh, double *fc) {
-    const double Ra = s.row(FD_RADIUS)[a] > 0 ? s.row(FD_RADIUS)[a] : cp->dem_radius;
-    const double Rb = s.row(FD_RADIUS)[b] > 0 ? s.row(FD_RADIUS)[b] : cp->dem_radius;
-    double dx[3] = {0, 0, 0}, r = 0.0;
-#pragma unroll
-    for (int k = 0; k < ND; k++) {
-        dx[k] = s.row(FD_R + k)[a] - image_pos(s.row(FD_R + k)[b], sh[k], cp->rmin[k], cp->rmax[k]);
-        r += dx[k] * dx[k];
-    }
-    r = sqrt(r);
-    const double overlap = (Ra + Rb) - r;
-    if (!(overlap > 0.0)) return false;
-    const double ma = s.row(FD_MASS)[a];
-    double odot = 0.0;
-#pragma unroll
-    for (int k = 0; k < ND; k++) odot -= (s.row(FD_VHAT + k)[a] - s.row(FD_VHAT + k)[b]) * (dx[k] / r);
-    const double sN = cp->dem_k * overlap + cp->dem_gamma * odot;
-#pragma unroll
-    for (int k = 0; k < ND; k++) fc[k] += (sN * (dx[k] / r)) / ma;
-    return true;
-}
-
-/* TAP: a warp's passing candidates of one round go to the owner's fixed
- * slots (out, per of them) in lane order; every lane calls it once per
- * round of the warp-uniform candidate loop */
-__device__ __forceinline__ void tap_flush(bool &hit, int &ent, int *out, int per, int &k) {
-    const unsigned m = __ballot_sync(0xffffffffu, hit);
-    const int pos = k + __popc(m & ((1u << (threadIdx.x & 31)) - 1u));
-    if (hit && out && pos < per) out[pos] = ent;
-    k += __popc(m);
-    hit = false;
-}
-
-/* Update of DEM particle a from its warp-reduced FPI and contact sums
- * (calcFPI normalisation, sph.h:1708-1792; Di Felice drag, sph.h:1575-1631,
- * with the drag coefficient in FP32); state accumulation in FP64 */
-template <int ND>
-__device__ __noinline__ void dem_end_update(const DevCfg *__restrict__ cp, const DevState s, int a, float sum,
-                                            float por, const float *fpfb, const float *fv, const float *fvel,
-                                            const double *fc) {
-    double f[3] = {0, 0, 0}, fpv[3] = {0, 0, 0};
-    float vel[3] = {0.f, 0.f, 0.f}, fdrag_out[3] = {0.f, 0.f, 0.f};
-    float pr = por;
-#pragma unroll
-    for (int k = 0; k < ND; k++) {
-        f[k] = s.row(FD_F + k)[a];
-        fpv[k] = s.row(FD_FP + k)[a];
-        vel[k] = fvel[k];
-    }
-    if (sum > 0.5f) {
-        const float rsum = 1.f / sum;
-        float fpfbd[3] = {0.f, 0.f, 0.f}, fvd[3] = {0.f, 0.f, 0.f};
-#pragma unroll
-        for (int k = 0; k < ND; k++) {
-            fpfbd[k] = fpfb[k] * rsum;
-            fvd[k] = fv[k] * rsum;
-            vel[k] *= rsum;
-            s.row(FD_FB + k)[a] = fpfbd[k];
-            s.row(FD_FV + k)[a] = fvd[k];
-        }
-        pr *= rsum;
-        float dv[3] = {0.f, 0.f, 0.f}, vd2 = 0.f;
-#pragma unroll
-        for (int k = 0; k < ND; k++) {
-            dv[k] = pr * (vel[k] - (float)s.row(FD_VHAT + k)[a]);
-            vd2 += dv[k] * dv[k];
-        }
-        const float vdiff = sqrtf(vd2);
-        float fdv[3] = {0.f, 0.f, 0.f};
-        if (vdiff != 0.f) {
-            const float A = (float)(cp->pi * (cp->dem_radius * cp->dem_radius));
-            const float Re = (float)(2.0 * cp->dem_radius / cp->viscosity) * vdiff;
-            const float lg = 1.5f - log10f(Re);
-            const float dragGamma = 3.7f - 0.65f * expf(-(lg * lg) / 2.f);
-            const float cc0 = 0.63f + 4.8f / sqrtf(Re);
-            const float sc = 0.5f * A * (cc0 * cc0) * vdiff;
-            const float pw = powf(pr, -dragGamma) * (float)cp->drag_scale;
-#pragma unroll
-            for (int k = 0; k < ND; k++) fdv[k] = sc * dv[k] * pw;
-        }
-        const double ma = s.row(FD_MASS)[a];
-        const float vm = (float)(cp->dem_vol / ma), dm = (float)(cp->dens / ma);
-#pragma unroll
-        for (int k = 0; k < ND; k++) {
-            fdrag_out[k] = vm * (fvd[k] + fpfbd[k]) + dm * fdv[k];
-            f[k] += fdrag_out[k];
-        }
-    }
-    for (int k = 0; k < 3; k++) {
-        s.row(FD_FVEL + k)[a] = vel[k];
-        s.row(FD_FDRAG + k)[a] = fdrag_out[k];
-    }
-    s.row(FD_POR)[a] = pr;
-    s.row(FD_SHEP)[a] = sum;
-#pragma unroll
-    for (int k = 0; k < ND; k++) {
-        s.row(FD_F + k)[a] = f[k] + fc[k];
-        s.row(FD_FP + k)[a] = fpv[k] + fc[k];
-    }
-}
-
-/* ---------------------------------------------------------------------- */
-/* calcFPI + calcParticleDrag + calcDEMContacts, one warp per DEM particle.
- * The candidates of the 3^d SPH buckets and of the 3^d DEM buckets come from
- * range tables (one lane per bucket run, all loaded at once) and are spread
- * flat over the lanes; sums are reduced over the warp.  Contacts (the overlap
- * 2R - r cancels) and the state update are FP64; the Di Felice drag
- * coefficient is FP32. */
-/* TAP (adjoint replay only): the FPI partners and the contacts with positive
- * overlap of each DEM particle also go to the tap tables tf / tct of step
- * *tslot (DEM particle w of the DEM range owns slots w * per). */
-template <int ND, bool TAP>
-__global__ void __launch_bounds__(BLK) k_dem_end(DevCfg c, const DevCfg *__restrict__ cp, DevState s,
-                                                 const int *__restrict__ start, const int *__restrict__ skey,
-                                                 const DevGlobals *__restrict__ g, const float4 *__restrict__ P0,
-                                                 const float4 *__restrict__ P1, const float4 *__restrict__ P2,
-                                                 const float4 *__restrict__ Q0, const float4 *__restrict__ Q1,
-                                                 const float4 *__restrict__ Q2, const int *__restrict__ tg,
-                                                 const float4 *__restrict__ DS, TapTable tf, TapTable tct,
-                                                 const int *__restrict__ tslot, int64_t n_all) {
-    constexpr int Z = ND - 1;
-    constexpr unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    const int warps = (blockDim.x >> 5) * gridDim.x;
-    const int nsc = g->n_sph_cells;
-    const int dem0 = start[nsc], dem1 = start[nsc + c.n_dem_cells];
-    const int sdims[3] = {g->sdims[0], g->sdims[1], g->sdims[2]};
-    float cell[3], dcellf[3];
-    load_cell32(c, g, cell);
-    float cs2 = 0.f, cd2 = 0.f;
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-        dcellf[d] = (float)c.dcell[d];
-        if (d < ND) {
-            cs2 = fmaxf(cs2, 4.f * cell[d] * cell[d]);
-            cd2 = fmaxf(cd2, 4.f * dcellf[d] * dcellf[d]);
-        }
-    }
-    const float wcon = (float)c.wcon;
-    for (int a = dem0 + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5); a < dem1; a += warps) {
-        if ((tg[a] & 0xff) != T_DEM) continue;
-        const float4 pa = P0[a];
-        const float ha = pa.w;
-        /* tap state: this lane's pending entry, entries so far, owner slots */
-        bool thit = false;
-        int tent = 0, kf = 0, kc = 0, js = 0;
-        int *fout = nullptr, *cout = nullptr;
-        if (TAP) {
-            js = *tslot;
-            const int64_t w = a - dem0;
-            if ((w + 1) * tf.per <= tf.cap) fout = tf.nb + (int64_t)js * tf.cap + w * tf.per;
-            if ((w + 1) * tct.per <= tct.cap) cout = tct.nb + (int64_t)js * tct.cap + w * tct.per;
-        }
-        /* FPI over the SPH candidates: this particle in its SPH bucket's frame */
-        const float4 ds = DS[a];
-        int cs[3] = {0, 0, 0};
-        decode<ND>(__float_as_int(ds.w), sdims, cs);
-        const float oa[3] = {ds.x, ds.y, ds.z};
-        float sum = 0.f, por = 0.f;
-        float fpfb[3] = {0, 0, 0}, fv[3] = {0, 0, 0}, fvel[3] = {0, 0, 0};
-        {
-            const RangeEntry re = range_entry<ND>(lane, cs, cs[Z], cs[Z], sdims, c.periodic, cell, 0, start);
-            int total = 0;
-            const int excl = warp_excl_scan(re.cnt, lane, &total);
-            for (int t = 0; t < total; t += 32) {
-                if (TAP) tap_flush(thit, tent, fout, tf.per, kf);
-                const int j = t + lane;
-                const int src = warp_range_src(excl, j);
-                const int b0 = __shfl_sync(FULL, re.b0, src), ex = __shfl_sync(FULL, excl, src);
-                const int lin = __shfl_sync(FULL, re.lin, src), zoff = __shfl_sync(FULL, re.zoff, src);
-                const int shp = __shfl_sync(FULL, re.shp, src);
-                const float ox = __shfl_sync(FULL, re.ox, src), oy = __shfl_sync(FULL, re.oy, src);
-                if (j >= total) continue;
-                const int b = b0 + (j - ex);
-                const float4 pb = P0[b];
-                const int zrel = zoff + (skey[b] - lin);
-                float qv[3] = {pb.x, pb.y, pb.z};
-                if (Z > 0) qv[0] += ox;
-                if (Z > 1) qv[1] += oy;
-                qv[Z] += (float)zrel * cell[Z];
-                const float d0 = oa[0] - qv[0];
-                const float d1 = ND > 1 ? oa[1] - qv[1] : 0.f;
-                const float d2 = ND > 2 ? oa[2] - qv[2] : 0.f;
-                const float r2 = fmaf(d2, d2, fmaf(d1, d1, d0 * d0));
-                const float tt = 2.f * fmaxf(ha, pb.w);
-                const float T = tt * tt;
-                const float band = fp32_band(T, cs2);
-                if (r2 > T + band) continue;
-                const int sh[3] = {(shp & 3) - 1, ((shp >> 2) & 3) - 1, ((shp >> 4) & 3) - 1};
-                if (r2 >= T - band && !exact_pair<ND>(cp, s, a, b, sh[0], sh[1], sh[2], 0.0, 0)) continue;
-                const int tgb = tg[b];
-                if (shp != 0x15 && !img_ok<ND>(tgb >> 8, sh)) continue;
-                if ((tgb & 0xff) == T_BOUNDARY) continue;
-                const float4 vb = P1[b], xb = P2[b];
-                const float mb = fabsf(vb.w);
-                const float q = sqrtf(r2) * xb.w;
-                const float Wab = powi<ND>(xb.w) * wK32(q, wcon);
-                const float dvW = (mb / xb.x) * Wab, mW = mb * Wab;
-                const float4 q0 = Q0[b], q1 = Q1[b];
-                const float fvb[3] = {q0.w, q1.x, q1.y};
-                const float fb_[3] = {q0.x, q0.y, q0.z};
-#pragma unroll
-                for (int k = 0; k < ND; k++) {
-                    fpfb[k] += mW * fb_[k];
-                    fv[k] += mW * fvb[k] + dvW * fvb[k];
-                }
-                fvel[0] += dvW * vb.x;
-                fvel[1] += dvW * vb.y;
-                fvel[2] += dvW * vb.z;
-                por += dvW * xb.z;
-                sum += dvW;
-                if (TAP) {
-                    thit = true;
-                    tent = s.irow(FI_TAG)[b] | (shp << B_BITS);
-                }
-            }
-            if (TAP) tap_flush(thit, tent, fout, tf.per, kf);
-        }
-        sum = warp_sum(sum);
-        por = warp_sum(por);
-#pragma unroll
-        for (int k = 0; k < ND; k++) {
-            fpfb[k] = warp_sum(fpfb[k]);
-            fv[k] = warp_sum(fv[k]);
-            fvel[k] = warp_sum(fvel[k]);
-        }
-        /* DEM contacts over the DEM grid (sph.h:1676-1706), FP64 per contact */
-        int cdm[3] = {0, 0, 0};
-        decode<ND>(skey[a] - nsc, c.ddims, cdm);
-        const float od[3] = {pa.x, pa.y, pa.z};
-        const float Ra_f = P2[a].y;
-        double fc[3] = {0, 0, 0};
-        {
-            const RangeEntry re = range_entry<ND>(lane, cdm, cdm[Z], cdm[Z], c.ddims, c.periodic, dcellf, nsc, start);
-            int total = 0;
-            const int excl = warp_excl_scan(re.cnt, lane, &total);
-            for (int t = 0; t < total; t += 32) {
-                if (TAP) tap_flush(thit, tent, cout, tct.per, kc);
-                const int j = t + lane;
-                const int src = warp_range_src(excl, j);
-                const int b0 = __shfl_sync(FULL, re.b0, src), ex = __shfl_sync(FULL, excl, src);
-                const int lin = __shfl_sync(FULL, re.lin, src), zoff = __shfl_sync(FULL, re.zoff, src);
-                const int shp = __shfl_sync(FULL, re.shp, src);
-                const float ox = __shfl_sync(FULL, re.ox, src), oy = __shfl_sync(FULL, re.oy, src);
-                if (j >= total) continue;
-                const int b = b0 + (j - ex);
-                if (b == a && shp == 0x15) continue;
-                const int tgb = tg[b];
-                if ((tgb & 0xff) != T_DEM) continue;
-                const float4 pb = P0[b];
-                const int zrel = zoff + (skey[b] - lin);
-                float qv[3] = {pb.x, pb.y, pb.z};
-                if (Z > 0) qv[0] += ox;
-                if (Z > 1) qv[1] += oy;
-                qv[Z] += (float)zrel * dcellf[Z];
-                const float d0 = od[0] - qv[0];
-                const float d1 = ND > 1 ? od[1] - qv[1] : 0.f;
-                const float d2 = ND > 2 ? od[2] - qv[2] : 0.f;
-                const float r2 = fmaf(d2, d2, fmaf(d1, d1, d0 * d0));
-                const float tt = 2.f * fmaxf(ha, pb.w);
-                const float T = tt * tt;
-                const float band = fp32_band(T, cd2);
-                if (r2 > T + band) continue;
-                const int sh[3] = {(shp & 3) - 1, ((shp >> 2) & 3) - 1, ((shp >> 4) & 3) - 1};
-                if (r2 >= T - band && !exact_pair<ND>(cp, s, a, b, sh[0], sh[1], sh[2], 0.0, 0)) continue;
-                if (shp != 0x15 && !img_ok<ND>(tgb >> 8, sh)) continue;
-                if ((Ra_f + P2[b].y) * 1.0001f - sqrtf(r2) <= 0.f) continue;
-                const bool touch = dem_contact<ND>(cp, s, a, b, sh, fc);
-                if (TAP && touch) {
-                    thit = true;
-                    tent = s.irow(FI_TAG)[b] | (shp << B_BITS);
-                }
-            }
-            if (TAP) tap_flush(thit, tent, cout, tct.per, kc);
-        }
-        if (TAP && lane == 0) {
-            const int64_t w = a - dem0, at = (int64_t)js * n_all + s.irow(FI_TAG)[a];
-            tf.oc[at] = make_int2((int)(w * tf.per), fout && kf <= tf.per ? kf : 0);
-            if (!fout || kf > tf.per) atomicMax(tf.cnt + js, (int)tf.cap + 1);   /* marks the step overflowed */
-            tct.oc[at] = make_int2((int)(w * tct.per), cout && kc <= tct.per ? kc : 0);
-            if (!cout || kc > tct.per) atomicMax(tct.cnt + js, (int)tct.cap + 1);
-        }
-#pragma unroll
-        for (int k = 0; k < ND; k++)
-            for (int oo = 16; oo > 0; oo >>= 1) fc[k] += __shfl_xor_sync(FULL, fc[k], oo);
-        if (lane == 0) dem_end_update<ND>(cp, s, a, sum, por, fpfb, fv, fvel, fc);
-    }
-}
-
 /* rows of the neighbour list in tag order (count pass when idx == nullptr) */
 __global__ void k_list_export(DevState s, const int *tg, const int *nbr, const int *ncnt, int64_t ld, int64_t n,
                               int *cnt, const long long *offs, int *idx) {
@@ -2049,35 +1085,6 @@ __global__ void k_adj_pairs(DevState s, const DevGlobals *__restrict__ g, const 
     oc[(int64_t)js * n + s.irow(FI_TAG)[a]] = make_int2((int)off, room >= k ? k : 0);
 }
 
-int warp_blocks(int items) { return std::max(1, std::min(1 << 16, (items + (BLK / 32) - 1) / (BLK / 32))); }
-/* coupling passes: grid-stride over 32-particle slices, one wave of resident blocks */
-template <int ND, int MODE>
-int resident_blocks(int64_t particles) {
-    static int resident = 0;
-    if (!resident) {
-        int dev = 0, sms = 0, per_sm = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_couple<ND, MODE, false>, CP_WARPS * 32, 0);
-        resident = std::max(1, sms * per_sm);
-    }
-    const int64_t need = (particles + 32 * CP_WARPS - 1) / (32 * CP_WARPS);
-    return (int)std::max<int64_t>(1, std::min<int64_t>(resident, need));
-}
-
-template <int ND>
-int dem_end_blocks(int64_t particles) {
-    static int resident = 0;
-    if (!resident) {
-        int dev = 0, sms = 0, per_sm = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_dem_end<ND, false>, BLK, 0);
-        resident = std::max(1, sms * per_sm);
-    }
-    return std::max(1, std::min(resident, warp_blocks((int)std::min<int64_t>(particles, 1 << 22))));
-}
-
 /* list build: grid-stride over 32-particle slices, one wave of resident blocks */
 template <int ND, bool COUNT, int G>
 int nlist_blocks(int64_t particles) {
@@ -2115,42 +1122,15 @@ void mixed_adj_pairs(sphdem_ctx *c, int *nb, int2 *oc, int *cnt, int64_t cap, co
 }
 
 /* ---------------------------------------------------------------------- */
-#define SPHDEM_ND_DISPATCH(nd, F) \
-    do {                          \
-        if ((nd) == 3) {          \
-            F(3);                 \
-        } else if ((nd) == 2) {   \
-            F(2);                 \
-        } else {                  \
-            F(1);                 \
-        }                         \
-    } while (0)
 
 namespace mixed {
 
 void pack(sphdem_ctx *c, bool middle) {
-    const bool coupling = middle && c->cfg.liq_dem();
 #define L_(ND)                                                                                                  \
     SPHDEM_LAUNCH(c, "pack32", k_pack<ND>, grid_for(c->n, 256), 256, 0, c->cfg, c->A, c->buf.skey, c->g,         \
-                  c->mx_pos, c->mx_vel, c->mx_aux, c->mx_tg, c->mx_rc4, (int)coupling, (int)middle, c->mx_ds,      \
-                  c->mx_nb, c->n)
+                  c->mx_pos, c->mx_vel, c->mx_aux, c->mx_tg, (int)middle, c->mx_ds, c->mx_nb, c->n)
     SPHDEM_ND_DISPATCH(c->cfg.nd, L_);
 #undef L_
-    if (coupling) {
-#define L_(ND)                                                                                                  \
-    SPHDEM_LAUNCH(c, "couple_win", k_win<ND>, grid_for(3 * (int64_t)c->mx_win_cap, 256), 256, 0, c->cfg, c->g,   \
-                  c->mx_win, c->mx_win_cap)
-        SPHDEM_ND_DISPATCH(c->cfg.nd, L_);
-#undef L_
-    }
-}
-
-void zero_shep(sphdem_ctx *c) {
-    SPHDEM_CUDA_CHECK(cudaMemsetAsync(c->mx_shep32, 0, c->n * sizeof(float), c->stream));
-}
-
-void pack_fpi(sphdem_ctx *c) {
-    SPHDEM_LAUNCH(c, "pack_fpi32", k_pack_fpi, grid_for(c->n, 256), 256, 0, c->A, c->mx_q0, c->mx_q1, c->mx_q2, c->n);
 }
 
 void nlist(sphdem_ctx *c, int depth, bool soft) {
@@ -2282,59 +1262,6 @@ void dddt(sphdem_ctx *c) {
             LD_(3, true, false);
     }
 #undef LD_
-}
-
-/* the porosity (MODE 0) or DEM -> SPH drag (MODE 1) pass; while the
- * adjoint's replay graph is captured, the form that also writes the
- * coupling tap table */
-template <int MODE>
-void couple(sphdem_ctx *c, const char *name) {
-    const TapTable tt = c->tap ? c->tap->cpl : TapTable{};
-    const int *ts = c->tap ? c->tap->slot : nullptr;
-#define L_(ND)                                                                                                  \
-    do {                                                                                                        \
-        const int nb_ = std::max(1, resident_blocks<ND, MODE>(c->n) / c->grid_div);                             \
-        if (c->tap)                                                                                             \
-            SPHDEM_LAUNCH(c, name, (k_couple<ND, MODE, true>), nb_, CP_WARPS * 32, 0, c->cfg, c->dcfg, c->A,      \
-                          c->buf.start, c->buf.skey, c->g, c->mx_pos, c->mx_vel, c->mx_aux, c->mx_dp, c->mx_tg,   \
-                          c->mx_rc4, c->mx_win, c->mx_win_cap, c->mx_shep32, tt, ts, c->n);                       \
-        else                                                                                                    \
-            SPHDEM_LAUNCH(c, name, (k_couple<ND, MODE, false>), nb_, CP_WARPS * 32, 0, c->cfg, c->dcfg, c->A,     \
-                          c->buf.start, c->buf.skey, c->g, c->mx_pos, c->mx_vel, c->mx_aux, c->mx_dp, c->mx_tg,   \
-                          c->mx_rc4, c->mx_win, c->mx_win_cap, c->mx_shep32, tt, ts, c->n);                       \
-    } while (0)
-    SPHDEM_ND_DISPATCH(c->cfg.nd, L_);
-#undef L_
-}
-
-void porosity(sphdem_ctx *c) { couple<0>(c, "porosity32"); }
-
-void dem_drag(sphdem_ctx *c) {
-    SPHDEM_LAUNCH(c, "pack_dem_drag32", k_pack_dem_drag, grid_for(c->n, 256), 256, 0, c->A, c->mx_shep32, c->mx_vel,
-                  c->mx_dp, c->n);
-    couple<1>(c, "dem_drag32");
-}
-
-void dem_end(sphdem_ctx *c) {
-    pack_fpi(c);
-    /* one warp per DEM particle, grid-stride over the DEM range: one wave of
-     * resident blocks (a grid sized by the particle count would launch
-     * mostly empty warps) */
-    const TapTable tf = c->tap ? c->tap->fpi : TapTable{}, tct = c->tap ? c->tap->ct : TapTable{};
-    const int *ts = c->tap ? c->tap->slot : nullptr;
-#define L_(ND)                                                                                                  \
-    do {                                                                                                        \
-        if (c->tap)                                                                                             \
-            SPHDEM_LAUNCH(c, "dem_end32", (k_dem_end<ND, true>), dem_end_blocks<ND>(c->n), BLK, 0, c->cfg,        \
-                          c->dcfg, c->A, c->buf.start, c->buf.skey, c->g, c->mx_pos, c->mx_vel, c->mx_aux,        \
-                          c->mx_q0, c->mx_q1, c->mx_q2, c->mx_tg, c->mx_ds, tf, tct, ts, c->n);                   \
-        else                                                                                                    \
-            SPHDEM_LAUNCH(c, "dem_end32", (k_dem_end<ND, false>), dem_end_blocks<ND>(c->n), BLK, 0, c->cfg,       \
-                          c->dcfg, c->A, c->buf.start, c->buf.skey, c->g, c->mx_pos, c->mx_vel, c->mx_aux,        \
-                          c->mx_q0, c->mx_q1, c->mx_q2, c->mx_tg, c->mx_ds, tf, tct, ts, c->n);                   \
-    } while (0)
-    SPHDEM_ND_DISPATCH(c->cfg.nd, L_);
-#undef L_
 }
 
 }  // namespace mixed

@@ -1,6 +1,8 @@
 /*
- * FP64 pair passes: the reference arithmetic of every neighbour functor of
- * the hot path, one thread per target particle over the sorted bucket lists.
+ * FP64 EOS and DEM time step, and the coupling and contact passes of an FP64
+ * handle whose lengths lie outside FP32's range, so that it has no FP32 records
+ * to search (coupling.cu): one thread per target particle over the buckets,
+ * every candidate tested in FP64.
  *
  *   k_porosity  calcPorosity + calcShepSum        sph.h:1323-1341, 1303-1320
  *   k_dem_drag  calcDEMtoSPHDrag + finalisePorosity + setPorosityForBoundary
@@ -287,10 +289,18 @@ void zero_dem_shep(sphdem_ctx *c) {
     SPHDEM_LAUNCH(c, "zero_dem_shep", k_zero_dem_shep, grid_for(c->n, 256), 256, 0, c->A, c->n);
 }
 void run_porosity(sphdem_ctx *c) {
+    if (c->f64_dem) {
+        if (!c->only_dem) couple64(c, 0);
+        return;
+    }
     zero_dem_shep(c);
     SPHDEM_LAUNCH(c, "porosity_fp64", k_porosity, grid_for(c->n, BLK), BLK, 0, c->cfg, c->A, c->buf.start, c->g, c->n);
 }
 void run_dem_drag(sphdem_ctx *c) {
+    if (c->f64_dem) {
+        if (!c->only_dem) couple64(c, 1);
+        return;
+    }
     SPHDEM_LAUNCH(c, "dem_drag_fp64", k_dem_drag, grid_for(c->n, BLK), BLK, 0, c->cfg, c->A, c->buf.start, c->g, c->n);
 }
 void run_eos(sphdem_ctx *c) {
@@ -300,6 +310,10 @@ void run_dem_accel(sphdem_ctx *c) {
     SPHDEM_LAUNCH(c, "dem_accel", k_dem_accel, grid_for(c->n, BLK), BLK, 0, c->cfg, c->A, c->g, c->n);
 }
 void run_dem_end(sphdem_ctx *c) {
+    if (c->f64_dem) {
+        dem_end64(c, !c->only_dem);
+        return;
+    }
     SPHDEM_LAUNCH(c, "dem_end_fp64", k_dem_end, grid_for(c->n, BLK), BLK, 0, c->cfg, c->A, c->buf.start, c->g, c->n);
 }
 

@@ -142,6 +142,7 @@ int insert_particles(sphdem_ctx *c, const SphDemParticles *in, int64_t *out_idx)
     SPHDEM_CUDA_CHECK(cudaFreeAsync(d_slot, c->stream));
     SPHDEM_CUDA_CHECK(cudaStreamSynchronize(c->stream));
     c->n = next;
+    for (int64_t j = 0; j < k; j++) c->only_dem = c->only_dem && in->iam[j] == T_DEM;
     population_changed(c);
     if (out_idx) std::copy(slot.begin(), slot.end(), out_idx);
     return SPHDEM_OK;

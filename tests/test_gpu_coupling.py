@@ -1,0 +1,96 @@
+"""Coupling and contact passes at the edges of their queues and splits (-m
+gpu): more partners per fluid particle than a queue or the kept pairs hold,
+populations on both sides of the four-threads rule, contacts beyond a lane's
+queue, DEM without fluid.  Checked against the CPU oracle (FP64, 1e-11 of each
+field's 2-norm: sums of some hundred terms in another order) and, for mixed
+precision, against the FP64 path (FP32 terms of ~20 roundings, 1.2e-5)."""
+import numpy as np
+import pytest
+
+from oracle.port_api import OracleSim
+from sphdem import capi, cases
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def lib():
+    import __graft_entry__
+    __graft_entry__.build()
+    return capi.Library()
+
+
+def dense_bed(nx, spacing, seed=4):
+    """A sediment box whose upper half holds spheres `spacing` diameters apart
+    on a jittered lattice (spacing < 1: every sphere in contact)."""
+    case = cases.sediment3d(nx=nx, L=0.0025 * nx, height=0.005 * nx, n_dem=1)
+    p, cfg = case.particles, case.cfg
+    R, L = cfg["dem_radius"], cfg["rmax"][0]
+    m = int(L / (2 * R * spacing))
+    k = max(2, int((0.5 * cfg["rmax"][2] - 4 * R) / (2 * R * spacing)))
+    rng = np.random.default_rng(seed)
+    q = np.stack(np.meshgrid(np.arange(m), np.arange(m), np.arange(k), indexing="ij"), -1).reshape(-1, 3)
+    r = (q + 0.5) * np.array([L / m, L / m, 2 * R * spacing]) + rng.uniform(-0.02 * R, 0.02 * R, q.shape)
+    r[:, 2] += 0.5 * cfg["rmax"][2] + R
+    r[:, :2] %= L
+    n = len(r)
+    out = {key: np.concatenate([v[:-1], np.repeat(v[-1:], n, axis=0)]) for key, v in p.items()}
+    out["r"][-n:] = r
+    out["v"][-n:] = 0.02 * rng.standard_normal((n, 3))
+    out["tag"] = np.arange(1, out["iam"].size + 1, dtype=np.int32)
+    # the pore pressure at rest: the spheres take a good part of the volume
+    fluid = (out["iam"] == cases.SPH) & (out["r"][:, 2] > 0.5 * cfg["rmax"][2])
+    out["dens"][fluid] *= 1.0 - n * cfg["dem_vol"] / (L * L * 0.5 * cfg["rmax"][2])
+    return cfg, out
+
+
+FIELDS = ("f", "fp", "fdrag", "fvel", "porosity", "dporositydt", "grad_porosity", "shep_sum", "dddt")
+
+
+def norm_gap(a, b):
+    n = np.linalg.norm(b)
+    return np.linalg.norm(a - b) / n if n > 0 else np.linalg.norm(a)
+
+
+@pytest.mark.parametrize("spacing", [0.98, 1.3, 2.5])
+def test_dense_suspension_equals_oracle(lib, spacing):
+    cfg, p = dense_bed(12, spacing)
+    ora = OracleSim(cfg, p)
+    ora.step(1)
+    want = ora.get()
+    sim = capi.Simulation(lib, cfg, p, precision=cases.PREC_FP64)
+    sim.step(1)
+    got = sim.get()
+    for k in FIELDS:
+        assert norm_gap(got[k], want[k]) <= 1e-11, k
+
+
+@pytest.mark.parametrize("nx,spacing", [(12, 0.98), (30, 1.1), (32, 1.1)])
+def test_mixed_coupling_equals_fp64(lib, nx, spacing):
+    cfg, p = dense_bed(nx, spacing)
+    got = []
+    for prec in (cases.PREC_FP64, cases.PREC_MIXED):
+        sim = capi.Simulation(lib, cfg, p, precision=prec)
+        sim.step(1)
+        a = sim.get()
+        got.append({k: a[k].copy() for k in FIELDS})
+        sim.close()
+    for k in FIELDS:
+        assert norm_gap(got[1][k], got[0][k]) <= 1.2e-5, k
+
+
+@pytest.mark.parametrize("precision", [cases.PREC_FP64, cases.PREC_MIXED])
+def test_crowded_contacts_without_fluid(lib, precision):
+    """Spheres squeezed to half a diameter: more contacts per lane than its
+    queue holds (FP64 on both handles)."""
+    case = cases.dem_settling3d(lattice=(6, 6, 10), box=(0.0138, 0.0138, 0.023), spread=0.0, vel_amp=0.1)
+    p = case.particles
+    p["r"][:] = p["r"].mean(axis=0) + 0.45 * (p["r"] - p["r"].mean(axis=0))
+    ora = OracleSim(case.cfg, p)
+    ora.step(1)
+    want = ora.get()
+    sim = capi.Simulation(lib, case.cfg, p, precision=precision)
+    sim.step(1)
+    got = sim.get()
+    for k in ("f", "fp", "v", "r", "fdrag", "shep_sum"):
+        assert norm_gap(got[k], want[k]) <= 1e-11, k
