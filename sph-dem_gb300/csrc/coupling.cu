@@ -449,10 +449,15 @@ __device__ __forceinline__ R warp_sum16(R *v, int lane) {
 
 /* calcFPI's sums, one warp per DEM particle.  Candidates of the 3^d SPH buckets
  * come from a range table (one lane per bucket run) and are spread flat over the
- * lanes; partners are queued and taken 32 at a time.  The unnormalised sums go
+ * lanes; a lane queues its partners and the warp takes one of each lane at a
+ * time.  (A queue of the warp instead, taken 32 partners at a time, runs at full
+ * lanes but adds in another order, and the partial sums of a particle at rest in
+ * a swarm under drag cancel: its path over 10 steps moved by up to 2e-9 of the box.)
+ * The unnormalised sums go
  * to the particle's fvel, porosity and Shepard rows and, where calcFPI normalises
  * (Shepard sum > 0.5), its fb and fv rows.  TAP: the partners of DEM particle w
  * of the DEM range also go to slots w * per .. of table tf of step *tslot. */
+constexpr int FPI_QUEUE = 8;
 template <int ND, typename R, bool TAP>
 __global__ void __launch_bounds__(BLK) k_fpi(DevCfg c, const DevCfg *__restrict__ cp, DevState s,
                                              const int *__restrict__ start, const int *__restrict__ skey,
@@ -464,9 +469,8 @@ __global__ void __launch_bounds__(BLK) k_fpi(DevCfg c, const DevCfg *__restrict_
     constexpr int Z = ND - 1;
     constexpr unsigned FULL = 0xffffffffu;
     constexpr bool F64 = sizeof(R) == 8;
-    __shared__ int s_queue[BLK / 32][64];
+    __shared__ int s_queue[FPI_QUEUE][BLK];
     const int lane = threadIdx.x & 31;
-    int *const queue = s_queue[threadIdx.x >> 5];
     const int warps = (blockDim.x >> 5) * gridDim.x;
     const int nsc = g->n_sph_cells;
     const int dem0 = start[nsc], dem1 = start[nsc + c.n_dem_cells];
@@ -497,12 +501,20 @@ __global__ void __launch_bounds__(BLK) k_fpi(DevCfg c, const DevCfg *__restrict_
 #pragma unroll
         for (int k = 0; k < 16; k++) v[k] = 0;
         int qn = 0;
-        /* the terms of `m` queued partners */
-        auto take = [&](int m) {
-            __syncwarp();
-            if (lane < m) {
-                const int id = queue[lane], b = id & B_MASK, shp = (unsigned)id >> B_BITS;
-                if (TAP && fout && kf + lane < tf.per) fout[kf + lane] = s.irow(FI_TAG)[b] | (id & ~B_MASK);
+        /* the terms of the queued partners */
+        auto take = [&]() {
+            for (int t = 0; __any_sync(FULL, t < qn); t++) {
+                if (TAP) {
+                    const unsigned m = __ballot_sync(FULL, t < qn);
+                    const int at = kf + __popc(m & ((1u << lane) - 1u));
+                    if (t < qn && fout && at < tf.per) {
+                        const int id = s_queue[t][threadIdx.x];
+                        fout[at] = s.irow(FI_TAG)[id & B_MASK] | (id & ~B_MASK);
+                    }
+                    kf += __popc(m);
+                }
+                if (t >= qn) continue;
+                const int id = s_queue[t][threadIdx.x], b = id & B_MASK, shp = (unsigned)id >> B_BITS;
                 if constexpr (F64) {
                     double d[3] = {0, 0, 0};
                     pair_dx<ND>(c, s, ra, b, shp, d);
@@ -549,13 +561,7 @@ __global__ void __launch_bounds__(BLK) k_fpi(DevCfg c, const DevCfg *__restrict_
                     v[10] += dvW;
                 }
             }
-            if (TAP) kf += m;
-            /* the rest moves to the front */
-            int e = 0;
-            if (lane < qn - m) e = queue[m + lane];
-            __syncwarp();
-            if (lane < qn - m) queue[lane] = e;
-            qn -= m;
+            qn = 0;
         };
         const RangeEntry re = range_entry<ND>(lane, cs, cs[Z], cs[Z], sdims, c.periodic, cell, 0, start);
         int total = 0;
@@ -589,12 +595,10 @@ __global__ void __launch_bounds__(BLK) k_fpi(DevCfg c, const DevCfg *__restrict_
                           (r2 < T - band || exact_pair<ND>(cp, s, a, b, sh[0], sh[1], sh[2], 0.0, 0));
                 }
             }
-            const unsigned m = __ballot_sync(FULL, hit);
-            if (hit) queue[qn + __popc(m & ((1u << lane) - 1u))] = b | (shp << B_BITS);
-            qn += __popc(m);
-            if (qn >= 32) take(32);
+            if (hit) s_queue[qn++][threadIdx.x] = b | (shp << B_BITS);
+            if (__any_sync(FULL, qn == FPI_QUEUE)) take();
         }
-        if (qn) take(qn);
+        take();
         if (TAP && lane == 0) {
             const int64_t w = a - dem0, at = (int64_t)js * n_all + s.irow(FI_TAG)[a];
             tf.oc[at] = make_int2((int)(w * tf.per), fout && kf <= tf.per ? kf : 0);

@@ -47,9 +47,10 @@ struct Plain {
 struct Kahan2 {
     float2 s, n;
     __device__ __forceinline__ void init() { s = n = make_float2(0.f, 0.f); }
-    __device__ __forceinline__ void add(float2 x) {
+    /* adds a * b; the product is not rounded by itself */
+    __device__ __forceinline__ void add_product(float2 a, float2 b) {
         const float2 neg = make_float2(-1.f, -1.f);
-        const float2 y = __fadd2_rn(x, n);
+        const float2 y = __ffma2_rn(a, b, n);
         const float2 t = __fadd2_rn(s, y);
         n = __ffma2_rn(__ffma2_rn(s, neg, t), neg, y);
         s = t;
