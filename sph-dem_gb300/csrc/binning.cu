@@ -3,14 +3,15 @@
  * (dataLL.cpp:140-236) including the single-rank part of updateDomain
  * (dataLL.cpp:319-700).
  *
- *   k_migrate   periodic wrap / out-of-domain deletion (dataLL.cpp:371-404,
- *               464-516) and the next h_max (calcDomainLimits, 954-975)
- *   k_ghost     which periodic images exist (dataLL.cpp:522-582): the clipped
+ *   k_sweep     (with the elementwise work that precedes the rebuild in a step)
+ *               periodic wrap / out-of-domain deletion (dataLL.cpp:371-404,
+ *               464-516) and the next h_max (calcDomainLimits, 954-975);
+ *               which periodic images exist (dataLL.cpp:522-582): the clipped
  *               inCoords of every particle, against the ghost widths
  *               procGhostMax2H of the previous rebuild (Rc for DEM), and the
- *               per-slot maximum h that sets the next widths (688-693)
- *   k_finalize  new widths, h_max, the search-radius hysteresis (220-223)
- *               and the SPH bucket grid size
+ *               per-slot maximum h that sets the next widths (688-693); the
+ *               last block writes the new widths, h_max, the search-radius
+ *               hysteresis (220-223) and the SPH bucket grid size
  *   k_keys      bucket key of every particle: getCellI (dataLL.h:303-305) on
  *               non-periodic axes, an L/floor(L/2h) grid on periodic axes;
  *               DEM particles go to the DEM search grid
@@ -26,59 +27,12 @@
  * graph.  Roofline: HBM-bound; per particle it reads r (8d B) and writes a
  * key (4 B) twice, then the gather reads+writes every live row.
  */
-#include "internal.cuh"
+#include "elementwise.cuh"
 
 namespace sphdem {
 namespace {
 
 constexpr int BLK = 256;
-
-__global__ void k_migrate(DevCfg c, DevState s, DevGlobals *g, unsigned char *mark, int64_t n) {
-    __shared__ unsigned long long bmax;
-    if (threadIdx.x == 0) bmax = 0ull;
-    __syncthreads();
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    double h = -1.0;
-    if (i < n) {
-        int *iam = s.irow(FI_IAM);
-        if (mark[i]) {
-            /* markForDeletion (tag -111) is honoured first (dataLL.cpp:377-380) */
-            mark[i] = 0;
-            iam[i] = T_DEAD;
-        }
-        if (iam[i] != T_DEAD) {
-            int oc[3] = {1, 1, 1};
-            bool lost = false, out = false;
-            for (int d = 0; d < c.nd; d++) {
-                const double r = s.row(FD_R + d)[i];
-                oc[d] = trunc_index(r, c.dmin[d], c.dspace[d], c.rdspace_f[d], 1.0);
-                if (oc[d] > 2 || oc[d] < 0) lost = true;
-                if (oc[d] != 1) {
-                    out = true;
-                    if (!c.periodic[d]) lost = true;
-                }
-            }
-            if (lost) {
-                iam[i] = T_DEAD;
-                atomicAdd((unsigned long long *)&g->n_deleted, 1ull);
-            } else {
-                if (out) {
-                    for (int d = 0; d < c.nd; d++) {
-                        double *r = s.row(FD_R + d);
-                        if (oc[d] == 2) r[i] = dadd(dsub(c.rmin[d], c.rmax[d]), r[i]);
-                        else if (oc[d] == 0) r[i] = dadd(dsub(c.rmax[d], c.rmin[d]), r[i]);
-                    }
-                }
-                h = s.row(FD_H)[i];
-            }
-        }
-    }
-    /* block maximum of h, then one atomic per block */
-    for (int o = 16; o > 0; o >>= 1) h = fmax(h, __shfl_xor_sync(0xffffffffu, h, o));
-    if ((threadIdx.x & 31) == 0 && h >= 0.0) atomicMax(&bmax, dbits(h));
-    __syncthreads();
-    if (threadIdx.x == 0 && bmax) atomicMax(&g->hmax_bits, bmax);
-}
 
 __device__ __forceinline__ int slot_index(const int *co, int nd) {
     int sidx = 0;
@@ -86,138 +40,256 @@ __device__ __forceinline__ int slot_index(const int *co, int nd) {
     return sidx;
 }
 
-__global__ void k_ghost(DevCfg c, DevState s, DevGlobals *g, int64_t n) {
-    __shared__ unsigned long long smax[27];
-    if (threadIdx.x < 27) smax[threadIdx.x] = 0ull;
-    __syncthreads();
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i < n) {
-        const int t = s.irow(FI_IAM)[i];
-        int gcode = 0;
-        if (t != T_DEAD) {
-            const bool dem = c.liq_dem() && t == T_DEM;
-            int ic[3] = {1, 1, 1};
-            bool any = false;
-            for (int d = 0; d < c.nd; d++) {
-                if (!c.periodic[d]) continue;
-                const double r = s.row(FD_R + d)[i];
-                int v = dem ? trunc_index(r, c.dg_lo[d], c.dg_sp[d], c.dg_rsp_f[d], 1.0)
-                            : trunc_index(r, g->ghost_lo[d], g->ghost_sp[d], g->ghost_rsp_f[d], 1.0);
-                if (v > 2) v = 2;
-                if (v < 0) v = 0;
-                ic[d] = v;
-                any |= v != 1;
-            }
-            for (int d = 0; d < c.nd; d++) gcode |= ic[d] << (2 * d);
-            if (any) {
-                const double h = s.row(FD_H)[i];
-                int lo3[3], hi3[3];
-                for (int d = 0; d < 3; d++) {
-                    lo3[d] = d < c.nd ? min(ic[d], 1) : 1;
-                    hi3[d] = d < c.nd ? max(ic[d], 1) : 1;
-                }
-                for (int a = lo3[0]; a <= hi3[0]; a++)
-                    for (int b = lo3[1]; b <= hi3[1]; b++)
-                        for (int e = lo3[2]; e <= hi3[2]; e++) {
-                            const int dc[3] = {a, b, e};
-                            bool centre = true;
-                            for (int d = 0; d < c.nd; d++) centre &= dc[d] == 1;
-                            if (centre) continue;
-                            int sl[3];
-                            for (int d = 0; d < c.nd; d++) sl[d] = 2 - dc[d];
-                            atomicMax(&smax[slot_index(sl, c.nd)], dbits(h));
-                        }
-            }
-        }
-        s.irow(FI_GCODE)[i] = gcode;
+/* migration of particle i (dataLL.cpp:371-404, 464-516): the particle's type
+ * after it, its h (dead: -1) in *h */
+__device__ __forceinline__ int migrate_particle(const DevCfg &c, const DevState &s, DevGlobals *g, unsigned char *mark,
+                                                int64_t i, int t, double *h) {
+    int *iam = s.irow(FI_IAM);
+    *h = -1.0;
+    if (mark[i]) {
+        /* markForDeletion (tag -111) is honoured first (dataLL.cpp:377-380) */
+        mark[i] = 0;
+        iam[i] = T_DEAD;
+        return T_DEAD;
     }
-    __syncthreads();
-    if (threadIdx.x < 27 && smax[threadIdx.x]) atomicMax(&g->slot_bits[threadIdx.x], smax[threadIdx.x]);
+    if (t == T_DEAD) return t;
+    int oc[3] = {1, 1, 1};
+    bool lost = false, out = false;
+    for (int d = 0; d < c.nd; d++) {
+        const double r = s.row(FD_R + d)[i];
+        oc[d] = trunc_index(r, c.dmin[d], c.dspace[d], c.rdspace_f[d], 1.0);
+        if (oc[d] > 2 || oc[d] < 0) lost = true;
+        if (oc[d] != 1) {
+            out = true;
+            if (!c.periodic[d]) lost = true;
+        }
+    }
+    if (lost) {
+        iam[i] = T_DEAD;
+        atomicAdd((unsigned long long *)&g->n_deleted, 1ull);
+        return T_DEAD;
+    }
+    if (out) {
+        for (int d = 0; d < c.nd; d++) {
+            double *r = s.row(FD_R + d);
+            if (oc[d] == 2) r[i] = dadd(dsub(c.rmin[d], c.rmax[d]), r[i]);
+            else if (oc[d] == 0) r[i] = dadd(dsub(c.rmax[d], c.rmin[d]), r[i]);
+        }
+    }
+    *h = s.row(FD_H)[i];
+    return t;
 }
 
-__global__ void k_finalize(DevCfg c, DevGlobals *g) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+/* ghost images of particle i (dataLL.cpp:522-582): its clipped inCoords, and its
+ * h into the maxima of the neighbour slots its images go to */
+__device__ __forceinline__ void ghost_particle(const DevCfg &c, const DevState &s, const DevGlobals *g, int64_t i, int t,
+                                               unsigned long long *smax) {
+    int gcode = 0;
+    if (t != T_DEAD) {
+        const bool dem = c.liq_dem() && t == T_DEM;
+        int ic[3] = {1, 1, 1};
+        bool any = false;
+        for (int d = 0; d < c.nd; d++) {
+            if (!c.periodic[d]) continue;
+            const double r = s.row(FD_R + d)[i];
+            int v = dem ? trunc_index(r, c.dg_lo[d], c.dg_sp[d], c.dg_rsp_f[d], 1.0)
+                        : trunc_index(r, g->ghost_lo[d], g->ghost_sp[d], g->ghost_rsp_f[d], 1.0);
+            if (v > 2) v = 2;
+            if (v < 0) v = 0;
+            ic[d] = v;
+            any |= v != 1;
+        }
+        for (int d = 0; d < c.nd; d++) gcode |= ic[d] << (2 * d);
+        if (any) {
+            const double h = s.row(FD_H)[i];
+            int lo3[3], hi3[3];
+            for (int d = 0; d < 3; d++) {
+                lo3[d] = d < c.nd ? min(ic[d], 1) : 1;
+                hi3[d] = d < c.nd ? max(ic[d], 1) : 1;
+            }
+            for (int a = lo3[0]; a <= hi3[0]; a++)
+                for (int b = lo3[1]; b <= hi3[1]; b++)
+                    for (int e = lo3[2]; e <= hi3[2]; e++) {
+                        const int dc[3] = {a, b, e};
+                        bool centre = true;
+                        for (int d = 0; d < c.nd; d++) centre &= dc[d] == 1;
+                        if (centre) continue;
+                        int sl[3];
+                        for (int d = 0; d < c.nd; d++) sl[d] = 2 - dc[d];
+                        atomicMax(&smax[slot_index(sl, c.nd)], dbits(h));
+                    }
+        }
+    }
+    s.irow(FI_GCODE)[i] = gcode;
+}
+
+/* The new ghost widths, h_max, the search-radius hysteresis (dataLL.cpp:220-223,
+ * 688-693) and the SPH bucket grid, by one warp: a lane per neighbour slot, then
+ * a lane per axis, so that the FP64 divisions of the axes run side by side. */
+__device__ __forceinline__ void finalize_grid(const DevCfg &c, DevGlobals *g) {
+    const int lane = threadIdx.x & 31;
+    volatile DevGlobals *v = g;
+    const double hmax = __longlong_as_double((long long)v->hmax_bits), hmax_old = g->hmax;
     bool any_periodic = false;
     for (int d = 0; d < c.nd; d++) any_periodic |= c.periodic[d] != 0;
     const int ns = c.nd == 3 ? 27 : (c.nd == 2 ? 9 : 3);
-    if (any_periodic) {
-        for (int sidx = 0; sidx < ns; sidx++) {
-            int co[3], t = sidx;
-            for (int d = c.nd - 1; d >= 0; d--) {
-                co[d] = t % 3;
-                t /= 3;
+    double gw = lane < 27 ? g->gw[lane] : 0.0;
+    int off_centre = 0;
+    if (lane < ns) {
+        int t = lane;
+        bool has = true;
+        for (int d = c.nd - 1; d >= 0; d--) {
+            if (t % 3 != 1) {
+                off_centre++;
+                if (!c.periodic[d]) has = false;
             }
-            bool centre = true, has = true;
-            for (int d = 0; d < c.nd; d++)
-                if (co[d] != 1) {
-                    centre = false;
-                    if (!c.periodic[d]) has = false;
+            t /= 3;
+        }
+        if (any_periodic && off_centre && has) {
+            const double smax = __longlong_as_double((long long)v->slot_bits[lane]);
+            gw = 2.0 * (smax > hmax_old ? smax : hmax_old);
+        }
+        if (off_centre == 1 && gw < hmax) gw = 2.0 * hmax;
+        g->gw[lane] = gw;
+    }
+    __syncwarp(); /* the axes' lanes read the slots' widths */
+    double sr = g->sr;
+    if (hmax > sr || hmax < 0.9 * sr) sr = hmax;
+    const double sr2 = 2.0 * sr;
+    int dim = 1, bad = 0;
+    if (lane < 3) {
+        const int d = lane;
+        /* face slots of the axis: their widths sit in lanes lo and hi */
+        int lo = 0, hi = 0;
+        for (int k = 0; k < c.nd; k++) {
+            lo = lo * 3 + (k == d ? 0 : 1);
+            hi = hi * 3 + (k == d ? 2 : 1);
+        }
+        if (d < c.nd) {
+            const double glo = g->gw[lo], ghi = g->gw[hi];
+            /* SPH ghost test of the next rebuild (dataLL.cpp:338-364) */
+            g->ghost_lo[d] = c.dmin[d] + glo;
+            double sp = c.dspace[d] - glo;
+            sp -= ghi;
+            g->ghost_sp[d] = sp;
+            g->ghost_rsp_f[d] = (float)(1.0 / sp);
+            const double ext = c.dmax[d] - c.dmin[d];
+            if (c.periodic[d]) {
+                dim = (int)floor(ext / (sr2 * (1.0 + 1e-12)));
+                if (dim < 3) {
+                    bad = 1;
+                    dim = 3;
                 }
-            if (centre || !has) continue;
-            const double smax = __longlong_as_double((long long)g->slot_bits[sidx]);
-            const double maxh = smax > g->hmax ? smax : g->hmax;
-            g->gw[sidx] = 2.0 * maxh;
-        }
-    }
-    const double hmax = __longlong_as_double((long long)g->hmax_bits);
-    g->hmax = hmax;
-    for (int d = 0; d < c.nd; d++) {
-        for (int side = 0; side <= 2; side += 2) {
-            int co[3] = {1, 1, 1};
-            co[d] = side;
-            int sidx = 0;
-            for (int k = 0; k < c.nd; k++) sidx = sidx * 3 + co[k];
-            if (g->gw[sidx] < hmax) g->gw[sidx] = 2.0 * hmax;
-        }
-    }
-    if (hmax > g->sr || hmax < 0.9 * g->sr) g->sr = hmax;
-    g->sr2 = 2.0 * g->sr;
-    g->rsr2_f = (float)(1.0 / g->sr2);
-    /* SPH ghost test of the next rebuild (dataLL.cpp:338-364) */
-    for (int d = 0; d < c.nd; d++) {
-        int co[3] = {1, 1, 1};
-        co[d] = 0;
-        int slo = 0, shi = 0;
-        for (int k = 0; k < c.nd; k++) slo = slo * 3 + co[k];
-        co[d] = 2;
-        for (int k = 0; k < c.nd; k++) shi = shi * 3 + co[k];
-        g->ghost_lo[d] = c.dmin[d] + g->gw[slo];
-        double sp = c.dspace[d] - g->gw[slo];
-        sp -= g->gw[shi];
-        g->ghost_sp[d] = sp;
-        g->ghost_rsp_f[d] = (float)(1.0 / sp);
-    }
-    int tot = 1;
-    for (int d = 0; d < 3; d++) {
-        if (d >= c.nd) {
-            g->sdims[d] = 1;
-            g->scell[d] = 1.0;
-            continue;
-        }
-        const double ext = c.dmax[d] - c.dmin[d];
-        if (c.periodic[d]) {
-            int m = (int)floor(ext / (2.0 * g->sr * (1.0 + 1e-12)));
-            if (m < 3) {
-                set_err(g, SPHDEM_ERR_CAPACITY, 100 + d);
-                m = 3;
+                g->scell[d] = ext / dim;
+                g->rscell[d] = dim / ext;
+            } else {
+                dim = (int)(ext / sr2) + 8;
+                g->scell[d] = sr2;
             }
-            g->sdims[d] = m;
-            g->scell[d] = ext / m;
-            g->rscell[d] = m / ext;
         } else {
-            g->sdims[d] = (int)(ext / (2.0 * g->sr)) + 8;
-            g->scell[d] = 2.0 * g->sr;
+            g->scell[d] = 1.0;
         }
-        tot *= g->sdims[d];
+        g->sdims[d] = dim;
+        if (bad) set_err(g, SPHDEM_ERR_CAPACITY, 100 + d);
     }
-    if (tot > c.sph_cells_cap) {
-        set_err(g, SPHDEM_ERR_CAPACITY, tot);
-        tot = c.sph_cells_cap;
+    int tot = __shfl_sync(0xffffffffu, dim, 0) * __shfl_sync(0xffffffffu, dim, 1) * __shfl_sync(0xffffffffu, dim, 2);
+    if (lane == 0) {
+        if (tot > c.sph_cells_cap) {
+            set_err(g, SPHDEM_ERR_CAPACITY, tot);
+            tot = c.sph_cells_cap;
+        }
+        g->hmax = hmax;
+        g->sr = sr;
+        g->sr2 = sr2;
+        g->rsr2_f = (float)(1.0 / sr2);
+        g->n_sph_cells = tot;
+        g->n_total_cells = tot + c.n_dem_cells + 1;
+        g->hmax_bits = 0ull;
     }
-    g->n_sph_cells = tot;
-    g->n_total_cells = tot + c.n_dem_cells + 1;
-    g->hmax_bits = 0ull;
-    for (int k = 0; k < 27; k++) g->slot_bits[k] = 0ull;
+    if (lane < 27) g->slot_bits[lane] = 0ull;
+}
+
+/* One pass over the particles before a rebuild: the elementwise work PRE that
+ * precedes it in a whole step, migration (with the next h_max), ghost images;
+ * the last block to finish writes the step globals and the new grid.  A step
+ * has two of these instead of five elementwise passes, three global updates and
+ * two each of migration, ghost and grid passes.  Bound by launches below some
+ * 100,000 particles (a step of 23,000: 39 launches -> 24, 163 -> 142 us), by
+ * the rows it reads and writes above (1.08 M particles: 147 and 119 us). */
+enum SweepWork : int {
+    SW_NONE = 0,      /* a rebuild by itself */
+    SW_START,         /* step count, start(), beforeMiddle hook, begin of middle() */
+    SW_MIDDLE_TAIL    /* dt, end of middle(), beforeEnd hook, begin of end() */
+};
+template <int PRE>
+__global__ void __launch_bounds__(BLK) k_sweep(DevCfg c, DevState s, DevGlobals *g, unsigned char *mark, int64_t n) {
+    __shared__ unsigned long long smax[27], bmax, bacc;
+    __shared__ int last;
+    if (threadIdx.x < 27) smax[threadIdx.x] = 0ull;
+    if (threadIdx.x == 0) {
+        bmax = 0ull;
+        bacc = ~0ull;
+    }
+    __syncthreads();
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    double h = -1.0, new_dt = 0.0;
+    const double old_dt = g->dt;
+    double dt = old_dt;
+    if (PRE == SW_MIDDLE_TAIL) dt = choose_dt(c, g, &new_dt);
+    if (i < n) {
+        int t = s.irow(FI_IAM)[i];
+        if (PRE == SW_START) {
+            start_particle(c, s, i, t, dt);
+            hook_before_middle_particle(c, s, i, t);
+        }
+        if (PRE == SW_MIDDLE_TAIL) {
+            middle_tail_particle(c, s, i, t, dt, old_dt, g->time);
+            hook_before_end_particle(c, s, i, t, g->time);
+            end_drift_particle(c, s, i, t, dt);
+        }
+        t = migrate_particle(c, s, g, mark, i, t, &h);
+        if (PRE == SW_START && c.liq_dem() && t == T_DEM) {
+            /* accelCondition of the DEM particles (sph.h:566-568): their force is
+             * still the last step's when middle() takes it */
+            double f2 = 0.0;
+            for (int d = 0; d < c.nd; d++) f2 += s.row(FD_F + d)[i] * s.row(FD_F + d)[i];
+            const double b = 0.25 * sqrt(s.row(FD_H)[i] / sqrt(f2));
+            if (b >= 0.0) atomicMin(&bacc, dbits(b));
+            s.row(FD_SHEP)[i] = 0.0; /* the porosity pass adds into it */
+        }
+        ghost_particle(c, s, g, i, t, smax);
+    }
+    /* block maximum of h, then one atomic per block */
+    for (int o = 16; o > 0; o >>= 1) h = fmax(h, __shfl_xor_sync(0xffffffffu, h, o));
+    if ((threadIdx.x & 31) == 0 && h >= 0.0) atomicMax(&bmax, dbits(h));
+    __syncthreads();
+    if (threadIdx.x == 0 && bmax) atomicMax(&g->hmax_bits, bmax);
+    if (PRE == SW_START && threadIdx.x == 0 && bacc != ~0ull) atomicMin(&g->dem_acc_bits, bacc);
+    if (threadIdx.x < 27 && smax[threadIdx.x]) atomicMax(&g->slot_bits[threadIdx.x], smax[threadIdx.x]);
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(&g->blocks_done, 1) == (int)gridDim.x - 1;
+    __syncthreads();
+    if (!last || threadIdx.x >= 32) return;
+    __threadfence();
+    finalize_grid(c, g);
+    if (threadIdx.x) return;
+    g->blocks_done = 0;
+    if (PRE == SW_START) {
+        g->step += 1;
+        g->time = g->time + dt / 2;
+        g->new_dt = g->maxdt;
+        const unsigned long long acc = *(volatile unsigned long long *)&g->dem_acc_bits;
+        g->new_dt_bits = acc < dbits(g->maxdt) ? acc : dbits(g->maxdt);
+        g->dem_acc_bits = ~0ull;
+    }
+    if (PRE == SW_MIDDLE_TAIL) {
+        g->new_dt = new_dt;
+        g->old_dt = old_dt;
+        g->dt = dt;
+        g->time = g->time + dt / 2;
+        if (c.liq_dem()) g->dem_dt = g->maxdt;
+    }
 }
 
 __device__ __forceinline__ int dem_grid_cell(const DevCfg &c, const double *r, int *cc) {
@@ -232,7 +304,7 @@ __device__ __forceinline__ int dem_grid_cell(const DevCfg &c, const double *r, i
     return lin;
 }
 
-__global__ void k_keys(DevCfg c, DevState s, DevGlobals *g, int *key, int *cnt, int64_t n) {
+__global__ void k_keys(DevCfg c, DevState s, DevGlobals *g, int *key, int *off, int *cnt, int64_t n) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int t = s.irow(FI_IAM)[i];
@@ -272,10 +344,11 @@ __global__ void k_keys(DevCfg c, DevState s, DevGlobals *g, int *key, int *cnt, 
         }
     }
     key[i] = k;
-    atomicAdd(&cnt[k], 1);
+    off[i] = atomicAdd(&cnt[k], 1); /* a slot of the bucket; k_rank orders them */
 }
 
-/* three-phase exclusive scan of cnt[0..m) into start[0..m], start[m] = total */
+/* three-phase exclusive scan of cnt[0..m) into start[0..m], start[m] = total;
+ * cnt is left zero for the next rebuild's count */
 constexpr int SCAN_BLK = 1024;
 constexpr int SCAN_ITEMS = 4;
 constexpr int SCAN_TILE = SCAN_BLK * SCAN_ITEMS;
@@ -334,7 +407,7 @@ __global__ void k_scan_blocks(int *bsum, int nblocks) {
     }
 }
 
-__global__ void k_scan_down(const int *cnt, const DevGlobals *g, const int *bsum, int *start, int *fill) {
+__global__ void k_scan_down(int *cnt, const DevGlobals *g, const int *bsum, int *start) {
     __shared__ int ws[32];
     const int m = g->n_total_cells;
     const int64_t base = (int64_t)blockIdx.x * SCAN_TILE;
@@ -350,7 +423,7 @@ __global__ void k_scan_down(const int *cnt, const DevGlobals *g, const int *bsum
         const int64_t j = base + threadIdx.x * SCAN_ITEMS + k;
         if (j < m) {
             start[j] = run;
-            fill[j] = 0;
+            cnt[j] = 0;
         } else if (j == m) {
             start[j] = run;
         }
@@ -360,18 +433,58 @@ __global__ void k_scan_down(const int *cnt, const DevGlobals *g, const int *bsum
     if (base + (int64_t)(threadIdx.x + 1) * SCAN_ITEMS == m) start[m] = run;
 }
 
+/* the same by one block, for grids that start at up to SCAN_ONE buckets: one
+ * launch in place of three.  It is bound by its chain of tiles (6 us at 2,000
+ * buckets, 14 us at 57,000); there the three launches make a step 3 us per
+ * rebuild faster, while an ensemble of small members gains 2 % by one. */
+constexpr int64_t SCAN_ONE = 32768;
+__global__ void __launch_bounds__(SCAN_BLK) k_scan_one(int *cnt, const DevGlobals *g, int *start) {
+    __shared__ int ws[32];
+    const int m = g->n_total_cells;
+    auto load = [&](int j) {
+        if (j + 3 < m) return *reinterpret_cast<const int4 *>(cnt + j);
+        return make_int4(j < m ? cnt[j] : 0, j + 1 < m ? cnt[j + 1] : 0, j + 2 < m ? cnt[j + 2] : 0, 0);
+    };
+    int carry = 0;
+    int4 next = load(threadIdx.x * 4);
+    for (int base = 0; base < m; base += SCAN_BLK * 4) {
+        const int j = base + threadIdx.x * 4;
+        const int4 v = next;
+        next = load(j + SCAN_BLK * 4); /* in flight during the scan */
+        int total;
+        int4 run;
+        run.x = carry + block_exclusive_scan(v.x + v.y + v.z + v.w, ws, &total);
+        run.y = run.x + v.x;
+        run.z = run.y + v.y;
+        run.w = run.z + v.z;
+        if (j + 3 < m) {
+            *reinterpret_cast<int4 *>(start + j) = run;
+            *reinterpret_cast<int4 *>(cnt + j) = make_int4(0, 0, 0, 0);
+        } else {
+            const int r[3] = {run.x, run.y, run.z};
+            for (int k = 0; k < 3 && j + k < m; k++) {
+                start[j + k] = r[k];
+                cnt[j + k] = 0;
+            }
+        }
+        carry += total;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) start[m] = carry;
+}
+
 /* order-preserving integer image of a double (integer compares are full rate) */
 __device__ __forceinline__ unsigned long long order_key(double x) {
     const unsigned long long b = (unsigned long long)__double_as_longlong(x);
     return (b >> 63) ? ~b : (b | 0x8000000000000000ull);
 }
 
-__global__ void k_scatter(const int *key, const int *start, int *fill, int *slot, const int *tag, const double *rz,
+__global__ void k_scatter(const int *key, const int *start, const int *off, int *slot, const int *tag, const double *rz,
                           int *slot_tag, unsigned long long *slot_z, int64_t n) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int k = key[i];
-    const int pos = start[k] + atomicAdd(&fill[k], 1);
+    const int pos = start[k] + off[i];
     slot[pos] = (int)i;
     slot_tag[pos] = tag[i];
     slot_z[pos] = order_key(rz[i]);
@@ -457,21 +570,21 @@ void setup_rebuild_buffers(sphdem_ctx *c) {
     c->buf.n_fields_i = (int)fi.size();
 }
 
-void rebuild(sphdem_ctx *c) {
+/* buckets, sort and gather, after a sweep */
+static void sort_particles(sphdem_ctx *c) {
     const int64_t n = c->n;
     const int gb = grid_for(n, BLK);
     Buffers &b = c->buf;
-    SPHDEM_LAUNCH(c, "rebuild_migrate", k_migrate, gb, BLK, 0, c->cfg, c->A, c->g, c->delmark, n);
-    SPHDEM_LAUNCH(c, "rebuild_ghost", k_ghost, gb, BLK, 0, c->cfg, c->A, c->g, n);
-    SPHDEM_LAUNCH(c, "rebuild_finalize", k_finalize, 1, 32, 0, c->cfg, c->g);
-    SPHDEM_CUDA_CHECK(cudaMemsetAsync(b.cnt, 0, (size_t)b.cells_cap * sizeof(int), c->stream));
-    SPHDEM_LAUNCH(c, "rebuild_keys", k_keys, gb, BLK, 0, c->cfg, c->A, c->g, b.key, b.cnt, n);
-    const int nscan = (b.cells_cap + SCAN_TILE - 1) / SCAN_TILE;
-    SPHDEM_LAUNCH(c, "rebuild_scan_reduce", k_scan_reduce, nscan, SCAN_BLK, 0, b.cnt, c->g, b.bsum);
-    SPHDEM_LAUNCH(c, "rebuild_scan_blocks", k_scan_blocks, 1, SCAN_BLK, 0, b.bsum, nscan);
-    SPHDEM_LAUNCH(c, "rebuild_scan_down", k_scan_down, nscan, SCAN_BLK, 0, b.cnt, c->g, b.bsum, b.start, b.fill);
-    SPHDEM_CUDA_CHECK(cudaMemsetAsync(b.perm, 0, (size_t)n * sizeof(int), c->stream));
-    SPHDEM_LAUNCH(c, "rebuild_scatter", k_scatter, gb, BLK, 0, b.key, b.start, b.fill, b.slot, c->A.irow(FI_TAG),
+    SPHDEM_LAUNCH(c, "rebuild_keys", k_keys, gb, BLK, 0, c->cfg, c->A, c->g, b.key, b.off, b.cnt, n);
+    if (c->cells_start <= SCAN_ONE) {
+        SPHDEM_LAUNCH(c, "rebuild_scan", k_scan_one, 1, SCAN_BLK, 0, b.cnt, c->g, b.start);
+    } else {
+        const int nscan = (b.cells_cap + SCAN_TILE - 1) / SCAN_TILE;
+        SPHDEM_LAUNCH(c, "rebuild_scan_reduce", k_scan_reduce, nscan, SCAN_BLK, 0, b.cnt, c->g, b.bsum);
+        SPHDEM_LAUNCH(c, "rebuild_scan_blocks", k_scan_blocks, 1, SCAN_BLK, 0, b.bsum, nscan);
+        SPHDEM_LAUNCH(c, "rebuild_scan_down", k_scan_down, nscan, SCAN_BLK, 0, b.cnt, c->g, b.bsum, b.start);
+    }
+    SPHDEM_LAUNCH(c, "rebuild_scatter", k_scatter, gb, BLK, 0, b.key, b.start, b.off, b.slot, c->A.irow(FI_TAG),
                   c->A.row(FD_R + c->cfg.nd - 1), b.slot_tag, b.slot_z, n);
     SPHDEM_LAUNCH(c, "rebuild_rank", k_rank, gb, BLK, 0, b.key, b.start, b.slot, b.slot_tag, b.slot_z, b.perm,
                   b.skey, c->g, n);
@@ -480,6 +593,22 @@ void rebuild(sphdem_ctx *c) {
                   b.n_fields_d, b.fields_i, b.n_fields_i, n);
     std::swap(c->A, c->B);
     c->flipped = !c->flipped;
+}
+
+void rebuild(sphdem_ctx *c) {
+    SPHDEM_LAUNCH(c, "rebuild_sweep", k_sweep<SW_NONE>, grid_for(c->n, BLK), BLK, 0, c->cfg, c->A, c->g, c->delmark, c->n);
+    sort_particles(c);
+}
+
+void start_and_rebuild(sphdem_ctx *c) {
+    SPHDEM_LAUNCH(c, "start_sweep", k_sweep<SW_START>, grid_for(c->n, BLK), BLK, 0, c->cfg, c->A, c->g, c->delmark, c->n);
+    sort_particles(c);
+}
+
+void middle_tail_and_rebuild(sphdem_ctx *c) {
+    SPHDEM_LAUNCH(c, "middle_sweep", k_sweep<SW_MIDDLE_TAIL>, grid_for(c->n, BLK), BLK, 0, c->cfg, c->A, c->g,
+                  c->delmark, c->n);
+    sort_particles(c);
 }
 
 }  // namespace sphdem

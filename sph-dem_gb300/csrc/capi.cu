@@ -267,7 +267,7 @@ void free_ctx(sphdem_ctx *c) {
     cudaFree(c->g);
     Buffers &b = c->buf;
     cudaFree(b.slot_z);
-    for (int *p : {b.skey, b.perm, b.slot, b.slot_tag, b.key, b.cnt, b.start, b.fill, b.bsum, b.fields_d, b.fields_i,
+    for (int *p : {b.skey, b.perm, b.slot, b.slot_tag, b.key, b.cnt, b.start, b.off, b.bsum, b.fields_d, b.fields_i,
                    b.pair_cnt})
         cudaFree(p);
     cudaFree(c->mx_pos);
@@ -336,55 +336,63 @@ void alloc_lists64(sphdem_ctx *c, double hmax, bool fluid) {
     if (get(&c->mx_nbr, (size_t)depth * ((cap + 31) / 32 * 32) * sizeof(int))) c->f64_maxn = depth;
 }
 
-void run_phase_mixed(sphdem_ctx *c, int phase) {
-    const bool liq = c->cfg.liq_dem();
-    const bool lists = c->mx_maxn > 0;
-    switch (phase) {
-        case SPHDEM_PHASE_MIDDLE:
-            globals_op(c, OP_MIDDLE_BEGIN);
-            rebuild(c);
-            mixed::pack(c);
-            if (lists) mixed::nlist(c, c->mx_maxn);
-            /* calcInvM in FP64 once per rebuild; the pair passes apply it in FP32 */
-            if (corrected_gradient(c)) run_invm(c);
-            if (liq) {
-                mixed::porosity(c);
-                mixed::dem_drag(c);
-            }
-            if (lists) {
-                /* elementwise EOS; Omega (VAR_H_CORRECTION) is summed inside the force pass */
-                mixed::omega_eos(c, false, true);
-                mixed::force(c);
-            }
-            if (liq) run_dem_accel(c);
-            globals_op(c, OP_SET_DT);
-            run_middle_tail(c);
-            break;
-        case SPHDEM_PHASE_END:
-            run_end_drift(c);
-            rebuild(c);
-            mixed::pack(c, false);
-            if (lists) mixed::nlist(c, c->mx_maxn);
-            if (corrected_gradient(c)) run_invm(c);
-            if (lists) {
-                mixed::dddt(c);  /* Omega (VAR_H_CORRECTION) is summed inside the continuity pass */
-            }
-            if (liq) mixed::dem_end(c);
-            if (c->host_cfg.flags & SPHDEM_F_DEM_BLOCK) run_dem_block(c);
-            run_end_tail(c);
-            break;
-    }
-}
-
-void run_phase(sphdem_ctx *c, int phase) {
+/* the pair passes of the middle and end phases, after their rebuild; whole: as
+ * part of a whole step, whose sweep has taken the DEM accelCondition */
+void middle_passes(sphdem_ctx *c, bool whole) {
     const bool liq = c->cfg.liq_dem();
     /* a DEM-only handle has no FP32 pair pass: its contacts are FP64 on both
      * paths, so the mixed handle runs the FP64 phases */
-    if (c->cfg.precision == SPHDEM_PREC_MIXED && !c->mx_dem_only &&
-        (phase == SPHDEM_PHASE_MIDDLE || phase == SPHDEM_PHASE_END)) {
-        run_phase_mixed(c, phase);
-        return;
+    if (c->cfg.precision == SPHDEM_PREC_MIXED && !c->mx_dem_only) {
+        const bool lists = c->mx_maxn > 0;
+        mixed::pack(c);
+        if (lists) mixed::nlist(c, c->mx_maxn);
+        /* calcInvM in FP64 once per rebuild; the pair passes apply it in FP32 */
+        if (corrected_gradient(c)) run_invm(c);
+        if (liq) {
+            mixed::porosity(c);
+            mixed::dem_drag(c);
+        }
+        if (lists) {
+            /* elementwise EOS; Omega (VAR_H_CORRECTION) is summed inside the force pass */
+            mixed::omega_eos(c, false, true);
+            mixed::force(c);
+        }
+    } else {
+        run_lists64(c, true);
+        if (liq) {
+            run_porosity(c);
+            run_dem_drag(c);
+        }
+        if (!c->only_dem) {
+            if (corrected_gradient(c)) run_invm(c);
+            run_eos(c);
+            run_force(c);  /* Omega (VAR_H_CORRECTION) is summed inside */
+        }
     }
+    if (liq && !whole) run_dem_accel(c);
+}
+
+void end_passes(sphdem_ctx *c) {
+    const bool liq = c->cfg.liq_dem();
+    if (c->cfg.precision == SPHDEM_PREC_MIXED && !c->mx_dem_only) {
+        const bool lists = c->mx_maxn > 0;
+        mixed::pack(c, false);
+        if (lists) mixed::nlist(c, c->mx_maxn);
+        if (corrected_gradient(c)) run_invm(c);
+        if (lists) mixed::dddt(c);  /* Omega (VAR_H_CORRECTION) is summed inside the continuity pass */
+        if (liq) mixed::dem_end(c);
+    } else {
+        run_lists64(c, false);
+        if (!c->only_dem) {
+            if (corrected_gradient(c)) run_invm(c);
+            run_dddt(c);   /* Omega (VAR_H_CORRECTION) is summed inside */
+        }
+        if (liq) run_dem_end(c);
+    }
+    if (c->host_cfg.flags & SPHDEM_F_DEM_BLOCK) run_dem_block(c);
+}
+
+void run_phase(sphdem_ctx *c, int phase) {
     switch (phase) {
         case SPHDEM_HOOK_BEFORE_START:
             globals_op(c, OP_STEP_INC);
@@ -400,17 +408,7 @@ void run_phase(sphdem_ctx *c, int phase) {
         case SPHDEM_PHASE_MIDDLE:
             globals_op(c, OP_MIDDLE_BEGIN);
             rebuild(c);
-            run_lists64(c, true);
-            if (liq) {
-                run_porosity(c);
-                run_dem_drag(c);
-            }
-            if (!c->only_dem) {
-                if (corrected_gradient(c)) run_invm(c);
-                run_eos(c);
-                run_force(c);  /* Omega (VAR_H_CORRECTION) is summed inside */
-            }
-            if (liq) run_dem_accel(c);
+            middle_passes(c, false);
             globals_op(c, OP_SET_DT);
             run_middle_tail(c);
             break;
@@ -420,13 +418,7 @@ void run_phase(sphdem_ctx *c, int phase) {
         case SPHDEM_PHASE_END:
             run_end_drift(c);
             rebuild(c);
-            run_lists64(c, false);
-            if (!c->only_dem) {
-                if (corrected_gradient(c)) run_invm(c);
-                run_dddt(c);   /* Omega (VAR_H_CORRECTION) is summed inside */
-            }
-            if (liq) run_dem_end(c);
-            if (c->host_cfg.flags & SPHDEM_F_DEM_BLOCK) run_dem_block(c);
+            end_passes(c);
             run_end_tail(c);
             break;
         case SPHDEM_HOOK_AFTER_END:
@@ -435,8 +427,23 @@ void run_phase(sphdem_ctx *c, int phase) {
     }
 }
 
+/* A whole step: the phases above with the elementwise work of neighbouring
+ * phases and hooks in one pass (a step that re-initialises the density rebuilds
+ * between start() and its hook and takes those by themselves). */
 void run_full_step(sphdem_ctx *c) {
-    for (int p = SPHDEM_HOOK_BEFORE_START; p <= SPHDEM_HOOK_AFTER_END; p++) run_phase(c, p);
+    const bool reinit = reinit_due(c->host_cfg, c->host_step + 1);
+    if (reinit) {
+        for (int p = SPHDEM_HOOK_BEFORE_START; p <= SPHDEM_HOOK_BEFORE_MIDDLE; p++) run_phase(c, p);
+        globals_op(c, OP_MIDDLE_BEGIN);
+        rebuild(c);
+    } else {
+        c->host_step++;
+        start_and_rebuild(c);
+    }
+    middle_passes(c, !reinit);
+    middle_tail_and_rebuild(c);
+    end_passes(c);
+    run_step_tail(c);
 }
 
 }  // namespace
@@ -526,21 +533,23 @@ int sphdem_create(const SphDemConfig *cfg, const SphDemParticles *init, int64_t 
         double hmax0 = 0;
         for (int64_t i = 0; i < n; i++) hmax0 = std::max(hmax0, init->h[i]);
         const double sr_min = 0.5 * std::min(cfg->h, hmax0);
-        long long sc = 1;
+        long long sc = 1, sc0 = 1;
         for (int d = 0; d < cfg->ndim; d++) {
-            const long long nd = (long long)((cfg->domain_max[d] - cfg->domain_min[d]) / (2.0 * sr_min)) + 9;
-            sc *= nd;
+            const double ext = cfg->domain_max[d] - cfg->domain_min[d];
+            sc *= (long long)(ext / (2.0 * sr_min)) + 9;
+            sc0 *= (long long)(ext / (2.0 * hmax0)) + 9;
         }
         if (sc > (1ll << 30)) throw std::string("bucket grid too large for the domain / smoothing length");
         c->cfg.sph_cells_cap = (int)sc;
+        c->cells_start = sc0 + c->cfg.n_dem_cells;
         Buffers &b = c->buf;
         b.cells_cap = (int)sc + c->cfg.n_dem_cells + 2;
         SPHDEM_CUDA_CHECK(cudaMalloc(&b.slot_z, capacity * sizeof(unsigned long long)));
-        for (int **p : {&b.skey, &b.perm, &b.slot, &b.slot_tag, &b.key})
+        for (int **p : {&b.skey, &b.perm, &b.slot, &b.slot_tag, &b.key, &b.off})
             SPHDEM_CUDA_CHECK(cudaMalloc(p, capacity * sizeof(int)));
         SPHDEM_CUDA_CHECK(cudaMalloc(&b.cnt, (size_t)b.cells_cap * sizeof(int)));
         SPHDEM_CUDA_CHECK(cudaMalloc(&b.start, ((size_t)b.cells_cap + 1) * sizeof(int)));
-        SPHDEM_CUDA_CHECK(cudaMalloc(&b.fill, (size_t)b.cells_cap * sizeof(int)));
+        SPHDEM_CUDA_CHECK(cudaMemset(b.cnt, 0, (size_t)b.cells_cap * sizeof(int)));
         SPHDEM_CUDA_CHECK(cudaMalloc(&b.bsum, ((size_t)b.cells_cap / 4096 + 2) * sizeof(int)));
         setup_rebuild_buffers(c);
         if (cfg->flags & SPHDEM_F_CORRECTED_GRADIENT)
@@ -562,6 +571,7 @@ int sphdem_create(const SphDemConfig *cfg, const SphDemParticles *init, int64_t 
         hg.dem_dt = cfg->maxdt;
         hg.sr = cfg->h;
         hg.hmax = cfg->h;
+        hg.dem_acc_bits = ~0ull;
         for (int k = 0; k < 27; k++) hg.gw[k] = 1.1 * 2.0 * cfg->h;
         for (int d = 0; d < 3; d++) {
             hg.ghost_lo[d] = c->cfg.dmin[d] + hg.gw[0];

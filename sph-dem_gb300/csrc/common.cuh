@@ -104,6 +104,8 @@ struct DevGlobals {
     double sr;                        /* sph_search_radius (dataLL.h:351) */
     double hmax;                      /* CdataLL::hmax */
     unsigned long long hmax_bits;     /* reduction target for the next hmax */
+    unsigned long long dem_acc_bits;  /* reduction target of the DEM accelCondition */
+    int blocks_done;                  /* blocks of the running sweep that are done */
     double gw[27];                    /* procGhostMax2H per neighbour slot */
     unsigned long long slot_bits[27]; /* max ghost h per slot (reduction) */
     int sdims[3];                     /* SPH bucket grid extents */

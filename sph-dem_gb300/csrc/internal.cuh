@@ -31,12 +31,12 @@ struct Buffers {
     int *key = nullptr;      /* bucket key of each particle, previous order */
     int *cnt = nullptr;      /* bucket counts                             */
     int *start = nullptr;    /* bucket starts (exclusive scan)            */
-    int *fill = nullptr;     /* scatter cursors                           */
+    int *off = nullptr;      /* slot of each particle in its bucket, before the sort */
     int *bsum = nullptr;     /* scan block sums                           */
     int *fields_d = nullptr; /* FP64 rows to gather at a rebuild          */
     int *fields_i = nullptr; /* int rows to gather                        */
     int n_fields_d = 0, n_fields_i = 0;
-    int cells_cap = 0;       /* capacity of cnt/start/fill                */
+    int cells_cap = 0;       /* capacity of cnt/start                     */
     /* export scratch */
     int *pair_cnt = nullptr;
 };
@@ -72,6 +72,7 @@ struct sphdem_ctx {
     bool flipped = false;    /* odd number of rebuilds so far              */
     sphdem::DevGlobals *g = nullptr;
     sphdem::Buffers buf;
+    int64_t cells_start = 0; /* buckets of the grid of the initial h       */
     cudaStream_t stream = nullptr;
     std::string err;
     /* CUDA graphs of one full step, keyed by the state parity at its start
@@ -168,6 +169,10 @@ void launch_end(sphdem_ctx *c);
 
 /* binning.cu */
 void rebuild(sphdem_ctx *c);
+/* in a whole step: step count, start(), its hook and the begin of middle() with
+ * the rebuild; dt, the end of middle(), its hook and the begin of end() with it */
+void start_and_rebuild(sphdem_ctx *c);
+void middle_tail_and_rebuild(sphdem_ctx *c);
 void setup_rebuild_buffers(sphdem_ctx *c);
 
 /* integrate.cu: elementwise phases and built-in hooks */
@@ -178,6 +183,7 @@ void run_hook_before_middle(sphdem_ctx *c);
 void run_middle_tail(sphdem_ctx *c);
 void run_end_drift(sphdem_ctx *c);
 void run_end_tail(sphdem_ctx *c);
+void run_step_tail(sphdem_ctx *c);     /* run_end_tail + run_hook_after_end */
 void run_hook_before_end(sphdem_ctx *c);
 void run_hook_after_end(sphdem_ctx *c);
 void run_h_derived(sphdem_ctx *c);
