@@ -66,6 +66,10 @@ struct AdjointData {
     int blk = 0;                    /* block the current segment's tape is in */
     int taped = 0;                  /* the blocks hold the forward pass's tapes */
     int64_t n = 0;
+    /* what the allocations and the replay graphs follow beside n, K and mode */
+    int64_t tape_mem = 0;
+    long long population_gen = 0;
+    bool scan_taps = false;
     std::vector<double *> ckpt;     /* state at steps 0, K, 2K, ... and the final state */
     std::vector<DevGlobals> ckpt_g;
     double *seg = nullptr;          /* (K + 1) states of one segment */
@@ -193,8 +197,16 @@ __device__ __forceinline__ void grad_factor32(float wcon, float r, float iha, fl
     Gp *= 0.5f;
 }
 
+/* entries of a per-step table for `now` pairs: room for half as many again */
+inline int64_t table_need(int64_t now) { return now + now / 2 + 4096; }
+/* allocated with a sixteenth more, so that a later pass from a state of a few
+ * more pairs finds its tables large enough */
+inline int64_t table_room(int64_t need) { return need + need / 16; }
+
 /* adjoint_cpl.cu: the coupled step */
-void cpl_count_tables(sphdem_ctx *c, AdjointData *a);          /* sizes cpl / fpi / contacts (synchronises) */
+bool cpl_scan_taps();                                          /* SPHDEM_ADJ_SCAN_TAPS */
+/* sizes cpl / fpi / contacts (synchronises); false: the tables that are there are too small */
+bool cpl_count_tables(sphdem_ctx *c, AdjointData *a);
 void cpl_alloc(sphdem_ctx *c, AdjointData *a);
 void cpl_free(AdjointData *a);
 void cpl_reset_segment(sphdem_ctx *c, AdjointData *a);         /* empty tables before a segment's replay */

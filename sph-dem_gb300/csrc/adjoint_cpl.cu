@@ -1803,10 +1803,11 @@ __global__ void __launch_bounds__(128) k_cp_force32_vh(DevCfg c, int64_t n, cons
 
 }  // namespace
 
-void cpl_count_tables(sphdem_ctx *c, AdjointData *a) {
+bool cpl_count_tables(sphdem_ctx *c, AdjointData *a) {
+    const bool kept = a->dpos != nullptr;
     /* the coupling pairs of the current buckets, counted with the tap's own
      * scan (a->slot is a device int the replay resets before use) */
-    SPHDEM_CUDA_CHECK(cudaMalloc(&a->dpos, (size_t)c->n * sizeof(float4)));
+    if (!kept) SPHDEM_CUDA_CHECK(cudaMalloc(&a->dpos, (size_t)c->n * sizeof(float4)));
     SPHDEM_CUDA_CHECK(cudaMemsetAsync(a->slot, 0, sizeof(int), c->stream));
     k_cp_dpos<<<grid_for(c->n, 256), 256, 0, c->stream>>>(c->A, c->g, c->n, a->dpos);
     k_cp_cpl_table<<<grid_for(c->n, CB), CB, 0, c->stream>>>(c->cfg, c->A, c->buf.start, c->g, c->n, a->dpos,
@@ -1814,18 +1815,22 @@ void cpl_count_tables(sphdem_ctx *c, AdjointData *a) {
     int nc = 0;
     SPHDEM_CUDA_CHECK(cudaMemcpyAsync(&nc, a->slot, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     SPHDEM_CUDA_CHECK(cudaStreamSynchronize(c->stream));
-    a->cpl.cap = (int64_t)nc + nc / 2 + 4096;
+    const int64_t need = table_need(nc);
+    if (kept && need > a->cpl.cap) return false;
+    if (!kept) a->cpl.cap = table_room(need);
     std::vector<int> iam(c->n), tags;
     field_get_int(c, FI_IAM, iam.data());   /* tag order */
     for (int64_t i = 0; i < c->n; i++)
         if (iam[i] == T_DEM) tags.push_back((int)i);
+    if (kept && (int)tags.size() != a->n_dem) return false;
     a->n_dem = (int)tags.size();
     a->fpi.cap = (int64_t)std::max(1, a->n_dem) * CP_FPI_PER;
     a->ct_cap = (int64_t)std::max(1, a->n_dem) * ADJ_MAX_CONTACTS;
     if (!tags.empty()) {
-        SPHDEM_CUDA_CHECK(cudaMalloc(&a->dem_tags, tags.size() * sizeof(int)));
+        if (!a->dem_tags) SPHDEM_CUDA_CHECK(cudaMalloc(&a->dem_tags, tags.size() * sizeof(int)));
         SPHDEM_CUDA_CHECK(cudaMemcpy(a->dem_tags, tags.data(), tags.size() * sizeof(int), cudaMemcpyHostToDevice));
     }
+    return true;
 }
 
 void cpl_alloc(sphdem_ctx *c, AdjointData *a) {
@@ -1902,12 +1907,15 @@ void cpl_reset_segment(sphdem_ctx *c, AdjointData *a) {
     }
 }
 
-const TapTables *cpl_forward_taps(sphdem_ctx *c, AdjointData *a) {
-    if (c->cfg.precision != SPHDEM_PREC_MIXED || c->mx_maxn <= 0) return nullptr;
+bool cpl_scan_taps() {
     /* SPHDEM_ADJ_SCAN_TAPS=1: scan for the tables after each phase as FP64
      * handles do (the tests compare both forms) */
     const char *e = getenv("SPHDEM_ADJ_SCAN_TAPS");
-    if (e && e[0] == '1') return nullptr;
+    return e && e[0] == '1';
+}
+
+const TapTables *cpl_forward_taps(sphdem_ctx *c, AdjointData *a) {
+    if (c->cfg.precision != SPHDEM_PREC_MIXED || c->mx_maxn <= 0 || a->scan_taps) return nullptr;
     TapTables &t = a->tap;
     t.cpl = TapTable{a->cpl.nb, a->cpl.oc, a->cpl.cnt, a->cpl.cap, 0};
     t.fpi = TapTable{a->fpi.nb, a->fpi.oc, a->fpi.cnt, a->fpi.cap, CP_FPI_PER};

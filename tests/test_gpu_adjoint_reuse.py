@@ -1,0 +1,59 @@
+"""Repeated gradient passes on one handle (-m gpu).  The buffers and replay
+graphs of a pass serve the next one of the same form; passes of another length
+or tape memory, from a state of more pairs, and after an insertion are opened
+anew.  Each must give the gradients of the same pass on a fresh handle: bit for
+bit in the position gradients, whose sums have a fixed order; the scalar
+gradient is summed by atomics over the warps (1e-9)."""
+import numpy as np
+import pytest
+
+from sphdem import capi, cases
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def lib():
+    import __graft_entry__
+    __graft_entry__.build()
+    return capi.Library()
+
+
+def one_pass(sim, r, steps, every, mem, seed):
+    sim.set(capi.ParticleBuffers(sim.n, {"r": r}, fields=("r",)), capi.FIELD_R)
+    sim.rebuild()
+    sim.rebuild()
+    sim.adjoint_set_tape_memory(mem)
+    sim.adjoint_forward(steps, every)
+    g, dr, dv, dvh = sim.adjoint_backward(dL_dr=seed, dL_dv=0.1 * seed)
+    return dr, dv, dvh, g.viscosity
+
+
+@pytest.mark.parametrize("prec", [cases.PREC_FP64, cases.PREC_MIXED])
+def test_repeated_passes_equal_fresh_handles(lib, prec):
+    case = cases.dambreak2d(dx=0.05)
+    rng = np.random.default_rng(9)
+    n, fluid = case.n, case.particles["iam"] == cases.SPH
+    seed = rng.standard_normal((n, 3)) * fluid[:, None]
+    seed[:, 2] = 0.0
+    r0 = case.particles["r"].copy()
+    squeezed = r0.copy()
+    squeezed[fluid, 1] *= 0.6          # more pairs than the first pass's tables hold
+    shifted = r0 + 1e-3 * rng.standard_normal(r0.shape) * fluid[:, None] * np.array([1.0, 1.0, 0.0])
+    plan = [(r0, 4, 2, -1), (shifted, 4, 2, -1), (r0, 4, 2, -1), (squeezed, 4, 2, -1), (r0, 4, 2, 0), (r0, 3, 2, 0),
+            (shifted, 3, 2, 0)]
+    kept = capi.Simulation(lib, case.cfg, case.particles, precision=prec)
+    start = kept.get()
+    state = {k: np.array(start[k]) for k in ("v", "vhat", "f", "dens", "dddt")}
+    for r, steps, every, mem in plan:
+        got = []
+        for sim in (kept, capi.Simulation(lib, case.cfg, case.particles, precision=prec)):
+            buf = capi.ParticleBuffers(n, state, fields=tuple(state))
+            sim.set(buf, capi.FIELD_V | capi.FIELD_VHAT | capi.FIELD_F | capi.FIELD_DENS | capi.FIELD_DDDT)
+            got.append(one_pass(sim, r, steps, every, mem, seed))
+            if sim is not kept:
+                sim.close()
+        for a, b in zip(got[0][:3], got[1][:3]):
+            assert np.array_equal(a, b)
+        assert abs(got[0][3] - got[1][3]) <= 1e-9 * abs(got[1][3])
+    kept.close()
