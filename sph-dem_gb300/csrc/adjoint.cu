@@ -61,6 +61,7 @@
 #include <vector>
 
 #include "adjoint.cuh"
+#include "mixed.cuh"
 
 namespace sphdem {
 
@@ -262,14 +263,24 @@ __device__ __forceinline__ int sph_pairs_of(const DevCfg &c, const DevState &s, 
  * nb[slot * cap + ...] = partner entries, oc[slot * n + tag_a] = (offset,
  * count), cnt[slot] = entries used.  One atomic per warp reserves the warp's
  * entries.  With nb == nullptr only cnt[0] is counted.  An overflowing
- * particle records count 0 and the caller sees cnt > cap. */
+ * particle records count 0 and the caller sees cnt > cap.  An FP64 scan of the
+ * buckets costs as much as the step's force pass, so a tape reads the phase's
+ * neighbour lists (nbr; a step with its tape 0.51 -> 0.28 ms at 23,018 particles). */
 __global__ void k_sph_pairs(DevCfg c, DevState s, const int *start, const int *skey, const DevGlobals *g, int64_t n,
-                            int *nb, int2 *oc, int *cnt, int64_t cap, const int *slot) {
+                            int *nb, int2 *oc, int *cnt, int64_t cap, const int *slot, const int *nbr, const int *ncnt,
+                            int64_t ld) {
     const int64_t a = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     const int dims[3] = {g->sdims[0], g->sdims[1], g->sdims[2]};
     const bool live = a < n && is_sph_or_sphb(s.irow(FI_IAM)[a]);
     const int j = slot ? *slot : 0;
-    const int k = live ? sph_pairs_of<false>(c, s, start, skey, dims, a, nullptr, 0) : 0;
+    /* from the phase's neighbour list where the particle has one */
+    const int m = live && nbr ? ncnt[a] : -1;
+    int k = 0;
+    if (m >= 0) {
+        for (int q = 0; q < m; q++) k += nbr[nl_at(a, q, ld)] >= 0;
+    } else if (live) {
+        k = sph_pairs_of<false>(c, s, start, skey, dims, a, nullptr, 0);
+    }
     const int lane = threadIdx.x & 31;
     int incl = k;
     for (int o = 1; o < 32; o <<= 1) {
@@ -284,7 +295,20 @@ __global__ void k_sph_pairs(DevCfg c, DevState s, const int *start, const int *s
     const int64_t off = (int64_t)base + incl - k;
     const int64_t room = cap - off;
     int *out = nb + (int64_t)j * cap + off;
-    sph_pairs_of<true>(c, s, start, skey, dims, a, out, room > 0 ? room : 0);
+    if (m < 0) {
+        sph_pairs_of<true>(c, s, start, skey, dims, a, out, room > 0 ? room : 0);
+    } else {
+        const CellCoord cc = decode_cell(skey[a], dims, c.nd);
+        int w = 0;
+        for (int q = 0; q < m && w < room; q++) {
+            const int e = nbr[nl_at(a, q, ld)];
+            if (e < 0) continue;
+            int o[3], sh[3] = {0, 0, 0};
+            nl_decode_code(e >> B_BITS, o);
+            for (int d = 0; d < c.nd; d++) sh[d] = cc.c[d] + o[d] < 0 ? -1 : (cc.c[d] + o[d] >= dims[d] ? 1 : 0);
+            out[w++] = s.irow(FI_TAG)[e & B_MASK] | shift_code(sh);
+        }
+    }
     oc[(int64_t)j * n + s.irow(FI_TAG)[a]] = make_int2((int)off, room >= k ? k : 0);
 }
 
@@ -412,24 +436,23 @@ __global__ void k_vjp_assemble(int64_t n, double dt, double *adj, const double *
 
 /* VJP of the force of the ordered pair (x, y) on x,
  *   T = [m_y Pi - m_y (pdr2_x + pdr2_y)] G(r) d,  d = r_x - r_y, w = vh_x - vh_y,
- * against the adjoint Fb of f_x.  Adds sign * dT/dd^T Fb to Db and
+ * against the adjoint Fb of f_x (ir = 1/r, rs = 1/(rho_x + rho_y)).  Adds sign * dT/dd^T Fb to Db and
  * sign * dT/dw^T Fb to Wb (sign -1 when the caller is y), and the adjoints of
  * rho_x (= that of rho_y) to Rb, of pdr2_x (= pdr2_y) to Qb, of alpha to Ab. */
-__device__ __forceinline__ void force_pair_vjp(const DevCfg &c, const double *d, const double *w, double r,
-                                               double G, double Gp, const double *Fb, double my, double rhox,
-                                               double rhoy, double pdr2x, double pdr2y, double sign, double *Db,
+__device__ __forceinline__ void force_pair_vjp(const DevCfg &c, const double *d, const double *w,
+                                               double ir, double rs, double G, double Gp, const double *Fb,
+                                               double my, double pdr2x, double pdr2y, double sign, double *Db,
                                                double *Wb, double &Rb, double &Qb, double &Ab) {
     double P = 0.0, vdr = 0.0;
     for (int k = 0; k < c.nd; k++) {
         P += Fb[k] * d[k];
         vdr += d[k] * w[k];
     }
-    const double ir = 1.0 / r;
     double s = -my * (pdr2x + pdr2y);
     Qb += -my * G * P;
     double coefw = 0.0, coefd = 0.0;
     if (vdr < 0.0) {
-        const double viss = vdr * ir, rs = 1.0 / (rhox + rhoy);
+        const double viss = vdr * ir;
         const double Pi = c.alpha_art * viss * (2.0 * c.spsound - 4.0 * viss) * rs;
         const double dPi = c.alpha_art * (2.0 * c.spsound - 8.0 * viss) * rs;
         const double K = G * P;
@@ -462,18 +485,23 @@ __global__ void k_sadj_pre(DevCfg c, int64_t n, double dt, const double *s0, con
     o[7] = c.prb * (q2 * q2 * q2 * q - 1.0) / (rho * rho);
 }
 
-/* continuity (end phase, pairs at r1): adjoints of r1 and vh1, then of f1 */
+/* continuity (end phase, pairs at r1): adjoints of r1 and vh1, then of f1.  This
+ * and k_sadj_mid were bound by the FP64 pipe, mostly by the divisions and the
+ * root of a pair: 0.66 ms a step of 23,018 particles in 2D, 0.27 with rcp_pos and
+ * sqrt_pos, the kernel's closed form and ADJ_LANES lanes per particle. */
 __global__ void k_sadj_end(DevCfg c, int64_t n, double dt, const double *s1, const double *mass, const double *hh,
                            const int *typ, const int *nb, const int2 *oc, const double *adj, double *racc,
                            double *vh1b, double *fbar) {
-    const int64_t a = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (a >= n) return;
+    const int64_t t = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / ADJ_LANES;
+    const int sub = threadIdx.x % ADJ_LANES;
+    const bool act = t < n;
+    const int64_t a = act ? t : 0;
     const double hd = 0.5 * dt;
     const double *xa = s1 + a * ADJ_NC, *aa = adj + a * ADJ_NC;
     const double Da = aa[13] + hd * aa[12], ma = mass[a], ha = hh[a];
     double rb[3] = {0, 0, 0}, wb[3] = {0, 0, 0};
-    const int2 o = oc[a];
-    for (int k = 0; k < o.y; k++) {
+    const int2 o = act ? oc[a] : make_int2(0, 0);
+    for (int k = sub; k < o.y; k += ADJ_LANES) {
         const int e = nb[o.x + k];
         const int b = e & ((1 << SH_SHIFT) - 1);
         const int code = (int)((unsigned)e >> SH_SHIFT);
@@ -486,17 +514,23 @@ __global__ void k_sadj_end(DevCfg c, int64_t n, double dt, const double *s1, con
             r2 += d[q] * d[q];
             wd += w[q] * d[q];
         }
-        const double r = sqrt(r2);
+        double ir;
+        const double r = sqrt_pos(r2, &ir);
         if (!(r > 0.0)) continue;
         double G, Gp;
         grad_factor(c, r, ha, hh[b], G, Gp);
         /* own term m_b D_a and the partner's m_a D_b: d and w flip sign together */
         const double coef = mass[b] * Da + ma * (ab[13] + hd * ab[12]);
         for (int q = 0; q < c.nd; q++) {
-            rb[q] += coef * (G * w[q] + Gp * wd * d[q] / r);
+            rb[q] += coef * (G * w[q] + Gp * wd * d[q] * ir);
             wb[q] += coef * G * d[q];
         }
     }
+    for (int q = 0; q < 3; q++) {
+        rb[q] = lane_sum<ADJ_LANES>(rb[q]);
+        wb[q] = lane_sum<ADJ_LANES>(wb[q]);
+    }
+    if (!act || sub) return;
     const bool sph = typ[a] == T_SPH;
     for (int q = 0; q < 3; q++) {
         const double rt = aa[q] + rb[q];                 /* r1 = r_s + hd vh1 */
@@ -512,45 +546,56 @@ __global__ void k_sadj_end(DevCfg c, int64_t n, double dt, const double *s1, con
 __global__ void k_sadj_mid(DevCfg c, int64_t n, double dt, const double *aux, const double *mass, const double *hh,
                            const int *typ, const int *nb, const int2 *oc, const double *fbar, const double *racc,
                            const double *vh1b, double *adj, double *grads) {
-    const int64_t a = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t t = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / ADJ_LANES;
+    const int sub = threadIdx.x % ADJ_LANES;
+    const bool act = t < n;
+    const int64_t a = act ? t : 0;
     double Ab = 0.0;
-    if (a < n) {
-        const double hd = 0.5 * dt;
-        const double *xa = aux + a * ADJ_AUX;
-        const double ma = mass[a], ha = hh[a];
-        const bool sph_a = typ[a] == T_SPH;
-        double Fa[3] = {0, 0, 0};
-        for (int q = 0; q < c.nd; q++) Fa[q] = fbar[a * 3 + q];
-        double Db[3] = {0, 0, 0}, Wb[3] = {0, 0, 0}, Rb = 0.0, Qb = 0.0, Adum = 0.0;
-        const int2 o = oc[a];
-        for (int k = 0; k < o.y; k++) {
-            const int e = nb[o.x + k];
-            const int b = e & ((1 << SH_SHIFT) - 1);
-            const int code = (int)((unsigned)e >> SH_SHIFT);
-            const int sh[3] = {(code & 3) - 1, ((code >> 2) & 3) - 1, ((code >> 4) & 3) - 1};
-            const double *xb = aux + (int64_t)b * ADJ_AUX;
-            double d[3] = {0, 0, 0}, w[3] = {0, 0, 0}, md[3] = {0, 0, 0}, mw[3] = {0, 0, 0}, r2 = 0.0;
-            for (int q = 0; q < c.nd; q++) {
-                d[q] = xa[q] - image_pos(xb[q], sh[q], c.rmin[q], c.rmax[q]);
-                w[q] = xa[3 + q] - xb[3 + q];
-                md[q] = -d[q];
-                mw[q] = -w[q];
-                r2 += d[q] * d[q];
-            }
-            const double r = sqrt(r2);
-            if (!(r > 0.0)) continue;
-            double G, Gp;
-            grad_factor(c, r, ha, hh[b], G, Gp);
-            /* a's own pair (a, b); an SPHB particle's force is read by nothing */
-            if (sph_a)
-                force_pair_vjp(c, d, w, r, G, Gp, Fa, mass[b], xa[6], xb[6], xa[7], xb[7], 1.0, Db, Wb, Rb, Qb, Ab);
-            /* the partner's pair (b, a): r_a and vh_a enter it with a minus sign */
-            if (typ[b] == T_SPH) {
-                double Fbv[3] = {0, 0, 0};
-                for (int q = 0; q < c.nd; q++) Fbv[q] = fbar[(int64_t)b * 3 + q];
-                force_pair_vjp(c, md, mw, r, G, Gp, Fbv, ma, xb[6], xa[6], xb[7], xa[7], -1.0, Db, Wb, Rb, Qb, Adum);
-            }
+    const double hd = 0.5 * dt;
+    const double *xa = aux + a * ADJ_AUX;
+    const double ma = mass[a], ha = hh[a];
+    const bool sph_a = typ[a] == T_SPH;
+    double Fa[3] = {0, 0, 0};
+    for (int q = 0; q < c.nd; q++) Fa[q] = fbar[a * 3 + q];
+    double Db[3] = {0, 0, 0}, Wb[3] = {0, 0, 0}, Rb = 0.0, Qb = 0.0, Adum = 0.0;
+    const int2 o = act ? oc[a] : make_int2(0, 0);
+    for (int k = sub; k < o.y; k += ADJ_LANES) {
+        const int e = nb[o.x + k];
+        const int b = e & ((1 << SH_SHIFT) - 1);
+        const int code = (int)((unsigned)e >> SH_SHIFT);
+        const int sh[3] = {(code & 3) - 1, ((code >> 2) & 3) - 1, ((code >> 4) & 3) - 1};
+        const double *xb = aux + (int64_t)b * ADJ_AUX;
+        double d[3] = {0, 0, 0}, w[3] = {0, 0, 0}, md[3] = {0, 0, 0}, mw[3] = {0, 0, 0}, r2 = 0.0;
+        for (int q = 0; q < c.nd; q++) {
+            d[q] = xa[q] - image_pos(xb[q], sh[q], c.rmin[q], c.rmax[q]);
+            w[q] = xa[3 + q] - xb[3 + q];
+            md[q] = -d[q];
+            mw[q] = -w[q];
+            r2 += d[q] * d[q];
         }
+        double ir;
+        const double r = sqrt_pos(r2, &ir);
+        if (!(r > 0.0)) continue;
+        const double rs = rcp_pos(xa[6] + xb[6]);
+        double G, Gp;
+        grad_factor(c, r, ha, hh[b], G, Gp);
+        /* a's own pair (a, b); an SPHB particle's force is read by nothing */
+        if (sph_a)
+            force_pair_vjp(c, d, w, ir, rs, G, Gp, Fa, mass[b], xa[7], xb[7], 1.0, Db, Wb, Rb, Qb, Ab);
+        /* the partner's pair (b, a): r_a and vh_a enter it with a minus sign */
+        if (typ[b] == T_SPH) {
+            double Fbv[3] = {0, 0, 0};
+            for (int q = 0; q < c.nd; q++) Fbv[q] = fbar[(int64_t)b * 3 + q];
+            force_pair_vjp(c, md, mw, ir, rs, G, Gp, Fbv, ma, xb[7], xa[7], -1.0, Db, Wb, Rb, Qb, Adum);
+        }
+    }
+    for (int q = 0; q < 3; q++) {
+        Db[q] = lane_sum<ADJ_LANES>(Db[q]);
+        Wb[q] = lane_sum<ADJ_LANES>(Wb[q]);
+    }
+    Rb = lane_sum<ADJ_LANES>(Rb);
+    Qb = lane_sum<ADJ_LANES>(Qb);
+    if (act && sub == 0) {
         /* EOS: d pdr2 / d rho = PRB (5 x^7 + 2) / rho^3, x = rho / refd */
         const double rho = xa[6], x = rho / c.refd, x2 = x * x;
         const double dpdr2 = c.prb * (5.0 * (x2 * x2 * x2 * x) + 2.0) / (rho * rho * rho);
@@ -616,14 +661,15 @@ __device__ __forceinline__ void force_pair_vjp32(float alpha, float c0, const fl
     for (int k = 0; k < ND; k++) Db[k].add(sign * (s * (G * Fb[k] + gpd * d[k]) + coefw * w[k] + coefd * d[k]));
 }
 
-/* decode a table entry: partner tag and the image displacement to add */
+/* decode a table entry: partner tag and the image displacement to add; L: the
+ * periods */
 template <int ND>
-__device__ __forceinline__ int entry_of(const DevCfg &c, int e, float *img) {
+__device__ __forceinline__ int entry_of(const float *L, int e, float *img) {
     const int code = (int)((unsigned)e >> SH_SHIFT);
 #pragma unroll
     for (int q = 0; q < ND; q++) {
         const int sh = ((code >> (2 * q)) & 3) - 1;
-        img[q] = sh == 0 ? 0.f : (float)(sh * (c.rmax[q] - c.rmin[q]));
+        img[q] = sh == 0 ? 0.f : (sh > 0 ? L[q] : -L[q]);
     }
     return e & ((1 << SH_SHIFT) - 1);
 }
@@ -659,17 +705,22 @@ template <int ND>
 __global__ void __launch_bounds__(128) k_sadj_end32(DevCfg c, int64_t n, double dt, const int *typ,
                                                     const int *__restrict__ nb, const int2 *__restrict__ oc,
                                                     const double *adj, double *racc, double *vh1b, float4 *rec) {
-    const int64_t a = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (a >= n) return;
+    const int64_t t = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / ADJ_LANES;
+    const int sub = threadIdx.x % ADJ_LANES;
+    const bool act = t < n;
+    const int64_t a = act ? t : 0;
     const float4 *E0 = rec + R_E0 * n, *E1 = rec + R_E1 * n, *E2 = rec + R_E2 * n;
+    float L[ND];
+#pragma unroll
+    for (int q = 0; q < ND; q++) L[q] = (float)(c.rmax[q] - c.rmin[q]);
     const float wcon = (float)c.wcon;
     const float4 p0 = E0[a], p1 = E1[a], p2 = E2[a];
     const float pa[3] = {p0.x, p0.y, p0.z}, la[3] = {p1.x, p1.y, p1.z}, va[3] = {p2.x, p2.y, p2.z};
     Kf rb[ND], wb[ND];
-    const int2 o = oc[a];
-    for (int k = 0; k < o.y; k++) {
+    const int2 o = act ? oc[a] : make_int2(0, 0);
+    for (int k = sub; k < o.y; k += ADJ_LANES) {
         float img[3];
-        const int b = entry_of<ND>(c, __ldg(nb + o.x + k), img);
+        const int b = entry_of<ND>(L, __ldg(nb + o.x + k), img);
         const float4 q0 = E0[b], q1 = E1[b], q2 = E2[b];
         const float pb[3] = {q0.x, q0.y, q0.z}, lb[3] = {q1.x, q1.y, q1.z}, vb[3] = {q2.x, q2.y, q2.z};
         float d[3], w[3], r2 = 0.f, wd = 0.f;
@@ -692,13 +743,20 @@ __global__ void __launch_bounds__(128) k_sadj_end32(DevCfg c, int64_t n, double 
             wb[q].add(coef * G * d[q]);
         }
     }
+    double rt_[ND], wt_[ND];
+#pragma unroll
+    for (int q = 0; q < ND; q++) {
+        rt_[q] = rb[q].total();
+        wt_[q] = wb[q].total();
+    }
+    if (!act || sub) return;
     const double hd = 0.5 * dt;
     const double *aa = adj + a * ADJ_NC;
     const bool sph = typ[a] == T_SPH;
     float F[3] = {0.f, 0.f, 0.f};
     for (int q = 0; q < 3; q++) {
-        const double rt = aa[q] + (q < ND ? rb[q].value() : 0.0);
-        const double vt = aa[6 + q] + (q < ND ? wb[q].value() : 0.0) + hd * rt;
+        const double rt = aa[q] + (q < ND ? rt_[q] : 0.0);
+        const double vt = aa[6 + q] + (q < ND ? wt_[q] : 0.0) + hd * rt;
         racc[a * 3 + q] = rt;
         vh1b[a * 3 + q] = vt;
         F[q] = sph ? (float)(aa[9 + q] + dt * (vt + aa[3 + q])) : 0.f;
@@ -713,53 +771,66 @@ __global__ void __launch_bounds__(128) k_sadj_mid32(DevCfg c, int64_t n, double 
                                                     const int2 *__restrict__ oc, const double *racc,
                                                     const double *vh1b, const float4 *__restrict__ rec, double *adj,
                                                     double *grads) {
-    const int64_t a = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t t = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / ADJ_LANES;
+    const int sub = threadIdx.x % ADJ_LANES;
+    const bool act = t < n;
+    const int64_t a = act ? t : 0;
     float Ab = 0.f;
-    if (a < n) {
-        const float4 *M0 = rec + R_M0 * n, *M1 = rec + R_M1 * n, *M2 = rec + R_M2 * n, *M3 = rec + R_M3 * n;
-        const float wcon = (float)c.wcon, alpha = (float)c.alpha_art, c0 = (float)c.spsound;
-        const float4 p0 = M0[a], p1 = M1[a], p2 = M2[a], p3 = M3[a];
-        const float pa[3] = {p0.x, p0.y, p0.z}, la[3] = {p1.x, p1.y, p1.z}, va[3] = {p2.x, p2.y, p2.z};
-        const float Fa[3] = {p3.x, p3.y, p3.z};
-        const bool own = Fa[0] != 0.f || Fa[1] != 0.f || Fa[2] != 0.f;
-        Kf Db[ND], Wb[ND], Rb, Qb;
-        float Adum = 0.f;
-        const int2 o = oc[a];
-        for (int k = 0; k < o.y; k++) {
-            float img[3];
-            const int b = entry_of<ND>(c, __ldg(nb + o.x + k), img);
-            const float4 q0 = M0[b], q1 = M1[b], q2 = M2[b], q3 = M3[b];
-            const float pb[3] = {q0.x, q0.y, q0.z}, lb[3] = {q1.x, q1.y, q1.z}, vb[3] = {q2.x, q2.y, q2.z};
-            const float Fb[3] = {q3.x, q3.y, q3.z};
-            float d[3], w[3], md[3], mw[3], r2 = 0.f;
+    const float4 *M0 = rec + R_M0 * n, *M1 = rec + R_M1 * n, *M2 = rec + R_M2 * n, *M3 = rec + R_M3 * n;
+    float L[ND];
 #pragma unroll
-            for (int q = 0; q < ND; q++) {
-                d[q] = ((pa[q] - pb[q]) + (la[q] - lb[q])) - img[q];
-                w[q] = va[q] - vb[q];
-                md[q] = -d[q];
-                mw[q] = -w[q];
-                r2 = fmaf(d[q], d[q], r2);
-            }
-            if (!(r2 > 0.f)) continue;
-            const float r = sqrtf(r2);
-            float G, Gp;
-            grad_factor32<ND>(wcon, r, p0.w, q0.w, G, Gp);
-            if (own)
-                force_pair_vjp32<ND>(alpha, c0, d, w, r, G, Gp, Fa, q1.w, p2.w, q2.w, p3.w, q3.w, 1.f, Db, Wb, Rb, Qb,
-                                     Ab);
-            if (Fb[0] != 0.f || Fb[1] != 0.f || Fb[2] != 0.f)
-                force_pair_vjp32<ND>(alpha, c0, md, mw, r, G, Gp, Fb, p1.w, q2.w, p2.w, q3.w, p3.w, -1.f, Db, Wb, Rb,
-                                     Qb, Adum);
+    for (int q = 0; q < ND; q++) L[q] = (float)(c.rmax[q] - c.rmin[q]);
+    const float wcon = (float)c.wcon, alpha = (float)c.alpha_art, c0 = (float)c.spsound;
+    const float4 p0 = M0[a], p1 = M1[a], p2 = M2[a], p3 = M3[a];
+    const float pa[3] = {p0.x, p0.y, p0.z}, la[3] = {p1.x, p1.y, p1.z}, va[3] = {p2.x, p2.y, p2.z};
+    const float Fa[3] = {p3.x, p3.y, p3.z};
+    const bool own = Fa[0] != 0.f || Fa[1] != 0.f || Fa[2] != 0.f;
+    Kf Db[ND], Wb[ND], Rb, Qb;
+    float Adum = 0.f;
+    const int2 o = act ? oc[a] : make_int2(0, 0);
+    for (int k = sub; k < o.y; k += ADJ_LANES) {
+        float img[3];
+        const int b = entry_of<ND>(L, __ldg(nb + o.x + k), img);
+        const float4 q0 = M0[b], q1 = M1[b], q2 = M2[b], q3 = M3[b];
+        const float pb[3] = {q0.x, q0.y, q0.z}, lb[3] = {q1.x, q1.y, q1.z}, vb[3] = {q2.x, q2.y, q2.z};
+        const float Fb[3] = {q3.x, q3.y, q3.z};
+        float d[3], w[3], md[3], mw[3], r2 = 0.f;
+#pragma unroll
+        for (int q = 0; q < ND; q++) {
+            d[q] = ((pa[q] - pb[q]) + (la[q] - lb[q])) - img[q];
+            w[q] = va[q] - vb[q];
+            md[q] = -d[q];
+            mw[q] = -w[q];
+            r2 = fmaf(d[q], d[q], r2);
         }
+        if (!(r2 > 0.f)) continue;
+        const float r = sqrtf(r2);
+        float G, Gp;
+        grad_factor32<ND>(wcon, r, p0.w, q0.w, G, Gp);
+        if (own)
+            force_pair_vjp32<ND>(alpha, c0, d, w, r, G, Gp, Fa, q1.w, p2.w, q2.w, p3.w, q3.w, 1.f, Db, Wb, Rb, Qb,
+                                 Ab);
+        if (Fb[0] != 0.f || Fb[1] != 0.f || Fb[2] != 0.f)
+            force_pair_vjp32<ND>(alpha, c0, md, mw, r, G, Gp, Fb, p1.w, q2.w, p2.w, q3.w, p3.w, -1.f, Db, Wb, Rb,
+                                 Qb, Adum);
+    }
+    double Dt[ND], Wt[ND];
+#pragma unroll
+    for (int q = 0; q < ND; q++) {
+        Dt[q] = Db[q].total();
+        Wt[q] = Wb[q].total();
+    }
+    const double Rt = Rb.total(), Qt = Qb.total();
+    if (act && sub == 0) {
         const double hd = 0.5 * dt;
         const double *x0 = s0 + a * ADJ_NC;
         const double rho = x0[12] + hd * x0[13], x = rho / c.refd, x2 = x * x;
         const double dpdr2 = c.prb * (5.0 * (x2 * x2 * x2 * x) + 2.0) / (rho * rho * rho);
         double *aa = adj + a * ADJ_NC;
-        const double rhos_b = aa[12] + Rb.value() + Qb.value() * dpdr2;
+        const double rhos_b = aa[12] + Rt + Qt * dpdr2;
         const bool sph_a = typ[a] == T_SPH;
         for (int q = 0; q < 3; q++) {
-            const double D = q < ND ? Db[q].value() : 0.0, W = q < ND ? Wb[q].value() : 0.0;
+            const double D = q < ND ? Dt[q] : 0.0, W = q < ND ? Wt[q] : 0.0;
             const double rs_b = racc[a * 3 + q] + D;
             aa[q] = rs_b;
             aa[6 + q] = vh1b[a * 3 + q] + W + hd * rs_b;
@@ -801,7 +872,8 @@ int one_step(sphdem_ctx *c) {
 void sph_pairs(sphdem_ctx *c, int *nb, int2 *oc, int *cnt, const int *slot) {
     AdjointData *a = c->adj;
     k_sph_pairs<<<grid_for(c->n, 128), 128, 0, c->stream>>>(c->cfg, c->A, c->buf.start, c->buf.skey, c->g, c->n, nb,
-                                                            oc, cnt, a->pair_cap, slot);
+                                                            oc, cnt, a->pair_cap, slot, nb && c->f64_maxn > 0 ? c->mx_nbr : nullptr,
+                                                            c->mx_ncnt, c->f64_maxn);
 }
 
 /* One replayed fluid or coupled step with its taps, as a CUDA graph (one per
@@ -907,9 +979,9 @@ void backward_sph(sphdem_ctx *c, AdjointData *a, int steps, double dt) {
                                                                     a->typ, a->rec);
 #define L_(ND)                                                                                                  \
     do {                                                                                                        \
-        k_sadj_end32<ND><<<grid_for(n, 128), 128, 0, c->stream>>>(c->cfg, n, dt, a->typ, nbe, oce, a->adj, a->racc, \
+        k_sadj_end32<ND><<<grid_for(n * ADJ_LANES, 128), 128, 0, c->stream>>>(c->cfg, n, dt, a->typ, nbe, oce, a->adj, a->racc, \
                                                                   a->vmacc, a->rec);                             \
-        k_sadj_mid32<ND><<<grid_for(n, 128), 128, 0, c->stream>>>(c->cfg, n, dt, s0, a->typ, nbm, ocm, a->racc,     \
+        k_sadj_mid32<ND><<<grid_for(n * ADJ_LANES, 128), 128, 0, c->stream>>>(c->cfg, n, dt, s0, a->typ, nbm, ocm, a->racc,     \
                                                                   a->vmacc, a->rec, a->adj, a->grads);           \
     } while (0)
             if (c->cfg.nd == 3) L_(3);
@@ -919,9 +991,9 @@ void backward_sph(sphdem_ctx *c, AdjointData *a, int steps, double dt) {
             continue;
         }
         k_sadj_pre<<<grid_for(n, ABLK), ABLK, 0, c->stream>>>(c->cfg, n, dt, s0, a->typ, a->aux);
-        k_sadj_end<<<grid_for(n, 128), 128, 0, c->stream>>>(c->cfg, n, dt, s1, a->mass, a->hh, a->typ, nbe, oce,
+        k_sadj_end<<<grid_for(n * ADJ_LANES, 128), 128, 0, c->stream>>>(c->cfg, n, dt, s1, a->mass, a->hh, a->typ, nbe, oce,
                                                             a->adj, a->racc, a->vmacc, a->fbar);
-        k_sadj_mid<<<grid_for(n, 128), 128, 0, c->stream>>>(c->cfg, n, dt, a->aux, a->mass, a->hh, a->typ, nbm, ocm,
+        k_sadj_mid<<<grid_for(n * ADJ_LANES, 128), 128, 0, c->stream>>>(c->cfg, n, dt, a->aux, a->mass, a->hh, a->typ, nbm, ocm,
                                                             a->fbar, a->racc, a->vmacc, a->adj, a->grads);
     }
 }

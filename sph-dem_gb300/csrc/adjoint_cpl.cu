@@ -329,14 +329,14 @@ __global__ void k_cp_tap_r(DevState s, int64_t n, double *rmid, const int *slot)
 /* ---- reverse pass of one step ------------------------------------------ */
 
 __device__ __forceinline__ void image_d(const DevCfg &c, const double *ra, const double *rb, const int *sh,
-                                        double *d, double &r) {
+                                        double *d, double &r, double *ir = nullptr) {
     double r2 = 0.0;
     for (int q = 0; q < 3; q++) d[q] = 0.0;
     for (int q = 0; q < c.nd; q++) {
         d[q] = ra[q] - image_pos(rb[q], sh[q], c.rmin[q], c.rmax[q]);
         r2 += d[q] * d[q];
     }
-    r = sqrt(r2);
+    r = sqrt_pos(r2, ir);
 }
 
 /* coupling kernel W_c(r) = C_c K(2r/Rc) and dW_c/dr (sph.h:1246-1256) */
@@ -573,17 +573,14 @@ __device__ __noinline__ double difelice_vjp(const DevCfg &c, const double *dv, d
  * particle's share.  Delta_i's adjoint is that of f1 + fdrag1.  Pair math in
  * M, per-particle math in FP64. */
 template <typename M>
-__global__ void k_cp_fpi(DevCfg c, int n_dem, const int *dem_tags, double dt, const double *s1, const double *aux,
-                         const double *cmid, const double *mass, const int *nb, const int2 *oc,
-                         const typename MT<M>::V4 *g4, const M *gw, const double *adj, double *cacc, double *coef,
-                         double *grads) {
+__global__ void k_cp_fpi_sums(DevCfg c, int n_dem, const int *dem_tags, const double *s1, const double *aux,
+                              const double *cmid, const double *mass, const int *nb, const int2 *oc, const M *gw,
+                              double *coef) {
     using Acc = typename MT<M>::Acc;
     const int w = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
     if (w >= n_dem) return;
     const int64_t i = dem_tags[w];
-    const double *ai = adj + i * ADJ_NC;
-    const double *vhm = aux + i * ADJ_AUX + 3;
     double *cf = coef + i * CP_NCOEF;
     const int2 o = oc[i];
     Acc sum, Npor, Nfp[3], Nfv[3], Nvel[3];
@@ -601,65 +598,104 @@ __global__ void k_cp_fpi(DevCfg c, int n_dem, const int *dem_tags, double dt, co
             Nvel[q3].add(dW * (M)xb[AS_VH + q3]);
         }
     }
-    const double sumv = warp_sum_d(sum.value());
-    if (!(sumv > 0.5)) {             /* no drag, Delta = 0 (uniform over the warp) */
-        if (lane == 0) cf[CF_ON] = 0.0;
-        return;
-    }
-    double npor = warp_sum_d(Npor.value()), nfp[3], nfv[3], nvel[3];
+    /* sum, porosity, fp, fv, velocity */
+    const double t0 = warp_sum_d(sum.value()), t1 = warp_sum_d(Npor.value());
+    double t[9];
     for (int q = 0; q < 3; q++) {
-        nfp[q] = warp_sum_d(Nfp[q].value());
-        nfv[q] = warp_sum_d(Nfv[q].value());
-        nvel[q] = warp_sum_d(Nvel[q].value());
+        t[q] = warp_sum_d(Nfp[q].value());
+        t[3 + q] = warp_sum_d(Nfv[q].value());
+        t[6 + q] = warp_sum_d(Nvel[q].value());
     }
-    /* the particle's own FP64 math (drag law and its VJP, with its
-     * transcendentals) once per warp, on lane 0; the lanes take the adjoints
-     * of the sums from its coefficient record */
-    if (lane == 0) {
-        const double mi = mass[i], rs = 1.0 / sumv;
-        const double por = npor * rs;
-        double fvel[3] = {0, 0, 0}, fpfb[3] = {0, 0, 0}, fvv[3] = {0, 0, 0}, dv[3] = {0, 0, 0}, Db[3] = {0, 0, 0};
-        for (int q = 0; q < c.nd; q++) {
-            fvel[q] = nvel[q] * rs;
-            fpfb[q] = nfp[q] * rs;
-            fvv[q] = nfv[q] * rs;
-            dv[q] = por * (fvel[q] - vhm[q]);
-            Db[q] = ai[AS_F + q] + dt * (ai[AS_V + q] + ai[AS_VH + q]) + ai[AS_FDRAG + q];
-        }
-        /* Delta = (V/m)(fv + fpfb) + (rho0/m) kappa Phi */
-        double phi[3];
-        difelice(c, dv, por, phi);
-        double Pb[3] = {0, 0, 0}, dvb[3] = {0, 0, 0}, porb = 0.0, gkap = 0.0;
-        for (int q = 0; q < c.nd; q++) {
-            Pb[q] = (c.dens / mi) * c.drag_scale * Db[q];
-            gkap += (c.dens / mi) * Db[q] * phi[q];
-        }
-        const double gnu = difelice_vjp(c, dv, por, Pb, dvb, porb);
-        double fvelb[3] = {0, 0, 0};
-        double *acc = cacc + i * CP_NACC;
-        for (int q = 0; q < c.nd; q++) {
-            fvelb[q] = por * dvb[q];
-            acc[CA_VH1 + q] += -por * dvb[q];
-            porb += (fvel[q] - vhm[q]) * dvb[q];
-        }
-        const double vm = c.dem_vol / mi;
-        double sumb = -porb * por;
-        cf[CF_ON] = 1.0;
+    if (lane) return;
+    cf[0] = t0;
+    cf[1] = t1;
+    for (int q = 0; q < 9; q++) cf[2 + q] = t[q];
+}
+
+/* the drag law and its VJP from the sums of k_cp_fpi_sums, which the record
+ * holds on entry: FP64 transcendentals, a thread per DEM particle (on one lane
+ * of a warp per particle they took 16 cycles of the FP64 pipe an instruction:
+ * the three passes 132 us for 5,000 particles, 270 in one) */
+__global__ void k_cp_fpi_drag(DevCfg c, int n_dem, const int *dem_tags, double dt, const double *aux,
+                              const double *mass, const double *adj, double *cacc, double *coef, double *grads) {
+    const int w = (int)(blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
+    double gnu = 0.0, gkap = 0.0;
+    if (w < n_dem) {
+        const int64_t i = dem_tags[w];
+        const double *ai = adj + i * ADJ_NC;
+        const double *vhm = aux + i * ADJ_AUX + 3;
+        double *cf = coef + i * CP_NCOEF;
+        const double sumv = cf[0], npor = cf[1];
+        double nfp[3], nfv[3], nvel[3];
         for (int q = 0; q < 3; q++) {
-            const bool on = q < c.nd;
-            if (on) sumb -= vm * Db[q] * fpfb[q] + vm * Db[q] * fvv[q] + fvelb[q] * fvel[q];
-            cf[CF_FP + q] = on ? vm * Db[q] * rs : 0.0;
-            cf[CF_FV + q] = on ? vm * Db[q] * rs : 0.0;
-            cf[CF_VEL + q] = on ? fvelb[q] * rs : 0.0;
+            nfp[q] = cf[2 + q];
+            nfv[q] = cf[5 + q];
+            nvel[q] = cf[8 + q];
         }
-        cf[CF_SUM] = sumb * rs;
-        cf[CF_POR] = porb * rs;
-        if (gnu != 0.0 || gkap != 0.0) {
-            atomicAdd(&grads[3], gnu);
-            atomicAdd(&grads[4], gkap);
+        if (!(sumv > 0.5)) { /* no drag, Delta = 0 */
+            cf[CF_ON] = 0.0;
+        } else {
+            const double mi = mass[i], rs = 1.0 / sumv;
+            const double por = npor * rs;
+            double fvel[3] = {0, 0, 0}, fpfb[3] = {0, 0, 0}, fvv[3] = {0, 0, 0}, dv[3] = {0, 0, 0}, Db[3] = {0, 0, 0};
+            for (int q = 0; q < c.nd; q++) {
+                fvel[q] = nvel[q] * rs;
+                fpfb[q] = nfp[q] * rs;
+                fvv[q] = nfv[q] * rs;
+                dv[q] = por * (fvel[q] - vhm[q]);
+                Db[q] = ai[AS_F + q] + dt * (ai[AS_V + q] + ai[AS_VH + q]) + ai[AS_FDRAG + q];
+            }
+            /* Delta = (V/m)(fv + fpfb) + (rho0/m) kappa Phi */
+            double phi[3];
+            difelice(c, dv, por, phi);
+            double Pb[3] = {0, 0, 0}, dvb[3] = {0, 0, 0}, porb = 0.0;
+            for (int q = 0; q < c.nd; q++) {
+                Pb[q] = (c.dens / mi) * c.drag_scale * Db[q];
+                gkap += (c.dens / mi) * Db[q] * phi[q];
+            }
+            gnu = difelice_vjp(c, dv, por, Pb, dvb, porb);
+            double fvelb[3] = {0, 0, 0};
+            double *acc = cacc + i * CP_NACC;
+            for (int q = 0; q < c.nd; q++) {
+                fvelb[q] = por * dvb[q];
+                acc[CA_VH1 + q] += -por * dvb[q];
+                porb += (fvel[q] - vhm[q]) * dvb[q];
+            }
+            const double vm = c.dem_vol / mi;
+            double sumb = -porb * por;
+            cf[CF_ON] = 1.0;
+            for (int q = 0; q < 3; q++) {
+                const bool on = q < c.nd;
+                if (on) sumb -= vm * Db[q] * fpfb[q] + vm * Db[q] * fvv[q] + fvelb[q] * fvel[q];
+                cf[CF_FP + q] = on ? vm * Db[q] * rs : 0.0;
+                cf[CF_FV + q] = on ? vm * Db[q] * rs : 0.0;
+                cf[CF_VEL + q] = on ? fvelb[q] * rs : 0.0;
+            }
+            cf[CF_SUM] = sumb * rs;
+            cf[CF_POR] = porb * rs;
         }
     }
-    __syncwarp();
+    gnu = warp_sum_d(gnu);
+    gkap = warp_sum_d(gkap);
+    if ((threadIdx.x & 31) == 0 && (gnu != 0.0 || gkap != 0.0)) {
+        atomicAdd(&grads[3], gnu);
+        atomicAdd(&grads[4], gkap);
+    }
+}
+
+/* the particle's own end position: its lanes split the partners */
+template <typename M>
+__global__ void k_cp_fpi_own(DevCfg c, int n_dem, const int *dem_tags, const double *s1, const double *aux,
+                             const double *cmid, const double *mass, const int *nb, const int2 *oc,
+                             const typename MT<M>::V4 *g4, double *cacc, const double *coef) {
+    using Acc = typename MT<M>::Acc;
+    const int w = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
+    const int lane = threadIdx.x & 31;
+    if (w >= n_dem) return;
+    const int64_t i = dem_tags[w];
+    const double *cf = coef + i * CP_NCOEF;
+    if (cf[CF_ON] == 0.0) return;
+    const int2 o = oc[i];
     const M sumbM = (M)cf[CF_SUM], NporBM = (M)cf[CF_POR];
     M NfpBM[3], NfvBM[3], NvelBM[3];
     for (int q = 0; q < 3; q++) {
@@ -870,19 +906,21 @@ __global__ void k_cp_dem(DevCfg c, int64_t n, double dt, const double *s1, const
 __global__ void k_cp_end(DevCfg c, int64_t n, double dt, const double *s1, const double *mass, const double *hh,
                          const int *typ, const int *nb, const int2 *oc, const double *adj, const double *cacc,
                          double *cend) {
-    const int64_t a = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (a >= n || !is_fluid(typ[a])) return;
+    const int64_t t = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / ADJ_LANES;
+    const int sub = threadIdx.x % ADJ_LANES;
+    const bool act = t < n && is_fluid(typ[t]);
+    const int64_t a = act ? t : 0;
     const double hd = 0.5 * dt;
     const double *xa = s1 + a * ADJ_NC, *aa = adj + a * ADJ_NC, *ac = cacc + a * CP_NACC;
     const double Da = aa[AS_DDDT] + hd * aa[AS_DENS], ma = mass[a], ha = hh[a];
     double rb[3] = {0, 0, 0}, wb[3] = {0, 0, 0};
-    const int2 o = oc[a];
-    for (int k = 0; k < o.y; k++) {
+    const int2 o = act ? oc[a] : make_int2(0, 0);
+    for (int k = sub; k < o.y; k += ADJ_LANES) {
         int sh[3];
         const int b = table_entry(nb[o.x + k], sh);
         const double *xb = s1 + (int64_t)b * ADJ_NC, *ab = adj + (int64_t)b * ADJ_NC;
-        double d[3], r, w[3] = {0, 0, 0}, wd = 0.0;
-        image_d(c, xa, xb, sh, d, r);
+        double d[3], r, ir, w[3] = {0, 0, 0}, wd = 0.0;
+        image_d(c, xa, xb, sh, d, r, &ir);
         if (!(r > 0.0)) continue;
         for (int q = 0; q < c.nd; q++) {
             w[q] = xa[AS_VH + q] - xb[AS_VH + q];
@@ -892,10 +930,15 @@ __global__ void k_cp_end(DevCfg c, int64_t n, double dt, const double *s1, const
         grad_factor(c, r, ha, hh[b], G, Gp);
         const double coef = mass[b] * Da + ma * (ab[AS_DDDT] + hd * ab[AS_DENS]);
         for (int q = 0; q < c.nd; q++) {
-            rb[q] += coef * (G * w[q] + Gp * wd * d[q] / r);
+            rb[q] += coef * (G * w[q] + Gp * wd * d[q] * ir);
             wb[q] += coef * G * d[q];
         }
     }
+    for (int q = 0; q < 3; q++) {
+        rb[q] = lane_sum<ADJ_LANES>(rb[q]);
+        wb[q] = lane_sum<ADJ_LANES>(wb[q]);
+    }
+    if (!act || sub) return;
     const bool sph = typ[a] == T_SPH;
     double *ce = cend + a * CP_NEND;
     for (int q = 0; q < 3; q++) {
@@ -948,34 +991,43 @@ __device__ __forceinline__ void cp_force_pair(const DevCfg &c, const double *d, 
 __global__ void k_cp_force(DevCfg c, int64_t n, const double *aux, const double *mass, const double *hh,
                            const int *typ, const int *nb, const int2 *oc, const double *adj, const double *cend,
                            double *cmid, double *cacc, double *grads) {
-    const int64_t a = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t t = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / ADJ_LANES;
+    const int sub = threadIdx.x % ADJ_LANES;
+    const bool act = t < n && is_fluid(typ[t]);
+    const int64_t a = act ? t : 0;
     double gnu = 0.0;
-    if (a < n && is_fluid(typ[a])) {
-        const double *xa = aux + a * ADJ_AUX, *ea = cend + a * CP_NEND;
-        const double ma = mass[a], ha = hh[a], rhoa = xa[6], pa = cmid[a * CP_NMID + CM_PDR2];
-        double Db[3] = {0, 0, 0}, Wb[3] = {0, 0, 0}, Rb = 0.0, Qb = 0.0, dum = 0.0;
-        const int2 o = oc[a];
-        for (int k = 0; k < o.y; k++) {
-            int sh[3];
-            const int b = table_entry(nb[o.x + k], sh);
-            const double *xb = aux + (int64_t)b * ADJ_AUX, *eb = cend + (int64_t)b * CP_NEND;
-            double d[3], r, w[3] = {0, 0, 0}, md[3] = {0, 0, 0}, mw[3] = {0, 0, 0};
-            image_d(c, xa, xb, sh, d, r);
-            if (!(r > 0.0)) continue;
-            for (int q = 0; q < c.nd; q++) {
-                w[q] = xa[3 + q] - xb[3 + q];
-                md[q] = -d[q];
-                mw[q] = -w[q];
-            }
-            double G, Gp;
-            grad_factor(c, r, ha, hh[b], G, Gp);
-            const double hbar = 0.5 * (ha + hh[b]);
-            const double rhob = xb[6], pb = cmid[(int64_t)b * CP_NMID + CM_PDR2];
-            cp_force_pair(c, d, w, r, G, Gp, hbar, ea + CE_P, ea + CE_V, mass[b], rhoa, rhob, pa, pb, 1.0, Db, Wb,
-                          Rb, Qb, gnu);
-            cp_force_pair(c, md, mw, r, G, Gp, hbar, eb + CE_P, eb + CE_V, ma, rhob, rhoa, pb, pa, -1.0, Db, Wb, Rb,
-                          Qb, dum);
+    const double *xa = aux + a * ADJ_AUX, *ea = cend + a * CP_NEND;
+    const double ma = mass[a], ha = hh[a], rhoa = xa[6], pa = cmid[a * CP_NMID + CM_PDR2];
+    double Db[3] = {0, 0, 0}, Wb[3] = {0, 0, 0}, Rb = 0.0, Qb = 0.0, dum = 0.0;
+    const int2 o = act ? oc[a] : make_int2(0, 0);
+    for (int k = sub; k < o.y; k += ADJ_LANES) {
+        int sh[3];
+        const int b = table_entry(nb[o.x + k], sh);
+        const double *xb = aux + (int64_t)b * ADJ_AUX, *eb = cend + (int64_t)b * CP_NEND;
+        double d[3], r, w[3] = {0, 0, 0}, md[3] = {0, 0, 0}, mw[3] = {0, 0, 0};
+        image_d(c, xa, xb, sh, d, r);
+        if (!(r > 0.0)) continue;
+        for (int q = 0; q < c.nd; q++) {
+            w[q] = xa[3 + q] - xb[3 + q];
+            md[q] = -d[q];
+            mw[q] = -w[q];
         }
+        double G, Gp;
+        grad_factor(c, r, ha, hh[b], G, Gp);
+        const double hbar = 0.5 * (ha + hh[b]);
+        const double rhob = xb[6], pb = cmid[(int64_t)b * CP_NMID + CM_PDR2];
+        cp_force_pair(c, d, w, r, G, Gp, hbar, ea + CE_P, ea + CE_V, mass[b], rhoa, rhob, pa, pb, 1.0, Db, Wb,
+                      Rb, Qb, gnu);
+        cp_force_pair(c, md, mw, r, G, Gp, hbar, eb + CE_P, eb + CE_V, ma, rhob, rhoa, pb, pa, -1.0, Db, Wb, Rb,
+                      Qb, dum);
+    }
+    for (int q = 0; q < 3; q++) {
+        Db[q] = lane_sum<ADJ_LANES>(Db[q]);
+        Wb[q] = lane_sum<ADJ_LANES>(Wb[q]);
+    }
+    Rb = lane_sum<ADJ_LANES>(Rb);
+    Qb = lane_sum<ADJ_LANES>(Qb);
+    if (act && sub == 0) {
         const double eps = cmid[a * CP_NMID + CM_EPS];
         const double x = rhoa / (c.refd * eps), x2 = x * x, x7 = x2 * x2 * x2 * x;
         const double dp_drho = c.prb * (5.0 * x7 + 2.0) / (rhoa * rhoa * rhoa);
@@ -1354,11 +1406,24 @@ __global__ void k_cp_pack32(int64_t n, double dt, const double *aux, const doubl
     }
 }
 
+
+/* periods in FP32, and the image displacement of a shift.  (Taken per pair and
+ * axis, the FP64 subtraction and product bound the passes: at 107,618 particles
+ * continuity 255 -> 128 us, forces 300 -> 254 with fewer divisions.)  Both passes
+ * are bound by latency of their gathers now; records of a particle side by side,
+ * which take fewer sectors, measured the same. */
 template <int ND>
-__device__ __forceinline__ void image32(const DevCfg &c, const int *sh, float *img) {
+struct Periods32 {
+    float p[ND];
+    __device__ __forceinline__ explicit Periods32(const DevCfg &c) {
 #pragma unroll
-    for (int q = 0; q < ND; q++) img[q] = sh[q] == 0 ? 0.f : (float)(sh[q] * (c.rmax[q] - c.rmin[q]));
-}
+        for (int q = 0; q < ND; q++) p[q] = (float)(c.rmax[q] - c.rmin[q]);
+    }
+    __device__ __forceinline__ void image(const int *sh, float *img) const {
+#pragma unroll
+        for (int q = 0; q < ND; q++) img[q] = sh[q] == 0 ? 0.f : (sh[q] > 0 ? p[q] : -p[q]);
+    }
+};
 
 /* continuity (end pairs) in FP32, then the FP64 totals of r1, vh1 and the
  * adjoints of f1, fp, fv (k_cp_end) */
@@ -1366,19 +1431,22 @@ template <int ND>
 __global__ void __launch_bounds__(128) k_cp_end32(DevCfg c, int64_t n, double dt, const int *typ,
                                                   const int *__restrict__ nb, const int2 *__restrict__ oc,
                                                   const double *adj, const double *cacc, double *cend, float4 *rec) {
-    const int64_t a = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (a >= n || !is_fluid(typ[a])) return;
+    const int64_t t = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / ADJ_LANES;
+    const int sub = threadIdx.x % ADJ_LANES;
+    const bool act = t < n && is_fluid(typ[t]);
+    const int64_t a = act ? t : 0;
     const float4 *E0 = rec + R_E0 * n, *E1 = rec + R_E1 * n, *E2 = rec + R_E2 * n;
+    const Periods32<ND> L(c);
     const float wcon = (float)c.wcon;
     const float4 p0 = E0[a], p1 = E1[a], p2 = E2[a];
     const float pa[3] = {p0.x, p0.y, p0.z}, la[3] = {p1.x, p1.y, p1.z}, va[3] = {p2.x, p2.y, p2.z};
     Kf rb[ND], wb[ND];
-    const int2 o = oc[a];
-    for (int k = 0; k < o.y; k++) {
+    const int2 o = act ? oc[a] : make_int2(0, 0);
+    for (int k = sub; k < o.y; k += ADJ_LANES) {
         int sh[3];
         const int b = table_entry(__ldg(nb + o.x + k), sh);
         float img[3];
-        image32<ND>(c, sh, img);
+        L.image(sh, img);
         const float4 q0 = E0[b], q1 = E1[b], q2 = E2[b];
         const float pb[3] = {q0.x, q0.y, q0.z}, lb[3] = {q1.x, q1.y, q1.z}, vb[3] = {q2.x, q2.y, q2.z};
         float d[3], w[3], r2 = 0.f, wd = 0.f;
@@ -1401,14 +1469,21 @@ __global__ void __launch_bounds__(128) k_cp_end32(DevCfg c, int64_t n, double dt
             wb[q].add(coef * G * d[q]);
         }
     }
+    double rt_[ND], wt_[ND];
+#pragma unroll
+    for (int q = 0; q < ND; q++) {
+        rt_[q] = rb[q].total();
+        wt_[q] = wb[q].total();
+    }
+    if (!act || sub) return;
     const double hd = 0.5 * dt;
     const double *aa = adj + a * ADJ_NC, *ac = cacc + a * CP_NACC;
     const bool sph = typ[a] == T_SPH;
     double *ce = cend + a * CP_NEND;
     float P[3] = {0.f, 0.f, 0.f}, V[3] = {0.f, 0.f, 0.f};
     for (int q = 0; q < 3; q++) {
-        const double rt = aa[AS_R + q] + ac[CA_R1 + q] + (q < ND ? rb[q].value() : 0.0);
-        const double vt = aa[AS_VH + q] + ac[CA_VH1 + q] + (q < ND ? wb[q].value() : 0.0) + hd * rt;
+        const double rt = aa[AS_R + q] + ac[CA_R1 + q] + (q < ND ? rt_[q] : 0.0);
+        const double vt = aa[AS_VH + q] + ac[CA_VH1 + q] + (q < ND ? wt_[q] : 0.0) + hd * rt;
         const double F = sph ? aa[AS_F + q] + dt * (vt + aa[AS_V + q]) : 0.0;
         ce[CE_R1 + q] = rt;
         ce[CE_VH1 + q] = vt;
@@ -1423,29 +1498,30 @@ __global__ void __launch_bounds__(128) k_cp_end32(DevCfg c, int64_t n, double dt
     M4[a] = make_float4(V[0], V[1], V[2], M4[a].w);
 }
 
-/* cp_force_pair in FP32 with Kahan sums */
+/* cp_force_pair in FP32 with Kahan sums; ir = 1/r, den = 1/(r^2 + eta^2) and
+ * irr = 1/(rho_x rho_y) are those of either orientation.  VT receives the sum
+ * of c_xy phi Vb.w, of which the adjoints of rho_self and nu are -1/rho_self and
+ * 1/nu times, and nub the same of the particle's own orientation. */
 template <int ND>
-__device__ __forceinline__ void cp_force_pair32(float nu, float rho0, const float *d, const float *w, float r,
-                                                float G, float Gp, float hbar, const float *Pb, const float *Vb,
-                                                float my, float rhox, float rhoy, float pdr2x, float pdr2y,
-                                                float sign, Kf *Db, Kf *Wb, Kf &Rb, Kf &Qb, float &nub) {
+__device__ __forceinline__ void cp_force_pair32(float nu, float rho0, const float *d, const float *w, float r, float ir,
+                                                float den, float irr, float eta2, float G, float Gp, const float *Pb,
+                                                const float *Vb, float my, float pdr2x, float pdr2y, float sign,
+                                                Kf *Db, Kf *Wb, Kf &VT, Kf &Qb, float &nub) {
     float P = 0.f, Vw = 0.f;
 #pragma unroll
     for (int q = 0; q < ND; q++) {
         P = fmaf(Pb[q], d[q], P);
         Vw = fmaf(Vb[q], w[q], Vw);
     }
-    const float ir = 1.f / r;
     const float s = -my * (pdr2x + pdr2y);
     Qb.add(-my * G * P);
-    const float gpd = Gp * P * ir;
-    const float eta2 = 0.01f * hbar * hbar, r2 = r * r, den = 1.f / (r2 + eta2);
+    const float gpd = Gp * P * ir, r2 = r * r;
     const float phi = G * r2 * den;
     const float dphi = Gp * r2 * den + G * 2.f * r * eta2 * den * den;
-    const float cxy = 2.f * nu * rho0 * my / (rhox * rhoy);
-    const float VT = cxy * phi * Vw;
-    Rb.add(-VT / (sign > 0.f ? rhox : rhoy));
-    nub += VT / nu;
+    const float cxy = 2.f * nu * rho0 * my * irr;
+    const float vt = cxy * phi * Vw;
+    VT.add(vt);
+    nub += vt;
     const float cv = cxy * Vw * dphi * ir;
 #pragma unroll
     for (int q = 0; q < ND; q++) {
@@ -1461,49 +1537,61 @@ __global__ void __launch_bounds__(128) k_cp_force32(DevCfg c, int64_t n, const i
                                                     const double *aux, const double *cend,
                                                     const float4 *__restrict__ rec, double *cmid, double *cacc,
                                                     double *grads) {
-    const int64_t a = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t t = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / ADJ_LANES;
+    const int sub = threadIdx.x % ADJ_LANES;
+    const bool act = t < n && is_fluid(typ[t]);
+    const int64_t a = act ? t : 0;
     float gnu = 0.f;
-    if (a < n && is_fluid(typ[a])) {
-        const float4 *M0 = rec + R_M0 * n, *M1 = rec + R_M1 * n, *M2 = rec + R_M2 * n, *M3 = rec + R_M3 * n,
-                     *M4 = rec + R_M4 * n;
-        const float wcon = (float)c.wcon, nu = (float)c.viscosity, rho0 = (float)c.dens;
-        const float4 p0 = M0[a], p1 = M1[a], p2 = M2[a], p3 = M3[a], p4 = M4[a];
-        const float pa[3] = {p0.x, p0.y, p0.z}, la[3] = {p1.x, p1.y, p1.z}, va[3] = {p2.x, p2.y, p2.z};
-        const float Pa[3] = {p3.x, p3.y, p3.z}, Va[3] = {p4.x, p4.y, p4.z};
-        const bool own = Pa[0] != 0.f || Pa[1] != 0.f || Pa[2] != 0.f || Va[0] != 0.f || Va[1] != 0.f ||
-                         Va[2] != 0.f;
-        Kf Db[ND], Wb[ND], Rb, Qb;
-        float dum = 0.f;
-        const int2 o = oc[a];
-        for (int k = 0; k < o.y; k++) {
-            int sh[3];
-            const int b = table_entry(__ldg(nb + o.x + k), sh);
-            float img[3];
-            image32<ND>(c, sh, img);
-            const float4 q0 = M0[b], q1 = M1[b], q2 = M2[b], q3 = M3[b], q4 = M4[b];
-            const float pb[3] = {q0.x, q0.y, q0.z}, lb[3] = {q1.x, q1.y, q1.z}, vb[3] = {q2.x, q2.y, q2.z};
-            const float Pbv[3] = {q3.x, q3.y, q3.z}, Vbv[3] = {q4.x, q4.y, q4.z};
-            float d[3], w[3], md[3], mw[3], r2 = 0.f;
+    const float4 *M0 = rec + R_M0 * n, *M1 = rec + R_M1 * n, *M2 = rec + R_M2 * n, *M3 = rec + R_M3 * n,
+                 *M4 = rec + R_M4 * n;
+    const Periods32<ND> L(c);
+    const float wcon = (float)c.wcon, nu = (float)c.viscosity, rho0 = (float)c.dens;
+    const float4 p0 = M0[a], p1 = M1[a], p2 = M2[a], p3 = M3[a], p4 = M4[a];
+    const float pa[3] = {p0.x, p0.y, p0.z}, la[3] = {p1.x, p1.y, p1.z}, va[3] = {p2.x, p2.y, p2.z};
+    const float Pa[3] = {p3.x, p3.y, p3.z}, Va[3] = {p4.x, p4.y, p4.z};
+    const bool own = Pa[0] != 0.f || Pa[1] != 0.f || Pa[2] != 0.f || Va[0] != 0.f || Va[1] != 0.f ||
+                     Va[2] != 0.f;
+    Kf Db[ND], Wb[ND], VT, Qb;
+    float dum = 0.f;
+    const int2 o = act ? oc[a] : make_int2(0, 0);
+    for (int k = sub; k < o.y; k += ADJ_LANES) {
+        int sh[3];
+        const int b = table_entry(__ldg(nb + o.x + k), sh);
+        float img[3];
+        L.image(sh, img);
+        const float4 q0 = M0[b], q1 = M1[b], q2 = M2[b], q3 = M3[b], q4 = M4[b];
+        const float pb[3] = {q0.x, q0.y, q0.z}, lb[3] = {q1.x, q1.y, q1.z}, vb[3] = {q2.x, q2.y, q2.z};
+        const float Pbv[3] = {q3.x, q3.y, q3.z}, Vbv[3] = {q4.x, q4.y, q4.z};
+        float d[3], w[3], md[3], mw[3], r2 = 0.f;
 #pragma unroll
-            for (int q = 0; q < ND; q++) {
-                d[q] = ((pa[q] - pb[q]) + (la[q] - lb[q])) - img[q];
-                w[q] = va[q] - vb[q];
-                md[q] = -d[q];
-                mw[q] = -w[q];
-                r2 = fmaf(d[q], d[q], r2);
-            }
-            if (!(r2 > 0.f)) continue;
-            const float r = sqrtf(r2);
-            float G, Gp;
-            grad_factor32<ND>(wcon, r, p0.w, q0.w, G, Gp);
-            const float hbar = 0.5f * (p4.w + q4.w);
-            if (own)
-                cp_force_pair32<ND>(nu, rho0, d, w, r, G, Gp, hbar, Pa, Va, q1.w, p2.w, q2.w, p3.w, q3.w, 1.f, Db, Wb,
-                                    Rb, Qb, gnu);
-            if (Pbv[0] != 0.f || Pbv[1] != 0.f || Pbv[2] != 0.f || Vbv[0] != 0.f || Vbv[1] != 0.f || Vbv[2] != 0.f)
-                cp_force_pair32<ND>(nu, rho0, md, mw, r, G, Gp, hbar, Pbv, Vbv, p1.w, q2.w, p2.w, q3.w, p3.w, -1.f, Db,
-                                    Wb, Rb, Qb, dum);
+        for (int q = 0; q < ND; q++) {
+            d[q] = ((pa[q] - pb[q]) + (la[q] - lb[q])) - img[q];
+            w[q] = va[q] - vb[q];
+            md[q] = -d[q];
+            mw[q] = -w[q];
+            r2 = fmaf(d[q], d[q], r2);
         }
+        if (!(r2 > 0.f)) continue;
+        const float r = sqrtf(r2);
+        float G, Gp;
+        grad_factor32<ND>(wcon, r, p0.w, q0.w, G, Gp);
+        const float hbar = 0.5f * (p4.w + q4.w), eta2 = 0.01f * hbar * hbar;
+        const float ir = 1.f / r, den = 1.f / (r * r + eta2), irr = 1.f / (p2.w * q2.w);
+        if (own)
+            cp_force_pair32<ND>(nu, rho0, d, w, r, ir, den, irr, eta2, G, Gp, Pa, Va, q1.w, p3.w, q3.w, 1.f, Db, Wb, VT,
+                                Qb, gnu);
+        if (Pbv[0] != 0.f || Pbv[1] != 0.f || Pbv[2] != 0.f || Vbv[0] != 0.f || Vbv[1] != 0.f || Vbv[2] != 0.f)
+            cp_force_pair32<ND>(nu, rho0, md, mw, r, ir, den, irr, eta2, G, Gp, Pbv, Vbv, p1.w, q3.w, p3.w, -1.f, Db, Wb,
+                                VT, Qb, dum);
+    }
+    double Dt[ND], Wt[ND];
+#pragma unroll
+    for (int q = 0; q < ND; q++) {
+        Dt[q] = Db[q].total();
+        Wt[q] = Wb[q].total();
+    }
+    const double Vt = VT.total(), Qt = Qb.total();
+    if (act && sub == 0) {
         const double rhoa = aux[a * ADJ_AUX + 6];
         const double eps = cmid[a * CP_NMID + CM_EPS];
         const double x = rhoa / (c.refd * eps), x2 = x * x, x7 = x2 * x2 * x2 * x;
@@ -1511,13 +1599,13 @@ __global__ void __launch_bounds__(128) k_cp_force32(DevCfg c, int64_t n, const i
         const double dp_deps = -7.0 * c.prb * x7 / (eps * rhoa * rhoa);
         double *ac = cacc + a * CP_NACC;
         const double *aa = adj + a * ADJ_NC, *ea = cend + a * CP_NEND;
-        const double Qv = Qb.value();
-        ac[CA_RHOS] = aa[AS_DENS] + ac[CA_RHO] + Rb.value() + Qv * dp_drho;
+        const double Qv = Qt;
+        ac[CA_RHOS] = aa[AS_DENS] + ac[CA_RHO] - Vt / rhoa + Qv * dp_drho;
         const double epsb = ac[CA_EPS] + Qv * dp_deps;
         ac[CA_EBAR] = cmid[a * CP_NMID + CM_CLAMP] != 0.0 ? 0.0 : -epsb;
         for (int q = 0; q < 3; q++) {
-            ac[CA_RS + q] = ea[CE_R1 + q] + (q < ND ? Db[q].value() : 0.0);
-            cmid[a * CP_NMID + CM_VHS + q] = q < ND ? Wb[q].value() : 0.0;
+            ac[CA_RS + q] = ea[CE_R1 + q] + (q < ND ? Dt[q] : 0.0);
+            cmid[a * CP_NMID + CM_VHS + q] = q < ND ? Wt[q] : 0.0;
         }
     }
     gnu += __shfl_xor_sync(0xffffffffu, gnu, 16);
@@ -1525,7 +1613,7 @@ __global__ void __launch_bounds__(128) k_cp_force32(DevCfg c, int64_t n, const i
     gnu += __shfl_xor_sync(0xffffffffu, gnu, 4);
     gnu += __shfl_xor_sync(0xffffffffu, gnu, 2);
     gnu += __shfl_xor_sync(0xffffffffu, gnu, 1);
-    if ((threadIdx.x & 31) == 0 && gnu != 0.f) atomicAdd(&grads[3], (double)gnu);
+    if ((threadIdx.x & 31) == 0 && gnu != 0.f) atomicAdd(&grads[3], (double)gnu / c.viscosity);
 }
 
 
@@ -1578,20 +1666,23 @@ __global__ void __launch_bounds__(128) k_cp_end32_vh(DevCfg c, int64_t n, double
                                                      const int *__restrict__ nb, const int2 *__restrict__ oc,
                                                      const double *adj, const double *s1, double *cacc, double *cend,
                                                      float4 *rec) {
-    const int64_t a = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (a >= n || !is_fluid(typ[a])) return;
+    const int64_t t = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / ADJ_LANES;
+    const int sub = threadIdx.x % ADJ_LANES;
+    const bool act = t < n && is_fluid(typ[t]);
+    const int64_t a = act ? t : 0;
     const float4 *E0 = rec + R_E0 * n, *E1 = rec + R_E1 * n, *E2 = rec + R_E2 * n, *O = rec + R_O * n;
+    const Periods32<ND> L(c);
     const float wcon = (float)c.wcon;
     const float4 p0 = E0[a], p1 = E1[a], p2 = E2[a], oa = O[a];
     const float pa[3] = {p0.x, p0.y, p0.z}, la[3] = {p1.x, p1.y, p1.z}, va[3] = {p2.x, p2.y, p2.z};
     const float ma = p1.w, da = p2.w / oa.y, ka = oa.w;   /* delta_a = Dbar / Omega_e, kappa_e */
     Kf rb[ND], wb[ND], hb;
-    const int2 o = oc[a];
-    for (int k = 0; k < o.y; k++) {
+    const int2 o = act ? oc[a] : make_int2(0, 0);
+    for (int k = sub; k < o.y; k += ADJ_LANES) {
         int sh[3];
         const int b = table_entry(__ldg(nb + o.x + k), sh);
         float img[3];
-        image32<ND>(c, sh, img);
+        L.image(sh, img);
         const float4 q0 = E0[b], q1 = E1[b], q2 = E2[b], ob = O[b];
         const float pb[3] = {q0.x, q0.y, q0.z}, lb[3] = {q1.x, q1.y, q1.z}, vb[3] = {q2.x, q2.y, q2.z};
         float d[3], w[3], r2 = 0.f, wd = 0.f;
@@ -1615,6 +1706,14 @@ __global__ void __launch_bounds__(128) k_cp_end32_vh(DevCfg c, int64_t n, double
         }
         hb.add(da * mb * wd * ka_.Fh + ka * mb * ka_.Whh);
     }
+    double rt_[ND], wt_[ND];
+#pragma unroll
+    for (int q = 0; q < ND; q++) {
+        rt_[q] = rb[q].total();
+        wt_[q] = wb[q].total();
+    }
+    const double hbt = hb.total();
+    if (!act || sub) return;
     const double hd = 0.5 * dt;
     const double *aa = adj + a * ADJ_NC, *x1 = s1 + a * ADJ_NC;
     double *ac = cacc + a * CP_NACC;
@@ -1623,14 +1722,14 @@ __global__ void __launch_bounds__(128) k_cp_end32_vh(DevCfg c, int64_t n, double
     /* Omega_e's own h and rho: Omega - 1 = h S / (rho d) */
     const double rho = rec[R_M2 * n + a].w, ih = p0.w, h = 1.0 / ih;
     const double ombar = (double)ka * rho * ND * ih;
-    ac[CA_HB] += hb.value() + ombar * ((double)oa.y - 1.0) * ih +
+    ac[CA_HB] += hbt + ombar * ((double)oa.y - 1.0) * ih +
                  (double)ka * ma * (double)ker_vh<ND>(wcon, 0.f, p0.w).Whh;
     ac[CA_RHO] += -ombar * ((double)oa.y - 1.0) / rho;
     float P[3] = {0.f, 0.f, 0.f}, V[3] = {0.f, 0.f, 0.f};
     double pf = 0.0;   /* Pbar.fp + Vbar.fv of the middle forces */
     for (int q = 0; q < 3; q++) {
-        const double rt = aa[AS_R + q] + ac[CA_R1 + q] + (q < ND ? rb[q].value() : 0.0);
-        const double vt = aa[AS_VH + q] + ac[CA_VH1 + q] + (q < ND ? wb[q].value() : 0.0) + hd * rt;
+        const double rt = aa[AS_R + q] + ac[CA_R1 + q] + (q < ND ? rt_[q] : 0.0);
+        const double vt = aa[AS_VH + q] + ac[CA_VH1 + q] + (q < ND ? wt_[q] : 0.0) + hd * rt;
         const double F = sph ? aa[AS_F + q] + dt * (vt + aa[AS_V + q]) : 0.0;
         ce[CE_R1 + q] = rt;
         ce[CE_VH1 + q] = vt;
@@ -1703,74 +1802,85 @@ __global__ void __launch_bounds__(128) k_cp_force32_vh(DevCfg c, int64_t n, cons
                                                        const double *adj, const double *aux, const double *cend,
                                                        const float4 *__restrict__ rec, double *cmid, double *cacc,
                                                        double *grads) {
-    const int64_t a = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t t = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / ADJ_LANES;
+    const int sub = threadIdx.x % ADJ_LANES;
+    const bool act = t < n && is_fluid(typ[t]);
+    const int64_t a = act ? t : 0;
     float gnu = 0.f;
-    if (a < n && is_fluid(typ[a])) {
-        const float4 *M0 = rec + R_M0 * n, *M1 = rec + R_M1 * n, *M2 = rec + R_M2 * n, *M3 = rec + R_M3 * n,
-                     *M4 = rec + R_M4 * n, *O = rec + R_O * n;
-        const float wcon = (float)c.wcon, nu = (float)c.viscosity, rho0 = (float)c.dens;
-        const float4 p0 = M0[a], p1 = M1[a], p2 = M2[a], p3 = M3[a], p4 = M4[a], oa = O[a];
-        const float pa[3] = {p0.x, p0.y, p0.z}, la[3] = {p1.x, p1.y, p1.z}, va[3] = {p2.x, p2.y, p2.z};
-        const float ioa = 1.f / oa.x;
-        const float Pa[3] = {p3.x * ioa, p3.y * ioa, p3.z * ioa}, Va[3] = {p4.x * ioa, p4.y * ioa, p4.z * ioa};
-        const bool own = p3.x != 0.f || p3.y != 0.f || p3.z != 0.f || p4.x != 0.f || p4.y != 0.f || p4.z != 0.f;
-        const float ma = p1.w, ka = oa.z;
-        Kf Db[ND], Wb[ND], Rb, Qb, Hb;
-        const int2 o = oc[a];
-        for (int k = 0; k < o.y; k++) {
-            int sh[3];
-            const int b = table_entry(__ldg(nb + o.x + k), sh);
-            float img[3];
-            image32<ND>(c, sh, img);
-            const float4 q0 = M0[b], q1 = M1[b], q2 = M2[b], q3 = M3[b], q4 = M4[b], ob = O[b];
-            const float pb[3] = {q0.x, q0.y, q0.z}, lb[3] = {q1.x, q1.y, q1.z}, vb[3] = {q2.x, q2.y, q2.z};
-            float d[3], w[3], md[3], mw[3], r2 = 0.f;
+    const float4 *M0 = rec + R_M0 * n, *M1 = rec + R_M1 * n, *M2 = rec + R_M2 * n, *M3 = rec + R_M3 * n,
+                 *M4 = rec + R_M4 * n, *O = rec + R_O * n;
+    const Periods32<ND> L(c);
+    const float wcon = (float)c.wcon, nu = (float)c.viscosity, rho0 = (float)c.dens;
+    const float4 p0 = M0[a], p1 = M1[a], p2 = M2[a], p3 = M3[a], p4 = M4[a], oa = O[a];
+    const float pa[3] = {p0.x, p0.y, p0.z}, la[3] = {p1.x, p1.y, p1.z}, va[3] = {p2.x, p2.y, p2.z};
+    const float ioa = 1.f / oa.x;
+    const float Pa[3] = {p3.x * ioa, p3.y * ioa, p3.z * ioa}, Va[3] = {p4.x * ioa, p4.y * ioa, p4.z * ioa};
+    const bool own = p3.x != 0.f || p3.y != 0.f || p3.z != 0.f || p4.x != 0.f || p4.y != 0.f || p4.z != 0.f;
+    const float ma = p1.w, ka = oa.z;
+    Kf Db[ND], Wb[ND], Rb, Qb, Hb;
+    const int2 o = act ? oc[a] : make_int2(0, 0);
+    for (int k = sub; k < o.y; k += ADJ_LANES) {
+        int sh[3];
+        const int b = table_entry(__ldg(nb + o.x + k), sh);
+        float img[3];
+        L.image(sh, img);
+        const float4 q0 = M0[b], q1 = M1[b], q2 = M2[b], q3 = M3[b], q4 = M4[b], ob = O[b];
+        const float pb[3] = {q0.x, q0.y, q0.z}, lb[3] = {q1.x, q1.y, q1.z}, vb[3] = {q2.x, q2.y, q2.z};
+        float d[3], w[3], md[3], mw[3], r2 = 0.f;
+#pragma unroll
+        for (int q = 0; q < ND; q++) {
+            d[q] = ((pa[q] - pb[q]) + (la[q] - lb[q])) - img[q];
+            w[q] = va[q] - vb[q];
+            md[q] = -d[q];
+            mw[q] = -w[q];
+            r2 = fmaf(d[q], d[q], r2);
+        }
+        if (!(r2 > 0.f)) continue;
+        const float r = sqrtf(r2), ir = 1.f / r;
+        const KerVH<ND> kA = ker_vh<ND>(wcon, r, p0.w), kB = ker_vh<ND>(wcon, r, q0.w);
+        const float hav = 0.5f * (p4.w + q4.w);
+        const float mb = q1.w;
+        if (own) {
+            const PairVH<ND> t = force_pair_vh<ND>(nu, rho0, d, w, r, kA, kB, hav, Pa, Va, mb, p2.w, q2.w, p3.w,
+                                                   q3.w);
 #pragma unroll
             for (int q = 0; q < ND; q++) {
-                d[q] = ((pa[q] - pb[q]) + (la[q] - lb[q])) - img[q];
-                w[q] = va[q] - vb[q];
-                md[q] = -d[q];
-                mw[q] = -w[q];
-                r2 = fmaf(d[q], d[q], r2);
+                Db[q].add(t.Dd[q]);
+                Wb[q].add(t.Dw[q]);
             }
-            if (!(r2 > 0.f)) continue;
-            const float r = sqrtf(r2), ir = 1.f / r;
-            const KerVH<ND> kA = ker_vh<ND>(wcon, r, p0.w), kB = ker_vh<ND>(wcon, r, q0.w);
-            const float hav = 0.5f * (p4.w + q4.w);
-            const float mb = q1.w;
-            if (own) {
-                const PairVH<ND> t = force_pair_vh<ND>(nu, rho0, d, w, r, kA, kB, hav, Pa, Va, mb, p2.w, q2.w, p3.w,
-                                                       q3.w);
-#pragma unroll
-                for (int q = 0; q < ND; q++) {
-                    Db[q].add(t.Dd[q]);
-                    Wb[q].add(t.Dw[q]);
-                }
-                Rb.add(t.Rx);
-                Qb.add(t.Qx);
-                Hb.add(t.Hx);
-                gnu += t.nu;
-            }
-            if (q3.x != 0.f || q3.y != 0.f || q3.z != 0.f || q4.x != 0.f || q4.y != 0.f || q4.z != 0.f) {
-                const float iob = 1.f / ob.x;
-                const float Pb_[3] = {q3.x * iob, q3.y * iob, q3.z * iob}, Vb_[3] = {q4.x * iob, q4.y * iob, q4.z * iob};
-                const PairVH<ND> t = force_pair_vh<ND>(nu, rho0, md, mw, r, kB, kA, hav, Pb_, Vb_, ma, q2.w, p2.w,
-                                                       q3.w, p3.w);
-#pragma unroll
-                for (int q = 0; q < ND; q++) {
-                    Db[q].add(-t.Dd[q]);
-                    Wb[q].add(-t.Dw[q]);
-                }
-                Rb.add(t.Ry);
-                Qb.add(t.Qy);
-                Hb.add(t.Hy);
-            }
-            /* Omega_m's pair terms */
-            const float cR = (ka * mb * kA.Whr + ob.z * ma * kB.Whr) * ir;
-#pragma unroll
-            for (int q = 0; q < ND; q++) Db[q].add(cR * d[q]);
-            Hb.add(ka * mb * kA.Whh);
+            Rb.add(t.Rx);
+            Qb.add(t.Qx);
+            Hb.add(t.Hx);
+            gnu += t.nu;
         }
+        if (q3.x != 0.f || q3.y != 0.f || q3.z != 0.f || q4.x != 0.f || q4.y != 0.f || q4.z != 0.f) {
+            const float iob = 1.f / ob.x;
+            const float Pb_[3] = {q3.x * iob, q3.y * iob, q3.z * iob}, Vb_[3] = {q4.x * iob, q4.y * iob, q4.z * iob};
+            const PairVH<ND> t = force_pair_vh<ND>(nu, rho0, md, mw, r, kB, kA, hav, Pb_, Vb_, ma, q2.w, p2.w,
+                                                   q3.w, p3.w);
+#pragma unroll
+            for (int q = 0; q < ND; q++) {
+                Db[q].add(-t.Dd[q]);
+                Wb[q].add(-t.Dw[q]);
+            }
+            Rb.add(t.Ry);
+            Qb.add(t.Qy);
+            Hb.add(t.Hy);
+        }
+        /* Omega_m's pair terms */
+        const float cR = (ka * mb * kA.Whr + ob.z * ma * kB.Whr) * ir;
+#pragma unroll
+        for (int q = 0; q < ND; q++) Db[q].add(cR * d[q]);
+        Hb.add(ka * mb * kA.Whh);
+    }
+    double Dt[ND], Wt[ND];
+#pragma unroll
+    for (int q = 0; q < ND; q++) {
+        Dt[q] = Db[q].total();
+        Wt[q] = Wb[q].total();
+    }
+    const double Rt = Rb.total(), Qt = Qb.total(), Ht = Hb.total();
+    if (act && sub == 0) {
         const double rhoa = aux[a * ADJ_AUX + 6];
         const double eps = cmid[a * CP_NMID + CM_EPS];
         const double x = rhoa / (c.refd * eps), x2 = x * x, x7 = x2 * x2 * x2 * x;
@@ -1778,19 +1888,19 @@ __global__ void __launch_bounds__(128) k_cp_force32_vh(DevCfg c, int64_t n, cons
         const double dp_deps = -7.0 * c.prb * x7 / (eps * rhoa * rhoa);
         double *ac = cacc + a * CP_NACC;
         const double *aa = adj + a * ADJ_NC, *ea = cend + a * CP_NEND;
-        const double Qv = Qb.value();
+        const double Qv = Qt;
         /* Omega_m's own h and rho, then h = hfac (m / rho)^(1/d) */
         const double ih = p0.w, h = 1.0 / ih;
         const double ombar = (double)ka * (double)p2.w * ND * ih;
-        const double hbar = ac[CA_HB] + Hb.value() + ombar * ((double)oa.x - 1.0) * ih +
+        const double hbar = ac[CA_HB] + Ht + ombar * ((double)oa.x - 1.0) * ih +
                             (double)ka * ma * (double)ker_vh<ND>(wcon, 0.f, p0.w).Whh;
-        ac[CA_RHOS] = aa[AS_DENS] + ac[CA_RHO] + Rb.value() + Qv * dp_drho - ombar * ((double)oa.x - 1.0) / rhoa -
+        ac[CA_RHOS] = aa[AS_DENS] + ac[CA_RHO] + Rt + Qv * dp_drho - ombar * ((double)oa.x - 1.0) / rhoa -
                       hbar * h / (ND * rhoa);
         const double epsb = ac[CA_EPS] + Qv * dp_deps;
         ac[CA_EBAR] = cmid[a * CP_NMID + CM_CLAMP] != 0.0 ? 0.0 : -epsb;
         for (int q = 0; q < 3; q++) {
-            ac[CA_RS + q] = ea[CE_R1 + q] + (q < ND ? Db[q].value() : 0.0);
-            cmid[a * CP_NMID + CM_VHS + q] = q < ND ? Wb[q].value() : 0.0;
+            ac[CA_RS + q] = ea[CE_R1 + q] + (q < ND ? Dt[q] : 0.0);
+            cmid[a * CP_NMID + CM_VHS + q] = q < ND ? Wt[q] : 0.0;
         }
     }
     gnu += __shfl_xor_sync(0xffffffffu, gnu, 16);
@@ -1984,8 +2094,12 @@ void cpl_backward_coupling(sphdem_ctx *c, AdjointData *a, int sl, const double *
         transpose<true>(c, a, nbf, ocf, a->fpiT);
         SPHDEM_LAUNCH(c, "adj_shep", k_cp_shep<M>, gd, CB, 0, nd, a->dem_tags, a->aux, a->mass, a->cplT.nb, a->cplT.ix,
                       a->cplT.oc, gwc, a->cmid);
-        SPHDEM_LAUNCH(c, "adj_fpi_dem", k_cp_fpi<M>, gd, CB, 0, c->cfg, nd, a->dem_tags, dt, s1, a->aux, a->cmid,
-                      a->mass, nbf, ocf, g4f, gwf, a->adj, a->cacc, a->coef, a->grads);
+        SPHDEM_LAUNCH(c, "adj_fpi_sums", k_cp_fpi_sums<M>, gd, CB, 0, c->cfg, nd, a->dem_tags, s1, a->aux, a->cmid,
+                      a->mass, nbf, ocf, gwf, a->coef);
+        SPHDEM_LAUNCH(c, "adj_fpi_drag", k_cp_fpi_drag, grid_for(nd, 64), 64, 0, c->cfg, nd, a->dem_tags, dt, a->aux,
+                      a->mass, a->adj, a->cacc, a->coef, a->grads);
+        SPHDEM_LAUNCH(c, "adj_fpi_own", k_cp_fpi_own<M>, gd, CB, 0, c->cfg, nd, a->dem_tags, s1, a->aux, a->cmid,
+                      a->mass, nbf, ocf, g4f, a->cacc, a->coef);
         if (c->cfg.var_h())
             SPHDEM_LAUNCH(c, "adj_fpi_fluid", (k_cp_fpi_fluid<M, true>), g, CB, 0, n, c->cfg.nd, s1, a->aux, a->cmid,
                           a->mass, a->typ, a->fpiT.nb, a->fpiT.ix, a->fpiT.oc, g4f, gwf, a->coef, a->cacc, hp,
@@ -2018,7 +2132,7 @@ void cpl_backward_step(sphdem_ctx *c, AdjointData *a, int j, double dt) {
     auto ocp = [&](const PairTable &t) { return t.oc + (size_t)sl * n; };
     const int *nbm = a->nb_mid + (size_t)sl * a->pair_cap, *nbe = a->nb_end + (size_t)sl * a->pair_cap;
     const int2 *ocm = a->oc_mid + (size_t)sl * n, *oce = a->oc_end + (size_t)sl * n;
-    const int g = grid_for(n, CB), g256 = grid_for(n, 256);
+    const int g = grid_for(n, CB), g256 = grid_for(n, 256), gl = grid_for(n * ADJ_LANES, CB);
     const bool mixed = a->crec != nullptr, vh = c->cfg.var_h();
     /* the step's smoothing lengths: h_s under VAR_H_CORRECTION, else constant */
     const double *hp = vh ? a->hs : a->hh;
@@ -2037,14 +2151,14 @@ void cpl_backward_step(sphdem_ctx *c, AdjointData *a, int j, double dt) {
 #define L_(ND)                                                                                                   \
     do {                                                                                                         \
         if (vh) {                                                                                                \
-            SPHDEM_LAUNCH(c, "adj_end32", k_cp_end32_vh<ND>, g, CB, 0, c->cfg, n, dt, a->typ, nbe, oce, a->adj,   \
+            SPHDEM_LAUNCH(c, "adj_end32", k_cp_end32_vh<ND>, gl, CB, 0, c->cfg, n, dt, a->typ, nbe, oce, a->adj,   \
                           s1, a->cacc, a->cend, a->crec);                                                         \
-            SPHDEM_LAUNCH(c, "adj_force32", k_cp_force32_vh<ND>, g, CB, 0, c->cfg, n, a->typ, nbm, ocm, a->adj,   \
+            SPHDEM_LAUNCH(c, "adj_force32", k_cp_force32_vh<ND>, gl, CB, 0, c->cfg, n, a->typ, nbm, ocm, a->adj,   \
                           a->aux, a->cend, a->crec, a->cmid, a->cacc, a->grads);                                  \
         } else {                                                                                                 \
-            SPHDEM_LAUNCH(c, "adj_end32", k_cp_end32<ND>, g, CB, 0, c->cfg, n, dt, a->typ, nbe, oce, a->adj,      \
+            SPHDEM_LAUNCH(c, "adj_end32", k_cp_end32<ND>, gl, CB, 0, c->cfg, n, dt, a->typ, nbe, oce, a->adj,      \
                           a->cacc, a->cend, a->crec);                                                             \
-            SPHDEM_LAUNCH(c, "adj_force32", k_cp_force32<ND>, g, CB, 0, c->cfg, n, a->typ, nbm, ocm, a->adj,      \
+            SPHDEM_LAUNCH(c, "adj_force32", k_cp_force32<ND>, gl, CB, 0, c->cfg, n, a->typ, nbm, ocm, a->adj,      \
                           a->aux, a->cend, a->crec, a->cmid, a->cacc, a->grads);                                  \
         }                                                                                                        \
     } while (0)
@@ -2054,9 +2168,9 @@ void cpl_backward_step(sphdem_ctx *c, AdjointData *a, int j, double dt) {
 #undef L_
         cpl_backward_coupling<float>(c, a, sl, s0, s1, dt, true, hp);
     } else {
-        SPHDEM_LAUNCH(c, "adj_end", k_cp_end, g, CB, 0, c->cfg, n, dt, s1, a->mass, a->hh, a->typ, nbe, oce, a->adj,
+        SPHDEM_LAUNCH(c, "adj_end", k_cp_end, gl, CB, 0, c->cfg, n, dt, s1, a->mass, a->hh, a->typ, nbe, oce, a->adj,
                       a->cacc, a->cend);
-        SPHDEM_LAUNCH(c, "adj_force", k_cp_force, g, CB, 0, c->cfg, n, a->aux, a->mass, a->hh, a->typ, nbm, ocm,
+        SPHDEM_LAUNCH(c, "adj_force", k_cp_force, gl, CB, 0, c->cfg, n, a->aux, a->mass, a->hh, a->typ, nbm, ocm,
                       a->adj, a->cend, a->cmid, a->cacc, a->grads);
         cpl_backward_coupling<double>(c, a, sl, s0, s1, dt, true, hp);
     }

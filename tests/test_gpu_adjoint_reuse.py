@@ -57,3 +57,27 @@ def test_repeated_passes_equal_fresh_handles(lib, prec):
             assert np.array_equal(a, b)
         assert abs(got[0][3] - got[1][3]) <= 1e-9 * abs(got[1][3])
     kept.close()
+
+
+def test_fp64_pair_tables_beyond_the_list_depth(lib):
+    """The FP64 gradient takes its pair tables from the neighbour lists, and by a
+    bucket scan for a particle whose list is too short: a handle squeezed
+    beyond the depth its lists were given at creation gives the gradients of one
+    created at the squeezed positions.  Only the order of FP64 sums differs
+    (2^-53 a sum of ~100 terms, three steps): 1e-11 of each 2-norm."""
+    case = cases.dambreak2d(dx=0.05)
+    rng = np.random.default_rng(5)
+    n, fluid = case.n, case.particles["iam"] == cases.SPH
+    two = np.array([1.0, 1.0, 0.0])
+    r = case.particles["r"] + 0.003 * rng.standard_normal((n, 3)) * fluid[:, None] * two
+    r[fluid, 1] = 0.02 + 0.3 * (r[fluid, 1] - r[fluid, 1].min())
+    v = 0.1 * rng.standard_normal((n, 3)) * fluid[:, None] * two
+    seed = rng.standard_normal((n, 3)) * fluid[:, None] * two
+    got = []
+    for start in (case.particles["r"], r):
+        sim = capi.Simulation(lib, case.cfg, dict(case.particles, r=start), precision=cases.PREC_FP64)
+        sim.set(capi.ParticleBuffers(n, {"v": v, "vhat": v}, fields=("v", "vhat")), capi.FIELD_V | capi.FIELD_VHAT)
+        got.append(one_pass(sim, r, 3, 3, 0, seed))
+        sim.close()
+    for a, b in zip(*got):
+        assert np.linalg.norm(a - b) <= 1e-11 * np.linalg.norm(b)
