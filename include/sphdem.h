@@ -384,7 +384,7 @@ int sphdem_batch_step(sphdem_batch b, int nsteps);
 int sphdem_batch_time_steps(sphdem_batch b, int nsteps, double *ms);
 /* Autotuner: for every member, times steps_per_trial graph-replayed steps
  * alone for each candidate launch configuration (block size of the
- * list-consumer passes 64 / 128, grid of the slice passes full or 1/4,
+ * list-consumer passes 64 / 128, grid of the list build full or 1/4,
  * neighbour tiles of the force and continuity passes staged in shared
  * memory or read through L1 -- mixed 2D / 3D handles) and keeps the
  * fastest.  Choices are remembered per (dimension, precision, feature

@@ -10,7 +10,7 @@
  * step and error flags; nothing is shared between them.
  *
  * The autotuner (sphdem_batch_tune) picks, per member, the block size of the
- * list-consumer passes, the grid of the slice passes and whether the force
+ * list-consumer passes, the grid of the list build and whether the force
  * and continuity passes stage their neighbour tiles in shared memory, by
  * timing a few graph-replayed steps of that member alone for every
  * candidate; the choice is remembered per dimension, precision, feature

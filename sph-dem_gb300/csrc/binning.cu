@@ -18,9 +18,8 @@
  *   k_scan_*    bucket starts
  *   k_scatter + k_rank   deterministic counting sort by bucket, and within
  *               a bucket by the coordinate on the last axis (ties by tag), so
- *               that a run of consecutive buckets along that axis is sorted
- *               by it and the slice passes can cut their candidate ranges
- *               by binary search
+ *               that the order of the particles, and with it of every sum,
+ *               follows from their positions alone
  *   k_gather    one launch moves every live field row into sorted order
  *
  * All sizes and widths live in DevGlobals, so the sequence replays in a CUDA

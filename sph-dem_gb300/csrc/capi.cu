@@ -354,7 +354,7 @@ void middle_passes(sphdem_ctx *c, bool whole) {
         }
         if (lists) {
             /* elementwise EOS; Omega (VAR_H_CORRECTION) is summed inside the force pass */
-            mixed::omega_eos(c, false, true);
+            mixed::eos(c);
             mixed::force(c);
         }
     } else {

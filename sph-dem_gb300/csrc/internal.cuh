@@ -125,7 +125,7 @@ struct sphdem_ctx {
     /* launch knobs chosen by the batch autotuner */
     int blk_pair = 128;         /* block size of the list-consumer passes (<= 128) */
     bool force_tile = false;    /* force / continuity: neighbour records staged in shared memory */
-    int grid_div = 1;           /* divides the resident-block grid of the slice passes */
+    int grid_div = 1;           /* divides the resident-block grid of the list build */
     int *mx_bandn = nullptr;    /* per particle: list candidates FP32 could not decide */
     sphdem::DevCfg *dcfg = nullptr;  /* device copy of cfg for out-of-line helpers */
     /* staging buffer for field transfers in tag order */
@@ -142,8 +142,9 @@ struct sphdem_ctx {
 
 namespace sphdem {
 
-/* coupling passes: populations below this take four threads per fluid particle;
- * pairs a thread keeps (a partner's bucket column gives one thread of four most
+/* coupling passes: populations below this take four threads per fluid particle
+ * (porosity + drag, us, with four / one: 3,768 particles 35 + 10 / 63 + 12, 33,400
+ * 48 + 33 / 80 + 14, 63,450 73 + 22 / 71 + 14, 206,287 183 + 49 / 130 + 24); pairs a thread keeps (a partner's bucket column gives one thread of four most
  * of a particle's pairs at times); entries and threads to allocate for */
 constexpr int64_t CP_SPLIT_BELOW = 60000;
 __host__ __device__ constexpr int kept_pairs(int threads_per_particle) { return threads_per_particle > 1 ? 16 : 32; }
@@ -217,7 +218,7 @@ void nlist(sphdem_ctx *c, int depth, bool soft = false);
 /* once per process, outside stream capture: kernel attributes of the step */
 void prepare(sphdem_ctx *c);
 int nlist_max_count(sphdem_ctx *c);
-void omega_eos(sphdem_ctx *c, bool omega, bool eos);
+void eos(sphdem_ctx *c);
 /* lists32.cu: the force / continuity passes specialised on the physics class;
  * false when the handle's class has none */
 bool force_lists(sphdem_ctx *c);

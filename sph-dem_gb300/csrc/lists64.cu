@@ -23,7 +23,11 @@
  * closed form F(r, h) = -10 C / h^(d+2) (2 - r/h)^3 (no division by q), square
  * roots and reciprocals start from an FP32 estimate, constant factors are
  * applied to the sums, calcOmega shares the loop, and G lanes share a particle
- * so that every SM has its part of the pairs.
+ * so that every SM has its part of the pairs.  Before (a thread scanning its
+ * stencil) / now, us: coupled step of 69,758 particles, force 24,856 / 1,136,
+ * continuity and Omega 16,795 / 502 (3D, ~85 neighbours); dam break of 23,018
+ * (2D), force 742 / 90, continuity 385 / 31; of 8,753 with CORRECTED_GRADIENT
+ * and density re-initialisation, k_invm twice 1,577 / 101, k_reinit_dens 1,192 / 79.
  */
 #include "fp64.cuh"
 #include "mixed.cuh"
@@ -31,7 +35,10 @@
 namespace sphdem {
 namespace {
 
-/* lanes per particle: about four pairs each in 2D, fourteen in 3D (1D has few) */
+/* lanes per particle: about five pairs each in 2D, eleven in 3D (1D has few).
+ * Force / continuity, us, with 2 / 4 / 8 lanes in 2D: 1,418 particles 38 / 27 / 21
+ * and 20 / 14 / 12, 23,018 80 / 90 / 104 and 35 / 31 / 37; with 4 / 8 / 16 in 3D:
+ * 69,758 1142 / 1142 / 1295 and 493 / 509 / 529. */
 template <int ND>
 constexpr int LANES64 = ND == 3 ? 8 : (ND == 2 ? 4 : 1);
 

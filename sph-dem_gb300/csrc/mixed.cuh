@@ -30,7 +30,6 @@ struct Kahan {
         c = (t - s) - y;
         s = t;
     }
-    __device__ __forceinline__ double value() const { return (double)s - (double)c; }
 };
 
 /* A plain FP32 sum with the same interface, for sums whose rounding does

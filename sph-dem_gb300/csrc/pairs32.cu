@@ -9,19 +9,18 @@
  * the dimension so per-axis arrays live in registers.
  *
  *   k_nlist      after each rebuild, the exact neighbour list of every
- *                sph/sphBoundary particle: a warp stages the 3^d stencil's
- *                candidates of 32 particles in shared memory and tests them in
- *                FP32 with a proven error bound; candidates inside the bound
- *                are settled there by the reference's FP64 predicate
- *                (particle.h:236-238).  Periodic
+ *                sph/sphBoundary particle: candidates of the 3^d stencil in
+ *                FP32 with a proven error bound; those inside the bound are
+ *                settled by the reference's FP64 predicate (particle.h:236-238).
+ *                Periodic
  *                images only where the reference holds a ghost.  Entries
  *                b | stencil code << 26 in tiles of 32 particles x 8 slots
  *                (nl_at).
- *   k_omega_eos  calcOmega over the list + the FP64 EOS (its (rho/rho0)^7-1
- *                cancels too much for FP32)
- *   k_force      calcForce + the Courant/viscous/accel dt conditions
- *   k_dddt       calcDddtDudt
- * The SPH-DEM coupling and contact passes are in coupling.cu.
+ *   k_eos32      the FP64 EOS (its (rho/rho0)^7-1 cancels too much for FP32)
+ *   k_force      calcForce + the Courant/viscous/accel dt conditions, any form
+ *   k_dddt       calcDddtDudt, with CORRECTED_GRADIENT and in 1D
+ * The force and continuity passes of the usual forms are in lists32.cu, the
+ * SPH-DEM coupling and contact passes in coupling.cu.
  *
  * Sums are Kahan-compensated in FP32 and added to the FP64 state once per
  * particle.  Roofline: the list passes are FP32-pipe-bound on 3D workloads
@@ -129,7 +128,10 @@ __global__ void k_pack(DevCfg c, DevState s, const int *__restrict__ skey, const
  * the band of doubt is settled on the spot (settle_band), which also takes
  * the particle itself out, so the lists hold exactly the neighbours.  The
  * lane only keeps the smallest margin of 32 candidates; the rare 32 with a
- * doubtful one (or the particle itself) are gone over again. */
+ * doubtful one (or the particle itself) are gone over again.
+ * Bound by instruction issue: the two builds of a coupled step of 1.08 M
+ * particles take 1.25 ms; tests into a bit mask, entries then spread over the
+ * warp and a second kernel for the candidates in doubt took 2.68. */
 constexpr int NL_WARPS = 4;
 constexpr int NL_CAP = 128;   /* staged candidates per warp before they are tested */
 constexpr int NL_QN = 64;     /* queue slots per lane: moved on when over 32 are taken, 32 come at most per round */
@@ -569,77 +571,32 @@ __global__ void __launch_bounds__(NL_WARPS * 32, 5) k_nlist(DevCfg c, const DevC
 }
 
 /* ---------------------------------------------------------------------- */
-template <int ND>
-__global__ void __launch_bounds__(BLK) k_omega_eos(DevCfg c, DevState s, const DevGlobals *__restrict__ g,
-                                                   const float4 *__restrict__ P0, const float4 *__restrict__ P1,
-                                                   float4 *__restrict__ P2, const int *__restrict__ tg,
-                                                   const int *__restrict__ nbr, const int *__restrict__ ncnt,
-                                                   int64_t ld, int64_t n, int do_omega, int do_eos,
-                                                   float *__restrict__ om32) {
-    const float4 *shift = stencil_shifts(c, g);
+__global__ void __launch_bounds__(BLK) k_eos32(DevCfg c, DevState s, float4 *__restrict__ P2, const int *__restrict__ tg,
+                                              int64_t n) {
     const int64_t a = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (a >= n) return;
     if (!is_sph_or_sphb(tg[a] & 0xff)) return;
-    if (do_omega) {
-        const float wcon = (float)c.wcon;
-        const float4 pa = P0[a];
-        const float iha = 1.f / pa.w;
-        const float ihna = powi<ND>(iha);
-        const float pd_coef = ND * ihna * iha;
-        Kahan om;
-        om.init(-P1[a].w * pd_coef * wK32(0.f, wcon));
-        const int cnt = ncnt[a];
-        /* 8 entries at a time from the particle's list tiles (two int4 loads) */
-        const int4 *tile = reinterpret_cast<const int4 *>(nbr + nl_at(a, 0, ld));
-        int4 q0 = make_int4(-1, -1, -1, -1), q1 = q0;
-#pragma unroll 2
-        for (int j = 0; j < cnt; j++) {
-            if ((j & 7) == 0) {
-                q0 = __ldg(tile + (j >> 3) * 64);
-                q1 = __ldg(tile + (j >> 3) * 64 + 1);
-            }
-            const int e = q0.x;
-            q0 = make_int4(q0.y, q0.z, q0.w, q1.x);
-            q1 = make_int4(q1.y, q1.z, q1.w, -1);
-            if (e < 0) continue;
-            const int b = e & B_MASK;
-            const float4 pb = P0[b];
-            const float mb = fabsf(P1[b].w);
-            const int tb = tg[b] & 0xff;
-            float d[3];
-            nb_delta_t<ND>(e, shift, pa, pb, d);
-            const float q = sqrtf(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]) * iha;
-            const float pdkh = -q * wdK32(q, wcon) * iha;
-            if (is_sph_or_sphb(tb)) om.add(mb * (ihna * pdkh - pd_coef * wK32(q, wcon)));
-        }
-        /* Omega = 1 + h*sum/(rho*NDIM): an O(1) number, FP32 is ample */
-        const float omega = 1.f + pa.w * om.s / (P2[a].x * ND);
-        s.row(FD_OMEGA)[a] = omega;
-        om32[a] = omega;
+    /* FP64: p = PRB((rho/rho0)^7 - 1) cancels; one FP64 reciprocal by
+     * an FP32 estimate and a Newton step, integer powers */
+    const double densa = s.row(FD_DENS)[a];
+    const double rho0 = c.liq_dem() ? c.refd * s.row(FD_POR)[a] : c.refd;
+    double r0 = (double)(1.0f / (float)rho0);
+    r0 = r0 * (2.0 - rho0 * r0);
+    const double x = densa * r0;
+    double xg;
+    if (!c.liq_dem() || c.gamma == 7.0) {
+        const double x2 = x * x;
+        xg = x2 * x2 * x2 * x;
+    } else {
+        xg = pow(x, c.gamma);
     }
-    if (do_eos) {
-        /* FP64: p = PRB((rho/rho0)^7 - 1) cancels; one FP64 reciprocal by
-         * an FP32 estimate and a Newton step, integer powers */
-        const double densa = s.row(FD_DENS)[a];
-        const double rho0 = c.liq_dem() ? c.refd * s.row(FD_POR)[a] : c.refd;
-        double r0 = (double)(1.0f / (float)rho0);
-        r0 = r0 * (2.0 - rho0 * r0);
-        const double x = densa * r0;
-        double xg;
-        if (!c.liq_dem() || c.gamma == 7.0) {
-            const double x2 = x * x;
-            xg = x2 * x2 * x2 * x;
-        } else {
-            xg = pow(x, c.gamma);
-        }
-        double rd = (double)(1.0f / (float)densa);
-        rd = rd * (2.0 - densa * rd);
-        const double press = c.prb * (xg - 1.0);
-        const double pdr2 = press * (rd * rd);
-        s.row(FD_PRESS)[a] = press;
-        s.row(FD_PDR2)[a] = pdr2;
-        P2[a].y = (float)pdr2;
-    }
+    double rd = (double)(1.0f / (float)densa);
+    rd = rd * (2.0 - densa * rd);
+    const double press = c.prb * (xg - 1.0);
+    const double pdr2 = press * (rd * rd);
+    s.row(FD_PRESS)[a] = press;
+    s.row(FD_PDR2)[a] = pdr2;
+    P2[a].y = (float)pdr2;
 }
 
 /* ---------------------------------------------------------------------- */
@@ -896,9 +853,7 @@ __global__ void __launch_bounds__(BLK) k_force(DevCfg c, const DevCfg *__restric
     block_min_atomic(ndt, &g->new_dt_bits);
 }
 
-/* VH: VAR_H_CORRECTION known at compile time (1 on, 0 off) or read from
- * the configuration (-1) */
-template <int ND, bool CG, int VH, bool TILE>
+template <int ND, bool CG, bool TILE>
 __global__ void __launch_bounds__(BLK) k_dddt(DevCfg c, DevState s, const DevGlobals *__restrict__ g,
                                               const float4 *__restrict__ P0, const float4 *__restrict__ P1,
                                               const float4 *__restrict__ P2, float *__restrict__ om32,
@@ -907,7 +862,7 @@ __global__ void __launch_bounds__(BLK) k_dddt(DevCfg c, DevState s, const DevGlo
                                               const double *__restrict__ cgrows,
                                               const int *__restrict__ start, const int *__restrict__ skey) {
     const float4 *shift = stencil_shifts(c, g);
-    const bool var_h = VH < 0 ? c.var_h() : VH == 1;
+    const bool var_h = c.var_h();
     extern __shared__ float4 st_smem[];
     Staged st = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, false};
     if constexpr (TILE) {
@@ -1176,14 +1131,8 @@ int nlist_max_count(sphdem_ctx *c) {
     return m;
 }
 
-void omega_eos(sphdem_ctx *c, bool omega, bool eos) {
-#define L_(ND)                                                                                                  \
-    SPHDEM_LAUNCH(c, omega ? "omega_eos32" : "eos32", k_omega_eos<ND>, grid_for(c->n, c->blk_pair), c->blk_pair, 0, \
-                  c->cfg, c->A, \
-                  c->g, c->mx_pos, c->mx_vel, c->mx_aux, c->mx_tg, c->mx_nbr, c->mx_ncnt, (int64_t)c->mx_maxn, c->n,         \
-                  (int)omega, (int)eos, c->mx_om)
-    SPHDEM_ND_DISPATCH(c->cfg.nd, L_);
-#undef L_
+void eos(sphdem_ctx *c) {
+    SPHDEM_LAUNCH(c, "eos32", k_eos32, grid_for(c->n, c->blk_pair), c->blk_pair, 0, c->cfg, c->A, c->mx_aux, c->mx_tg, c->n);
 }
 
 void force(sphdem_ctx *c) {
@@ -1227,7 +1176,7 @@ void prepare(sphdem_ctx *) {
 #undef A_
     const int bytes2 = (int)(2 * ST_CAP * sizeof(float4));
 #define D_(ND) \
-    SPHDEM_CUDA_CHECK(cudaFuncSetAttribute(k_dddt<ND, true, -1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes2))
+    SPHDEM_CUDA_CHECK(cudaFuncSetAttribute(k_dddt<ND, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes2))
     D_(2);
     D_(3);
 #undef D_
@@ -1242,7 +1191,7 @@ void dddt(sphdem_ctx *c) {
     const bool tile = c->cfg.nd > 1 && c->force_tile;
     const size_t st_bytes = tile ? (size_t)2 * ST_CAP * sizeof(float4) : 0;
 #define LD_(ND, CGF, T)                                                                                         \
-    SPHDEM_LAUNCH(c, "dddt32", (k_dddt<ND, CGF, -1, T>), grid_for(c->n, c->blk_pair), c->blk_pair, st_bytes,   \
+    SPHDEM_LAUNCH(c, "dddt32", (k_dddt<ND, CGF, T>), grid_for(c->n, c->blk_pair), c->blk_pair, st_bytes,   \
                   c->cfg, c->A, c->g, c->mx_pos, c->mx_vel, c->mx_aux, c->mx_om, c->mx_tg, c->mx_nbr,          \
                   c->mx_ncnt, (int64_t)c->mx_maxn, c->n, cgrows, c->buf.start, c->buf.skey)
     if (c->cfg.nd == 1) {
