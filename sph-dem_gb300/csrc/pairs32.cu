@@ -129,7 +129,8 @@ __global__ void k_pack(DevCfg c, DevState s, const int *__restrict__ skey, const
  * the particle itself out, so the lists hold exactly the neighbours.  The
  * lane only keeps the smallest margin of 32 candidates; the rare 32 with a
  * doubtful one (or the particle itself) are gone over again.
- * Bound by instruction issue: the two builds of a coupled step of 1.08 M
+ * Bound by instruction issue, and from a lattice at rest (eight exact ties a
+ * particle) by the chains of the FP64 decisions: the two builds of a coupled step of 1.08 M
  * particles take 1.25 ms; tests into a bit mask, entries then spread over the
  * warp and a second kernel for the candidates in doubt took 2.68. */
 constexpr int NL_WARPS = 4;
