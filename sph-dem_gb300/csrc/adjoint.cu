@@ -1174,7 +1174,8 @@ bool open_pass(sphdem_ctx *c, int nsteps, int K, int mode) {
         /* size the per-step pair lists from the pairs of the current buckets */
         if (!a->slot) SPHDEM_CUDA_CHECK(cudaMalloc(&a->slot, sizeof(int)));
         SPHDEM_CUDA_CHECK(cudaMemsetAsync(a->slot, 0, sizeof(int), c->stream));
-        sph_pairs(c, nullptr, nullptr, a->slot, nullptr);
+        if (c->mx_maxn > 0 || c->f64_maxn > 0) mixed::nlist_pairs(c, a->slot);
+        else sph_pairs(c, nullptr, nullptr, a->slot, nullptr);
         int n0 = 0;
         SPHDEM_CUDA_CHECK(cudaMemcpyAsync(&n0, a->slot, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
         SPHDEM_CUDA_CHECK(cudaStreamSynchronize(c->stream));

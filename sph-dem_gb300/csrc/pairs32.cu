@@ -965,6 +965,13 @@ __global__ void __launch_bounds__(BLK) k_dddt(DevCfg c, DevState s, const DevGlo
     s.row(FD_DDDT)[a] += (double)(acc.s * roma);
 }
 
+/* total += sum of x */
+__global__ void k_sum(int64_t n, const int *__restrict__ x, int *total) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int v = __reduce_add_sync(0xffffffffu, i < n ? x[i] : 0);
+    if ((threadIdx.x & 31) == 0 && v) atomicAdd(total, v);
+}
+
 /* rows of the neighbour list in tag order (count pass when idx == nullptr) */
 __global__ void k_list_export(DevState s, const int *tg, const int *nbr, const int *ncnt, int64_t ld, int64_t n,
                               int *cnt, const long long *offs, int *idx) {
@@ -1115,7 +1122,8 @@ void nlist(sphdem_ctx *c, int depth, bool soft) {
 /* largest neighbour count at the current positions (sizes the lists); band
  * candidates and the particle itself count as neighbours, so this is an upper
  * bound */
-int nlist_max_count(sphdem_ctx *c) {
+/* neighbour counts of the current buckets and records into mx_ncnt */
+static void nlist_count(sphdem_ctx *c) {
     SPHDEM_CUDA_CHECK(cudaMemsetAsync(c->mx_ncnt, 0, c->n * sizeof(int), c->stream));
 #define L_(ND)                                                                                                    \
     k_nlist<ND, true, 1><<<nlist_blocks<ND, true, 1>(c->n), NL_WARPS * 32, 0, c->stream>>>(                           \
@@ -1124,6 +1132,18 @@ int nlist_max_count(sphdem_ctx *c) {
     SPHDEM_ND_DISPATCH(c->cfg.nd, L_);
 #undef L_
     SPHDEM_CUDA_CHECK(cudaGetLastError());
+}
+
+void nlist_pairs(sphdem_ctx *c, int *total) {
+    if (c->cfg.precision == SPHDEM_PREC_MIXED) pack(c, false);
+    else pack_positions(c, false);
+    nlist_count(c);
+    k_sum<<<grid_for(c->n, 256), 256, 0, c->stream>>>(c->n, c->mx_ncnt, total);
+    SPHDEM_CUDA_CHECK(cudaGetLastError());
+}
+
+int nlist_max_count(sphdem_ctx *c) {
+    nlist_count(c);
     std::vector<int> h(c->n);
     SPHDEM_CUDA_CHECK(cudaMemcpyAsync(h.data(), c->mx_ncnt, c->n * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     SPHDEM_CUDA_CHECK(cudaStreamSynchronize(c->stream));
