@@ -1133,8 +1133,8 @@ namespace {
 
 /* The buffers and replay graphs of the handle's last pass serve the next one of
  * the same form (steps, checkpoint interval, tape memory, population), as a loss
- * is minimised over repeated passes: 8 coupled steps of 107,618 particles take
- * 15.8 ms forward with allocation, capture and instantiation, 11.6 without.  One
+ * is minimised over repeated passes: allocation, capture and instantiation took
+ * 4.2 ms of a forward pass over 8 coupled steps of 107,618 particles (9.3 now).  One
  * pass's buffers are held, as before; they go with the handle, a pass of another
  * form or a change of the population. */
 bool same_form(const sphdem_ctx *c, const AdjointData *a, int nsteps, int K, int mode) {
