@@ -57,7 +57,7 @@ UNIT = "particle-steps/s"
 SM_COUNT = 152
 FP32_LANES = 128
 # FLOPs per listed pair of the force pass (kernel evaluations for h_a and h_b,
-# Morris viscosity, pressure; counted from k_force32's FP32 instruction mix)
+# Morris viscosity, pressure; counted from the general force pass's FP32 instruction mix)
 FORCE_FLOP_PER_PAIR = 80.0
 
 
