@@ -601,7 +601,12 @@ int sphdem_create(const SphDemConfig *cfg, const SphDemParticles *init, int64_t 
             SPHDEM_CUDA_CHECK(cudaMalloc(&c->mx_dp, capacity * sizeof(float4)));
             SPHDEM_CUDA_CHECK(cudaMalloc(&c->mx_ds, capacity * sizeof(float4)));
             SPHDEM_CUDA_CHECK(cudaMalloc(&c->mx_nb, 3 * capacity * sizeof(float4)));
-            if (c->cfg.liq_dem()) {
+            c->mx_dem_only = true;
+            for (int64_t i = 0; i < n; i++) c->mx_dem_only = c->mx_dem_only && init->iam[i] == T_DEM;
+            /* kept pairs of the mixed coupling passes; a handle of DEM only runs the
+             * FP64 passes, whose kernel values are doubles, and keeps none: should
+             * fluid be inserted, its drag pass searches again */
+            if (c->cfg.liq_dem() && !c->mx_dem_only) {
                 SPHDEM_CUDA_CHECK(cudaMalloc(&c->cp_id, kept_entries(capacity) * sizeof(int)));
                 SPHDEM_CUDA_CHECK(cudaMalloc(&c->cp_w, kept_entries(capacity) * sizeof(float)));
                 SPHDEM_CUDA_CHECK(cudaMalloc(&c->cp_num, 4 * capacity * sizeof(int)));
@@ -618,8 +623,6 @@ int sphdem_create(const SphDemConfig *cfg, const SphDemParticles *init, int64_t 
              * so off by default) */
             const char *ft = std::getenv("SPHDEM_FORCE_TILE");
             c->force_tile = ft && ft[0] == '1';
-            c->mx_dem_only = true;
-            for (int64_t i = 0; i < init->n; i++) c->mx_dem_only = c->mx_dem_only && init->iam[i] == T_DEM;
             mixed::pack(c);
             const int m = mixed::nlist_max_count(c);
             if (m > 0) {

@@ -94,3 +94,31 @@ def test_crowded_contacts_without_fluid(lib, precision):
     got = sim.get()
     for k in ("f", "fp", "v", "r", "fdrag", "shep_sum"):
         assert norm_gap(got[k], want[k]) <= 1e-11, k
+
+
+@pytest.mark.parametrize("nx", [12, 32])
+def test_fluid_inserted_into_a_handle_of_dem_only(lib, nx):
+    """A mixed handle of DEM only runs the FP64 passes, also once fluid has been
+    inserted up to its capacity, with more partners per fluid particle than the
+    kept pairs hold (four threads a particle, and one): the step of an FP64
+    handle created with all particles.  Both sum in FP64; the mixed handle takes
+    h and the reciprocals of the equation of state by a Newton step good to
+    1e-14, which the pressure (x^7 - 1) and its differences enlarge by up to
+    some 1e4: 1e-9 of each field's 2-norm."""
+    cfg, p = dense_bed(nx, 0.98)
+    order = np.argsort(p["iam"] != cases.DEM, kind="stable")
+    p = {k: v[order] for k, v in p.items()}
+    n, nd = p["iam"].size, int((p["iam"] == cases.DEM).sum())
+    whole = capi.Simulation(lib, cfg, p, precision=cases.PREC_FP64)
+    mixed = capi.Simulation(lib, cfg, {k: v[:nd] for k, v in p.items()}, precision=cases.PREC_MIXED, capacity=n)
+    assert np.array_equal(mixed.insert({k: v[nd:] for k, v in p.items()}), np.arange(nd, n))
+    got = []
+    for sim in (mixed, whole):
+        sim.rebuild()
+        sim.rebuild()   # the ghost widths of both handles follow the same h
+        sim.step(1)
+        a = sim.get()
+        got.append({k: a[k].copy() for k in FIELDS})
+        sim.close()
+    for k in FIELDS:
+        assert np.linalg.norm(got[1][k]) > 0 and norm_gap(got[0][k], got[1][k]) <= 1e-9, k
