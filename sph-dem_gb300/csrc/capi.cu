@@ -344,7 +344,7 @@ void middle_passes(sphdem_ctx *c, bool whole) {
      * paths, so the mixed handle runs the FP64 phases */
     if (c->cfg.precision == SPHDEM_PREC_MIXED && !c->mx_dem_only) {
         const bool lists = c->mx_maxn > 0;
-        mixed::pack(c);
+        mixed::pack(c, true);
         if (lists) mixed::nlist(c, c->mx_maxn);
         /* calcInvM in FP64 once per rebuild; the pair passes apply it in FP32 */
         if (corrected_gradient(c)) run_invm(c);
@@ -623,7 +623,7 @@ int sphdem_create(const SphDemConfig *cfg, const SphDemParticles *init, int64_t 
              * so off by default) */
             const char *ft = std::getenv("SPHDEM_FORCE_TILE");
             c->force_tile = ft && ft[0] == '1';
-            mixed::pack(c);
+            mixed::pack(c, false);
             const int m = mixed::nlist_max_count(c);
             if (m > 0) {
                 /* a run that outgrows the depth stops with SPHDEM_ERR_CAPACITY
@@ -752,7 +752,7 @@ int sphdem_rebuild(sphdem_handle h) {
     try {
         rebuild(h);
         if (h->mx_maxn > 0) {
-            mixed::pack(h);
+            mixed::pack(h, false); /* no porosity pass follows: the Shepard sums stay */
             mixed::nlist(h, h->mx_maxn);
         }
     } catch (const std::string &e) {

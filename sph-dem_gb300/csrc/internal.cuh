@@ -209,9 +209,9 @@ void mixed_list_export(sphdem_ctx *c, int *cnt, const long long *offs, int *idx)
 
 /* pairs32.cu: mixed-precision passes */
 namespace mixed {
-/* pack the FP32 records of the middle phase (which also starts the Shepard sums
- * at zero) or those of the end phase */
-void pack(sphdem_ctx *c, bool middle = true);
+/* pack the FP32 records of the middle phase, whose porosity pass follows (it also
+ * starts the Shepard sums at zero), or those of the end phase and of the searches */
+void pack(sphdem_ctx *c, bool middle);
 /* the neighbour lists of the last rebuild, `depth` entries per particle; more
  * neighbours are an error, or (soft) leave the particle without a list */
 void nlist(sphdem_ctx *c, int depth, bool soft = false);

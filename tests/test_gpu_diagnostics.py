@@ -62,3 +62,22 @@ def test_output_vars_match_reference(lib, name, precision):
         scale = np.abs(refv).max()
         err = np.abs(a[ours_name] - refv).max()
         assert err <= ftol * max(scale, 1e-300), f"{name}:{key} err {err:.3e} scale {scale:.3e}"
+
+
+@pytest.mark.parametrize("precision", [cases.PREC_FP64, cases.PREC_MIXED])
+@pytest.mark.parametrize("kind", ["sediment3d_small", "dem_small", "dambreak2d_own_small"])
+def test_rebuild_keeps_every_field(lib, kind, precision):
+    """sphdem_rebuild after a step finds every particle where the step's own
+    rebuild left it: no field changes, the Shepard sums of the spheres among
+    them (bit for bit)."""
+    case = cases.workload(kind)
+    sim = capi.Simulation(lib, case.cfg, case.particles, precision=precision)
+    sim.step(3)
+    before = {k: v.copy() for k, v in sim.get().arrays.items()}
+    sim.rebuild()
+    after = sim.get().arrays
+    for k, v in before.items():
+        assert np.array_equal(after[k], v), k
+    if kind == "sediment3d_small":
+        assert (before["shep_sum"][case.particles["iam"] == cases.DEM] > 0).all()
+    sim.close()
