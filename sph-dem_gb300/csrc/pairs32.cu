@@ -168,7 +168,8 @@ __device__ __forceinline__ void queue_append(unsigned &qa, int e, float margin) 
     asm volatile(
         "{\n .reg .pred p;\n setp.ge.f32 p, %2, 0f00000000;\n @p st.shared.u32 [%0], %1;\n @p add.u32 %0, %0, 128;\n}\n"
         : "+r"(qa)
-        : "r"(e), "f"(margin));
+        : "r"(e), "f"(margin)
+        : "memory");
 }
 
 /* G lanes per particle: a warp takes 32 / G consecutive particles and each of
