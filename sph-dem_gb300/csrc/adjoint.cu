@@ -1242,6 +1242,7 @@ int adjoint_forward(sphdem_ctx *c, int nsteps, int K, int mode) {
         rc = forward_pass(c, nsteps, K, mode);
     } catch (...) {
         adjoint_free(c);
+        cudaGetLastError(); /* a refused allocation is reported by this call, not by the next */
         throw;
     }
     if (rc != SPHDEM_OK) adjoint_free(c);

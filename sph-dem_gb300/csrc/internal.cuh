@@ -217,9 +217,9 @@ void pack(sphdem_ctx *c, bool middle);
 void nlist(sphdem_ctx *c, int depth, bool soft = false);
 /* once per process, outside stream capture: kernel attributes of the step */
 void prepare(sphdem_ctx *c);
+/* the largest neighbour count of the current buckets (sizes the lists), and their
+ * sum added to *total (device; packs the records): upper bounds, see nlist_count */
 int nlist_max_count(sphdem_ctx *c);
-/* adds the number of listed pairs of the current buckets to *total (device);
- * packs the records and overwrites the counts of the last list */
 void nlist_pairs(sphdem_ctx *c, int *total);
 void eos(sphdem_ctx *c);
 /* lists32.cu: the force / continuity passes specialised on the physics class;

@@ -1120,33 +1120,34 @@ void nlist(sphdem_ctx *c, int depth, bool soft) {
 #undef LG_
 }
 
-/* largest neighbour count at the current positions (sizes the lists); band
- * candidates and the particle itself count as neighbours, so this is an upper
- * bound */
-/* neighbour counts of the current buckets and records into mx_ncnt */
-static void nlist_count(sphdem_ctx *c) {
-    SPHDEM_CUDA_CHECK(cudaMemsetAsync(c->mx_ncnt, 0, c->n * sizeof(int), c->stream));
+/* neighbour counts of the current buckets and records, into scratch of the
+ * rebuild: mx_ncnt holds the counts of the lists that are there.  Candidates FP32
+ * cannot decide and the particle itself count as neighbours, so these are upper
+ * bounds */
+static int *nlist_count(sphdem_ctx *c) {
+    int *cnt = c->buf.slot;
+    SPHDEM_CUDA_CHECK(cudaMemsetAsync(cnt, 0, c->n * sizeof(int), c->stream));
 #define L_(ND)                                                                                                    \
     k_nlist<ND, true, 1><<<nlist_blocks<ND, true, 1>(c->n), NL_WARPS * 32, 0, c->stream>>>(                           \
-        c->cfg, c->dcfg, c->A, c->buf.start, c->buf.skey, c->g, c->mx_pos, c->mx_tg, c->mx_nbr,      \
-        c->mx_ncnt, 0, 0, nullptr)
+        c->cfg, c->dcfg, c->A, c->buf.start, c->buf.skey, c->g, c->mx_pos, c->mx_tg, nullptr,        \
+        cnt, 0, 0, nullptr)
     SPHDEM_ND_DISPATCH(c->cfg.nd, L_);
 #undef L_
     SPHDEM_CUDA_CHECK(cudaGetLastError());
+    return cnt;
 }
 
 void nlist_pairs(sphdem_ctx *c, int *total) {
     if (c->cfg.precision == SPHDEM_PREC_MIXED) pack(c, false);
     else pack_positions(c, false);
-    nlist_count(c);
-    k_sum<<<grid_for(c->n, 256), 256, 0, c->stream>>>(c->n, c->mx_ncnt, total);
+    k_sum<<<grid_for(c->n, 256), 256, 0, c->stream>>>(c->n, nlist_count(c), total);
     SPHDEM_CUDA_CHECK(cudaGetLastError());
 }
 
 int nlist_max_count(sphdem_ctx *c) {
-    nlist_count(c);
+    const int *cnt = nlist_count(c);
     std::vector<int> h(c->n);
-    SPHDEM_CUDA_CHECK(cudaMemcpyAsync(h.data(), c->mx_ncnt, c->n * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    SPHDEM_CUDA_CHECK(cudaMemcpyAsync(h.data(), cnt, c->n * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     SPHDEM_CUDA_CHECK(cudaStreamSynchronize(c->stream));
     int m = 0;
     for (int v : h) m = std::max(m, v);

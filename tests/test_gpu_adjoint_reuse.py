@@ -81,3 +81,30 @@ def test_fp64_pair_tables_beyond_the_list_depth(lib):
         sim.close()
     for a, b in zip(*got):
         assert np.linalg.norm(a - b) <= 1e-11 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("kind", ["dambreak", "coupled"])
+def test_refused_pass_leaves_the_lists(lib, kind):
+    """A gradient pass sizes its tables by a count of the present pairs before it
+    allocates them.  When the allocation is refused (tapes of 1e8 steps are some
+    terabytes) the handle's neighbour lists are the ones of before, and it steps
+    on as if nothing had been asked."""
+    if kind == "dambreak":
+        case = cases.dambreak2d(dx=0.05)
+    else:
+        case = cases.sediment3d(nx=12, L=0.03, height=0.06, n_dem=60, floor="sphb3", var_h=False)
+    sims = [capi.Simulation(lib, case.cfg, case.particles, precision=cases.PREC_MIXED) for _ in range(2)]
+    for sim in sims:
+        sim.step(2)
+    want = sims[0].pairs(capi.PAIRS_SPH)
+    with pytest.raises(capi.SphDemError, match="CUDA"):
+        sims[0].adjoint_forward(10 ** 8, 10 ** 8)
+    got = sims[0].pairs(capi.PAIRS_SPH)
+    assert want[1].size > 0 and all(np.array_equal(a, b) for a, b in zip(got, want))
+    for sim in sims:
+        sim.step(1)
+    a, b = (sim.get() for sim in sims)
+    # coupled: the Shepard sums' atomics turn FP32 roundings, 2e-7 a step
+    tol = 0.0 if kind == "dambreak" else 6e-7
+    for k in ("r", "v", "f", "dens"):
+        assert np.linalg.norm(a[k] - b[k]) <= tol * np.linalg.norm(b[k]), k
