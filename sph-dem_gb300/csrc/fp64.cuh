@@ -7,6 +7,7 @@
 #include <cfloat>
 
 #include "internal.cuh"
+#include "series.cuh"
 
 namespace sphdem {
 namespace {
@@ -56,19 +57,17 @@ __device__ __forceinline__ void block_min_atomic(double v, unsigned long long *t
     }
 }
 
-/* 1/x for x > 0: an FP32 estimate y (relative error d ~ 1e-7) and one step of
- * the series 1/x = y (1 + e + e^2 + ..), e = 1 - x y, which leaves d^3 */
+/* 1/x for x > 0 (rcp_series) */
 __device__ __forceinline__ double rcp_pos(double x) {
     const float xf = (float)x;
     if (!(xf > 1e-30f && xf < 1e30f)) return 1.0 / x;
     float yf;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(yf) : "f"(xf));
-    const double y = (double)yf, e = fma(-x, y, 1.0);
-    return fma(y, fma(e, e, e), y);
+    return rcp_series(x, (double)yf);
 }
 
-/* sqrt(x) and, where asked, 1/sqrt(x) of x >= 0: an FP32 estimate y of 1/sqrt
- * and one step of the series 1/sqrt(1 - e) = 1 + e/2 + 3 e^2/8 + .., e = 1 - x y^2 */
+/* sqrt(x) and, where asked, 1/sqrt(x) of x >= 0 (sqrt_series; FULL: sqrt_series_full) */
+template <bool FULL = false>
 __device__ __forceinline__ double sqrt_pos(double x, double *inv = nullptr) {
     const float xf = (float)x;
     if (!(xf > 1e-30f && xf < 1e30f)) {
@@ -78,10 +77,8 @@ __device__ __forceinline__ double sqrt_pos(double x, double *inv = nullptr) {
     }
     float yf;
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(yf) : "f"(xf));
-    const double y = (double)yf, s = x * y;
-    const double e = fma(-s, y, 1.0), k = e * fma(e, 0.375, 0.5);
-    if (inv) *inv = fma(y, k, y);
-    return fma(s, k, s);
+    if (FULL) return sqrt_series_full(x, (double)yf, inv);
+    return sqrt_series(x, (double)yf, inv);
 }
 
 /* max(x, 0) by the sign bit (an integer operation) */

@@ -1,0 +1,68 @@
+"""The reciprocals and roots that the pass kernels take from a hardware estimate
+(csrc/series.cuh), on the CPU against wider arithmetic.  The estimates are FP32
+numbers up to 2 ulp off (the instructions' stated error).  Bound: half an ulp for the
+last rounding, the series' first dropped term ((2.4e-7)^3 and 5/16 of it,
+below 1e-4 ulp) and the roundings of a correction of 2e-7 of the result (below
+1e-6 ulp): 0.501 ulp; the short form of the root lets half of the rounding of s = x y
+in as well, half an ulp of s: 0.751 ulp of the root, which shares s's binade, and
+1.001 of its reciprocal, whose ulp may be half as large relative to it."""
+import os
+import subprocess
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "sph-dem_gb300", "csrc")
+
+HARNESS = r"""
+#include <algorithm>
+#include <cfloat>
+#include <cstdio>
+#include <random>
+#include "series.cuh"
+
+/* |got - want| in units of the last place of want */
+static double ulps(double got, long double want) {
+    const double w = (double)want;
+    return (double)(fabsl((long double)got - want) / (std::nextafter(fabs(w), INFINITY) - fabs(w)));
+}
+static float off(float x, int n) {
+    for (; n > 0; n--) x = std::nextafterf(x, INFINITY);
+    for (; n < 0; n++) x = std::nextafterf(x, 0.f);
+    return x;
+}
+
+int main() {
+    std::mt19937_64 rng(7);
+    std::uniform_real_distribution<double> ex(-29.0, 29.0);
+    double worst[5] = {0, 0, 0, 0, 0};
+    for (int k = 0; k < 400000; k++) {
+        const double x = std::pow(10.0, ex(rng));
+        const int n = (int)(rng() % 5) - 2;
+        const float yr = off((float)(1.0 / x), n), ys = off((float)(1.0 / std::sqrt(x)), n);
+        worst[0] = std::max(worst[0], ulps(sphdem::rcp_series(x, yr), 1.0L / (long double)x));
+        double inv = 0.0;
+        const long double root = sqrtl((long double)x);
+        worst[1] = std::max(worst[1], ulps(sphdem::sqrt_series_full(x, ys, &inv), root));
+        worst[2] = std::max(worst[2], ulps(inv, 1.0L / root));
+        worst[3] = std::max(worst[3], ulps(sphdem::sqrt_series(x, ys, &inv), root));
+        worst[4] = std::max(worst[4], ulps(inv, 1.0L / root));
+    }
+    for (double w : worst) printf("%.6f ", w);
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def errors(tmp_path_factory):
+    d = tmp_path_factory.mktemp("series")
+    src, exe = d / "series.cpp", d / "series"
+    src.write_text(HARNESS)
+    # series.cuh says what it fuses: no contraction of its own by the compiler
+    subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", f"-I{CSRC}", str(src), "-o", str(exe)], check=True)
+    return [float(v) for v in subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.split()]
+
+
+@pytest.mark.parametrize("k,what,bound", [(0, "reciprocal", 0.501), (1, "root", 0.501), (2, "reciprocal root", 0.501),
+                                          (3, "root, short form", 0.751), (4, "reciprocal root, short form", 1.001)])
+def test_fp64_series(errors, k, what, bound):
+    assert 0.4 < errors[k] <= bound, what
