@@ -43,4 +43,21 @@ SPHDEM_HD double sqrt_series_full(double x, double y, double *inv) {
     return fma(fma(-s, s, x) * y, k, s);
 }
 
+/* num / den from an estimate y of 1/den (FP32 scalars or pairs), the remainder
+ * of the quotient taken back once: 0.5 ulp, where num y by itself is off by up to
+ * two.  For numbers whose quotient is in range; infinities give NaN. */
+SPHDEM_HD float fused(float a, float b, float c) { return fmaf(a, b, c); }
+SPHDEM_HD float times(float a, float b) { return a * b; }
+SPHDEM_HD float minus(float a) { return -a; }
+#ifdef __CUDACC__
+__device__ __forceinline__ float2 fused(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+__device__ __forceinline__ float2 times(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 minus(float2 a) { return make_float2(-a.x, -a.y); }
+#endif
+template <class V>
+SPHDEM_HD V quotient(V num, V den, V y) {
+    const V q = times(num, y);
+    return fused(fused(minus(q), den, num), y, q);
+}
+
 }  // namespace sphdem
