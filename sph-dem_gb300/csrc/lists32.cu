@@ -345,9 +345,7 @@ __global__ void __launch_bounds__(BLK, 4) k_force_list(DevCfg c, const DevCfg *_
     for (int k = 0; k < ND; k++) {
         tp[k] = fp[k].template total<G>();
         tv[k] = fv[k].template total<G>();
-        tb[k] = fb[k].s;
-#pragma unroll
-        for (int o = 1; o < G; o <<= 1) tb[k] += __shfl_xor_sync(0xffffffffu, tb[k], o);
+        tb[k] = fb[k].template total<G>();
     }
     float omt = om.x + om.y;
     if (VARH) {

@@ -18,6 +18,27 @@ constexpr int BLK = 128;
 constexpr int B_BITS = 26;
 constexpr int B_MASK = (1 << B_BITS) - 1;
 
+/* a + b = r + e, e the rounding error */
+__device__ __forceinline__ void two_sum(float a, float b, float &r, float &e) {
+    r = a + b;
+    const float bb = r - a;
+    e = (a - (r - bb)) + (b - bb);
+}
+
+/* the sum of t + c over G consecutive lanes, c a small correction of t */
+template <int G>
+__device__ __forceinline__ float join_lanes(float t, float c) {
+#pragma unroll
+    for (int o = 1; o < G; o <<= 1) {
+        const float to = __shfl_xor_sync(0xffffffffu, t, o), co = __shfl_xor_sync(0xffffffffu, c, o);
+        float u, e;
+        two_sum(t, to, u, e);
+        t = u;
+        c = (c + co) + e;
+    }
+    return t + c;
+}
+
 struct Kahan {
     float s, c;
     __device__ __forceinline__ void init(float v) {
@@ -29,6 +50,12 @@ struct Kahan {
         const float t = s + y;
         c = (t - s) - y;
         s = t;
+    }
+    /* the total of G consecutive lanes' sums (all lanes of the warp call it) with
+     * the additions' rounding errors kept */
+    template <int G>
+    __device__ __forceinline__ float total() const {
+        return join_lanes<G>(s, -c);
     }
 };
 
@@ -60,21 +87,7 @@ struct Kahan2 {
     __device__ __forceinline__ float total() const {
         float t, e;
         two_sum(s.x, s.y, t, e);
-        float c = e + (n.x + n.y);
-#pragma unroll
-        for (int o = 1; o < G; o <<= 1) {
-            const float to = __shfl_xor_sync(0xffffffffu, t, o), co = __shfl_xor_sync(0xffffffffu, c, o);
-            float u;
-            two_sum(t, to, u, e);
-            t = u;
-            c = (c + co) + e;
-        }
-        return t + c;
-    }
-    static __device__ __forceinline__ void two_sum(float a, float b, float &r, float &e) {
-        r = a + b;
-        const float bb = r - a;
-        e = (a - (r - bb)) + (b - bb);
+        return join_lanes<G>(t, e + (n.x + n.y));
     }
 };
 
