@@ -564,11 +564,11 @@ __device__ __noinline__ double difelice_vjp(const DevCfg &c, const double *dv, d
     return Pd * dgPsi_dRe * (-Re / c.viscosity);
 }
 
-/* FPI + Di Felice drag of each DEM particle (end phase), one warp per DEM
- * particle: the lanes split its fluid partners for the forward sums (warp
- * reductions), every lane then runs the drag VJP on the reduced values and
- * the lanes split the partners again for the particle's own position
- * adjoint.  The adjoints of the normalised sums go to the particle's
+/* FPI + Di Felice drag of each DEM particle (end phase) in three passes: the
+ * forward sums over its fluid partners (k_cp_fpi_sums, one warp per DEM particle),
+ * the drag law and its VJP on them (k_cp_fpi_drag, a thread each), and the
+ * particle's own position adjoint over the partners (k_cp_fpi_own, a warp each).
+ * The sums, then the adjoints of the normalised sums, stand in the particle's
  * coefficient record (CF_*), from which k_cp_fpi_fluid gathers each fluid
  * particle's share.  Delta_i's adjoint is that of f1 + fdrag1.  Pair math in
  * M, per-particle math in FP64. */

@@ -229,8 +229,9 @@ std::string validate(const SphDemConfig *cfg, const SphDemParticles *p, int64_t 
     if ((cfg->flags & SPHDEM_F_LIQ_DEM) && !(cfg->dem_search_radius > 0 && cfg->coupling_radius > 0))
         return "LIQ_DEM needs dem_search_radius and coupling_radius";
     if ((cfg->flags & SPHDEM_F_LIQ_DEM) && cfg->precision == SPHDEM_PREC_MIXED) {
-        /* the mixed coupling pass packs reference DEM bucket indices (of
-         * particles and their periodic images) into 10 bits per axis */
+        /* a limit of the mixed path's interface: reference DEM bucket indices (of
+         * particles and their periodic images) of 10 bits per axis.  The present
+         * passes would take more */
         for (int d = 0; d < cfg->ndim; d++) {
             const double w = 2 * cfg->dem_search_radius;
             const double off = 2 * cfg->coupling_radius / cfg->dem_search_radius - 1;
@@ -274,7 +275,6 @@ void free_ctx(sphdem_ctx *c) {
     cudaFree(c->mx_vel);
     cudaFree(c->mx_aux);
     cudaFree(c->mx_tg);
-    cudaFree(c->mx_om);
     cudaFree(c->mx_nbr);
     cudaFree(c->mx_ncnt);
     cudaFree(c->stage);
@@ -594,7 +594,6 @@ int sphdem_create(const SphDemConfig *cfg, const SphDemParticles *init, int64_t 
             SPHDEM_CUDA_CHECK(cudaMalloc(&c->mx_vel, capacity * sizeof(float4)));
             SPHDEM_CUDA_CHECK(cudaMalloc(&c->mx_aux, capacity * sizeof(float4)));
             SPHDEM_CUDA_CHECK(cudaMalloc(&c->mx_tg, capacity * sizeof(int)));
-            SPHDEM_CUDA_CHECK(cudaMalloc(&c->mx_om, capacity * sizeof(float)));
             SPHDEM_CUDA_CHECK(cudaMalloc(&c->mx_ncnt, capacity * sizeof(int)));
             SPHDEM_CUDA_CHECK(cudaMalloc(&c->mx_q0, capacity * sizeof(float4)));
             SPHDEM_CUDA_CHECK(cudaMalloc(&c->mx_q1, capacity * sizeof(float2)));
@@ -613,7 +612,6 @@ int sphdem_create(const SphDemConfig *cfg, const SphDemParticles *init, int64_t 
             }
             SPHDEM_CUDA_CHECK(cudaMalloc(&c->mx_bandn, capacity * sizeof(int)));
             SPHDEM_CUDA_CHECK(cudaMemset(c->mx_bandn, 0, capacity * sizeof(int)));
-            SPHDEM_CUDA_CHECK(cudaMemset(c->mx_om, 0, capacity * sizeof(float)));
             SPHDEM_CUDA_CHECK(cudaMemset(c->mx_ncnt, 0, capacity * sizeof(int)));
             SPHDEM_CUDA_CHECK(cudaDeviceSynchronize());
             mixed::prepare(c);

@@ -97,7 +97,6 @@ struct sphdem_ctx {
     /* mixed precision: packed FP32 particle records and neighbour lists */
     float4 *mx_pos = nullptr, *mx_vel = nullptr, *mx_aux = nullptr;
     int *mx_tg = nullptr;       /* type | ghost code << 8 */
-    float *mx_om = nullptr;     /* Omega (VAR_H_CORRECTION) */
     int *mx_nbr = nullptr;      /* lists in tiles of 32 particles x 8 slots, mx_maxn x cap (rounded to 32) */
     int *mx_ncnt = nullptr;
     int mx_maxn = 0;
@@ -199,8 +198,8 @@ void run_lists64(sphdem_ctx *c, bool middle);
 void run_force(sphdem_ctx *c);         /* calcForce + calcOmega + accelCondition */
 void run_dem_accel(sphdem_ctx *c);
 void run_dddt(sphdem_ctx *c);          /* calcDddtDudt                      */
-void run_invm(sphdem_ctx *c);
-void run_dem_block(sphdem_ctx *c);     /* DEM_BLOCK: mean DEM force     */          /* calcInvM (CORRECTED_GRADIENT)     */
+void run_invm(sphdem_ctx *c);          /* calcInvM (CORRECTED_GRADIENT)     */
+void run_dem_block(sphdem_ctx *c);     /* DEM_BLOCK: mean DEM force         */
 void run_reinit_density(sphdem_ctx *c); /* reset + ten rounds of calcHFromDens and calcDensity */
 void run_dem_end(sphdem_ctx *c);       /* calcFPI + calcDEMContacts         */
 

@@ -78,7 +78,7 @@ __device__ __forceinline__ float2 omega_poly(float2 q, float2 t3) {
 
 /* visit a lane's share of a particle's list: body(std::bool_constant masked,
  * e0, e1), two entries at a time, the lane's next group of 8 in flight.  In a
- * masked call either entry may be < 0 (none). */
+ * masked call the second entry may be < 0 (none). */
 template <int G, class Body>
 __device__ __forceinline__ void visit_list(const int *__restrict__ nbr, int64_t a, int64_t ld, int cnt, int sub, Body &&body) {
     const int4 *tile = reinterpret_cast<const int4 *>(nbr + nl_at(a, 0, ld));
@@ -117,7 +117,7 @@ template <int ND, int VISC, bool VARH, int G, bool TILE>
 __global__ void __launch_bounds__(BLK, 4) k_force_list(DevCfg c, const DevCfg *__restrict__ cp, DevState s,
                                                     DevGlobals *__restrict__ g, const float4 *__restrict__ P0,
                                                     const float4 *__restrict__ P1, const float4 *__restrict__ P2,
-                                                    float *__restrict__ om32, const int *__restrict__ tg,
+                                                    const int *__restrict__ tg,
                                                     const int *__restrict__ nbr, const int *__restrict__ ncnt,
                                                     int64_t ld, int64_t n, const float4 *__restrict__ NB,
                                                     const int *__restrict__ start, const int *__restrict__ skey) {
@@ -322,7 +322,6 @@ __global__ void __launch_bounds__(BLK, 4) k_force_list(DevCfg c, const DevCfg *_
             const float sum = hd1 * (omt * wcon - va.w * ND * wK32(0.f, wcon));
             const float omega = 1.f + ha * sum / (densa * ND);
             s.row(FD_OMEGA)[a] = omega;
-            om32[a] = omega;
             roma = 1.f / omega;
         }
         float fsum2 = 0.f;
@@ -349,7 +348,7 @@ __global__ void __launch_bounds__(BLK, 4) k_force_list(DevCfg c, const DevCfg *_
 template <int ND, bool VARH, int G, bool TILE>
 __global__ void __launch_bounds__(BLK) k_dddt_list(DevCfg c, DevState s, DevGlobals *__restrict__ g,
                                                    const float4 *__restrict__ P0, const float4 *__restrict__ P1,
-                                                   const float4 *__restrict__ P2, float *__restrict__ om32,
+                                                   const float4 *__restrict__ P2,
                                                    const int *__restrict__ tg, const int *__restrict__ nbr,
                                                    const int *__restrict__ ncnt, int64_t ld, int64_t n,
                                                    const int *__restrict__ start, const int *__restrict__ skey) {
@@ -446,7 +445,6 @@ __global__ void __launch_bounds__(BLK) k_dddt_list(DevCfg c, DevState s, DevGlob
         const float o = hd1 * (omt * wcon - va.w * ND * wK32(0.f, wcon));
         const float omega = 1.f + ha * o / (xa.x * ND);
         s.row(FD_OMEGA)[a] = omega;
-        om32[a] = omega;
         rate = sum * cFa / omega;
     }
     s.row(FD_DDDT)[a] += (double)rate;
@@ -510,7 +508,7 @@ bool force_lists(sphdem_ctx *c) {
     const int lanes = force_lanes(c->n, c->cfg.nd);
 #define LK_(ND, V, H, G, T)                                                                                       \
     SPHDEM_LAUNCH(c, "force32", (k_force_list<ND, V, H, G, T>), grid_for(c->n * G, c->blk_pair), c->blk_pair, st_bytes, \
-                  c->cfg, c->dcfg, c->A, c->g, c->mx_pos, c->mx_vel, c->mx_aux, c->mx_om, c->mx_tg, c->mx_nbr,     \
+                  c->cfg, c->dcfg, c->A, c->g, c->mx_pos, c->mx_vel, c->mx_aux, c->mx_tg, c->mx_nbr,     \
                   c->mx_ncnt, (int64_t)c->mx_maxn, c->n, c->mx_nb, c->buf.start, c->buf.skey)
 #define LG_(ND, G, T) FORCE_CLASS_(LK_, ND, G, T)
     if (c->cfg.nd == 3)
@@ -529,7 +527,7 @@ bool dddt_lists(sphdem_ctx *c) {
     const int lanes = dddt_lanes(c->n, c->cfg.nd);
 #define LK_(ND, H, G, T)                                                                                          \
     SPHDEM_LAUNCH(c, "dddt32", (k_dddt_list<ND, H, G, T>), grid_for(c->n * G, c->blk_pair), c->blk_pair, st_bytes, \
-                  c->cfg, c->A, c->g, c->mx_pos, c->mx_vel, c->mx_aux, c->mx_om, c->mx_tg, c->mx_nbr, c->mx_ncnt,  \
+                  c->cfg, c->A, c->g, c->mx_pos, c->mx_vel, c->mx_aux, c->mx_tg, c->mx_nbr, c->mx_ncnt,  \
                   (int64_t)c->mx_maxn, c->n, c->buf.start, c->buf.skey)
 #define LG_(ND, G, T)              \
     do {                           \

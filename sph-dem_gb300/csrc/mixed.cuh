@@ -110,12 +110,6 @@ __device__ __forceinline__ float powi(float x) {
     return r;
 }
 
-__device__ __forceinline__ float warp_sum(float v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
 template <int ND>
 __device__ __forceinline__ void decode(int key, const int *dims, int *cc) {
     if (ND == 3) {

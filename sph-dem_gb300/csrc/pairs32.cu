@@ -40,11 +40,11 @@ namespace {
  * particles that are neither sph / sphBoundary nor DEM), P2 = (dens, pdr2, cF,
  * 1/h) for the middle phase and (dens, cF, porosity, 1/h) for the end phase,
  * where cF = -10 C / h^(d+2) is the factor of the Wendland gradient F(r, h) =
- * cF (2 - r/h)^3 and a DEM particle's second place holds its radius,
- * tg = type | gcode << 8.  cF follows from the FP32 1/h next to it, so that factor
- * and argument belong to one kernel: with cF of the FP64 h the rounding of 1/h
- * stays in (2 - r/h)^3 alone, an error of one sign in a run with constant h (of
- * the pairs' moment sum F r^2, rms over h: 1.3e-7 in 3D, in this form 2.9e-8) */
+ * cF (2 - r/h)^3, tg = type | gcode << 8.  cF follows from the FP32 1/h next to
+ * it, so that factor and argument belong to one kernel: with cF of the FP64 h the
+ * rounding of 1/h stays in (2 - r/h)^3 alone, an error of one sign in a run with
+ * constant h (of the pairs' moment sum F r^2, rms over h: 1.3e-7 in 3D, in this
+ * form 2.9e-8) */
 template <int ND>
 __global__ void k_pack(DevCfg c, DevState s, const int *__restrict__ skey, const DevGlobals *__restrict__ g,
                        float4 *__restrict__ P0, float4 *__restrict__ P1, float4 *__restrict__ P2,
@@ -78,14 +78,12 @@ __global__ void k_pack(DevCfg c, DevState s, const int *__restrict__ skey, const
      * load the type row only for those (walls) */
     const float mpk = (float)s.row(FD_MASS)[i];
     P1[i] = make_float4(vh[0], vh[1], vh[2], (is_sph_or_sphb(t) || dem) ? mpk : -mpk);
-    /* a DEM particle's pdr2 slot holds its radius (the contact pre-test) */
-    const double rad = s.row(FD_RADIUS)[i] > 0 ? s.row(FD_RADIUS)[i] : c.dem_radius;
     const float ih = (float)s.row(FD_IH)[i];
     double ihn2 = (double)ih * (double)ih;
 #pragma unroll
     for (int d = 0; d < ND; d++) ihn2 *= (double)ih;
     const float cF = (float)(-10.0 * c.wcon * ihn2);
-    P2[i] = make_float4((float)s.row(FD_DENS)[i], t == T_DEM ? (float)rad : (middle ? (float)s.row(FD_PDR2)[i] : cF),
+    P2[i] = make_float4((float)s.row(FD_DENS)[i], middle ? (float)s.row(FD_PDR2)[i] : cF,
                         middle ? cF : (float)s.row(FD_POR)[i], ih);
     if (is_boundary(t)) {
         float nv[3][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
@@ -646,7 +644,7 @@ struct Cg32 {
 template <int ND, int PHYS, bool TILE>
 __global__ void __launch_bounds__(BLK) k_force(DevCfg c, const DevCfg *__restrict__ cp, DevState s, DevGlobals *__restrict__ g,
                                                const float4 *__restrict__ P0, const float4 *__restrict__ P1,
-                                               const float4 *__restrict__ P2, float *__restrict__ om32,
+                                               const float4 *__restrict__ P2,
                                                const int *__restrict__ tg, const int *__restrict__ nbr,
                                                const int *__restrict__ ncnt, int64_t ld, int64_t n,
                                                const float4 *__restrict__ NB, const double *__restrict__ cgrows,
@@ -840,7 +838,6 @@ __global__ void __launch_bounds__(BLK) k_force(DevCfg c, const DevCfg *__restric
             /* Omega = 1 + h*sum/(rho*NDIM): an O(1) number, FP32 is ample */
             const float omega = 1.f + ha * om.s / (densa * ND);
             s.row(FD_OMEGA)[a] = omega;
-            om32[a] = omega;
             roma = 1.f / omega;
         }
         float fsum2 = 0.f;
@@ -865,7 +862,7 @@ __global__ void __launch_bounds__(BLK) k_force(DevCfg c, const DevCfg *__restric
 template <int ND, bool CG, bool TILE>
 __global__ void __launch_bounds__(BLK) k_dddt(DevCfg c, DevState s, const DevGlobals *__restrict__ g,
                                               const float4 *__restrict__ P0, const float4 *__restrict__ P1,
-                                              const float4 *__restrict__ P2, float *__restrict__ om32,
+                                              const float4 *__restrict__ P2,
                                               const int *__restrict__ tg, const int *__restrict__ nbr,
                                               const int *__restrict__ ncnt, int64_t ld, int64_t n,
                                               const double *__restrict__ cgrows,
@@ -967,7 +964,6 @@ __global__ void __launch_bounds__(BLK) k_dddt(DevCfg c, DevState s, const DevGlo
     if (var_h) {
         const float omega = 1.f + ha * om.s / (P2[a].x * ND);
         s.row(FD_OMEGA)[a] = omega;
-        om32[a] = omega;
         roma = 1.f / omega;
     }
     s.row(FD_DDDT)[a] += (double)(acc.s * roma);
@@ -1173,7 +1169,7 @@ void force(sphdem_ctx *c) {
     const size_t st_bytes = tile ? (size_t)3 * ST_CAP * sizeof(float4) : 0;
 #define LP_(ND, P, T)                                                                                           \
     SPHDEM_LAUNCH(c, "force32", (k_force<ND, P, T>), grid_for(c->n, c->blk_pair), c->blk_pair, st_bytes, c->cfg, \
-                  c->dcfg, c->A, c->g, c->mx_pos, c->mx_vel, c->mx_aux, c->mx_om, c->mx_tg, c->mx_nbr,         \
+                  c->dcfg, c->A, c->g, c->mx_pos, c->mx_vel, c->mx_aux, c->mx_tg, c->mx_nbr,         \
                   c->mx_ncnt, (int64_t)c->mx_maxn, c->n, c->mx_nb, cgrows, c->buf.start, c->buf.skey)
 #define L_(ND)                              \
     do {                                    \
@@ -1222,7 +1218,7 @@ void dddt(sphdem_ctx *c) {
     const size_t st_bytes = tile ? (size_t)2 * ST_CAP * sizeof(float4) : 0;
 #define LD_(ND, CGF, T)                                                                                         \
     SPHDEM_LAUNCH(c, "dddt32", (k_dddt<ND, CGF, T>), grid_for(c->n, c->blk_pair), c->blk_pair, st_bytes,   \
-                  c->cfg, c->A, c->g, c->mx_pos, c->mx_vel, c->mx_aux, c->mx_om, c->mx_tg, c->mx_nbr,          \
+                  c->cfg, c->A, c->g, c->mx_pos, c->mx_vel, c->mx_aux, c->mx_tg, c->mx_nbr,          \
                   c->mx_ncnt, (int64_t)c->mx_maxn, c->n, cgrows, c->buf.start, c->buf.skey)
     if (c->cfg.nd == 1) {
         if (cgrows)
