@@ -68,6 +68,28 @@ struct Duo {
     }
 };
 
+/* One pair by the general passes' own expressions (pairs32.cu): the kernel
+ * gradient in its expanded form, which the 8-lane passes of the coupled case take.
+ * It is neither faster (3,768 particles: force 26.7 us a launch against 23.0 in the
+ * closed form, continuity 14.1 against 11.7) nor nearer to FP64: it keeps the
+ * results of small boxes where they have been.  In those a few stiff spheres amplify
+ * a rounding within ten steps, and the closed form moves the paths by 0.4e-9 to
+ * 1.1e-9 of the box, as far as either form is from FP64 (0.9e-9 to 1.6e-9). */
+template <int ND>
+struct PlainPair {
+    float d[3], r2, r, rinv;
+    __device__ __forceinline__ void set(int e, const float4 *shift, float4 pa, float4 pb) {
+        nb_delta_t<ND>(e, shift, pa, pb, d);
+        r2 = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
+        rinv = r2 > 0.f ? rsqrtf(r2) : 0.f;
+        r = r2 * rinv;
+    }
+    __device__ __forceinline__ float gradient(float h, float ih, float wcon) const {
+        const float ihn2 = powi<ND>(ih) * ih * ih, q = r * ih;
+        return q != 0.f ? ihn2 * wdK32(q, wcon) * (h * rinv) : 0.f;
+    }
+};
+
 /* d/dh of the kernel at b, W_h = C (10 q^2 - d t (1 + 2q)) t^3 / h^(d+1) with
  * t = 2 - q cut at 0 (calcOmega, sph.h:438-451), without C / h^(d+1) */
 template <int ND>
@@ -158,6 +180,7 @@ __global__ void __launch_bounds__(BLK, 4) k_force_list(DevCfg c, const DevCfg *_
     float hmin = FLT_MAX;  /* smallest hav of the fluid pairs */
     float hbest = FLT_MAX, vbest = 1.f; /* the pair with the smallest hav / vsig (artificial viscosity) */
     const float2 niha = both(-iha);
+    constexpr bool EXPANDED = G == 8 && VISC == SPHDEM_VISC_MORRIS;
     const float wcon = (float)c.wcon;
     auto fetch = [&](int e, float4 &p, float4 &v, float4 &x) {
         const int b = e & B_MASK;
@@ -217,20 +240,37 @@ __global__ void __launch_bounds__(BLK, 4) k_force_list(DevCfg c, const DevCfg *_
         /* F of b's kernel, cut at 2 h_b */
         float2 tb = make_float2(fmaxf(fmaf(q.r.x, -x0.w, 2.f), 0.f), fmaxf(fmaf(q.r.y, -x1.w, 2.f), 0.f));
         tb = __fmul2_rn(__fmul2_rn(tb, tb), tb);
-        const float2 Fb = make_float2(x0.z * tb.x, x1.z * tb.y);
-        const float2 Fa = __fmul2_rn(q.t3, both(cFa));
+        float2 Fb = make_float2(x0.z * tb.x, x1.z * tb.y);
+        float2 Fa = __fmul2_rn(q.t3, both(cFa));
+        if constexpr (EXPANDED) {
+            PlainPair<ND> u0, u1;
+            u0.set(e0, shift, pa, p0);
+            u1.set(e1, shift, pa, p1);
+            Fa = make_float2(u0.gradient(ha, iha, wcon), u1.gradient(ha, iha, wcon));
+            Fb = make_float2(u0.gradient(p0.w, x0.w, wcon), u1.gradient(p1.w, x1.w, wcon));
+        }
         const float2 cM = __fmul2_rn(__fadd2_rn(Fa, Fb), both(0.5f)); /* 0.5 (gA + gB) = d cM */
         float2 pc;
         if constexpr (VARH) {
-            pc = make_float2(x0.y * Fb.x, x1.y * Fb.y);
-            pc = __ffma2_rn(both(pdr2a), Fa, pc);
+            if constexpr (EXPANDED) {
+                pc = make_float2(pdr2a * Fa.x + x0.y * Fb.x, pdr2a * Fa.y + x1.y * Fb.y);
+            } else {
+                pc = make_float2(x0.y * Fb.x, x1.y * Fb.y);
+                pc = __ffma2_rn(both(pdr2a), Fa, pc);
+            }
             om = __ffma2_rn(m, omega_poly<ND>(__fmul2_rn(q.r, both(iha)), q.t3), om);
         } else {
             pc = __fmul2_rn(make_float2(pdr2a + x0.y, pdr2a + x1.y), cM);
         }
-        pc = __fmul2_rn(pc, make_float2(-m.x, -m.y));
+        const float2 nm = make_float2(-m.x, -m.y);
+        if constexpr (EXPANDED) {
 #pragma unroll
-        for (int k = 0; k < ND; k++) fp[k].add_product(pc, q.d[k]);
+            for (int k = 0; k < ND; k++) fp[k].add_product(nm, __fmul2_rn(pc, q.d[k]));
+        } else {
+            pc = __fmul2_rn(pc, nm);
+#pragma unroll
+            for (int k = 0; k < ND; k++) fp[k].add_product(pc, q.d[k]);
+        }
         if constexpr (VISC == SPHDEM_VISC_MORRIS) {
             /* m_b visc dg / (r^2 + 0.01 hav^2), visc = num / (rho_a rho_b) */
             float2 num = __fmul2_rn(__fmul2_rn(q.r2, cM), mv);
@@ -377,6 +417,7 @@ __global__ void __launch_bounds__(BLK) k_dddt_list(DevCfg c, DevState s, DevGlob
     acc.init();
     float2 om = both(0.f);
     const float2 niha = both(-iha);
+    constexpr bool EXPANDED = G == 8 && VARH;
     const float wcon = (float)c.wcon;
     auto body = [&](auto masked, int e0, int e1) {
         constexpr bool MASK = decltype(masked)::value;
@@ -423,6 +464,14 @@ __global__ void __launch_bounds__(BLK) k_dddt_list(DevCfg c, DevState s, DevGlob
         if constexpr (VARH) {
             F = q.t3; /* times cFa / Omega_a at the end */
             om = __ffma2_rn(mo, omega_poly<ND>(__fmul2_rn(q.r, both(iha)), q.t3), om);
+            if constexpr (EXPANDED) {
+                PlainPair<ND> u0, u1;
+                u0.set(e0, shift, pa, p0);
+                u1.set(e1, shift, pa, p1);
+                F = make_float2(u0.gradient(ha, iha, wcon), u1.gradient(ha, iha, wcon));
+                vdr = make_float2((va.x - v0.x) * u0.d[0] + (va.y - v0.y) * u0.d[1] + (va.z - v0.z) * u0.d[2],
+                                  (va.x - v1.x) * u1.d[0] + (va.y - v1.y) * u1.d[1] + (va.z - v1.z) * u1.d[2]);
+            }
         } else {
             const float4 x0 = P2[b0], x1 = P2[b1];
             float2 tb = make_float2(fmaxf(fmaf(q.r.x, -x0.w, 2.f), 0.f), fmaxf(fmaf(q.r.y, -x1.w, 2.f), 0.f));
@@ -445,7 +494,7 @@ __global__ void __launch_bounds__(BLK) k_dddt_list(DevCfg c, DevState s, DevGlob
         const float o = hd1 * (omt * wcon - va.w * ND * wK32(0.f, wcon));
         const float omega = 1.f + ha * o / (xa.x * ND);
         s.row(FD_OMEGA)[a] = omega;
-        rate = sum * cFa / omega;
+        rate = EXPANDED ? sum / omega : sum * cFa / omega;
     }
     s.row(FD_DDDT)[a] += (double)rate;
 }
@@ -456,7 +505,9 @@ __global__ void __launch_bounds__(BLK) k_dddt_list(DevCfg c, DevState s, DevGlob
  * 91k 135 / 114 / 141, 724k 530 / 684 / 978; 2D 6.5k 14.5 / 11.7 / 11.9, 23k
  * 13.4 / 17.3 / 22.  Continuity pass: 3D 3.8k 29 / 14 / 12, 23k 33 / 21 / 25,
  * 47k 36 / 37; 2D 6.5k 10.4 / 9.5, 23k 10.5 / 10.0.  (In 3D the force pass's
- * longest chains are those of the particles at a repulsive floor.) */
+ * longest chains are those of the particles at a repulsive floor.  All in the
+ * closed form: the coupled case's 8 lanes take the expanded one, 3.8k 26.7 and
+ * 14.1 us, so that its continuity pass gains nothing over 4 lanes there.) */
 int force_lanes(int64_t n, int nd) { return nd == 2 ? (n < 10000 ? 4 : 1) : (n < 12000 ? 8 : (n < 130000 ? 4 : 1)); }
 int dddt_lanes(int64_t n, int nd) { return nd == 2 ? (n < 10000 ? 4 : 1) : (n < 12000 ? 8 : (n < 40000 ? 4 : 1)); }
 
