@@ -203,6 +203,8 @@ void build_devcfg(const SphDemConfig &h, DevCfg &c) {
         const double t = 2.0 - q;
         c.k_anti = q <= 2.0 ? c.wcon * std::pow(t, 4) * (1.0 + 2.0 * q) : 0.0;
     }
+    c.f_grad[0] = (float)(-10.0 * c.wcon);
+    c.f_grad[1] = (float)(-10.0 * c.wcon - (double)c.f_grad[0]);
     c.f_pi = (float)h.pi;
     c.f_c0 = (float)h.spsound;
     c.f_rpsep = h.psep > 0 ? (float)(1.0 / h.psep) : 0.f;

@@ -91,6 +91,7 @@ struct DevCfg {
     double k_anti;        /* K(1/HFAC) for anticlumping */
     /* FP32 copies for the mixed-precision boundary force */
     float f_pi, f_c0, f_rpsep, f_rdelp; /* PI, SPSOUND, 1/PSEP, 1/(BFAC*PSEP) */
+    float f_grad[2];      /* -10 wcon of the Wendland gradient: FP32 and what it leaves */
     __host__ __device__ bool liq_dem() const { return flags & SPHDEM_F_LIQ_DEM; }
     __host__ __device__ bool var_h() const { return flags & SPHDEM_F_VAR_H_CORRECTION; }
 };

@@ -23,7 +23,6 @@
 #include <type_traits>
 
 #include "mixed.cuh"
-#include "series.cuh"
 
 namespace sphdem {
 namespace {

@@ -10,6 +10,7 @@
 #include <climits>
 
 #include "internal.cuh"
+#include "series.cuh"
 
 namespace sphdem {
 namespace {

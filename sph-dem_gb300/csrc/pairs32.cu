@@ -79,10 +79,7 @@ __global__ void k_pack(DevCfg c, DevState s, const int *__restrict__ skey, const
     const float mpk = (float)s.row(FD_MASS)[i];
     P1[i] = make_float4(vh[0], vh[1], vh[2], (is_sph_or_sphb(t) || dem) ? mpk : -mpk);
     const float ih = (float)s.row(FD_IH)[i];
-    double ihn2 = (double)ih * (double)ih;
-#pragma unroll
-    for (int d = 0; d < ND; d++) ihn2 *= (double)ih;
-    const float cF = (float)(-10.0 * c.wcon * ihn2);
+    const float cF = scaled_power<ND + 2>(ih, c.f_grad[0], c.f_grad[1]);
     P2[i] = make_float4((float)s.row(FD_DENS)[i], middle ? (float)s.row(FD_PDR2)[i] : cF,
                         middle ? cF : (float)s.row(FD_POR)[i], ih);
     if (is_boundary(t)) {

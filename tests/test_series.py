@@ -1,5 +1,5 @@
-"""The reciprocals and roots that the pass kernels take from a hardware estimate
-(csrc/series.cuh), on the CPU against wider arithmetic.  The estimates are FP32
+"""The reciprocals, roots, quotients and powers of csrc/series.cuh, as the kernels
+take them, on the CPU against wider arithmetic.  The estimates are FP32
 numbers up to 2 ulp off (the instructions' stated error).  Bound: half an ulp for the
 last rounding, the series' first dropped term ((2.4e-7)^3 and 5/16 of it,
 below 1e-4 ulp) and the roundings of a correction of 2e-7 of the result (below
@@ -57,7 +57,24 @@ int main() {
         const float w = (float)want;
         q = std::max(q, fabs((double)sphdem::quotient(a, b, y) - want) / (double)(std::nextafterf(w, INFINITY) - w));
     }
+    /* the gradient factor -10 C x^N of an FP32 x */
+    double pw = 0.0;
+    std::uniform_real_distribution<float> e3(-5.f, 5.f);
+    for (int k = 0; k < 400000; k++) {
+        const float x = std::pow(10.f, e3(rng));
+        for (int n = 3; n <= 5; n++) {
+            const double c = -10.0 * (n == 4 ? 7.0 / (64.0 * 3.14159265) : 21.0 / (256.0 * 3.14159265));
+            const float g = (float)c, glo = (float)(c - (double)g);
+            const float got = n == 3 ? sphdem::scaled_power<3>(x, g, glo)
+                                     : (n == 4 ? sphdem::scaled_power<4>(x, g, glo) : sphdem::scaled_power<5>(x, g, glo));
+            double want = c;
+            for (int i = 0; i < n; i++) want *= (double)x;
+            const float w = fabsf((float)want);
+            pw = std::max(pw, fabs((double)got - want) / (double)(std::nextafterf(w, INFINITY) - w));
+        }
+    }
     for (double w : worst) printf("%.6f ", w);
+    printf("%.6f ", pw);
     printf("%.6f\n", q);
 }
 """
@@ -82,4 +99,10 @@ def test_fp64_series(errors, k, what, bound):
 def test_fp32_quotient(errors):
     """Half an ulp for the last rounding; the remainder (exact by fma) times an
     estimate 1.2e-7 off, of a correction of up to 2 ulp, is below 1e-6 ulp: 0.501."""
+    assert 0.4 < errors[6] <= 0.501
+
+
+def test_fp32_scaled_power(errors):
+    """Half an ulp for the last addition; what is carried along is of the size of
+    the products' roundings (five of 2^-24) and itself rounded: below 1e-5 ulp."""
     assert 0.4 < errors[5] <= 0.501
