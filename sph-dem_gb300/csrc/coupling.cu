@@ -789,10 +789,19 @@ __global__ void __launch_bounds__(BLK) k_dem_finish(DevCfg c, DevState s, const 
                     const int bb = id & B_MASK, sp = (unsigned)id >> B_BITS;
                     double dx[3] = {0, 0, 0};
                     pair_dx<ND>(c, s, ra, bb, sp, dx);
-                    const double r2 = exact_len2(dx, ND), hb = s.row(FD_H)[bb], t = 2.0 * (ha > hb ? ha : hb);
+                    const double r2 = exact_len2(dx, ND);
+                    /* r^2 <= (2 max h)^2: five FP32 roundings are below 4e-7, so FP32 decides
+                     * unless the two are nearly equal */
+                    const float hm = fmaxf(haf, P0[bb].w), r2f = (float)r2, T = 4.f * hm * hm;
+                    const bool fits = T > 1e-30f;
+                    bool near = fits && r2f < T * (1.f - 1e-6f);
+                    if (!near && !(fits && r2f > T * (1.f + 1e-6f))) {
+                        const double hb = s.row(FD_H)[bb], t = 2.0 * (ha > hb ? ha : hb);
+                        near = r2 <= dmul(t, t);
+                    }
                     int sh[3];
                     shift_of(sp, sh);
-                    if (r2 <= dmul(t, t) && (sp == 0x15 || img_ok<ND>(tg[bb] >> 8, sh))) {
+                    if (near && (sp == 0x15 || img_ok<ND>(tg[bb] >> 8, sh))) {
                         /* the overlap is a difference of r and the radii, and shows the last
                          * place of r: with the root to 0.75 ulp the paths of 50,000
                          * settling spheres were off by 2.1e-13, with 0.5 ulp by 1.7e-13 */

@@ -122,3 +122,35 @@ def test_fluid_inserted_into_a_handle_of_dem_only(lib, nx):
         sim.close()
     for k in FIELDS:
         assert np.linalg.norm(got[1][k]) > 0 and norm_gap(got[0][k], got[1][k]) <= 1e-9, k
+
+
+@pytest.mark.parametrize("precision", [cases.PREC_FP64, cases.PREC_MIXED])
+def test_contacts_at_the_edge_of_the_search(lib, precision):
+    """Pairs of spheres that overlap at distances around 2 max(h), where the
+    neighbour predicate decides whether they meet: from 2e-5 of the distance off
+    to the last places, both sides of the range in which FP32 decides.  The same
+    pairs touch as in the CPU oracle, with the same force (1e-11)."""
+    case = cases.dem_settling3d(lattice=(10, 10, 8), spread=0.0, vel_amp=0.0)
+    p, R = case.particles, case.cfg["dem_radius"]
+    n, h = case.n // 2, p["h"][0]
+    rng = np.random.default_rng(2)
+    way = rng.standard_normal((n, 3))
+    way /= np.linalg.norm(way, axis=1)[:, None]
+    off = np.concatenate([[0.0], *([s * 2.0 ** -k for k in range(16, 54)] for s in (1.0, -1.0))])
+    gap = 2.0 * h * (1.0 + off[np.arange(n) % off.size])
+    q = np.stack(np.unravel_index(np.arange(n), (10, 10, 4)), 1)
+    mid = (q + 1.0) * 8.0 * R + rng.uniform(-0.5, 0.5, (n, 3)) * R
+    p["r"][:n], p["r"][n:] = mid - 0.5 * gap[:, None] * way, mid + 0.5 * gap[:, None] * way
+    p["h"][n:] = h * rng.choice([0.7, 1.0], n)
+    p["radius"][:] = 1.1 * h
+    p["v"][:] = 0.0
+    ora = OracleSim(case.cfg, p)
+    ora.step(1)
+    want = ora.get()
+    sim = capi.Simulation(lib, case.cfg, p, precision=precision)
+    sim.step(1)
+    got = sim.get()
+    touch = np.abs(want["fp"]).sum(axis=1) > 0
+    assert 0.2 < touch.mean() < 0.8
+    assert np.array_equal(np.abs(got["fp"]).sum(axis=1) > 0, touch)
+    assert norm_gap(got["fp"], want["fp"]) <= 1e-11
