@@ -220,12 +220,13 @@ PASS_MODELS = {
     "force32": lambda owners, entries: (68.0 * owners + 4.0 * entries, 80.0 * entries),
     "dddt32": lambda owners, entries: (52.0 * owners + 4.0 * entries, 40.0 * entries),
 }
-# DRAM bytes (read + write) of one launch per particle of the whole state,
-# from ncu captures of the 270k sub-box of the same workload (traffic grows
-# in proportion to the particle count at fixed density)
+# DRAM bytes (read + write) of one launch per particle of the whole state, from
+# a one-pass ncu capture of the workload itself (1,080,400 particles; of the 270k
+# sub-box's list half stays in L2)
 PASS_DRAM_BYTES_PER_PARTICLE = {
-    "force32": (163.309824e6 + 12.316928e6) / 270100,
-    "nlist32": (37.5e6 + 121.9e6) / 270100,
+    "force32": (623.6e6 + 93.7e6) / 1080400,
+    "nlist32": (59.2e6 + 405.0e6) / 1080400,
+    "dddt32": (526.5e6 + 13.4e6) / 1080400,
 }
 
 

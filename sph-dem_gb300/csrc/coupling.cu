@@ -22,9 +22,9 @@
  *
  * All are bound by the search: latency of the bucket records below ~100,000
  * particles, instruction issue above.  Before / now, us: 1.08 M particles (mixed)
- * porosity 530 / 438, drag 328 / 91, FPI and contacts 571 / 408; 69,758 (FP64)
- * 1,303 / 188, 1,155 / 40, 3,737 / 133; contacts of 50,000 settling spheres (FP64)
- * 515 / 69.
+ * porosity 530 / 438, drag 328 / 94, FPI and contacts 571 / 385; 69,758 (FP64)
+ * 1,303 / 188, 1,155 / 42, 3,737 / 134; contacts of 50,000 settling spheres (FP64)
+ * 515 / 68.
  */
 #include <algorithm>
 
